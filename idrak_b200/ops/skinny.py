@@ -110,33 +110,50 @@ def skinny8_reference(x, w8, bias=None, residual=None, gate: Optional[str] = Non
     return y.to(x.dtype)
 
 
-def skinny8_linear(x: torch.Tensor, w8, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
-                   gate: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``x [M <= 64, K]`` times an int8 weight with one scale per output (``quant.Int8Weight``, ``[K, N]``) ->
-    ``[M, N]``; with ``gate`` the weight's outputs are ``[gate | up]`` and the result is ``act(gate) * up`` ``[M, N / 2]``.
-    The kernel reads the codes in their K-major copy (``Int8Weight.kmajor``) and expands them in shared memory."""
+def packed_supported(x: torch.Tensor, w, gate: Optional[str] = None) -> bool:
+    """Whether the few-row kernels take ``x @ W`` over this int8 / int4 weight: at most 64 bf16 rows, whole 16-byte chunks of
+    inputs (int8) or whole groups of 32 (int4), and a gated weight's up half on a 16-byte boundary of the codes."""
+    n_out = w.cols // 2 if gate is not None else w.cols
+    step = 16 if w.bits == 8 else 32
+    return (x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] <= MAX_ROWS and x.shape[1] == w.rows
+            and w.rows % step == 0 and _native.has("idrak_skinny_packed") and w.codes.is_cuda
+            and (w.bits == 8 or (w.ld % 4 == 0 and w.codes.data_ptr() % 16 == 0 and w.scale_ld % 8 == 0
+                                 and w.scales.data_ptr() % 16 == 0))
+            and (gate is None or (gate in _KINDS and w.cols % 2 == 0 and n_out % step == 0)))
+
+
+def packed_linear(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
+                  gate: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``x [M <= 64, K]`` times a packed int8 or int4 weight ``[K, N]`` (``packed_supported``) -> ``[M, N]``; with ``gate``
+    the outputs are ``[gate | up]`` and the result is ``act(gate) * up`` ``[M, N / 2]``. The kernels stream the codes as
+    they are stored and expand them on the way to the tensor cores."""
     M, K = x.shape
-    n_out = w8.cols // 2 if gate is not None else w8.cols
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and M <= 64 and K % 16 == 0 and K == w8.rows
-            and (gate is None or (gate in _KINDS and n_out % 8 == 0))):
-        res = skinny8_reference(x, w8, bias, residual, gate)
-        if out is not None:
-            out.copy_(res)
-            return out
-        return res
-    from ._util import ptr, stream_ptr
-    codes = w8.kmajor()
-    x = x if x.stride(1) == 1 and x.stride(0) % 8 == 0 else x.contiguous()
+    n_out = w.cols // 2 if gate is not None else w.cols
+    codes = w.tma_codes() if w.bits == 8 else w.codes
+    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
+        x = x.clone(memory_format=torch.contiguous_format)
     if out is None:
         out = torch.empty((M, n_out), dtype=torch.bfloat16, device=x.device)
     assert out.dtype == torch.bfloat16 and out.shape == (M, n_out) and out.stride(1) == 1
     if bias is not None:
-        assert bias.dtype == torch.bfloat16 and bias.numel() == w8.cols
+        assert bias.dtype == torch.bfloat16 and bias.numel() == w.cols
     if residual is not None:
         assert residual.dtype == torch.bfloat16 and residual.shape == (M, n_out) and residual.stride(1) == 1
-    rc = _native.lib().idrak_skinny8_gemm(x.data_ptr(), x.stride(0), codes.data_ptr(), codes.stride(0), w8.scales.data_ptr(),
-                                          out.data_ptr(), out.stride(0), M, n_out, K, ptr(bias), ptr(residual),
-                                          residual.stride(0) if residual is not None else 0,
-                                          _KINDS[gate] if gate is not None else -1, stream_ptr())
-    _native.check(rc, "idrak_skinny8_gemm")
+    rc = _native.lib().idrak_skinny_packed(x.data_ptr(), x.stride(0), codes.data_ptr(), codes.stride(0) * codes.element_size(),
+                                           w.scales.data_ptr(), w.scale_ld, w.bits, out.data_ptr(), out.stride(0), M, n_out, K,
+                                           ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
+                                           _KINDS[gate] if gate is not None else -1, stream_ptr())
+    _native.check(rc, "idrak_skinny_packed")
     return out
+
+
+def skinny8_linear(x: torch.Tensor, w8, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
+                   gate: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``packed_linear`` over an int8 weight, or its fp32 statement where the kernels do not take the call."""
+    if packed_supported(x, w8, gate):
+        return packed_linear(x, w8, bias, residual, gate, out)
+    res = skinny8_reference(x, w8, bias, residual, gate)
+    if out is not None:
+        out.copy_(res)
+        return out
+    return res

@@ -64,7 +64,7 @@ class Int8Weight:
         scale = amax / 127.0
         safe = torch.where(scale > 0, scale, torch.ones_like(scale))
         q = torch.clamp(torch.round(wf / safe), -127, 127).to(torch.int8)
-        ld = (cols + 7) // 8 * 8
+        ld = (cols + 15) // 16 * 16               # 16-byte rows: what TMA needs to read them
         codes = torch.zeros((rows, ld), dtype=torch.int8, device=w.device)
         codes[:, :cols] = q
         return cls(codes.contiguous(), scale.to(torch.float16).contiguous(), rows, cols)
@@ -75,15 +75,16 @@ class Int8Weight:
     def to(self, device) -> "Int8Weight":
         return Int8Weight(self.codes.to(device), self.scales.to(device), self.rows, self.cols)
 
-    def kmajor(self) -> torch.Tensor:
-        """The codes transposed to ``[out, in]`` with the input index contiguous (rows padded to 16 bytes): what the
-        few-row decode kernel streams. Made on first use and kept (it doubles the weight's code bytes)."""
-        t = getattr(self, "_kmajor", None)
+    def tma_codes(self) -> torch.Tensor:
+        """The codes with rows and base on 16-byte boundaries, as the few-row kernels read them: the codes themselves, or
+        for a weight that came with shorter rows (an older file) a padded copy, made on first use and kept."""
+        if self.codes.stride(0) % 16 == 0 and self.codes.data_ptr() % 16 == 0:
+            return self.codes
+        t = getattr(self, "_tma_codes", None)
         if t is None or t.device != self.codes.device:
-            kp = (self.rows + 15) // 16 * 16
-            t = torch.zeros((self.cols, kp), dtype=torch.int8, device=self.codes.device)
-            t[:, : self.rows] = self.codes[:, : self.cols].t()
-            self._kmajor = t
+            t = torch.zeros((self.rows, (self.cols + 15) // 16 * 16), dtype=torch.int8, device=self.codes.device)
+            t[:, : self.cols] = self.codes[:, : self.cols]
+            self._tma_codes = t
         return t
 
     @property
@@ -244,8 +245,7 @@ def _fp8_product(x2, w: "Fp8Weight", transposed, bias, residual, act, out):
 
 
 # --------------------------------------------------------------------------- the op
-FEW_ROW_INT8_KERNEL = True   # int8 weights, few rows: the few-row kernel that reads the codes directly (csrc/skinny8_gemm.cu)
-FEW_ROWS = 64           # up to this many rows (decode steps) the weight is unpacked first as well: see qgemm
+FEW_ROWS = 64           # up to this many rows (decode steps) the few-row kernels stream the codes: see qgemm
 DENSE_ROWS = 512        # from this many activation rows on, the weight is unpacked to bf16 first and multiplied densely
 
 
@@ -271,19 +271,18 @@ def qgemm(x2: torch.Tensor, w, transposed: bool = False, bias=None, residual=Non
             y = y + residual.float()
         y = y.to(x2.dtype)
         return (y, aux) if aux is not None else y
-    if (M <= FEW_ROWS and isinstance(w, Int8Weight) and not transposed and act is None and x2.is_cuda
-            and x2.dtype == torch.bfloat16 and K % 16 == 0 and x2.stride(0) % 8 == 0 and FEW_ROW_INT8_KERNEL
-            and _native.has("idrak_skinny8_gemm")):
-        # decode steps over int8 weights: the codes are streamed once (half the bytes of bf16) and expanded to bf16
-        # operand tiles inside the few-row kernel
-        from ..ops.skinny import skinny8_linear
-        return skinny8_linear(x2, w, bias, residual, out=out)
+    if M <= FEW_ROWS and not transposed and act is None and (out is None or out.dtype == x2.dtype):
+        # decode steps: the codes are streamed once, as stored (a half or a quarter of the bytes of bf16), and expanded on
+        # the way to the tensor cores
+        from ..ops.skinny import packed_linear, packed_supported
+        if packed_supported(x2, w):
+            return packed_linear(x2, w, bias, residual, out=out)
     if ((M >= DENSE_ROWS or M <= FEW_ROWS) and x2.dtype == torch.bfloat16 and w.cols % 8 == 0
             and x2.stride(0) % 8 == 0):
         # many rows: unpacking the weight once (a bandwidth-bound pass over it) and running the dense tensor-core GEMM
-        # beats unpacking inside the GEMM's producer warps. Few rows (decoding): the same holds, measured at 64 rows of
-        # a 4096 x 4096 int8 weight 81 us in the unpacking GEMM against 13 us to unpack (the bf16 copy of one
-        # projection stays in L2) plus 17 us for the split-K product over it
+        # beats unpacking inside the GEMM's producer warps. The same holds for the few-row products the few-row kernels do
+        # not take (transposed use): 64 rows of a 4096 x 4096 int8 weight measured 81 us in the unpacking GEMM against
+        # 13 us to unpack (the bf16 copy of one projection stays in L2) plus 17 us for the split-K product over it
         from ..ops.gemm import gemm
         return gemm(x2, dequantize_bf16(w), b_mn=not transposed, bias=bias, residual=residual, act=act, out=out)
     _bind()
