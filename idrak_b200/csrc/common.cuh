@@ -14,6 +14,7 @@
 #include <cuda.h>
 #include <stdint.h>
 #include <atomic>
+#include <cstdlib>
 #include <mutex>
 
 namespace idrak {
@@ -425,4 +426,25 @@ struct DeviceOnce {
 };
 // Every kernel launch made by this library is counted (read with idrak_launch_count()).
 void note_launches(int n);
+
+// Launches a kernel with programmatic serialization: its CTAs may be set up while the kernel before it in the stream
+// drains. Only for kernels that call pdl_wait() in every thread before they touch global memory. IDRAK_PDL=0 launches the
+// ordinary way.
+template <class... P, class... A>
+int launch_overlapped(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  static const bool pdl = [] { const char* e = getenv("IDRAK_PDL"); return !(e && e[0] == '0'); }();
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  const int rc = int(cudaLaunchKernelEx(&cfg, kern, P(args)...));
+  note_launches(1);
+  return rc;
+}
 }  // namespace idrak

@@ -13,6 +13,17 @@
 // order. The kernel is bound by the bytes of K and V (each is read once); warp-level MMAs are enough to keep up
 // with them - a 16-row tile cannot feed tcgen05's 128-row instruction - while the FMA pipes are not.
 //
+// The host knows only a bound on the lengths, so a share is at least `min_tiles` tiles and a sequence uses as many of the
+// splits as its own length fills; the other CTAs leave at once, and a sequence with one share is written out directly.
+// Short shares even out a batch whose contexts differ: 64 sequences of 128 to 2304 tokens (8 KV heads, head size 128,
+// 386 MB) took 95 us unsplit - 512 CTAs on 444 places, the longest alone at the end - and 84 us in shares of 1024 keys;
+// 16 of them 51 and 28.5 us in shares of 512.
+//
+// int8 cache: the codes enter the tensor core as exact bf16 numbers (code / 64, one permute and one fused multiply-add per
+// two codes); a key's scale multiplies its column of scores and a value's scale its column of probabilities, so nothing
+// is rounded that a bf16 cache would not round. Converting and scaling every element in fp32 had bound the kernel: 150
+// sequences of 606 tokens on average (192 MB) 152 us, now 88 us.
+//
 // Reference counterparts: attention_decode_{f32,int8,bf16} (split over blocks, last block merges;
 // src/Idrak.Gpu/Cuda/PtxKernels.Rows.cs:2047-2060), kv_write_{f32,bf16} (PtxKernels.Decoding.cs:12),
 // KeyValuePages (src/Idrak.Abstraction/Generation/KeyValuePages.cs:20-34) whose pages the reference copies into a
@@ -37,6 +48,7 @@ struct DecodeParams {
   __nv_bfloat16* out;            // [seqs, H, D]
   float* partial;                // [seqs, H, splits, D + 2]
   int H, Hkv, D, block_size, max_blocks, splits;
+  int min_tiles;                 // tiles per split at least
   float scale_log2;
   int window;                    // 0 = full; else attend to the last `window` positions only
 };
@@ -71,19 +83,30 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 // wait until at most one of this thread's committed groups is still in flight (groups complete in order)
 __device__ __forceinline__ void cp_async_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
-// 16 int8 codes times a scale -> 16 bf16 values (two 16-byte words)
-__device__ __forceinline__ void dequant16(const uint4& raw, float scale, uint4& lo, uint4& hi) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  uint32_t o[8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float a = float(int8_t(w[i] & 0xff)) * scale, b = float(int8_t((w[i] >> 8) & 0xff)) * scale;
-    const float c = float(int8_t((w[i] >> 16) & 0xff)) * scale, d = float(int8_t(w[i] >> 24)) * scale;
-    o[2 * i] = pack_bf16x2(a, b);
-    o[2 * i + 1] = pack_bf16x2(c, d);
-  }
-  lo = make_uint4(o[0], o[1], o[2], o[3]);
-  hi = make_uint4(o[4], o[5], o[6], o[7]);
+// 16 int8 codes -> 16 bf16 values code / 64 (two 16-byte words), exactly: an unsigned integer u < 256 in a 16-bit lane is,
+// read as bf16, u * 2^-133, and one fused multiply-add takes it to (u - 128) / 64.
+__device__ __forceinline__ uint32_t codes_pair(uint32_t t) {
+  const uint32_t mul = 0x7F007F00u, add = 0xC000C000u;      // 2^127, -128 / 64
+  const __nv_bfloat162 v = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&mul),
+                                   *reinterpret_cast<const __nv_bfloat162*>(&add));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ void expand16(const uint4& raw, uint4& lo, uint4& hi) {
+  const uint32_t a = raw.x ^ 0x80808080u, b = raw.y ^ 0x80808080u, c = raw.z ^ 0x80808080u, d = raw.w ^ 0x80808080u;
+  lo = make_uint4(codes_pair(__byte_perm(a, 0, 0x4140)), codes_pair(__byte_perm(a, 0, 0x4342)),
+                  codes_pair(__byte_perm(b, 0, 0x4140)), codes_pair(__byte_perm(b, 0, 0x4342)));
+  hi = make_uint4(codes_pair(__byte_perm(c, 0, 0x4140)), codes_pair(__byte_perm(c, 0, 0x4342)),
+                  codes_pair(__byte_perm(d, 0, 0x4140)), codes_pair(__byte_perm(d, 0, 0x4342)));
+}
+
+// The share of a sequence's tiles that each split takes, and how many splits that leaves with work.
+__device__ __forceinline__ int tiles_per_split(int span, int splits, int min_tiles) {
+  return max(min_tiles, (span + splits - 1) / splits);
+}
+__device__ __forceinline__ void key_span(int len, int window, int& first_tile, int& span) {
+  const int first_pos = (window > 0 && len > window) ? len - window : 0;
+  first_tile = first_pos / kDecTile;
+  span = (len + kDecTile - 1) / kDecTile - first_tile;
 }
 
 // KV8 = 1: the cache holds int8 codes with one scale per (slot, kv head) (norm_rope_kv's int8 mode). A tile's codes
@@ -93,6 +116,7 @@ __device__ __forceinline__ void dequant16(const uint4& raw, float scale, uint4& 
 template <int D, int KV8>
 __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const DecodeParams p) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
+  pdl_wait();
   constexpr int kRow = D * 2 + 16;                       // padded shared-memory row (bytes): conflict-free ldmatrix
   constexpr int kChunks = D / 8;                         // 16-byte chunks per key row
   constexpr int KS = D / 16;                             // k-steps of Q·K^T
@@ -110,11 +134,12 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
 
   const int len = p.seq_lens[seq];
   const int first_pos = (p.window > 0 && len > p.window) ? len - p.window : 0;
-  const int tiles = (len + kDecTile - 1) / kDecTile;
-  const int first_tile = first_pos / kDecTile;
-  const int span = tiles - first_tile;
-  const int per = (span + p.splits - 1) / p.splits;
-  const int t0 = first_tile + split * per, t1 = min(tiles, t0 + per);
+  int first_tile, span;
+  key_span(len, p.window, first_tile, span);
+  const int per = tiles_per_split(span, p.splits, p.min_tiles);
+  const bool alone = span <= per;                        // the only split of its sequence with work
+  if (split > 0 && split * per >= span) return;
+  const int t0 = first_tile + split * per, t1 = min(first_tile + span, t0 + per);
 
   // queries of the G heads of this KV head -> shared (bf16, rows padded to 16 with zeros)
   for (int i = threadIdx.x; i < 16 * kChunks; i += blockDim.x) {
@@ -175,12 +200,12 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
     }
     cp_async_commit();
   };
-  auto expand_row = [&](uint8_t* row, float scale) {     // this lane's row: codes -> bf16, front to back
+  auto expand_row = [&](uint8_t* row) {                  // this lane's row: codes -> bf16, front to back
 #pragma unroll
     for (int c = 0; c < kByteChunks; ++c) {
       const uint4 codes = *reinterpret_cast<const uint4*>(row + D + c * 16);
       uint4 lo, hi;
-      dequant16(codes, scale, lo, hi);
+      expand16(codes, lo, hi);
       *reinterpret_cast<uint4*>(row + c * 32) = lo;
       *reinterpret_cast<uint4*>(row + c * 32 + 16) = hi;
     }
@@ -202,13 +227,13 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
     // int8 cache: this lane's row scales (0 for a key past the end: the codes are zeros there anyway)
     float ks = 0.f, vs = 0.f;
     if (KV8 && next_slots >= 0) {
-      ks = p.k_scale[size_t(next_slots) * p.Hkv + kvh];
-      vs = p.v_scale[size_t(next_slots) * p.Hkv + kvh];
+      ks = p.k_scale[size_t(next_slots) * p.Hkv + kvh] * (64.f * p.scale_log2);
+      vs = p.v_scale[size_t(next_slots) * p.Hkv + kvh] * 64.f;
     }
     cp_async_wait_but_one();                             // this tile's keys have landed; its values may still fly
     __syncwarp();
     if (KV8) {
-      expand_row(sk + lane * kRow, ks);
+      expand_row(sk + lane * kRow);
       __syncwarp();
     }
     // ---- S[16 x 32] = Q · K^T: 4 n-tiles of 8 keys
@@ -238,8 +263,9 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
       for (int j = 0; j < 2; ++j) {
         const int pos = key0 + n * 8 + 2 * (lane & 3) + j;
         const bool valid = pos < len && pos >= first_pos;
-        s[n][j] = valid ? s[n][j] * p.scale_log2 : -INFINITY;
-        s[n][2 + j] = valid ? s[n][2 + j] * p.scale_log2 : -INFINITY;
+        const float f = KV8 ? __shfl_sync(0xffffffffu, ks, n * 8 + 2 * (lane & 3) + j) : p.scale_log2;
+        s[n][j] = valid ? s[n][j] * f : -INFINITY;
+        s[n][2 + j] = valid ? s[n][2 + j] * f : -INFINITY;
         mx0 = fmaxf(mx0, s[n][j]);
         mx1 = fmaxf(mx1, s[n][2 + j]);
       }
@@ -261,8 +287,10 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
       const float p11 = (mn1 == -INFINITY) ? 0.f : exp2f(s[n][3] - mn1);
       sum0 += p00 + p01;
       sum1 += p10 + p11;
-      pa[n >> 1][(n & 1) * 2 + 0] = pack_bf16x2(p00, p01);
-      pa[n >> 1][(n & 1) * 2 + 1] = pack_bf16x2(p10, p11);
+      const float v0 = KV8 ? __shfl_sync(0xffffffffu, vs, n * 8 + 2 * (lane & 3)) : 1.f;
+      const float v1 = KV8 ? __shfl_sync(0xffffffffu, vs, n * 8 + 2 * (lane & 3) + 1) : 1.f;
+      pa[n >> 1][(n & 1) * 2 + 0] = KV8 ? pack_bf16x2(p00 * v0, p01 * v1) : pack_bf16x2(p00, p01);
+      pa[n >> 1][(n & 1) * 2 + 1] = KV8 ? pack_bf16x2(p10 * v0, p11 * v1) : pack_bf16x2(p10, p11);
     }
     sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
     sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
@@ -277,7 +305,7 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
     cp_async_wait_but_one();                             // this tile's values have landed; the next keys may still fly
     __syncwarp();
     if (KV8) {
-      expand_row(sv + lane * kRow, vs);
+      expand_row(sv + lane * kRow);
       __syncwarp();
     }
     // ---- O[16 x D] += P[16 x 32] · V[32 x D]: V is [key][d], so its B fragments come through transposing loads
@@ -325,7 +353,7 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
       oo += src[d] * a;
     }
     const int head = kvh * G + g;
-    if (p.splits == 1) {
+    if (alone) {
       p.out[(size_t(seq) * p.H + head) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
     } else {
       float* pp = p.partial + ((size_t(seq) * p.H + head) * p.splits + split) * (D + 2);
@@ -335,24 +363,28 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
   }
 }
 
-// out[seq, head, :] = merge of the splits' partials, in split order
-__global__ void decode_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, int rows,
-                                    int splits, int D) {
+// out[seq, head, :] = merge of the partials of a sequence's splits, in split order
+__global__ void decode_merge_kernel(const DecodeParams p) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
-  const int row = blockIdx.x;
-  if (row >= rows) return;
-  const float* base = partial + size_t(row) * splits * (D + 2);
+  pdl_wait();
+  const int row = blockIdx.x, D = p.D;
+  int first_tile, span;
+  key_span(p.seq_lens[row / p.H], p.window, first_tile, span);
+  const int per = tiles_per_split(span, p.splits, p.min_tiles);
+  if (span <= per) return;                               // written out by its only split
+  const int used = (span + per - 1) / per;
+  const float* base = p.partial + size_t(row) * p.splits * (D + 2);
   float mm = -INFINITY;
-  for (int s = 0; s < splits; ++s) mm = fmaxf(mm, base[s * (D + 2) + D]);
+  for (int s = 0; s < used; ++s) mm = fmaxf(mm, base[s * (D + 2) + D]);
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     float ll = 0.f, oo = 0.f;
-    for (int s = 0; s < splits; ++s) {
+    for (int s = 0; s < used; ++s) {
       const float* src = base + s * (D + 2);
       const float a = (src[D] == -INFINITY) ? 0.f : exp2f(src[D] - mm);
       ll += src[D + 1] * a;
       oo += src[d] * a;
     }
-    out[size_t(row) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
+    p.out[size_t(row) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
   }
 }
 
@@ -390,11 +422,13 @@ IDRAK_API long long idrak_decode_partial_floats(int seqs, int H, int D, int spli
   return splits > 1 ? (long long)seqs * H * splits * (D + 2) : 0;
 }
 
-// The same over an int8 cache when k_scale / v_scale are given (one fp32 scale per (slot, kv head)).
+// Over an int8 cache when k_scale / v_scale are given (one fp32 scale per (slot, kv head)). A sequence's keys are shared by
+// at most `splits` CTAs per KV head, at least `min_keys` keys each (rounded up to tiles).
 IDRAK_API int idrak_paged_decode_kv(const void* q, long long q_stride, const void* k_cache, const void* v_cache,
                                     const float* k_scale, const float* v_scale, const int* block_table,
                                     const int* seq_lens, void* out, float* partial, int seqs, int H, int Hkv, int D,
-                                    int block_size, int max_blocks, int splits, float scale, int window, void* stream_) {
+                                    int block_size, int max_blocks, int splits, int min_keys, float scale, int window,
+                                    void* stream_) {
   if (D != 64 && D != 128) return -2;
   const bool kv8 = k_scale != nullptr;
   if (kv8 && !v_scale) return -6;
@@ -415,6 +449,7 @@ IDRAK_API int idrak_paged_decode_kv(const void* q, long long q_stride, const voi
   p.partial = partial;
   p.H = H; p.Hkv = Hkv; p.D = D; p.block_size = block_size; p.max_blocks = max_blocks;
   p.splits = splits < 1 ? 1 : splits;
+  p.min_tiles = min_keys <= kDecTile ? 1 : (min_keys + kDecTile - 1) / kDecTile;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.window = window;
   dim3 grid(seqs, Hkv, p.splits);
@@ -434,29 +469,13 @@ IDRAK_API int idrak_paged_decode_kv(const void* q, long long q_stride, const voi
         return int(e1);
       }))
     return e;
-  if (D == 64) {
-    if (kv8) paged_decode_kernel<64, 1><<<grid, kDecWarps * 32, decode_smem<64>(), s>>>(p);
-    else paged_decode_kernel<64, 0><<<grid, kDecWarps * 32, decode_smem<64>(), s>>>(p);
-  } else {
-    if (kv8) paged_decode_kernel<128, 1><<<grid, kDecWarps * 32, decode_smem<128>(), s>>>(p);
-    else paged_decode_kernel<128, 0><<<grid, kDecWarps * 32, decode_smem<128>(), s>>>(p);
-  }
-  note_launches(1);
-  int rc = int(cudaGetLastError());
-  if (rc) return rc;
-  if (p.splits > 1) {
-    decode_merge_kernel<<<seqs * H, D < 128 ? 64 : 128, 0, s>>>(partial, p.out, seqs * H, p.splits, D);
-    note_launches(1);
-    rc = int(cudaGetLastError());
-  }
+  const int threads = kDecWarps * 32;
+  int rc;
+  if (D == 64) rc = launch_overlapped(kv8 ? paged_decode_kernel<64, 1> : paged_decode_kernel<64, 0>, grid, threads, decode_smem<64>(), s, p);
+  else rc = launch_overlapped(kv8 ? paged_decode_kernel<128, 1> : paged_decode_kernel<128, 0>, grid, threads, decode_smem<128>(), s, p);
+  if (rc == 0 && p.splits > 1)
+    rc = launch_overlapped(decode_merge_kernel, dim3(unsigned(seqs * H)), D < 128 ? 64 : 128, 0, s, p);
   return rc;
-}
-
-IDRAK_API int idrak_paged_decode(const void* q, long long q_stride, const void* k_cache, const void* v_cache, const int* block_table,
-                                 const int* seq_lens, void* out, float* partial, int seqs, int H, int Hkv, int D,
-                                 int block_size, int max_blocks, int splits, float scale, int window, void* stream_) {
-  return idrak_paged_decode_kv(q, q_stride, k_cache, v_cache, nullptr, nullptr, block_table, seq_lens, out, partial, seqs,
-                               H, Hkv, D, block_size, max_blocks, splits, scale, window, stream_);
 }
 
 IDRAK_API int idrak_kv_write_paged(const void* k_src, const void* v_src, long long src_stride, const int* slots,

@@ -39,6 +39,8 @@ struct NormRopeKvParams {
 // One warp per (token, head); each lane owns PER = D / 32 elements: index e = lane + 32 j.
 template <int PER>
 __global__ void __launch_bounds__(256) norm_rope_kv_kernel(const NormRopeKvParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int heads_total = p.H + 2 * p.Hkv;
   const long long unit = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
   if (unit >= (long long)p.T * heads_total) return;
@@ -138,9 +140,6 @@ IDRAK_API int idrak_norm_rope_kv(void* qkv, long long row_stride, const int* pos
   const long long units = (long long)T * (H + 2 * Hkv);
   const int blocks = int((units + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  if (D == 64) norm_rope_kv_kernel<2><<<blocks, 256, 0, s>>>(p);
-  else if (D == 128) norm_rope_kv_kernel<4><<<blocks, 256, 0, s>>>(p);
-  else norm_rope_kv_kernel<8><<<blocks, 256, 0, s>>>(p);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(D == 64 ? norm_rope_kv_kernel<2> : (D == 128 ? norm_rope_kv_kernel<4> : norm_rope_kv_kernel<8>),
+                           dim3(unsigned(blocks)), 256, 0, s, p);
 }

@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(256) norm_fwd_block_kernel(const __nv_bfloat16
                                                              float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                              int rows, int C, float eps, int rms) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
+  pdl_wait();
   __shared__ float red[8];
   const int row = blockIdx.x;
   const size_t base = size_t(row) * C;
@@ -518,6 +519,7 @@ __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 __global__ void gated_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out, int rows,
                                  int H, int kind) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
+  pdl_wait();
   const int hv = H >> 3;
   const size_t total = size_t(rows) * hv;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -732,10 +734,8 @@ IDRAK_API int idrak_norm_fwd(const void* x, const void* residual, const void* w,
   const int blocks = (rows + 3) / 4;
   const int nvec = C / 8;
   if (rows <= 2 * sm_count() && nvec >= 128) {      // few long rows: a block per row
-    norm_fwd_block_kernel<<<rows, 256, 0, s>>>(CBF(x), CBF(residual), CBF(w), CBF(b), BF(out), BF(sum_out), mean, rstd,
-                                               rows, C, eps, rms);
-    note_launches(1);
-    return int(cudaGetLastError());
+    return launch_overlapped(norm_fwd_block_kernel, dim3(unsigned(rows)), 256, 0, s, CBF(x), CBF(residual), CBF(w), CBF(b),
+                             BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms);
   }
 #define NF(V) norm_fwd_kernel<V><<<blocks, 128, 0, s>>>(CBF(x), CBF(residual), CBF(w), CBF(b), BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms)
   if (nvec <= 32 * 1) NF(1);
@@ -877,10 +877,8 @@ IDRAK_API int idrak_gelu_bwd(const void* x, const void* dy, void* dx, long long 
 }
 IDRAK_API int idrak_gated_fwd(const void* gu, void* out, int rows, int H, int kind, void* stream_) {
   if (H % 8) return -2;
-  gated_fwd_kernel<<<grid_for(size_t(rows) * (H / 8), 256), 256, 0, static_cast<cudaStream_t>(stream_)>>>(
-      CBF(gu), BF(out), rows, H, kind);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(gated_fwd_kernel, dim3(unsigned(grid_for(size_t(rows) * (H / 8), 256))), 256, 0,
+                           static_cast<cudaStream_t>(stream_), CBF(gu), BF(out), rows, H, kind);
 }
 IDRAK_API int idrak_gated_bwd(const void* gu, const void* dout, void* dgu, int rows, int H, int kind,
                               void* stream_) {

@@ -26,8 +26,7 @@ def _bind():
         return
     vp, i, f, ll = C.c_void_p, C.c_int, C.c_float, C.c_longlong
     _native.bind("idrak_decode_partial_floats", ll, [i, i, i, i])
-    _native.bind("idrak_paged_decode", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, f, i, vp])
-    _native.bind("idrak_paged_decode_kv", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, f, i, vp])
+    _native.bind("idrak_paged_decode_kv", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, f, i, vp])
     _native.bind("idrak_norm_rope_kv", i, [vp, ll, vp, vp, vp, vp, vp, vp, vp, vp, f, f, f, i, i, i, i, i, i, vp])
     _native.bind("idrak_kv_write_paged", i, [vp, vp, ll, vp, vp, vp, i, i, vp])
     _native.bind("idrak_argmax_rows", i, [vp, i, i, i, ll, vp, vp])
@@ -154,11 +153,15 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     _, bs, Hkv, _ = k_cache.shape
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     lib = _native.lib()
+    min_keys = 0
     if splits is None:
-        # fill the machine: sequences x kv heads CTAs may be few; long contexts split along the keys
-        ctas = seqs * Hkv
+        # Shares of 128 keys (one tile per warp) to 1024: short ones so that few sequences fill the machine, long ones where
+        # there are CTAs enough, since a CTA costs about as much as 200 keys of a busy machine. 1024 CTAs if every sequence
+        # had the bound on the lengths (a power of two above them). Measured, us, shares of 128 / 512 / 1024 / unsplit:
+        # 1 sequence 9.8 / 11.8 / 11.8 / 11.8, 16 of 128 to 2304 tokens 41 / 28.5 / 40 / 51, 64 of those 145 / 91 / 84 / 95
         longest = max_len_hint if max_len_hint is not None else block_table.shape[1] * bs
-        splits = max(1, min(lib.idrak_sm_count() * 2 // max(ctas, 1), (longest + 255) // 256, 32))
+        min_keys = max(128, min(1024, (longest * seqs * Hkv // 1024 + 127) // 128 * 128))
+        splits = max(1, min((longest + min_keys - 1) // min_keys, 64))
     out = torch.empty(seqs, H, D, dtype=q.dtype, device=q.device)
     part = None
     if splits > 1:
@@ -168,7 +171,7 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     assert block_table.dtype == torch.int32 and seq_lens.dtype == torch.int32
     rc = lib.idrak_paged_decode_kv(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), ptr(k_scale),
                                    ptr(v_scale), block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), ptr(part),
-                                   seqs, H, Hkv, D, bs, block_table.shape[1], splits, float(scale), int(window),
+                                   seqs, H, Hkv, D, bs, block_table.shape[1], splits, min_keys, float(scale), int(window),
                                    stream_ptr())
     _native.check(rc, "idrak_paged_decode_kv")
     return out

@@ -175,3 +175,33 @@ def test_int8_kv_cache_write_and_decode(H, Hkv, Dh, splits):
     D.norm_rope_kv(qkv, H, Hkv, Dh, None, slots, kb, vb)
     exact = D.paged_decode_reference(q, kb, vb, table, lens_t)
     assert (out.float() - exact.float()).abs().max().item() < 6e-2
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("hint,window", [(None, 0), (4096, 0), (4096, 300)])
+def test_uneven_lengths_share_their_keys_by_the_built_in_rule(int8, Dh, hint, window):
+    """Lengths at the edges of tiles (32) and shares (128 to 512), empty and long ones in one batch, with the split that the
+    length bound gives. Probabilities enter the tensor core as bf16 (relative 2^-9) and the result is rounded to bf16:
+    2^-8 of the largest value, which is at most about 4 here."""
+    bs, Hkv, H = 16, 2, 8
+    lens = [0, 1, 31, 32, 33, 127, 128, 129, 511, 512, 513, 1025, 2000, 3000]
+    width = 256
+    need = [(n + bs - 1) // bs for n in lens]
+    order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(1)).tolist()
+    table, at = torch.zeros(len(lens), width, dtype=torch.int32), 0
+    for i, n in enumerate(need):
+        table[i, :n] = torch.tensor(order[at:at + n], dtype=torch.int32)
+        at += n
+    table, lens_t = table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    kc, vc, q = _rand((sum(need), bs, Hkv, Dh), 1), _rand((sum(need), bs, Hkv, Dh), 2), _rand((len(lens), H, Dh), 3)
+    scales = {}
+    if int8:
+        codes = [D.quantize_kv_reference(t.view(-1, Hkv, Dh)) for t in (kc, vc)]
+        (kc, ks), (vc, vs) = ((c.view(-1, bs, Hkv, Dh), s.view(-1, bs, Hkv).contiguous()) for c, s in codes)
+        scales = {"k_scale": ks, "v_scale": vs}
+    out = D.paged_decode(q, kc, vc, table, lens_t, window=window, max_len_hint=hint, **scales)
+    kd, vd = (kc.float() * ks[..., None], vc.float() * vs[..., None]) if int8 else (kc.float(), vc.float())
+    ref = D.paged_decode_reference(q.float(), kd, vd, table, lens_t, window=window)
+    assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * 4
+    assert torch.equal(out, D.paged_decode(q, kc, vc, table, lens_t, window=window, max_len_hint=hint, **scales))
