@@ -65,6 +65,7 @@ _SIGNATURES = {
     "idrak_wte_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "idrak_softmax_xent": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                    c_int, c_void_p]),
+    "idrak_scale_cast": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_ll, c_void_p]),
     "idrak_sum_rows": (c_int, [c_void_p, c_int, c_float, c_void_p, c_void_p]),
     "idrak_opt_chunk_elems": (c_int, []),
     "idrak_opt_tensor_bytes": (c_int, []),

@@ -44,6 +44,21 @@ def softmax_xent_(logits: torch.Tensor, targets: torch.Tensor, vocab: int, grad_
     return losses
 
 
+def _scaled(x: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``(x * scale).to(dtype)`` with a device scalar, in one pass for bf16 results outside a recorded backward."""
+    if (dtype == torch.bfloat16 and x.dtype in (torch.float32, torch.bfloat16) and x.is_cuda and x.is_contiguous()
+            and not torch.is_grad_enabled() and x.data_ptr() % 16 == 0
+            and (out is None or (out.is_contiguous() and out.data_ptr() % 16 == 0 and out.dtype == dtype))):
+        out = torch.empty_like(x, dtype=dtype) if out is None else out
+        scale = scale.float()
+        rc = _native.lib().idrak_scale_cast(x.data_ptr(), int(x.dtype == torch.float32), scale.data_ptr(), out.data_ptr(),
+                                            x.numel(), stream_ptr())
+        _native.check(rc, "idrak_scale_cast")
+        return out
+    y = (x * scale.to(x.dtype)).to(dtype)
+    return y if out is None else out.copy_(y)
+
+
 class _TokenCrossEntropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, targets, vocab, chunk_rows, ignore_index):
@@ -55,7 +70,7 @@ class _TokenCrossEntropy(torch.autograd.Function):
         t = targets.reshape(-1)
         # gradients are produced for d(mean loss) with upstream gradient 1; backward rescales them
         need_grad = hidden.requires_grad or weight.requires_grad
-        dh = torch.empty_like(h2) if need_grad else None
+        dh = torch.empty_like(h2) if hidden.requires_grad else None
         dw = None
         losses = []
         inv_dev = None
@@ -75,8 +90,9 @@ class _TokenCrossEntropy(torch.autograd.Function):
             r1 = min(rows, r0 + chunk_rows)
             logits = gemm(h2[r0:r1], weight)                       # [chunk, Vpad]
             losses.append(softmax_xent_(logits, t[r0:r1], vocab, inv, ignore_index, write_grad=need_grad))
-            if need_grad:
+            if dh is not None:
                 gemm(logits, weight, b_mn=True, out=dh[r0:r1])     # dH = dL @ W
+            if weight.requires_grad:                               # a frozen head has no gradient product
                 if dw is None:
                     dw = gemm(logits, h2[r0:r1], a_mn=True, b_mn=True, out_dtype=torch.float32)
                 else:
@@ -96,7 +112,7 @@ class _TokenCrossEntropy(torch.autograd.Function):
         dh, dw = ctx.saved_tensors
         if ctx.inv_dev is not None:
             dloss = dloss * ctx.inv_dev
-        gh = (dh * dloss.to(dh.dtype)).reshape(ctx.hshape) if dh is not None and ctx.needs_input_grad[0] else None
+        gh = _scaled(dh, dloss, dh.dtype).reshape(ctx.hshape) if dh is not None and ctx.needs_input_grad[0] else None
         gw = None
         if dw is not None and ctx.needs_input_grad[1]:
             tgt = _grad.target(ctx.param)
@@ -105,10 +121,10 @@ class _TokenCrossEntropy(torch.autograd.Function):
                 if accumulate:
                     g.add_((dw * dloss).to(g.dtype))
                 else:
-                    torch.mul(dw, dloss.to(dw.dtype), out=g) if g.dtype == dw.dtype else g.copy_(dw * dloss)
+                    torch.mul(dw, dloss.to(dw.dtype), out=g) if g.dtype == dw.dtype else _scaled(dw, dloss, g.dtype, g)
                 _grad.written(ctx.param)
             else:
-                gw = (dw * dloss).to(ctx.wdtype)
+                gw = _scaled(dw, dloss, ctx.wdtype)
         return gh, gw, None, None, None, None
 
 

@@ -73,6 +73,27 @@ def test_token_cross_entropy_chunked_matches_torch():
     assert (w.grad.float() - wr.grad).abs().max().item() < 3e-2 * wr.grad.abs().max().item() + 1e-5
 
 
+@pytest.mark.parametrize("train_hidden,train_head", [(True, True), (True, False), (False, True)])
+@pytest.mark.parametrize("C,V", [(64, 264), (72, 1000)])
+def test_token_cross_entropy_frozen_sides_and_upstream_scale(train_hidden, train_head, C, V):
+    """Gradients times an upstream factor, and none for a side that is frozen. The logit gradients are bf16 (relative 2^-9)
+    and sums of them are rounded to bf16 once more: 2^-7 of the sum of magnitudes bounds both."""
+    rows = 77
+    h, w = _rand((rows, C), 1.0, 1).requires_grad_(train_hidden), _rand((V, C), 0.1, 2).requires_grad_(train_head)
+    t = torch.randint(0, V, (rows,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    (ops.token_cross_entropy(h, w, t, vocab=V, chunk_rows=None, ignore_index=None) * 0.37).backward()
+    hd, wd = h.detach().double().requires_grad_(), w.detach().double().requires_grad_()
+    lg = (hd @ wd.t()).detach().requires_grad_()
+    (torch.nn.functional.cross_entropy(lg, t) * 0.37).backward()
+    d = lg.grad
+    for got, want, mag in ((h.grad, d @ wd, d.abs() @ wd.abs()), (w.grad, d.t() @ hd, d.abs().t() @ hd.abs())):
+        if got is None:
+            continue
+        # logits are rounded to bf16 before the softmax: up to 2^-8 of a logit (|logit| < 8) moves a probability by 2^-5
+        assert ((got.double() - want).abs() <= (2.0 ** -7 + 2.0 ** -5) * mag + 1e-7).all()
+    assert (h.grad is not None) == train_hidden and (w.grad is not None) == train_head
+
+
 def test_fused_adamw_matches_torch_adamw():
     torch.manual_seed(0)
     shapes = [(300, 77), (5000,), (64, 64), (3,)]
