@@ -94,8 +94,8 @@ def kernel_shapes() -> List[KernelShape]:
         KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128"),
         KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
                     "cta_group::2: each CTA holds half of the A rows and half of the B columns"),
-        KernelShape("skinny_gemm_kernel", "128 features x (16 | 32 | 64) tokens x 64, K over a cluster of up to 8", 4, 192,
-                    98304, 64, 2, "partial tiles summed through distributed shared memory"),
+        KernelShape("skinny_gemm_kernel", "128 features x (16 | 32 | 64) tokens x 64, K over a cluster of up to 8", 4, 320,
+                    100352, 64, 2, "partial tiles summed through distributed shared memory"),
         KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 100 * 1024, 256, 2, ""),
         KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 197 * 1024, 512, 1, ""),
         KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 160 * 1024, 320, 1, ""),

@@ -280,10 +280,7 @@ class ModelRunner:
         s, dev, bs = self.spec, self.device, self.block_size
         H, Hkv, D = s.heads, s.kv_heads, s.head_dim
         n = tokens.shape[0]
-        rows = torch.arange(n, device=dev)
-        blk_of = block_table[rows, (positions // bs).long()]
-        slots = (blk_of * bs + positions % bs).to(torch.int32)
-        lens = (positions + 1).to(torch.int32)
+        slots, lens = dops.decode_slots(positions, block_table, bs)
         x = self._embed(tokens, positions)
         if n <= 64 and self._few_row_path():
             return self._decode_few_rows(x.view(n, -1), positions, slots, block_table, lens, max_len_hint)
@@ -327,43 +324,59 @@ class ModelRunner:
             if not ok:
                 break
             rope = blk.attn.rope
-            ok = (not any(getattr(m, "adapters", None) is not None or getattr(m, "packed", None)
-                          for m in (blk.attn, blk.mlp)) and (rope is None or rope.scaling is None))
+            packed = [w for m in (blk.attn, blk.mlp) for w in (getattr(m, "packed", None) or {}).values()]
+            dense = [w for w in (blk.attn.qkv_weight, blk.attn.o_weight, blk.mlp.up_weight, blk.mlp.down_weight) if w is not None]
+            ok = (not any(getattr(m, "adapters", None) is not None for m in (blk.attn, blk.mlp))
+                  and (rope is None or rope.scaling is None)
+                  and (not packed or (self.few_row_packed and len(packed) == 4 and not dense
+                                      and all(self._streams(w, "silu" if w is blk.mlp.packed["up"] else None) for w in packed))))
         self._few_rows_ok = bool(ok)
         return self._few_rows_ok
 
+    few_row_packed = True          # the few-row path takes int8 / int4 weights too (a subclass with its own path may not)
+
+    def _streams(self, w, gate) -> bool:
+        """Whether the few-row kernels take a packed weight as it is stored (``ops.skinny.packed_supported``)."""
+        from ..ops.skinny import packed_supported
+        return (w.bits in (4, 8) and getattr(w, "kind", "int") == "int"
+                and packed_supported(torch.empty(1, w.rows, dtype=self.dtype, device=self.device), w, gate))
+
+    @staticmethod
+    def _few(x, owner, name, residual=None, gate=None, norm_eps=None):
+        """One few-row projection of a block: ``name`` in qkv / o / up / down of an attention or feed-forward module."""
+        from ..ops.skinny import packed_linear, skinny_linear
+        w, bias = getattr(owner, name + "_weight"), getattr(owner, name + "_bias")
+        if w is None:
+            return packed_linear(x, owner.packed[name], bias, residual, gate)
+        return skinny_linear(x, w, bias, residual, gate, norm_eps)
+
     def _decode_few_rows(self, x, positions, slots, block_table, lens, max_len_hint):
-        """Six or seven launches per layer: qkv (+norm) | norms of q, k + RoPE + cache write | paged attention
-        (+ its merge) | out + residual | gate/up (+norm) + activation | down + residual."""
-        from ..ops.skinny import few_row_linear, skinny_linear
+        """Six to eight launches per layer: (norm |) qkv | norms of q, k + RoPE + cache write | paged attention (+ its
+        merge) | out + residual | (norm |) gate/up + activation | down + residual."""
+        from ..ops.rowops import norm_forward
+        from ..ops.skinny import few_row_linear
         s, m = self.spec, self.model
         H, Hkv, D = s.heads, s.kv_heads, s.head_dim
         folded = bool(getattr(m, "_norms_folded", False))
         eps = s.norm_epsilon if folded else None
         n = x.shape[0]
+
+        def norm(layer, t):        # the layer's forward without an autograd node: a decode step is launch-bound on the host
+            return norm_forward(t, layer.effective_weight(), layer.bias, layer.eps, layer.kind != "layer")[0]
+
         for li, blk in enumerate(m.blocks):
             attn, mlp = blk.attn, blk.mlp
-            h = x if folded else blk.attn_norm(x)
-            qkv = skinny_linear(h, attn.qkv_weight, attn.qkv_bias, norm_eps=eps)
+            qkv = self._few(x if folded else norm(blk.attn_norm, x), attn, "qkv", norm_eps=eps)
             self._rotate_and_cache(attn, qkv, positions, slots, li)
             q = qkv[:, : H * D].unflatten(-1, (H, D))
             window = s.sliding_window if s.is_windowed(attn.layer) else 0
             o = dops.paged_decode(q, self.k_cache[li], self.v_cache[li], block_table, lens, attn.scale, window or 0,
                                   max_len_hint=max_len_hint, k_scale=self.k_scale[li], v_scale=self.v_scale[li])
-            x = skinny_linear(o.reshape(n, H * D), attn.o_weight, attn.o_bias, residual=x)
-            if folded:
-                g = skinny_linear(x, mlp.up_weight, mlp.up_bias, gate=s.activation, norm_eps=eps)
-            else:
-                # the stacked gate / up matrix is wide enough for the dense kernel to stream it faster (measured:
-                # 56 + 8 us against 74 us at 64 rows of the 8 B shape); the few-row kernel earns its place where the
-                # norm is folded in as well
-                gu = ops.gemm(blk.mlp_norm(x), mlp.up_weight, bias=mlp.up_bias)
-                g = ops.gated_activation(gu, s.activation)
-            x = skinny_linear(g, mlp.down_weight, mlp.down_bias, residual=x)
-        if folded:
-            logits = skinny_linear(x, m.head_weight(), m.head_bias, norm_eps=s.norm_epsilon)
-        else:
-            logits = few_row_linear(m.norm(x), m.head_weight(), m.head_bias)      # a wide head streams faster densely
+            x = self._few(o.reshape(n, H * D), attn, "o", residual=x)
+            g = self._few(x if folded else norm(blk.mlp_norm, x), mlp, "up", gate=s.activation, norm_eps=eps)
+            x = self._few(g, mlp, "down", residual=x)
+        h = x if folded else norm(m.norm, x)
+        logits = few_row_linear(h, m.head_weight(), m.head_bias, norm_eps=eps)
         return logits.reshape(-1, logits.shape[-1])
 
     # ------------------------------------------------------------------ decode as a replayed CUDA graph

@@ -36,6 +36,8 @@ class TPModelRunner(ModelRunner):
         self.vocab_offset = lo
         self.vocab_local = max(0, min(hi, self.full_spec.vocabulary) - lo)      # columns of the slice that are real tokens
 
+    few_row_packed = False         # its few-row path below is written over dense slices
+
     def _few_row_path(self) -> bool:
         """Decode steps of up to 64 sequences on the few-row projection kernels, as on one GPU, with the row-parallel
         products written straight into the symmetric buffer the all-reduce kernel reads."""

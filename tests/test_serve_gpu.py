@@ -91,3 +91,30 @@ def test_engine_end_to_end_on_device():
     assert all(len(r.logprobs) == 24 and max(r.logprobs) <= 0 for r in a)
     st = eng.stats()
     assert st["free_blocks"] == 256 and st["running"] == 0
+
+
+@pytest.mark.parametrize("quant", ["", "int8", "int4"])
+@pytest.mark.parametrize("rows", [1, 9, 40])
+def test_few_row_decode_agrees_with_the_layer_by_layer_path(quant, rows):
+    """The fused decode path (bf16 or packed projections) against the modules' own forwards over the same cache. Both round
+    activations to bf16 at every layer (relative 2^-9, ten roundings over two layers), the fused one at fewer places."""
+    from idrak_b200.models import DecoderSpec, build_decoder
+    from idrak_b200.quant import quantize_model
+    from idrak_b200.serve import ModelRunner
+    torch.manual_seed(0)
+    spec = DecoderSpec.llama(layers=2, dim=256, heads=4, kv_heads=2, ff_dim=512, vocab=500, max_positions=256, head_dim=64)
+    model = build_decoder(spec, seed=1).to("cuda", torch.bfloat16)
+    if quant:
+        quantize_model(model, quant)
+    runner = ModelRunner(model, rows * 4, 16)
+    for c in runner.k_cache + runner.v_cache:
+        c.copy_(torch.randn(c.shape, device="cuda"))
+    table = torch.randperm(rows * 4, device="cuda").to(torch.int32).view(rows, 4)
+    positions = torch.randint(0, 64, (rows,), device="cuda", dtype=torch.int32)
+    tokens = torch.randint(0, 500, (rows,), device="cuda", dtype=torch.int32)
+    assert runner._few_row_path()
+    fused = runner.decode(tokens, positions, table).float()
+    runner._few_rows_ok = False
+    plain = runner.decode(tokens, positions, table).float()
+    rms = plain.pow(2).mean().sqrt()
+    assert ((fused - plain).pow(2).mean().sqrt() <= 10 * 2.0 ** -9 * rms) and fused.isfinite().all()
