@@ -2,8 +2,9 @@
 // rotary embedding of both, and the write of the new keys / values into the paged cache - bf16, or int8 with one
 // scale per (token, kv head).
 //
-// The packed projection row of a token is [H query heads | Hkv key heads | Hkv value heads] x D. One warp takes one
-// (token, head); lane l holds elements l, l + 32, l + 64, ... of the head, so both members of a rotation pair
+// The packed projection row of a token is [H query heads | Hkv key heads | Hkv value heads] x D. One warp takes one token and
+// a run of heads, one after another, so that the angles (a power and a range-reduced sincos per pair) are taken once per run:
+// and four heads' loads are in flight at a time (one head per warp: 9712 tokens x 48 heads of 128 128 us, now 63). Lane l holds elements l, l + 32, l + 64, ... of the head, so both members of a rotation pair
 // (i, i + rot_dim / 2) sit in the same lane.
 //   query head   -> norm, rotate, written back in place (attention reads it from the projection buffer)
 //   key head     -> norm, rotate, written back in place (prefill attention reads it there) and into the cache slot
@@ -34,82 +35,127 @@ struct NormRopeKvParams {
   float theta, freq_scale;
   int rot_dim;                   // elements of a head that rotate (pairs i, i + rot_dim / 2); 0 = no rotation
   int T, H, Hkv, D, kv_int8;
+  int run;                       // heads per warp
 };
 
-// One warp per (token, head); each lane owns PER = D / 32 elements: index e = lane + 32 j.
-template <int PER>
+// One warp per token and run of heads, four heads in flight at a time; each lane owns PER = D / 32 elements of a head.
+// kPairs = 0: elements e = lane + 32 j (any rotary width that is a multiple of 64). kPairs = 1 (PER = 4, rotary width = the
+// whole head or none): e = 2 lane, 2 lane + 1 and the same plus D / 2, in four-byte accesses.
+template <int PER, int kPairs>
 __global__ void __launch_bounds__(256) norm_rope_kv_kernel(const NormRopeKvParams p) {
   pdl_launch_dependents();
   pdl_wait();
+  constexpr int kBatch = 4;
   const int heads_total = p.H + 2 * p.Hkv;
+  const int runs = (heads_total + p.run - 1) / p.run;
   const long long unit = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (unit >= (long long)p.T * heads_total) return;
-  const int t = int(unit / heads_total), h = int(unit - (long long)t * heads_total);
+  if (unit >= (long long)p.T * runs) return;
+  const int t = int(unit / runs), h0 = int(unit - (long long)t * runs) * p.run;
   const int lane = threadIdx.x & 31;
   const int D = p.D;
-  __nv_bfloat16* src = p.qkv + size_t(t) * p.row_stride + size_t(h) * D;
-  const bool is_q = h < p.H, is_k = !is_q && h < p.H + p.Hkv;
-  const int kvh = is_q ? 0 : (is_k ? h - p.H : h - p.H - p.Hkv);
-  float v[PER];
+  const bool rotate = p.rot_dim > 0 && p.positions;
+  const int hj = kPairs ? 2 : p.rot_dim >> 6;         // distance in j of a pair's members: half / 32, half = rot_dim / 2
+  auto element = [&](int j) { return kPairs ? 2 * lane + (j & 1) + (j >> 1) * (PER * 16) : lane + 32 * j; };
+  auto load = [&](const __nv_bfloat16* src, float (&v)[PER]) {
+    if constexpr (kPairs) {
 #pragma unroll
-  for (int j = 0; j < PER; ++j) v[j] = __bfloat162float(src[lane + 32 * j]);
-  if (is_q || is_k) {
-    const __nv_bfloat16* nw = is_q ? p.q_norm : p.k_norm;
-    if (nw) {
-      float ss = 0.f;
+      for (int j = 0; j < PER; j += 2) {
+        const float2 f = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(src + element(j)));
+        v[j] = f.x;
+        v[j + 1] = f.y;
+      }
+    } else {
 #pragma unroll
-      for (int j = 0; j < PER; ++j) ss += v[j] * v[j];
-      ss = warp_sum(ss);
-      const float r = rsqrtf(ss / float(D) + p.eps);
-#pragma unroll
-      for (int j = 0; j < PER; ++j)
-        v[j] = __bfloat162float(__float2bfloat16(v[j] * r * __bfloat162float(nw[lane + 32 * j])));   // as a separate norm would store it
+      for (int j = 0; j < PER; ++j) v[j] = __bfloat162float(src[element(j)]);
     }
-    if (p.rot_dim > 0 && p.positions) {
-      // element e < half pairs with e + half; with e = lane + 32 j the partner lives in the same lane at j + half / 32
-      const int half = p.rot_dim >> 1;
-      const int hj = half >> 5;                       // half % 32 == 0 (rot_dim % 64 == 0)
-      const float pos = float(p.positions[t]) * p.freq_scale;      // the arithmetic of rope_kernel, so results agree bit for bit
+  };
+  auto store = [&](__nv_bfloat16* dst, const float (&v)[PER]) {
+    if constexpr (kPairs) {
 #pragma unroll
-      for (int j = 0; j < PER / 2; ++j) {
-        if (j < hj) {
-          const int e = lane + 32 * j;
-          const float inv = __powf(p.theta, -2.0f * float(e) / float(p.rot_dim));
-          float sn, cs;
-          sincosf(pos * inv, &sn, &cs);
-          const float a = v[j], b = v[j + hj];
-          v[j] = a * cs - b * sn;
-          v[j + hj] = b * cs + a * sn;
-        }
+      for (int j = 0; j < PER; j += 2) *reinterpret_cast<uint32_t*>(dst + element(j)) = pack_bf16x2(v[j], v[j + 1]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) dst[element(j)] = __float2bfloat16(v[j]);
+    }
+  };
+  float sn[PER / 2], cs[PER / 2];
+  if (rotate && h0 < p.H + p.Hkv) {
+    const float pos = float(p.positions[t]) * p.freq_scale;      // the arithmetic of the rope kernels, so results agree bit for bit
+#pragma unroll
+    for (int j = 0; j < PER / 2; ++j) {
+      if (j < hj) {
+        const float inv = __powf(p.theta, -2.0f * float(element(j)) / float(p.rot_dim));
+        sincosf(pos * inv, &sn[j], &cs[j]);
       }
     }
-#pragma unroll
-    for (int j = 0; j < PER; ++j) src[lane + 32 * j] = __float2bfloat16(v[j]);
   }
-  if (is_q || !p.slots) return;
-  const int slot = p.slots[t];
-  if (slot < 0) return;
-  const size_t row = (size_t(slot) * p.Hkv + kvh) * D;
-  if (!p.kv_int8) {
-    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(is_k ? p.k_cache : p.v_cache) + row;
+  const int slot = p.slots ? p.slots[t] : -1;
+  __nv_bfloat16* row_base = p.qkv + size_t(t) * p.row_stride;
+  const int h1 = min(heads_total, h0 + p.run);
+  for (int hb = h0; hb < h1; hb += kBatch) {
+    float buf[kBatch][PER];
 #pragma unroll
-    for (int j = 0; j < PER; ++j) dst[lane + 32 * j] = __float2bfloat16(v[j]);
-  } else {
-    float mx = 0.f;
+    for (int i = 0; i < kBatch; ++i)
+      if (hb + i < h1) load(row_base + size_t(hb + i) * D, buf[i]);
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      v[j] = __bfloat162float(__float2bfloat16(v[j]));       // quantise what the bf16 cache would have held
-      mx = fmaxf(mx, fabsf(v[j]));
+    for (int i = 0; i < kBatch; ++i) {
+      const int h = hb + i;
+      if (h >= h1) break;
+      const bool is_q = h < p.H, is_k = !is_q && h < p.H + p.Hkv;
+      const int kvh = is_q ? 0 : (is_k ? h - p.H : h - p.H - p.Hkv);
+      float(&v)[PER] = buf[i];
+      if (is_q || is_k) {
+        const __nv_bfloat16* nw = is_q ? p.q_norm : p.k_norm;
+        if (nw) {
+          float ss = 0.f;
+#pragma unroll
+          for (int j = 0; j < PER; ++j) ss += v[j] * v[j];
+          ss = warp_sum(ss);
+          const float r = rsqrtf(ss / float(D) + p.eps);
+#pragma unroll
+          for (int j = 0; j < PER; ++j)
+            v[j] = __bfloat162float(__float2bfloat16(v[j] * r * __bfloat162float(nw[element(j)])));   // as a separate norm would store it
+        }
+        if (rotate) {
+#pragma unroll
+          for (int j = 0; j < PER / 2; ++j) {
+            if (j < hj) {
+              // v[j + hj] with hj = 1, 2 or 4: constant indices, so that v stays in registers
+#pragma unroll
+              for (int o = 1; o <= PER / 2; o <<= 1) {
+                if (o == hj && j + o < PER) {
+                  const float a = v[j], b = v[j + o];
+                  v[j] = a * cs[j] - b * sn[j];
+                  v[j + o] = b * cs[j] + a * sn[j];
+                }
+              }
+            }
+          }
+        }
+        store(row_base + size_t(h) * D, v);
+      }
+      if (is_q || slot < 0) continue;
+      const size_t row = (size_t(slot) * p.Hkv + kvh) * D;
+      if (!p.kv_int8) {
+        store(static_cast<__nv_bfloat16*>(is_k ? p.k_cache : p.v_cache) + row, v);
+      } else {
+        float mx = 0.f;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+          v[j] = __bfloat162float(__float2bfloat16(v[j]));       // quantise what the bf16 cache would have held
+          mx = fmaxf(mx, fabsf(v[j]));
+        }
+        mx = warp_max(mx);
+        const float scale = mx > 0.f ? mx / 127.f : 1.f;
+        int8_t* dst = static_cast<int8_t*>(is_k ? p.k_cache : p.v_cache) + row;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+          const int q = __float2int_rn(v[j] / scale);
+          dst[element(j)] = int8_t(max(-127, min(127, q)));
+        }
+        if (lane == 0) (is_k ? p.k_scale : p.v_scale)[size_t(slot) * p.Hkv + kvh] = scale;
+      }
     }
-    mx = warp_max(mx);
-    const float scale = mx > 0.f ? mx / 127.f : 1.f;
-    int8_t* dst = static_cast<int8_t*>(is_k ? p.k_cache : p.v_cache) + row;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int q = __float2int_rn(v[j] / scale);
-      dst[lane + 32 * j] = int8_t(max(-127, min(127, q)));
-    }
-    if (lane == 0) (is_k ? p.k_scale : p.v_scale)[size_t(slot) * p.Hkv + kvh] = scale;
   }
 }
 
@@ -159,9 +205,16 @@ IDRAK_API int idrak_norm_rope_kv(void* qkv, long long row_stride, const int* pos
   p.k_norm = static_cast<const __nv_bfloat16*>(k_norm);
   p.eps = eps; p.theta = theta; p.freq_scale = freq_scale; p.rot_dim = rot_dim;
   p.T = T; p.H = H; p.Hkv = Hkv; p.D = D; p.kv_int8 = kv_int8;
-  const long long units = (long long)T * (H + 2 * Hkv);
+  const int heads = H + 2 * Hkv;
+  p.run = 1;                     // longer runs as long as there are four warps for every scheduler of the device
+  while (p.run < 16 && (long long)T * ((heads + 2 * p.run - 1) / (2 * p.run)) >= (long long)sm_count() * 16) p.run *= 2;
+  const long long units = (long long)T * ((heads + p.run - 1) / p.run);
   const int blocks = int((units + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  return launch_overlapped(D == 64 ? norm_rope_kv_kernel<2> : (D == 128 ? norm_rope_kv_kernel<4> : norm_rope_kv_kernel<8>),
-                           dim3(unsigned(blocks)), 256, 0, s, p);
+  const bool pairs = D == 128 && (rot_dim == 0 || rot_dim == 128 || !positions) && row_stride % 2 == 0 &&
+                     (reinterpret_cast<uintptr_t>(qkv) & 3) == 0 && (reinterpret_cast<uintptr_t>(k_cache) & 3) == 0 &&
+                     (reinterpret_cast<uintptr_t>(v_cache) & 3) == 0;
+  auto kern = D == 64 ? norm_rope_kv_kernel<2, 0>
+                      : (D == 256 ? norm_rope_kv_kernel<8, 0> : (pairs ? norm_rope_kv_kernel<4, 1> : norm_rope_kv_kernel<4, 0>));
+  return launch_overlapped(kern, dim3(unsigned(blocks)), 256, 0, s, p);
 }

@@ -31,6 +31,11 @@ def _split_qkv(qkv, H, Hkv, D):
     return q, k, v
 
 
+def _query_key_heads(qkv, heads, D):
+    """The query and key heads of a packed projection as one ``[tokens, heads, D]`` view."""
+    return qkv[..., : heads * D].unflatten(-1, (heads, D)).flatten(0, 1)
+
+
 class _QkvAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, H, Hkv, D, causal, scale, rope_theta, rope_dim, rope_scale, positions, window=None,
@@ -38,9 +43,8 @@ class _QkvAttention(torch.autograd.Function):
         B, S, _ = qkv.shape
         q, k, v = _split_qkv(qkv, H, Hkv, D)
         if rope_theta is not None:
-            # the projection output is ours to overwrite: rotate q and k where they lie
-            for t, heads in ((q, H), (k, Hkv)):
-                rope_(t.flatten(0, 1), positions, rope_theta, rope_dim, rope_scale, False)
+            # the projection output is ours to overwrite: rotate q and k (neighbouring heads) where they lie
+            rope_(_query_key_heads(qkv, H + Hkv, D), positions, rope_theta, rope_dim, rope_scale, False)
         out, lse = flash_forward(q, k, v, causal, scale, window, row_start, softcap)
         ctx.save_for_backward(qkv, out, lse, positions)
         ctx.cfg = (H, Hkv, D, causal, scale, rope_theta, rope_dim, rope_scale)
@@ -60,8 +64,7 @@ class _QkvAttention(torch.autograd.Function):
         flash_backward(dout.reshape(B, S, H, D), q, k, v, out, lse, causal, scale, (dq, dk, dv), window, row_start,
                        softcap)
         if rope_theta is not None:
-            for t in (dq, dk):
-                rope_(t.flatten(0, 1), positions, rope_theta, rope_dim, rope_scale, True)
+            rope_(_query_key_heads(dqkv, H + Hkv, D), positions, rope_theta, rope_dim, rope_scale, True)
         return (dqkv,) + (None,) * 12
 
 

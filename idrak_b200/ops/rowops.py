@@ -76,8 +76,8 @@ def norm_forward(x, weight, bias, eps, rms, residual=None):
 
 
 def norm_backward(dy, x, weight, mean, rstd, rms, has_bias, dres=None, w_param=None, b_param=None,
-                  sums_of_dx: bool = False):
-    """Returns (dx, dweight, dbias). ``x`` is the tensor that was normalised. ``dres`` is added to dx.
+                  sums_of_dx: bool = False, frozen: bool = False):
+    """Returns (dx, dweight, dbias); with ``frozen`` (weight and bias take no gradient) the latter two may be None. ``x`` is the tensor that was normalised. ``dres`` is added to dx.
     When ``w_param`` (and ``b_param``) take direct gradient writes, dweight / dbias go straight into their
     ``.grad`` and come back as None. With ``sums_of_dx`` the column sums of dx (fp32) are attached to the returned
     dx as ``_idrak_colsum`` where the kernel produces them on the way (rows of up to 1024 elements): dx is the
@@ -100,6 +100,12 @@ def norm_backward(dy, x, weight, mean, rstd, rms, has_bias, dres=None, w_param=N
     lib = _native.lib()
     dy2, x2 = dy2.contiguous(), x2.contiguous()
     dx = torch.empty_like(x2)
+    if frozen and not (has_bias and sums_of_dx):
+        d2 = dres.reshape(-1, C).contiguous() if dres is not None else None
+        rc = lib.idrak_norm_bwd_fused(dy2.data_ptr(), x2.data_ptr(), weight.data_ptr(), ptr(mean), rstd.data_ptr(), ptr(d2),
+                                      dx.data_ptr(), None, None, None, None, 0, 0, rows, C, int(rms), stream_ptr())
+        _native.check(rc, "idrak_norm_bwd_fused")
+        return dx.reshape(x.shape), None, None
     blocks = lib.idrak_norm_bwd_blocks(rows)
     part = scratch("norm_bwd", 3 * blocks * C, torch.float32, x.device)
     from . import _grad
@@ -144,7 +150,8 @@ class _Norm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight, mean, rstd = ctx.saved_tensors
-        dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, None, *ctx.params)
+        dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, None, *ctx.params,
+                                   frozen=not any(ctx.needs_input_grad[1:3]))
         return dx, dw, db, None, None
 
 
@@ -167,7 +174,7 @@ class _NormBranch(torch.autograd.Function):
         if dy is None:
             return dres, None, None, None, None
         dx, dw, db = norm_backward(dy, x, weight, mean, rstd, ctx.rms, ctx.has_bias, dres, *ctx.params,
-                                   sums_of_dx=True)
+                                   sums_of_dx=True, frozen=not any(ctx.needs_input_grad[1:3]))
         return dx, dw, db, None, None
 
 

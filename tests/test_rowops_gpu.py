@@ -157,3 +157,51 @@ def test_embedding_forward_backward():
 def test_colsum():
     x = _rand((1000, 200), 1.0, 1)
     _close(ops.colsum(x), x.float().sum(0), 1e-2)
+
+
+@pytest.mark.parametrize("tokens,heads,D,rot", [(1, 1, 64, 64), (3, 5, 128, 128), (7, 40, 128, 64), (2000, 40, 128, 128),
+                                                (1500, 33, 64, 64), (50, 3, 64, 32), (9, 4, 256, 128)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_rope_of_a_packed_projection(tokens, heads, D, rot, inverse):
+    """A strided view of a packed projection, positions given: runs of heads per warp, partial rotary widths, and the
+    general kernel (rot 32). One bf16 rounding (2^-8 of the pair's magnitude covers it and the angle's fp32 error)."""
+    buf = _rand((tokens, heads * D + 2 * D), 1.0, 1)
+    keep = buf.clone()
+    x = buf[:, D: D + heads * D].unflatten(-1, (heads, D))
+    pos = torch.randint(0, 5000, (tokens,), device="cuda", dtype=torch.int32, generator=torch.Generator(device="cuda").manual_seed(2))
+    want = ops.rope_reference(x.clone(), pos, 10000.0, rot, 1.0, inverse).float()
+    ops.rope_(x, pos, 10000.0, rot, 1.0, inverse)
+    assert ((x.float() - want).abs() <= 2.0 ** -8 * 6 + 2e-3).all()
+    assert torch.equal(buf[:, :D], keep[:, :D]) and torch.equal(buf[:, D + heads * D:], keep[:, D + heads * D:])
+    assert torch.equal(x[..., rot:], keep[:, D: D + heads * D].unflatten(-1, (heads, D))[..., rot:])
+
+
+@pytest.mark.parametrize("rows,C", [(400, 2048), (301, 2056), (400, 4096), (333, 8192), (5, 1032)])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_of_long_rows_and_backward_with_a_frozen_weight(rows, C, rms):
+    x, w, dy = _rand((rows, C), 1.0, 1).requires_grad_(), _rand((C,), 1.0, 2), _rand((rows, C), 1.0, 3)
+    b = None if rms else _rand((C,), 1.0, 4)
+    y = ops.rms_norm(x, w, 1e-5) if rms else ops.layer_norm(x, w, b, 1e-5)
+    y.backward(dy)
+    xr = x.detach().double().requires_grad_()
+    if rms:
+        yr = xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    else:
+        yr = torch.nn.functional.layer_norm(xr, (C,), w.double(), b.double(), 1e-5)
+    yr.backward(dy.double())
+    # one bf16 rounding each (2^-9) and fp32 sums
+    assert ((y.double() - yr).abs() <= 2.0 ** -8 * yr.abs() + 1e-4).all()
+    assert ((x.grad.double() - xr.grad).abs() <= 2.0 ** -8 * xr.grad.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 2040), (5, 2048), (5, 2056), (70, 14336)])
+def test_gated_activation_at_the_edges_of_a_block(rows, H):
+    from idrak_b200.ops.rowops import GATE_KINDS, _gate_ref
+    gu, do = _rand((rows, 2 * H), 1.5, 3).requires_grad_(), _rand((rows, H), 1.0, 4)
+    o = ops.gated_activation(gu, "silu")
+    o.backward(do)
+    gr = gu.detach().float().requires_grad_()
+    ref = _gate_ref(gr[:, :H], GATE_KINDS["silu"]) * gr[:, H:]
+    ref.backward(do.float())
+    _close(o, ref)
+    _close(gu.grad, gr.grad)
