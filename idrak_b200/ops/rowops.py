@@ -238,14 +238,21 @@ def _gate_ref(g, kind):
     return torch.tanh(g)
 
 
+def gated_forward(gu2: torch.Tensor, kind: int) -> torch.Tensor:
+    """The kernel of ``gated_activation`` on a contiguous ``[rows, 2 H]`` bf16 matrix, ``kind`` one of ``GATE_KINDS``."""
+    H = gu2.shape[1] // 2
+    out = torch.empty((gu2.shape[0], H), dtype=gu2.dtype, device=gu2.device)
+    _native.check(_native.lib().idrak_gated_fwd(gu2.data_ptr(), out.data_ptr(), gu2.shape[0], H, kind, stream_ptr()),
+                  "gated_fwd")
+    return out
+
+
 class _Gated(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gu, kind):
         H = gu.shape[-1] // 2
         gu2 = gu.reshape(-1, 2 * H).contiguous()
-        out = torch.empty((gu2.shape[0], H), dtype=gu.dtype, device=gu.device)
-        _native.check(_native.lib().idrak_gated_fwd(gu2.data_ptr(), out.data_ptr(), gu2.shape[0], H, kind,
-                                                    stream_ptr()), "gated_fwd")
+        out = gated_forward(gu2, kind)
         ctx.save_for_backward(gu2)
         ctx.kind, ctx.shape = kind, gu.shape
         return out.reshape(*gu.shape[:-1], H)

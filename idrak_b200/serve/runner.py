@@ -20,6 +20,7 @@ import os
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -198,23 +199,11 @@ class ModelRunner:
     def prefill(self, items: Sequence[PrefillItem], all_logits: bool = False) -> torch.Tensor:
         """Computes the listed tokens of every item, fills the cache, and returns the logits of each item's last
         token ``[len(items), padded vocabulary]`` (or of every computed token, packed, when ``all_logits``)."""
-        s, dev, bs = self.spec, self.device, self.block_size
+        s, dev = self.spec, self.device
         H, Hkv, D = s.heads, s.kv_heads, s.head_dim
-        ids, pos, slots, bounds = [], [], [], [0]
-        for it in items:
-            n = len(it.tokens)
-            ids += it.tokens
-            for j in range(n):
-                p = it.start + j
-                pos.append(p)
-                slots.append(it.blocks[p // bs] * bs + p % bs)
-            bounds.append(bounds[-1] + n)
-        ids_t = torch.tensor(ids, dtype=torch.int32, device=dev)
-        pos_t = torch.tensor(pos, dtype=torch.int32, device=dev)
-        slots_t = torch.tensor(slots, dtype=torch.int32, device=dev)
+        ids_t, pos_t, slots_t, last, bounds = self._pack(items)
         tables = [torch.tensor(it.blocks, dtype=torch.long, device=dev) if it.start > 0 else None for it in items]
         x = self._embed(ids_t, pos_t)
-        layer_index = {id(blk.attn): i for i, blk in enumerate(self.model.blocks)}
         runs = []                                  # (first item, count, length) of >= 2 fresh prompts of equal length
         i = 0
         while i < len(items):
@@ -226,25 +215,31 @@ class ModelRunner:
                 runs.append((i, j - i + 1, len(items[i].tokens)))
             i = j + 1
 
-        def attend(attn, h, residual):
-            li = layer_index[id(attn)]
-            qkv = self._qkv(attn, h)
-            qkv2 = qkv.view(-1, qkv.shape[-1])
-            self._rotate_and_cache(attn, qkv2, pos_t, slots_t, li)
+        def attention(attn, qkv2, li):
+            """Attention of every item over its own keys: ``[T, H D]`` from the packed projection."""
             q = qkv2[:, : H * D].unflatten(-1, (H, D))
             k = qkv2[:, H * D: (H + Hkv) * D].unflatten(-1, (Hkv, D))
             v = qkv2[:, (H + Hkv) * D:].unflatten(-1, (Hkv, D))
             window = s.sliding_window if s.is_windowed(attn.layer) else None
             fast = window is None and s.attention_softcap is None
-            out = torch.empty(qkv2.shape[0], H * D, dtype=qkv.dtype, device=dev)
+            out = None
             done = set()
+
+            def put(a, b, o):
+                nonlocal out
+                if (a, b) == (0, qkv2.shape[0]):
+                    out = o.reshape(b - a, H * D)
+                    return
+                if out is None:
+                    out = torch.empty(qkv2.shape[0], H * D, dtype=qkv2.dtype, device=dev)
+                out[a:b] = o.reshape(b - a, H * D)
+
             if fast:
                 # runs of fresh prompts of one length are contiguous in the pack: one batched attention launch
                 for first, count, length in runs:
                     a, b = bounds[first], bounds[first + count]
-                    o = ops.attention(q[a:b].unflatten(0, (count, length)), k[a:b].unflatten(0, (count, length)),
-                                      v[a:b].unflatten(0, (count, length)), True, attn.scale)
-                    out[a:b] = o.reshape(b - a, H * D)
+                    put(a, b, self._flash(q[a:b].unflatten(0, (count, length)), k[a:b].unflatten(0, (count, length)),
+                                          v[a:b].unflatten(0, (count, length)), attn.scale))
                     done.update(range(first, first + count))
             for i, it in enumerate(items):
                 if i in done:
@@ -252,24 +247,61 @@ class ModelRunner:
                 a, b = bounds[i], bounds[i + 1]
                 qi = q[a:b][None]
                 if it.start > 0:     # queries see the shared prefix too: read keys / values back from the cache
-                    total = it.start + (b - a)
-                    ki, vi = self._cached_kv(li, tables[i], total, qkv.dtype)
+                    ki, vi = self._cached_kv(li, tables[i], it.start + (b - a), qkv2.dtype)
                 else:
                     ki, vi = k[a:b][None], v[a:b][None]
-                if fast:
-                    o = ops.attention(qi, ki, vi, True, attn.scale)
-                else:
-                    o = masked_attention(qi, ki, vi, attn.scale, window, s.attention_softcap)
-                out[a:b] = o.reshape(b - a, H * D)
-            return self._out(attn, out[None], residual)
+                put(a, b, self._flash(qi, ki, vi, attn.scale) if fast
+                    else masked_attention(qi, ki, vi, attn.scale, window, s.attention_softcap))
+            return out if out is not None else qkv2.new_empty(qkv2.shape[0], H * D)
+
+        if self.direct_prefill and self._few_row_path():
+            # the kernels of the modules' forwards, in their order, without the modules: a short prompt is bound by the host
+            x = self._row_blocks(x.view(ids_t.shape[0], -1), pos_t, slots_t, attention, self._dense)
+            return self._logits(self._norm(self.model.norm, x if all_logits else x[last]))
+
+        layer_index = {id(blk.attn): i for i, blk in enumerate(self.model.blocks)}
+
+        def attend(attn, h, residual):
+            li = layer_index[id(attn)]
+            qkv = self._qkv(attn, h)
+            qkv2 = qkv.view(-1, qkv.shape[-1])
+            self._rotate_and_cache(attn, qkv2, pos_t, slots_t, li)
+            return self._out(attn, attention(attn, qkv2, li)[None], residual)
 
         for blk in self.model.blocks:
             x = self._block(blk, x, attend)
         if all_logits:
             return self._logits(self.model.norm(x))
-        last = torch.tensor([b - 1 for b in bounds[1:]], dtype=torch.long, device=dev)
-        h = self.model.norm(x[0, last].contiguous()[None])
+        h = self.model.norm(x[0, last][None])
         return self._logits(h)
+
+    @staticmethod
+    def _flash(q, k, v, scale):
+        """Causal attention of a prefill: the kernel without an autograd node where it takes the call."""
+        if q.is_cuda and q.dtype == torch.bfloat16 and q.shape[-1] in (64, 128):
+            return ops.flash_forward(q, k, v, True, scale)[0]
+        return ops.attention(q, k, v, True, scale)
+
+    def _pack(self, items: Sequence[PrefillItem]):
+        """Token ids, positions and cache slots of the packed items (int32, on the device), the index of every item's last
+        token, and the items' bounds in the pack. One copy from pinned memory that the host does not wait for: a copy per
+        list from pageable memory made the GPU wait for the host before every prefill."""
+        bs = self.block_size
+        counts = [len(it.tokens) for it in items]
+        bounds = [0]
+        for n in counts:
+            bounds.append(bounds[-1] + n)
+        T = bounds[-1]
+        meta = torch.empty(3 * T + len(items), dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        m = meta.numpy()
+        for it, a, n in zip(items, bounds, counts):
+            p = np.arange(it.start, it.start + n)
+            m[a: a + n] = it.tokens
+            m[T + a: T + a + n] = p
+            m[2 * T + a: 2 * T + a + n] = np.asarray(it.blocks, dtype=np.int64)[p // bs] * bs + p % bs
+        m[3 * T:] = np.asarray(bounds[1:]) - 1
+        dev = meta.to(self.device, non_blocking=True)
+        return dev[:T], dev[T: 2 * T], dev[2 * T: 3 * T], dev[3 * T:], bounds
 
     # ------------------------------------------------------------------ decode
     @torch.no_grad()
@@ -350,33 +382,57 @@ class ModelRunner:
             return packed_linear(x, owner.packed[name], bias, residual, gate)
         return skinny_linear(x, w, bias, residual, gate, norm_eps)
 
-    def _decode_few_rows(self, x, positions, slots, block_table, lens, max_len_hint):
-        """Six to eight launches per layer: (norm |) qkv | norms of q, k + RoPE + cache write | paged attention (+ its
-        merge) | out + residual | (norm |) gate/up + activation | down + residual."""
+    @staticmethod
+    def _dense(x, owner, name, residual=None, gate=None):
+        """The same projection of any number of rows on the dense (or unpacking) product, as the modules' forwards run it."""
+        from ..ops.rowops import GATE_KINDS, gated_forward
+        from ..quant.weights import qgemm
+        w, bias = getattr(owner, name + "_weight"), getattr(owner, name + "_bias")
+        if w is None:
+            y = qgemm(x, owner.packed[name], False, bias, residual)
+        else:
+            y = ops.gemm(x, w, bias=bias, residual=residual)
+        return y if gate is None else gated_forward(y, GATE_KINDS[gate])
+
+    direct_prefill = True          # prefill calls the kernels directly (not for a subclass with its own blocks)
+
+    @staticmethod
+    def _norm(layer, t):
+        """A norm layer's forward without an autograd node."""
         from ..ops.rowops import norm_forward
-        from ..ops.skinny import few_row_linear
-        s, m = self.spec, self.model
-        H, Hkv, D = s.heads, s.kv_heads, s.head_dim
-        folded = bool(getattr(m, "_norms_folded", False))
-        eps = s.norm_epsilon if folded else None
-        n = x.shape[0]
+        return norm_forward(t, layer.effective_weight(), layer.bias, layer.eps, layer.kind != "layer")[0]
 
-        def norm(layer, t):        # the layer's forward without an autograd node: a decode step is launch-bound on the host
-            return norm_forward(t, layer.effective_weight(), layer.bias, layer.eps, layer.kind != "layer")[0]
-
-        for li, blk in enumerate(m.blocks):
+    def _row_blocks(self, x, positions, slots, attention, project, norm_eps=None):
+        """The blocks over rows ``x [n, dim]``: (norm |) qkv | norms of q, k + RoPE + cache write | attention | out + residual
+        | (norm |) gate/up, activation | down + residual. ``attention(attn, qkv, layer)`` gives ``[n, H D]`` from the packed
+        projection; ``project`` is ``_few`` (at most 64 rows) or ``_dense``. With ``norm_eps`` the norms run inside the
+        projections (folded weights, ``_few`` only)."""
+        fold = {"norm_eps": norm_eps} if norm_eps is not None else {}
+        for li, blk in enumerate(self.model.blocks):
             attn, mlp = blk.attn, blk.mlp
-            qkv = self._few(x if folded else norm(blk.attn_norm, x), attn, "qkv", norm_eps=eps)
+            qkv = project(x if fold else self._norm(blk.attn_norm, x), attn, "qkv", **fold)
             self._rotate_and_cache(attn, qkv, positions, slots, li)
-            q = qkv[:, : H * D].unflatten(-1, (H, D))
+            x = project(attention(attn, qkv, li), attn, "o", residual=x)
+            g = project(x if fold else self._norm(blk.mlp_norm, x), mlp, "up", gate=self.spec.activation, **fold)
+            x = project(g, mlp, "down", residual=x)
+        return x
+
+    def _decode_few_rows(self, x, positions, slots, block_table, lens, max_len_hint):
+        s = self.spec
+        H, D = s.heads, s.head_dim
+
+        def attention(attn, qkv, li):
             window = s.sliding_window if s.is_windowed(attn.layer) else 0
-            o = dops.paged_decode(q, self.k_cache[li], self.v_cache[li], block_table, lens, attn.scale, window or 0,
-                                  max_len_hint=max_len_hint, k_scale=self.k_scale[li], v_scale=self.v_scale[li])
-            x = self._few(o.reshape(n, H * D), attn, "o", residual=x)
-            g = self._few(x if folded else norm(blk.mlp_norm, x), mlp, "up", gate=s.activation, norm_eps=eps)
-            x = self._few(g, mlp, "down", residual=x)
-        h = x if folded else norm(m.norm, x)
-        logits = few_row_linear(h, m.head_weight(), m.head_bias, norm_eps=eps)
+            o = dops.paged_decode(qkv[:, : H * D].unflatten(-1, (H, D)), self.k_cache[li], self.v_cache[li], block_table, lens,
+                                  attn.scale, window or 0, max_len_hint=max_len_hint, k_scale=self.k_scale[li],
+                                  v_scale=self.v_scale[li])
+            return o.reshape(-1, H * D)
+
+        from ..ops.skinny import few_row_linear
+        m = self.model
+        eps = s.norm_epsilon if getattr(m, "_norms_folded", False) else None
+        x = self._row_blocks(x, positions, slots, attention, self._few, eps)
+        logits = few_row_linear(x if eps is not None else self._norm(m.norm, x), m.head_weight(), m.head_bias, norm_eps=eps)
         return logits.reshape(-1, logits.shape[-1])
 
     # ------------------------------------------------------------------ decode as a replayed CUDA graph

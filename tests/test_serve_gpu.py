@@ -118,3 +118,35 @@ def test_few_row_decode_agrees_with_the_layer_by_layer_path(quant, rows):
     plain = runner.decode(tokens, positions, table).float()
     rms = plain.pow(2).mean().sqrt()
     assert ((fused - plain).pow(2).mean().sqrt() <= 10 * 2.0 ** -9 * rms) and fused.isfinite().all()
+
+
+@pytest.mark.parametrize("quant", ["", "int8", "int4"])
+@pytest.mark.parametrize("lengths,shared", [((5,), 0), ((64,), 0), ((9, 300, 9), 0), ((16, 16), 0), ((20, 11), 16)])
+def test_prefill_calls_the_same_kernels_as_the_modules(quant, lengths, shared):
+    """Prefill through the kernels directly (fresh prompts, of equal length, behind a shared prefix) against the modules' own
+    forwards: the same kernels in the same order, so logits and caches agree bit for bit."""
+    from idrak_b200.models import DecoderSpec, build_decoder
+    from idrak_b200.quant import quantize_model
+    from idrak_b200.serve import ModelRunner, PrefillItem
+    spec = DecoderSpec.llama(layers=2, dim=256, heads=4, kv_heads=2, ff_dim=512, vocab=500, max_positions=512, head_dim=64)
+    model = build_decoder(spec, seed=1).to("cuda", torch.bfloat16)
+    if quant:
+        quantize_model(model, quant)
+    runner = ModelRunner(model, 40, 16)
+    g = torch.Generator().manual_seed(0)
+    items, block = [], 0
+    for n in lengths:
+        need = (shared + n + 15) // 16
+        items.append(PrefillItem(torch.randint(0, 500, (n,), generator=g).tolist(), shared, list(range(block, block + need))))
+        block += need
+    if shared:
+        for c in runner.k_cache + runner.v_cache:
+            c.copy_(torch.randn(c.shape, device="cuda"))
+    results = []
+    for few in (True, False):
+        runner._few_rows_ok = few
+        logits = runner.prefill(items).float()
+        results.append((logits, runner.prefill(items, all_logits=True).float(), [c.float().clone() for c in runner.k_cache + runner.v_cache]))
+    (a, a_all, a_cache), (b, b_all, b_cache) = results
+    for x, y in [(a, b), (a_all, b_all)] + list(zip(a_cache, b_cache)):
+        assert torch.equal(x, y) and x.isfinite().all()
