@@ -11,10 +11,14 @@
 //
 // Warp roles match the forward kernel: warp 0 feeds shared memory with TMA, warp 1 issues tcgen05.mma,
 // warps 2..9 do the element-wise work, two threads per tile row with 64 of the block's 128 columns each (the row
-// statistics come from the forward pass, so the halves are independent). The operand tiles the element-wise warps
-// produce (dS; P^T and dS^T) are double-buffered, each buffer with its own "product done" barrier, so the next block is
-// filled while the tensor cores still accumulate from the previous one. The same 128B-swizzled tile serves as a
-// K-major operand for one product and as an MN-major operand for the other, so nothing is transposed.
+// statistics come from the forward pass, so the halves are independent). dS (dQ) and P^T (dV) go back to tensor memory as
+// bf16 and are read there as the A operand of the product they enter; only dS^T is staged in shared memory. That leaves
+// room for two or three stages of every streamed tile at head size 128 too, so loads, products and element-wise steps of
+// neighbouring blocks overlap. With everything staged in shared memory there was one stage of each, and a block's load,
+// scores, element-wise step and accumulation ran one after the other. Measured, 8192 positions, 32 heads on 8, size 128,
+// causal: dQ 1330 -> 747 us, dK / dV 1884 -> 1299 us; 8 x 1024, 12 heads, size 64: 49 -> 47 and 84 -> 77 us.
+// A tile in shared memory serves as a K-major operand for one product and as an MN-major operand for the other, so nothing
+// is transposed.
 //
 // Reference counterparts: flash_tc_bwd_q_d{64,128}, flash_tc_bwd_kv_d{64,128}, flash_tc_delta
 // (src/Idrak.Gpu/Cuda/PtxKernels.FlashTensorCore.cs) and attn_bwd_{d,kv,q}_f32 (PtxKernels.Rows.cs:1222-1750).
@@ -88,15 +92,16 @@ __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ o, const __
 template <int D>
 struct BwdQSmem {
   static constexpr int kTile = 128 * D * 2;
-  // three K / V stages at head size 64: a stage is freed only by the dQ product of its block, and with two the load of
-  // block j + 2 (about 1500 cycles from L2) sat on the critical path of every block
-  static constexpr int kStages = (D == 64) ? 3 : 1;
+  // A key tile is freed only by the dQ product of its block, a value tile already by the dP product: with three and two
+  // stages neither load (about 1500 cycles from L2) sits on the path from one block to the next. dS stays in tensor memory,
+  // which is what makes the room for them at head size 128 (one stage of each before: every load, product and element-wise
+  // step of a block waited for the one before).
+  static constexpr int kKStages = 3, kVStages = 2;
   static constexpr int kQ = 0;
   static constexpr int kDO = kQ + kTile;
   static constexpr int kK = kDO + kTile;
-  static constexpr int kV = kK + kStages * kTile;
-  static constexpr int kDS = kV + kStages * kTile;          // two dS tiles: the next one is filled while the tensor
-  static constexpr int kBar = kDS + 2 * 32768;              // cores still read the previous one for dQ
+  static constexpr int kV = kK + kKStages * kTile;
+  static constexpr int kBar = kV + kVStages * kTile;
   static constexpr int kTotal = kBar + 256 + 1024;
 };
 
@@ -144,20 +149,22 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                    const FlashParams p) {
   using L = BwdQSmem<D>;
-  constexpr int NS = L::kStages;
+  constexpr int KS = L::kKStages, VS = L::kVStages;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* qdo_full = bars + 0;
-  uint64_t* kv_full = bars + 1;     // [3]
-  uint64_t* kv_empty = bars + 4;    // [3]
-  uint64_t* sdp_full = bars + 7;
-  uint64_t* ds_ready = bars + 8;
-  uint64_t* dq_done = bars + 9;     // [2]: one per dS tile
-  uint64_t* sdp_taken = bars + 11;  // the element-wise warps hold S and dP of the block in registers: TMEM may be rewritten
-  uint64_t* qdo_free = bars + 12;   // the unit's last score products have read Q and dO: the next unit's may land
-  uint64_t* dq_free = bars + 13;    // dQ of the unit sits in registers: the next unit may accumulate
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* k_full = bars + 1;      // [3]
+  uint64_t* k_empty = bars + 4;     // [3]
+  uint64_t* v_full = bars + 7;      // [2]
+  uint64_t* v_empty = bars + 9;     // [2]
+  uint64_t* sdp_full = bars + 11;
+  uint64_t* ds_ready = bars + 12;
+  uint64_t* dq_done = bars + 13;    // [2]: one per dS buffer
+  uint64_t* sdp_taken = bars + 15;  // the element-wise warps hold S and dP of the block in registers: TMEM may be rewritten
+  uint64_t* qdo_free = bars + 16;   // the unit's last score products have read Q and dO: the next unit's may land
+  uint64_t* dq_free = bars + 17;    // dQ of the unit sits in registers: the next unit may accumulate
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -168,9 +175,13 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (threadIdx.x == 0) {
     mbar_init(qdo_full, 1);
-    for (int s = 0; s < 3; ++s) {
-      mbar_init(&kv_full[s], 1);
-      mbar_init(&kv_empty[s], 1);
+    for (int s = 0; s < KS; ++s) {
+      mbar_init(&k_full[s], 1);
+      mbar_init(&k_empty[s], 1);
+    }
+    for (int s = 0; s < VS; ++s) {
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
     }
     mbar_init(sdp_full, 1);
     mbar_init(ds_ready, 256);
@@ -186,7 +197,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
   }
-  constexpr uint32_t kTmemCols = 512;   // S [0,128) | dP [128,256) | dQ [256, 256+D)
+  constexpr uint32_t kTmemCols = 512;   // S [0,128) | dP [128,256) | dS 2 x 64 [256,384) | dQ [384, 384+D)
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -195,7 +206,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dQ = tmem_base + 256;
+  const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dS = tmem_base + 256, tmem_dQ = tmem_base + 384;
 
   // Every role walks the same units and counts alike: n = units with work so far, g = key blocks so far over all units.
   if (warp == 0) {
@@ -215,15 +226,18 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           tma_load_4d(smem + L::kDO + c * 16384, &tmDO, qdo_full, c * 64, t.q0, t.head, t.batch);
         }
         for (int j = 0; j < t.nkv; ++j, ++g) {
-          const int st = g % NS;
-          const uint32_t ph = (g / NS) & 1;
-          if (!mbar_wait(&kv_empty[st], ph ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (3u << 16) | st)) { ok = false; break; }
-          mbar_expect_tx(&kv_full[st], 2 * L::kTile);
+          const int ks = g % KS, vs = g % VS;
+          const int key0 = (t.jlo + j) * 128;
+          if (!mbar_wait(&k_empty[ks], ((g / KS) & 1) ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (3u << 16) | ks)) { ok = false; break; }
+          mbar_expect_tx(&k_full[ks], L::kTile);
 #pragma unroll
-          for (int c = 0; c < D / 64; ++c) {
-            tma_load_4d(smem + L::kK + st * L::kTile + c * 16384, &tmK, &kv_full[st], c * 64, (t.jlo + j) * 128, t.kv_head, t.batch);
-            tma_load_4d(smem + L::kV + st * L::kTile + c * 16384, &tmV, &kv_full[st], c * 64, (t.jlo + j) * 128, t.kv_head, t.batch);
-          }
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_4d(smem + L::kK + ks * L::kTile + c * 16384, &tmK, &k_full[ks], c * 64, key0, t.kv_head, t.batch);
+          if (!mbar_wait(&v_empty[vs], ((g / VS) & 1) ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (3u << 16) | (4 + vs))) { ok = false; break; }
+          mbar_expect_tx(&v_full[vs], L::kTile);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c)
+            tma_load_4d(smem + L::kV + vs * L::kTile + c * 16384, &tmV, &v_full[vs], c * 64, key0, t.kv_head, t.batch);
         }
         ++n;
       }
@@ -233,18 +247,18 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_f16(128, 128, 0, 0, 1);
       constexpr uint32_t idesc_dq = make_idesc_f16(128, D, 0, 1, 1);
-      const uint32_t sq = smem_u32(smem + L::kQ), sdo = smem_u32(smem + L::kDO), sds = smem_u32(smem + L::kDS);
+      const uint32_t sq = smem_u32(smem + L::kQ), sdo = smem_u32(smem + L::kDO);
       int n = 0, g0 = 0;
       bool ok = true;
       // S and dP of global block g; within a unit they are issued one block ahead, as soon as the element-wise warps
       // have taken the previous block's S and dP into registers
       auto issue_scores = [&](int g) -> bool {
-        const int st = g % NS;
-        const uint32_t ph = (g / NS) & 1;
-        if (!mbar_wait(&kv_full[st], ph, abort_flag, p.st, kTimeoutSmemFull, (3u << 16) | st)) return false;
+        const int ks = g % KS, vs = g % VS;
+        if (!mbar_wait(&k_full[ks], (g / KS) & 1, abort_flag, p.st, kTimeoutSmemFull, (3u << 16) | ks)) return false;
+        if (!mbar_wait(&v_full[vs], (g / VS) & 1, abort_flag, p.st, kTimeoutSmemFull, (3u << 16) | (4 + vs))) return false;
         if (g > 0 && !mbar_wait(sdp_taken, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (3u << 16) | 13)) return false;
         tc_fence_after();
-        const uint32_t sk = smem_u32(smem + L::kK + st * L::kTile), sv = smem_u32(smem + L::kV + st * L::kTile);
+        const uint32_t sk = smem_u32(smem + L::kK + ks * L::kTile), sv = smem_u32(smem + L::kV + vs * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           tc_mma_f16_ss(tmem_S, kmajor_desc(sq, kk), kmajor_desc(sk, kk), idesc_s, kk > 0 ? 1u : 0u);
@@ -252,30 +266,23 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int kk = 0; kk < D / 16; ++kk)
           tc_mma_f16_ss(tmem_dP, kmajor_desc(sdo, kk), kmajor_desc(sv, kk), idesc_s, kk > 0 ? 1u : 0u);
         tc_commit(sdp_full);
+        tc_commit(&v_empty[vs]);
         return true;
       };
-      constexpr bool kAhead = NS >= 2;      // one stage: the next K / V cannot land before this block's dQ product is done
       for (int round = 0; round < snake_rounds(units) && ok; ++round) {
         const int u = snake_unit(round, units);
         if (u < 0) continue;
         const QUnit t = q_unit<MODES>(p, u, off, nqt);
         if (t.nkv <= 0) continue;
         if (!mbar_wait(qdo_full, n & 1, abort_flag, p.st, kTimeoutSmemFull, (3u << 16) | 8)) break;
-        if (kAhead) {
-          ok = issue_scores(g0);
-          if (ok && t.nkv == 1) tc_commit(qdo_free);
-        }
+        ok = issue_scores(g0);
+        if (ok && t.nkv == 1) tc_commit(qdo_free);
         for (int j = 0; j < t.nkv && ok; ++j) {
           const int g = g0 + j;
-          const int st = g % NS;
-          if (kAhead) {
-            if (j + 1 < t.nkv) {
-              if (!issue_scores(g + 1)) { ok = false; break; }
-              if (j + 2 == t.nkv) tc_commit(qdo_free);        // the unit's last score products are on their way
-            }
-          } else {
-            if (!issue_scores(g)) { ok = false; break; }
-            if (j + 1 == t.nkv) tc_commit(qdo_free);
+          const int ks = g % KS;
+          if (j + 1 < t.nkv) {
+            if (!issue_scores(g + 1)) { ok = false; break; }
+            if (j + 2 == t.nkv) tc_commit(qdo_free);        // the unit's last score products are on their way
           }
           if (!mbar_wait(ds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (3u << 16) | 9)) { ok = false; break; }
           if (j == 0 && n > 0) {
@@ -283,12 +290,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (!mbar_wait(dq_free, (n - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (3u << 16) | 15)) { ok = false; break; }
           }
           tc_fence_after();
-          const uint32_t sk = smem_u32(smem + L::kK + st * L::kTile);
-          const uint32_t sds_b = sds + (g & 1) * 32768;
+          const uint32_t sk = smem_u32(smem + L::kK + ks * L::kTile);
+          const uint32_t ds_b = tmem_dS + (g & 1) * 64;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            tc_mma_f16_ss(tmem_dQ, kmajor_desc(sds_b, kk), mnmajor_desc(sk, kk), idesc_dq, (j > 0 || kk > 0) ? 1u : 0u);
-          tc_commit(&kv_empty[st]);
+            tc_mma_f16_ts(tmem_dQ, ds_b + kk * 8, mnmajor_desc(sk, kk), idesc_dq, (j > 0 || kk > 0) ? 1u : 0u);
+          tc_commit(&k_empty[ks]);
           tc_commit(&dq_done[g & 1]);
         }
         g0 += t.nkv;
@@ -327,12 +334,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         lse2 = (l == -INFINITY) ? INFINITY : l * kLog2e;
         dlt = p.delta[idx];
       }
+      const float dlt_s = dlt * p.scale;       // dS = P * (dP * scale - delta * scale)
       const int row_lo = bounded ? flash_row_lo(p, t.batch, row, off) : 0;
       for (int j = 0; j < t.nkv && ok; ++j) {
         const int g = g0 + j;
         if (!mbar_wait(sdp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 10)) { ok = false; break; }
         tc_fence_after();
-        uint8_t* sDS = smem + L::kDS + (g & 1) * 32768;
         const int k0 = (t.jlo + j) * 128 + half * 64;          // first key of this thread's 64 columns
         int lim = p.Skv - k0;
         if (p.causal) lim = min(lim, row + off - k0 + 1);
@@ -348,43 +355,50 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_ld_wait();
         tc_fence_before();
         mbar_arrive(sdp_taken);
-        if (g >= 2) {
-          // the dQ product that last read this dS tile (block g - 2) must be complete
-          if (!mbar_wait(&dq_done[g & 1], uint32_t((g >> 1) - 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 11)) {
-            ok = false;
-            break;
-          }
-        }
+        uint32_t packed[32];
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           float ds[32];
           if (!special) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              float pr = fast_exp2(__uint_as_float(s[cc][i]) * p.scale_log2 - lse2);
-              float v = pr * (__uint_as_float(dp[cc][i]) - dlt) * p.scale;
-              ds[i] = (cc * 32 + i < lim) ? v : 0.f;
+              const float pr = fast_exp2(__uint_as_float(s[cc][i]) * p.scale_log2 - lse2);
+              ds[i] = pr * (__uint_as_float(dp[cc][i]) * p.scale - dlt_s);
             }
           } else {
             // lower key bound and / or soft-capped scores: u = cap * tanh(s * scale / cap), du/ds = scale * (1 - tanh^2)
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              float sc = __uint_as_float(s[cc][i]), gr = p.scale;
+              float sc = __uint_as_float(s[cc][i]), gr = 1.f;
               if (capped) {
                 const float th = tanh_fast(sc * cap_in);
                 sc = th * cap_l2;
-                gr *= 1.f - th * th;
+                gr -= th * th;
               } else {
                 sc *= p.scale_log2;
               }
-              float pr = fast_exp2(sc - lse2);
-              float v = pr * (__uint_as_float(dp[cc][i]) - dlt) * gr;
-              ds[i] = (cc * 32 + i < lim && cc * 32 + i >= lo) ? v : 0.f;
+              const float pr = fast_exp2(sc - lse2);
+              ds[i] = pr * (__uint_as_float(dp[cc][i]) * p.scale - dlt_s) * gr;
             }
           }
-          store_operand_chunk(sDS, r, half * 2 + cc, ds);
+          if (lim < 64 || lo > 0) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (cc * 32 + i >= lim || cc * 32 + i < lo) ds[i] = 0.f;
+          }
+#pragma unroll
+          for (int i = 0; i < 16; ++i) packed[cc * 16 + i] = pack_bf16x2(ds[2 * i], ds[2 * i + 1]);
         }
-        fence_proxy_async_smem();
+        if (g >= 2) {
+          // the dQ product that last read this dS buffer (block g - 2) must be complete
+          if (!mbar_wait(&dq_done[g & 1], uint32_t((g >> 1) - 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 11)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+        }
+        tmem_st_32x32b_x32(tmem_dS + (g & 1) * 64 + lane_addr + half * 32, packed);
+        tmem_st_wait();
         tc_fence_before();
         mbar_arrive(ds_ready);
       }
@@ -432,17 +446,16 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 template <int D>
 struct BwdKVSmem {
   static constexpr int kTile = 128 * D * 2;
-  static constexpr int kStages = (D == 64) ? 2 : 1;
+  static constexpr int kStages = 2;                         // Q and dO: the next block's load during this one's products
   static constexpr int kK = 0;
   static constexpr int kV = kK + kTile;
   static constexpr int kQ = kV + kTile;
   static constexpr int kDO = kQ + kStages * kTile;
-  // head size 64: two P^T / dS^T buffers, so the element-wise warps fill the next pair while the tensor cores still
-  // accumulate dV / dK from the previous one (224 KB in all; at head size 128 there is room for one pair only)
-  static constexpr int kPBufs = (D == 64) ? 2 : 1;
-  static constexpr int kPT = kDO + kStages * kTile;
-  static constexpr int kDST = kPT + kPBufs * 32768;
-  static constexpr int kStat = kDST + kPBufs * 32768;       // lse2[128], delta[128], lo[128]
+  // P^T is an operand in tensor memory; only dS^T is staged here, in two buffers at head size 64 and in the one that fits
+  // beside two Q / dO stages at head size 128 (227 KB in all)
+  static constexpr int kDSBufs = (D == 64) ? 2 : 1;
+  static constexpr int kDST = kDO + kStages * kTile;
+  static constexpr int kStat = kDST + kDSBufs * 32768;      // lse2[128], delta * scale [128], lo[128]
   static constexpr int kBar = kStat + 1536;
   static constexpr int kTotal = kBar + 256 + 1024;
 };
@@ -490,20 +503,25 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const FlashParams p) {
   using L = BwdKVSmem<D>;
   constexpr int NS = L::kStages;
-  constexpr int PB = L::kPBufs;
+  constexpr int DB = L::kDSBufs;
+  constexpr bool kAlias = D == 128;    // P^T lies over the scores it was made from (tensor memory is full)
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBar);
   uint64_t* kv_full = bars + 0;
   uint64_t* qdo_full = bars + 1;    // [2]
   uint64_t* qdo_empty = bars + 3;   // [2]
-  uint64_t* sdp_full = bars + 5;
-  uint64_t* pds_ready = bars + 6;
-  uint64_t* acc_done = bars + 7;    // [2]: one per P^T / dS^T buffer
-  uint64_t* sdp_taken = bars + 9;   // S^T and dP^T of the block are in registers: TMEM may be rewritten
-  uint64_t* kv_free = bars + 10;    // the unit's last score products have read K and V: the next unit's may land
-  uint64_t* acc_free = bars + 11;   // dV and dK of the unit sit in registers: the next unit may accumulate
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  uint64_t* s_full = bars + 5;
+  uint64_t* dp_full = bars + 6;
+  uint64_t* s_taken = bars + 7;     // S^T / dP^T of the block are in registers: TMEM may be rewritten
+  uint64_t* dp_taken = bars + 8;
+  uint64_t* p_ready = bars + 9;     // P^T is in tensor memory
+  uint64_t* ds_ready = bars + 10;   // dS^T is in shared memory
+  uint64_t* dv_done = bars + 11;    // the dV product has read P^T
+  uint64_t* dk_done = bars + 12;    // [2]: one per dS^T buffer
+  uint64_t* kv_free = bars + 14;    // the unit's last score products have read K and V: the next unit's may land
+  uint64_t* acc_free = bars + 15;   // dV and dK of the unit sit in registers: the next unit may accumulate
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* s_lse2 = reinterpret_cast<float*>(smem + L::kStat);
   float* s_delta = s_lse2 + 128;
@@ -522,11 +540,15 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(&qdo_full[s], 1);
       mbar_init(&qdo_empty[s], 1);
     }
-    mbar_init(sdp_full, 1);
-    mbar_init(pds_ready, 256);
-    mbar_init(&acc_done[0], 1);
-    mbar_init(&acc_done[1], 1);
-    mbar_init(sdp_taken, 256);
+    mbar_init(s_full, 1);
+    mbar_init(dp_full, 1);
+    mbar_init(s_taken, 256);
+    mbar_init(dp_taken, 256);
+    mbar_init(p_ready, 256);
+    mbar_init(ds_ready, 256);
+    mbar_init(dv_done, 1);
+    mbar_init(&dk_done[0], 1);
+    mbar_init(&dk_done[1], 1);
     mbar_init(kv_free, 1);
     mbar_init(acc_free, 256);
     *abort_flag = 0;
@@ -536,7 +558,10 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
   }
-  constexpr uint32_t kTmemCols = 512;   // S^T [0,128) | dP^T [128,256) | dV [256,256+D) | dK [256+D, 256+2D)
+  // S^T [0,128) | dP^T [128,256) | dV [256,256+D) | dK [256+D, 256+2D) | P^T: 64 more columns at D = 64; at D = 128 over
+  // the scores, each half of the queries in the first 32 columns of its own half
+  constexpr uint32_t kTmemCols = 512;
+  constexpr uint32_t kPHalf = kAlias ? 64 : 32;      // columns from the first 64 queries' part of P^T to the second's
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
@@ -546,7 +571,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_ST = tmem_base, tmem_dPT = tmem_base + 128, tmem_dV = tmem_base + 256,
-                 tmem_dK = tmem_base + 256 + D;
+                 tmem_dK = tmem_base + 256 + D, tmem_PT = kAlias ? tmem_base : tmem_base + 256 + 2 * D;
 
   // Every role walks the same units and counts the same things: n = units with work so far (parity of the per-unit
   // barriers), g = query blocks so far over all units (stage and parity of the per-block barriers).
@@ -589,67 +614,77 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       constexpr uint32_t idesc_s = make_idesc_f16(128, 128, 0, 0, 1);
       constexpr uint32_t idesc_acc = make_idesc_f16(128, D, 0, 1, 1);
       const uint32_t sk = smem_u32(smem + L::kK), sv = smem_u32(smem + L::kV);
-      const uint32_t spt = smem_u32(smem + L::kPT), sdst = smem_u32(smem + L::kDST);
+      const uint32_t sdst = smem_u32(smem + L::kDST);
       int n = 0, g0 = 0;
       bool ok = true;
-      // S^T and dP^T of global block g; within a unit they are issued one block ahead (two Q / dO stages), as soon as
-      // the element-wise warps hold the previous block's scores in registers
-      auto issue_scores = [&](int g) -> bool {
+      auto load_wait = [&](int g) -> bool {
         const int st = g % NS;
-        const uint32_t ph = (g / NS) & 1;
-        if (!mbar_wait(&qdo_full[st], ph, abort_flag, p.st, kTimeoutSmemFull, (4u << 16) | st)) return false;
-        if (g > 0 && !mbar_wait(sdp_taken, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (4u << 16) | 13)) return false;
+        return mbar_wait(&qdo_full[st], (g / NS) & 1, abort_flag, p.st, kTimeoutSmemFull, (4u << 16) | st);
+      };
+      // Scores of global block g, once their place is free: S^T of the block before was taken into registers or, where P^T
+      // lies over it, the dV product that reads P^T is complete.
+      auto issue_s = [&](int g) -> bool {
+        if (!load_wait(g)) return false;
+        if (g > 0 && !mbar_wait(kAlias ? dv_done : s_taken, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (4u << 16) | 13))
+          return false;
         tc_fence_after();
-        const uint32_t sq = smem_u32(smem + L::kQ + st * L::kTile), sdo = smem_u32(smem + L::kDO + st * L::kTile);
+        const uint32_t sq = smem_u32(smem + L::kQ + (g % NS) * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           tc_mma_f16_ss(tmem_ST, kmajor_desc(sk, kk), kmajor_desc(sq, kk), idesc_s, kk > 0 ? 1u : 0u);
+        tc_commit(s_full);
+        return true;
+      };
+      auto issue_dp = [&](int g) -> bool {
+        if (!load_wait(g)) return false;
+        if (g > 0 && !mbar_wait(dp_taken, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (4u << 16) | 16)) return false;
+        tc_fence_after();
+        const uint32_t sdo = smem_u32(smem + L::kDO + (g % NS) * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
           tc_mma_f16_ss(tmem_dPT, kmajor_desc(sv, kk), kmajor_desc(sdo, kk), idesc_s, kk > 0 ? 1u : 0u);
-        tc_commit(sdp_full);
+        tc_commit(dp_full);
         return true;
       };
-      constexpr bool kAhead = NS >= 2;
       for (int round = 0; round < snake_rounds(units) && ok; ++round) {
         const int u = snake_unit(round, units);
         if (u < 0) continue;
         const KvUnit t = kv_unit<MODES>(p, u, off, nq);
         if (t.iters == 0) continue;
         if (!mbar_wait(kv_full, n & 1, abort_flag, p.st, kTimeoutSmemFull, (4u << 16) | 8)) break;
-        if (kAhead) {
-          ok = issue_scores(g0);
-          if (ok && t.iters == 1) tc_commit(kv_free);
-        }
+        ok = issue_s(g0) && issue_dp(g0);
+        if (ok && t.iters == 1) tc_commit(kv_free);
         for (int it = 0; it < t.iters && ok; ++it) {
           const int g = g0 + it;
           const int st = g % NS;
-          if (kAhead) {
-            if (it + 1 < t.iters) {
-              if (!issue_scores(g + 1)) { ok = false; break; }
-              if (it + 2 == t.iters) tc_commit(kv_free);       // the unit's last score products are on their way
-            }
-          } else {
-            if (!issue_scores(g)) { ok = false; break; }
-            if (it + 1 == t.iters) tc_commit(kv_free);
-          }
-          if (!mbar_wait(pds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 9)) { ok = false; break; }
+          const bool more = it + 1 < t.iters;
+          // The next block's scores and dP go out between this block's two accumulations, so the element-wise warps find
+          // them when they are done with this block. Scores with a place of their own go first; scores that share it with
+          // P^T follow dP, whose product covers the wait for dV.
+          if (more && !kAlias && !issue_s(g + 1)) { ok = false; break; }
+          if (!mbar_wait(p_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 9)) { ok = false; break; }
           if (it == 0 && n > 0) {
             // dV and dK of the previous unit must have been read out before this unit starts its own sums
             if (!mbar_wait(acc_free, (n - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (4u << 16) | 15)) { ok = false; break; }
           }
           tc_fence_after();
           const uint32_t sq = smem_u32(smem + L::kQ + st * L::kTile), sdo = smem_u32(smem + L::kDO + st * L::kTile);
-          const int pb = g % PB;
-          const uint32_t spt_b = spt + pb * 32768, sdst_b = sdst + pb * 32768;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
-            tc_mma_f16_ss(tmem_dV, kmajor_desc(spt_b, kk), mnmajor_desc(sdo, kk), idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+            tc_mma_f16_ts(tmem_dV, tmem_PT + (kk >> 2) * kPHalf + (kk & 3) * 8, mnmajor_desc(sdo, kk), idesc_acc,
+                          (it > 0 || kk > 0) ? 1u : 0u);
+          tc_commit(dv_done);
+          if (more && !issue_dp(g + 1)) { ok = false; break; }
+          if (more && kAlias && !issue_s(g + 1)) { ok = false; break; }
+          if (it + 2 == t.iters) tc_commit(kv_free);               // the unit's last score products are on their way
+          if (!mbar_wait(ds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 17)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sdst_b = sdst + (g % DB) * 32768;
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)
             tc_mma_f16_ss(tmem_dK, kmajor_desc(sdst_b, kk), mnmajor_desc(sq, kk), idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
           tc_commit(&qdo_empty[st]);
-          tc_commit(&acc_done[pb]);
+          tc_commit(&dk_done[g % DB]);
         }
         g0 += t.iters;
         ++n;
@@ -664,7 +699,6 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
     bool ok = true;
     const bool capped = MODES && p.softcap > 0.f;
-    const bool special = bounded || capped;
     const float cap_in = capped ? p.scale / p.softcap : 0.f;
     const float cap_l2 = p.softcap * kLog2e;
     int n = 0, g0 = 0;
@@ -685,106 +719,144 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const size_t idx = (size_t(t.batch) * p.H + head) * p.Sq + qr;
             const float l = p.lse[idx];
             l2 = (l == -INFINITY) ? INFINITY : l * kLog2e;
-            dl = p.delta[idx];
+            dl = p.delta[idx] * p.scale;
           }
           lo = bounded ? flash_row_lo(p, t.batch, qr, off) : 0;
-        };
-        auto store_stats = [&](float l2, float dl, int lo) {
-          s_lse2[r] = l2;
-          s_delta[r] = dl;
-          s_lo[r] = lo;
         };
         // the previous unit's last block ended with a barrier after its statistics were last read
         if (half == 0) {
           float l2, dl;
           int lo;
           load_stats(0, l2, dl, lo);
-          store_stats(l2, dl, lo);
+          s_lse2[r] = l2;
+          s_lo[r] = lo;
+          s_delta[r] = dl;
         }
         softmax_bar_sync();
         for (int it = 0; it < t.iters; ++it) {
           const int g = g0 + it;
           const int qrow0 = (t.i_min + it % t.per_head) * 128;
-          const int pb = g % PB;
-          uint8_t* sPT = smem + L::kPT + pb * 32768;
-          uint8_t* sDST = smem + L::kDST + pb * 32768;
-          // the statistics of this query block were staged at the end of the previous block; those of the next are
-          // fetched now and stored at the end of this one, so their latency hides behind this block's arithmetic
+          // The statistics of the next query block are fetched now. Its lse replaces this block's once the probabilities
+          // are formed, its delta once dS is: each is written after one of the block's two barriers and read after the
+          // other, so neither barrier stands alone in the chain.
           float n_l2 = INFINITY, n_dl = 0.f;
           int n_lo = 0;
-          if (half == 0 && it + 1 < t.iters) load_stats(it + 1, n_l2, n_dl, n_lo);
-          if (ok && !mbar_wait(sdp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 10)) ok = false;
+          const bool fetch = half == 0 && it + 1 < t.iters;
+          if (fetch) load_stats(it + 1, n_l2, n_dl, n_lo);
+          if (ok && !mbar_wait(s_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 10)) ok = false;
           tc_fence_after();
           // query q (column) sees this key iff key <= q + off  <=>  q >= key - off
           const int first_q = p.causal ? (key - off - qrow0) : 0;    // columns below this are masked
-          // this thread's 64 columns: four loads in flight and one wait; the MMA warp may rewrite S^T and dP^T once
-          // every thread holds its part in registers
-          uint32_t s[2][32], dp[2][32];
-          if (ok) {
-            tmem_ld_32x32b_x32(tmem_ST + lane_addr + half * 64, s[0]);
-            tmem_ld_32x32b_x32(tmem_ST + lane_addr + half * 64 + 32, s[1]);
-            tmem_ld_32x32b_x32(tmem_dPT + lane_addr + half * 64, dp[0]);
-            tmem_ld_32x32b_x32(tmem_dPT + lane_addr + half * 64 + 32, dp[1]);
-            tmem_ld_wait();
-            tc_fence_before();
-            mbar_arrive(sdp_taken);
-          } else {
+          const bool diagonal = p.causal && t.k0 + 127 - off > qrow0;
+          float pr[2][32], gr[MODES ? 2 : 1][MODES ? 32 : 1];
+          {
+            uint32_t s[2][32], packed[32];
+            if (ok) {
+              tmem_ld_32x32b_x32(tmem_ST + lane_addr + half * 64, s[0]);
+              tmem_ld_32x32b_x32(tmem_ST + lane_addr + half * 64 + 32, s[1]);
+              tmem_ld_wait();
+              tc_fence_before();
+              if (!kAlias) mbar_arrive(s_taken);
+            } else {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) s[0][i] = s[1][i] = dp[0][i] = dp[1][i] = 0u;
+              for (int i = 0; i < 32; ++i) s[0][i] = s[1][i] = 0u;
+            }
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+              const int c0 = half * 64 + cc * 32;
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                const float4 l4 = *reinterpret_cast<const float4*>(&s_lse2[c0 + i]);
+                const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  float sc = __uint_as_float(s[cc][i + e]);
+                  if (MODES && capped) {
+                    // u = cap * tanh(s * scale / cap), du/ds = scale * (1 - tanh^2)
+                    const float th = tanh_fast(sc * cap_in);
+                    pr[cc][i + e] = fast_exp2(th * cap_l2 - l[e]);
+                    gr[MODES ? cc : 0][MODES ? i + e : 0] = 1.f - th * th;
+                  } else {
+                    pr[cc][i + e] = fast_exp2(sc * p.scale_log2 - l[e]);
+                  }
+                }
+              }
+              if (diagonal) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (c0 + i < first_q) pr[cc][i] = 0.f;
+              }
+              if (bounded) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                  if (key < s_lo[c0 + i]) pr[cc][i] = 0.f;
+              }
+#pragma unroll
+              for (int i = 0; i < 16; ++i) packed[cc * 16 + i] = pack_bf16x2(pr[cc][2 * i], pr[cc][2 * i + 1]);
+            }
+            if (!kAlias && ok && g > 0) {
+              // the dV product of the block before has read P^T (over the scores: they came after it)
+              if (!mbar_wait(dv_done, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 18)) ok = false;
+              tc_fence_after();
+            }
+            if (ok) {
+              tmem_st_32x32b_x32(tmem_PT + lane_addr + half * kPHalf, packed);
+              tmem_st_wait();
+              tc_fence_before();
+              mbar_arrive(p_ready);
+            }
           }
-          if (ok && g >= PB) {
-            // the accumulation that last read this P^T / dS^T buffer (block g - PB) must be complete
-            const uint32_t use = uint32_t(g / PB) - 1u;
-            if (!mbar_wait(&acc_done[pb], use & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 11)) ok = false;
+          softmax_bar_sync();    // this block's lse is no longer read; its delta is visible
+          if (fetch) {
+            s_lse2[r] = n_l2;
+            s_lo[r] = n_lo;
+          }
+          if (ok && !mbar_wait(dp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 19)) ok = false;
+          tc_fence_after();
+          uint8_t* sDST = smem + L::kDST + (g % DB) * 32768;
+          if (ok && g >= DB) {
+            // the dK product that last read this dS^T buffer (block g - DB) must be complete
+            if (!mbar_wait(&dk_done[g % DB], (uint32_t(g / DB) - 1u) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 11)) ok = false;
           }
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
-            const int c = half * 2 + cc;
-            float pt[32], dst[32];
-            if (!special) {
-#pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int col = c * 32 + i;
-                float pr = fast_exp2(__uint_as_float(s[cc][i]) * p.scale_log2 - s_lse2[col]);
-                if (col < first_q) pr = 0.f;
-                pt[i] = pr;
-                dst[i] = pr * (__uint_as_float(dp[cc][i]) - s_delta[col]) * p.scale;
+            const int c0 = half * 64 + cc * 32;
+            uint32_t dp[32];                       // 32 at a time: beside the 64 probabilities they stay in registers
+            if (ok) {
+              tmem_ld_32x32b_x32(tmem_dPT + lane_addr + c0, dp);
+              tmem_ld_wait();
+              if (cc == 1) {
+                tc_fence_before();
+                mbar_arrive(dp_taken);
               }
             } else {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int col = c * 32 + i;
-                float sc = __uint_as_float(s[cc][i]), gr = p.scale;
-                if (capped) {
-                  const float th = tanh_fast(sc * cap_in);
-                  sc = th * cap_l2;
-                  gr *= 1.f - th * th;
-                } else {
-                  sc *= p.scale_log2;
-                }
-                float pr = fast_exp2(sc - s_lse2[col]);
-                if (col < first_q || key < s_lo[col]) pr = 0.f;
-                pt[i] = pr;
-                dst[i] = pr * (__uint_as_float(dp[cc][i]) - s_delta[col]) * gr;
+              for (int i = 0; i < 32; ++i) dp[i] = 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+              const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[c0 + i]);
+              const float d[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                float v = pr[cc][i + e] * (__uint_as_float(dp[i + e]) * p.scale - d[e]);
+                if (MODES && capped) v *= gr[MODES ? cc : 0][MODES ? i + e : 0];
+                pr[cc][i + e] = v;
               }
             }
-            if (ok) {
-              store_operand_chunk(sPT, r, c, pt);
-              store_operand_chunk(sDST, r, c, dst);
-            }
+            if (ok) store_operand_chunk(sDST, r, half * 2 + cc, pr[cc]);
           }
           if (ok) {
             fence_proxy_async_smem();
             tc_fence_before();
-            mbar_arrive(pds_ready);
+            mbar_arrive(ds_ready);
           }
-          softmax_bar_sync();    // this block's statistics are no longer read
-          if (half == 0 && it + 1 < t.iters) store_stats(n_l2, n_dl, n_lo);
-          softmax_bar_sync();    // the next block's are visible
+          softmax_bar_sync();    // this block's delta is no longer read; the next block's lse is visible
+          if (fetch) s_delta[r] = n_dl;
         }
         if (ok) {
           const int last = g0 + t.iters - 1;
-          if (!mbar_wait(&acc_done[last % PB], uint32_t(last / PB) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 12))
+          if (!mbar_wait(&dk_done[last % DB], uint32_t(last / DB) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 12))
             ok = false;
         }
         tc_fence_after();

@@ -60,6 +60,29 @@ def test_flash_backward(B, Sq, Skv, H, Hkv, D, causal):
     _close(v.grad, vr.grad, 5e-2)
 
 
+@pytest.mark.parametrize("B,Sq,Skv,H,Hkv,D,causal", [
+    (3, 130, 130, 64, 64, 128, True),      # many units per CTA, of one block and of two, the last two rows tall
+    (2, 640, 640, 48, 16, 128, True),      # one to five blocks, three query heads on a key head
+    (2, 640, 640, 48, 16, 64, True),
+    (5, 128, 520, 40, 40, 128, False),     # one query block against five, the last eight keys wide
+    (5, 520, 128, 40, 40, 64, False),
+])
+def test_flash_backward_walks_many_units(B, Sq, Skv, H, Hkv, D, causal):
+    """Every CTA runs several units of different length one after the other: the next one's tiles, scores and sums come into
+    the buffers of the one before."""
+    q, k, v = _rand((B, Sq, H, D), 1), _rand((B, Skv, Hkv, D), 2), _rand((B, Skv, Hkv, D), 3)
+    do = _rand((B, Sq, H, D), 4)
+    out, lse = ops.flash_forward(q, k, v, causal)
+    grads = ops.flash_backward(do, q, k, v, out, lse, causal)
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    ops.attention_reference(qr, kr, vr, causal).backward(do.float())
+    for got, want in zip(grads, (qr.grad, kr.grad, vr.grad)):
+        # out, P (or dS) and the gradient are rounded to 8 bits of mantissa, each 2^-9 of the value: 4 * 2^-9 with delta's share
+        assert ((got.float() - want).norm() / want.norm()).item() < 2.0 ** -7
+    for a, b in zip(grads, ops.flash_backward(do, q, k, v, out, lse, causal)):
+        assert torch.equal(a, b)
+
+
 MODES = [  # B, S, H, Hkv, D, window, spans, softcap
     (2, 512, 4, 4, 64, 128, None, None),
     (1, 640, 4, 2, 128, 200, None, None),
