@@ -361,9 +361,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
           float ds[32];
           if (!special) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const float pr = fast_exp2(__uint_as_float(s[cc][i]) * p.scale_log2 - lse2);
-              ds[i] = pr * (__uint_as_float(dp[cc][i]) * p.scale - dlt_s);
+            for (int i = 0; i < 32; i += 2) {
+              const float2 x = fma2(as_float2(s[cc][i], s[cc][i + 1]), make_float2(p.scale_log2, p.scale_log2), make_float2(-lse2, -lse2));
+              const float2 d = fma2(as_float2(dp[cc][i], dp[cc][i + 1]), make_float2(p.scale, p.scale), make_float2(-dlt_s, -dlt_s));
+              const float2 v = mul2(make_float2(fast_exp2(x.x), fast_exp2(x.y)), d);
+              ds[i] = v.x;
+              ds[i + 1] = v.y;
             }
           } else {
             // lower key bound and / or soft-capped scores: u = cap * tanh(s * scale / cap), du/ds = scale * (1 - tanh^2)
@@ -455,7 +458,7 @@ struct BwdKVSmem {
   // beside two Q / dO stages at head size 128 (227 KB in all)
   static constexpr int kDSBufs = (D == 64) ? 2 : 1;
   static constexpr int kDST = kDO + kStages * kTile;
-  static constexpr int kStat = kDST + kDSBufs * 32768;      // lse2[128], delta * scale [128], lo[128]
+  static constexpr int kStat = kDST + kDSBufs * 32768;      // -lse * log2(e) [128], -delta * scale [128], lo[128]
   static constexpr int kBar = kStat + 1536;
   static constexpr int kTotal = kBar + 256 + 1024;
 };
@@ -713,13 +716,13 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         auto load_stats = [&](int it, float& l2, float& dl, int& lo) {
           const int head = t.kv_head * group + it / t.per_head;
           const int qr = (t.i_min + it % t.per_head) * 128 + r;
-          l2 = INFINITY;
+          l2 = -INFINITY;                       // both negated: the addends of the fused multiply-adds below
           dl = 0.f;
           if (qr < p.Sq) {
             const size_t idx = (size_t(t.batch) * p.H + head) * p.Sq + qr;
             const float l = p.lse[idx];
-            l2 = (l == -INFINITY) ? INFINITY : l * kLog2e;
-            dl = p.delta[idx] * p.scale;
+            l2 = (l == -INFINITY) ? -INFINITY : -(l * kLog2e);
+            dl = -(p.delta[idx] * p.scale);
           }
           lo = bounded ? flash_row_lo(p, t.batch, qr, off) : 0;
         };
@@ -739,7 +742,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // The statistics of the next query block are fetched now. Its lse replaces this block's once the probabilities
           // are formed, its delta once dS is: each is written after one of the block's two barriers and read after the
           // other, so neither barrier stands alone in the chain.
-          float n_l2 = INFINITY, n_dl = 0.f;
+          float n_l2 = -INFINITY, n_dl = 0.f;
           int n_lo = 0;
           const bool fetch = half == 0 && it + 1 < t.iters;
           if (fetch) load_stats(it + 1, n_l2, n_dl, n_lo);
@@ -769,16 +772,20 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                 const float4 l4 = *reinterpret_cast<const float4*>(&s_lse2[c0 + i]);
                 const float l[4] = {l4.x, l4.y, l4.z, l4.w};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  float sc = __uint_as_float(s[cc][i + e]);
+                for (int e = 0; e < 4; e += 2) {
+                  const float2 l2 = make_float2(l[e], l[e + 1]);
+                  float2 x;
                   if (MODES && capped) {
                     // u = cap * tanh(s * scale / cap), du/ds = scale * (1 - tanh^2)
-                    const float th = tanh_fast(sc * cap_in);
-                    pr[cc][i + e] = fast_exp2(th * cap_l2 - l[e]);
-                    gr[MODES ? cc : 0][MODES ? i + e : 0] = 1.f - th * th;
+                    const float t0 = tanh_fast(__uint_as_float(s[cc][i + e]) * cap_in), t1 = tanh_fast(__uint_as_float(s[cc][i + e + 1]) * cap_in);
+                    x = fma2(make_float2(t0, t1), make_float2(cap_l2, cap_l2), l2);
+                    gr[MODES ? cc : 0][MODES ? i + e : 0] = 1.f - t0 * t0;
+                    gr[MODES ? cc : 0][MODES ? i + e + 1 : 0] = 1.f - t1 * t1;
                   } else {
-                    pr[cc][i + e] = fast_exp2(sc * p.scale_log2 - l[e]);
+                    x = fma2(as_float2(s[cc][i + e], s[cc][i + e + 1]), make_float2(p.scale_log2, p.scale_log2), l2);
                   }
+                  pr[cc][i + e] = fast_exp2(x.x);
+                  pr[cc][i + e + 1] = fast_exp2(x.y);
                 }
               }
               if (diagonal) {
@@ -838,10 +845,12 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               const float4 d4 = *reinterpret_cast<const float4*>(&s_delta[c0 + i]);
               const float d[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                float v = pr[cc][i + e] * (__uint_as_float(dp[i + e]) * p.scale - d[e]);
-                if (MODES && capped) v *= gr[MODES ? cc : 0][MODES ? i + e : 0];
-                pr[cc][i + e] = v;
+              for (int e = 0; e < 4; e += 2) {
+                float2 v = fma2(as_float2(dp[i + e], dp[i + e + 1]), make_float2(p.scale, p.scale), make_float2(d[e], d[e + 1]));
+                v = mul2(make_float2(pr[cc][i + e], pr[cc][i + e + 1]), v);
+                if (MODES && capped) v = mul2(v, make_float2(gr[MODES ? cc : 0][MODES ? i + e : 0], gr[MODES ? cc : 0][MODES ? i + e + 1 : 0]));
+                pr[cc][i + e] = v.x;
+                pr[cc][i + e + 1] = v.y;
               }
             }
             if (ok) store_operand_chunk(sDST, r, half * 2 + cc, pr[cc]);

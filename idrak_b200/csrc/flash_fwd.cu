@@ -20,6 +20,7 @@
 // Reference counterparts: flash_tc_fwd_d{64,128} (src/Idrak.Gpu/Cuda/PtxKernels.FlashTensorCore.cs:318-321)
 // and Tensor.CausalAttention (src/Idrak.Abstraction/Tensors/Tensor.Decoding.cs:132).
 #include "flash_common.cuh"
+#include <type_traits>
 
 namespace idrak {
 
@@ -243,7 +244,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (p.causal) lim = min(lim, row + off - k0 + 1);
       lim = max(0, min(64, lim));
       const int lo = max(0, min(64, row_lo - k0));
-      const bool need_mask = lim < 64 || lo > 0;
+      // whether any row of the warp masks a column: only then are the columns compared one by one, which is half of the
+      // instructions of a block
+      const bool masked = __any_sync(0xffffffffu, lim < 64 || lo > 0);
       uint32_t s[2][32];
       if (ok) {
         const uint32_t s_addr = tmem_S + uint32_t(sb) * 128 + lane_addr + half * 64;
@@ -263,7 +266,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int i = 0; i < 32; ++i) s[c][i] = __float_as_uint(tanh_fast(__uint_as_float(s[c][i]) * cap_in));
       }
       float m2[2] = {-INFINITY, -INFINITY};
-      if (!need_mask) {
+      if (!masked) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           m2[0] = fmaxf(m2[0], __uint_as_float(s[0][i]));
@@ -315,21 +318,28 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
       // probabilities -> bf16 operand tile (K-major, 128B swizzle: chunk ^= row % 8), from the registers
+      auto probabilities = [&](auto with_mask) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        float l4[4] = {0.f, 0.f, 0.f, 0.f};
+        float2 l01 = make_float2(0.f, 0.f), l23 = l01;
         uint8_t* atom = sP + half * 16384 + r * 128;          // columns [64 half, 64 half + 64) are one 128-byte row
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           // eight exponentials, packed and stored at once: few values live at a time (96 registers per thread)
           float pv[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < 8; i += 2) {
             const int col = c * 32 + g * 8 + i;
-            float e = fast_exp2(__uint_as_float(s[c][g * 8 + i]) * sl2 - m_sub);
-            if (need_mask && (col >= lim || col < lo)) e = 0.f;
-            pv[i] = e;
-            l4[i & 3] += e;
+            const float2 x = fma2(as_float2(s[c][g * 8 + i], s[c][g * 8 + i + 1]), make_float2(sl2, sl2), make_float2(-m_sub, -m_sub));
+            float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+            if (decltype(with_mask)::value) {
+              if (col >= lim || col < lo) e.x = 0.f;
+              if (col + 1 >= lim || col + 1 < lo) e.y = 0.f;
+            }
+            pv[i] = e.x;
+            pv[i + 1] = e.y;
+            if (i & 2) l23 = add2(l23, e);
+            else l01 = add2(l01, e);
           }
           const int chunk = (c * 4 + g) ^ (r & 7);
           uint4 o;
@@ -339,8 +349,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           o.w = pack_bf16x2(pv[6], pv[7]);
           *reinterpret_cast<uint4*>(atom + chunk * 16) = o;
         }
-        l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+        l += (l01.x + l01.y) + (l23.x + l23.y);
       }
+      };
+      if (masked) probabilities(std::true_type{});
+      else probabilities(std::false_type{});
       if (ok) {
         fence_proxy_async_smem();
         tc_fence_before();
