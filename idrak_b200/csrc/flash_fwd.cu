@@ -5,11 +5,12 @@
 //   warp 0      TMA producer: Q once, then K and V blocks through two-stage rings (128B swizzle)
 //   warp 1      MMA issuer:   S = Q K^T into one of TWO score buffers in TMEM (tcgen05.mma, K-major x K-major), issued
 //                             one block ahead so the scores of block j+1 are being computed while block j is in the
-//                             softmax; then O += P V (P from shared memory, V as an MN-major operand, accumulator in TMEM)
+//                             softmax; then O += P V (P from TMEM, V as an MN-major operand, accumulator in TMEM)
 //   warps 2..9  softmax:      two threads per query row, each with 64 of the block's 128 score columns in registers
 //                             (two tcgen05.ld in flight, one wait); the score buffer goes back to the MMA warp at
 //                             once; the halves exchange row maxima through shared memory, take the online max /
-//                             sum in the log2 domain, write P as bf16 into the swizzled operand layout, rescale
+//                             sum in the log2 domain, write P as bf16 back to tensor memory (an A operand needs no
+//                             shared memory), rescale
 //                             their half of the TMEM accumulator only when the running max moved by more than 2^8
 //                             (warp-uniform decision), and finally normalise and store O plus the row
 //                             log-sum-exp for the backward pass. Eight softmax warps per CTA, two CTAs per SM at
@@ -27,16 +28,10 @@ namespace idrak {
 template <int D>
 struct FwdSmem {
   static constexpr int kTile = 128 * D * 2;        // one 128-row operand tile
-  static constexpr int kP = 128 * 128 * 2;
   static constexpr int kQ = 0;
-  // Head size 64 keeps ONE key stage: Q K^T of a block finishes before that block's softmax starts, so the next keys
-  // load during the softmax anyway, and the 16 KB saved are what lets two CTAs share an SM (2 x 100 KB): with one CTA
-  // per SM its set-up and write-out (about 6 us) ran unhidden, half of the time at 1024 tokens.
-  static constexpr int kKStages = (D == 64) ? 1 : 2;
-  static constexpr int kK = kQ + kTile;
-  static constexpr int kV = kK + kKStages * kTile;  // two stages
-  static constexpr int kPOff = kV + 2 * kTile;
-  static constexpr int kXch = kPOff + kP;          // row maxima / sums exchanged between the two halves: 2 x 2 x 128 floats
+  static constexpr int kK = kQ + kTile;             // two stages
+  static constexpr int kV = kK + 2 * kTile;         // two stages
+  static constexpr int kXch = kV + 2 * kTile;       // row maxima / sums exchanged between the two halves: 2 x 2 x 128 floats
   static constexpr int kBar = kXch + 2048;
   static constexpr int kTotal = kBar + 256 + 1024;
 };
@@ -60,8 +55,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* s_full = bars + 9;    // [2]
   uint64_t* s_empty = bars + 11;  // [2]
   uint64_t* p_ready = bars + 13;
-  uint64_t* o_done = bars + 14;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* o_done = bars + 14;   // [2]: the P V products of even and odd blocks
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -92,7 +87,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&s_empty[b], 256);
     }
     mbar_init(p_ready, 256);
-    mbar_init(o_done, 1);
+    mbar_init(&o_done[0], 1);
+    mbar_init(&o_done[1], 1);
     *abort_flag = 0;
     fence_barrier_init();
     if (nkv > 0) {
@@ -112,11 +108,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
     }
   }
-  // D = 64: one score buffer [0,128) and O at [128,192) in 256 columns, so two CTAs share an SM (one CTA's prologue and
-  // epilogue hide behind the other's main loop); the buffer is handed back as soon as the row sits in registers, which
-  // lets the next block's scores be computed during this block's softmax all the same.
-  // D = 128: two score buffers at [0,128) and [128,256), O at [256,384), one CTA per SM.
+  // D = 64: one score buffer [0,128), O at [128,192) and P at [192,256): 256 columns, so two CTAs share an SM (one CTA's
+  // prologue and epilogue hide behind the other's main loop); the score buffer is handed back as soon as the row sits in
+  // registers, which lets the next block's scores be computed during this block's softmax all the same.
+  // D = 128: two score buffers at [0,128) and [128,256), O at [256,384), two P buffers of 64 columns at [384,512), one CTA
+  // per SM.
   constexpr int kSBufs = (D == 64) ? 1 : 2;
+  constexpr int kPBufs = kSBufs;
   constexpr uint32_t kTmemCols = (D == 64) ? 256 : 512;
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -126,7 +124,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128 * kSBufs;
+  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 128 * kSBufs, tmem_P = tmem_O + D;
 
   if (warp == 0) {
     if (lane == 0 && nkv > 0) {
@@ -135,13 +133,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       for (int j = 1; j < nkv && ok; ++j) {          // block 0 was requested before the sync
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int kst = (L::kKStages == 2) ? st : 0;
-        const uint32_t kph = (L::kKStages == 2) ? ph : uint32_t(j & 1);
-        if (!mbar_wait(&k_empty[kst], kph ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (2u << 16) | kst)) { ok = false; break; }
-        mbar_expect_tx(&k_full[kst], L::kTile);
+        if (!mbar_wait(&k_empty[st], ph ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (2u << 16) | st)) { ok = false; break; }
+        mbar_expect_tx(&k_full[st], L::kTile);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c)
-          tma_load_4d(smem + L::kK + kst * L::kTile + c * 16384, &tmK, &k_full[kst], c * 64, (jlo + j) * 128, kv_head, batch);
+          tma_load_4d(smem + L::kK + st * L::kTile + c * 16384, &tmK, &k_full[st], c * 64, (jlo + j) * 128, kv_head, batch);
         inflight |= 1u << st;
         if (!mbar_wait(&v_empty[st], ph ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (2u << 16) | (2 + st))) { ok = false; break; }
         mbar_expect_tx(&v_full[st], L::kTile);
@@ -165,20 +161,17 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       constexpr uint32_t idesc_o = make_idesc_f16(128, D, 0, 1, 1);
       bool ok = mbar_wait(q_full, 0, abort_flag, p.st, kTimeoutSmemFull, (2u << 16) | 8);
       const uint32_t sq = smem_u32(smem + L::kQ);
-      const uint32_t sp = smem_u32(smem + L::kPOff);
       // scores of block j go to buffer j & 1; they are issued one block ahead of the P V product
       auto issue_scores = [&](int j) -> bool {
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int kst = (L::kKStages == 2) ? st : 0;
-        const uint32_t kph = (L::kKStages == 2) ? ph : uint32_t(j & 1);
-        if (!mbar_wait(&k_full[kst], kph, abort_flag, p.st, kTimeoutSmemFull, (2u << 16) | kst)) return false;
+        if (!mbar_wait(&k_full[st], ph, abort_flag, p.st, kTimeoutSmemFull, (2u << 16) | st)) return false;
         // the buffer's previous use (block j - 2) has been read out by the softmax warps
         const int sb = (kSBufs == 2) ? st : 0;
         const uint32_t sph = (kSBufs == 2) ? (ph ^ 1) : uint32_t((j + 1) & 1);     // the buffer's previous use: block j - kSBufs
         if (!mbar_wait(&s_empty[sb], sph, abort_flag, p.st, kTimeoutTmemEmpty, (2u << 16) | (12 + sb))) return false;
         tc_fence_after();
-        const uint32_t sk = smem_u32(smem + L::kK + kst * L::kTile);
+        const uint32_t sk = smem_u32(smem + L::kK + st * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t o = (kk >> 2) * 16384 + (kk & 3) * 32;
@@ -186,7 +179,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         idesc_s, kk > 0 ? 1u : 0u);
         }
         tc_commit(&s_full[sb]);
-        tc_commit(&k_empty[kst]);
+        tc_commit(&k_empty[st]);
         return true;
       };
       if (ok) ok = issue_scores(0);
@@ -200,12 +193,11 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t sv = smem_u32(smem + L::kV + st * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t da = make_smem_desc_sw128(sp + (kk >> 2) * 16384 + (kk & 3) * 32, 16, 1024);
           const uint64_t db = make_smem_desc_sw128(sv + kk * 2048, 16384, 1024);
-          tc_mma_f16_ss(tmem_O, da, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          tc_mma_f16_ts(tmem_O, tmem_P + ((kPBufs == 2) ? st * 64 : 0) + kk * 8, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
         }
         tc_commit(&v_empty[st]);
-        tc_commit(o_done);
+        tc_commit(&o_done[st]);
       }
     }
   } else {
@@ -220,7 +212,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int r = quarter * 32 + lane;           // row within the tile == TMEM lane
     const int row = q0 + r;                      // query position
     const uint32_t lane_addr = uint32_t(quarter * 32) << 16;
-    uint8_t* sP = smem + L::kPOff;
     float* xch = reinterpret_cast<float*>(smem + L::kXch);      // [2 parities][2 halves][128 rows]
     const uint32_t pair_bar = 1 + quarter;       // named barrier of the two warps of this lane quarter
     float m_used = -INFINITY;                    // max the accumulator and the running sum are scaled by
@@ -292,11 +283,16 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       // quarter hold the same rows and so decide alike)
       const bool need = (j > 0) && (m_new - m_used > 8.0f);
       const bool warp_rescale = __any_sync(0xffffffffu, need);
-      if (j > 0 && ok) {
-        // P of the previous block is still being read by its MMA until o_done completes
-        if (!mbar_wait(o_done, (j - 1) & 1, abort_flag, p.st, kTimeoutTmemFull, (2u << 16) | 11)) ok = false;
-        tc_fence_after();
+      // Block j - 1's P V product must be complete before the accumulator is rescaled, and before P is overwritten where
+      // there is one buffer; with two, P's buffer was read by block j - 2's.
+      if (ok && j >= kPBufs) {
+        const int last = j - kPBufs;
+        if (!mbar_wait(&o_done[last & 1], uint32_t(last >> 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (2u << 16) | 11)) ok = false;
       }
+      if (kPBufs == 2 && ok && warp_rescale) {
+        if (!mbar_wait(&o_done[(j - 1) & 1], uint32_t((j - 1) >> 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (2u << 16) | 14)) ok = false;
+      }
+      tc_fence_after();
       if (j == 0) {
         m_used = m_new;
       } else if (warp_rescale) {
@@ -317,12 +313,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         }
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
-      // probabilities -> bf16 operand tile (K-major, 128B swizzle: chunk ^= row % 8), from the registers
+      // probabilities -> bf16 A operand of the P V product in tensor memory, two columns of the row per 32-bit column
+      const uint32_t p_addr = tmem_P + ((kPBufs == 2) ? (j & 1) * 64 : 0) + lane_addr + half * 32;
       auto probabilities = [&](auto with_mask) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         float2 l01 = make_float2(0.f, 0.f), l23 = l01;
-        uint8_t* atom = sP + half * 16384 + r * 128;          // columns [64 half, 64 half + 64) are one 128-byte row
+        uint32_t packed[16];
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           // eight exponentials, packed and stored at once: few values live at a time (96 registers per thread)
@@ -341,27 +338,23 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (i & 2) l23 = add2(l23, e);
             else l01 = add2(l01, e);
           }
-          const int chunk = (c * 4 + g) ^ (r & 7);
-          uint4 o;
-          o.x = pack_bf16x2(pv[0], pv[1]);
-          o.y = pack_bf16x2(pv[2], pv[3]);
-          o.z = pack_bf16x2(pv[4], pv[5]);
-          o.w = pack_bf16x2(pv[6], pv[7]);
-          *reinterpret_cast<uint4*>(atom + chunk * 16) = o;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) packed[g * 4 + i] = pack_bf16x2(pv[2 * i], pv[2 * i + 1]);
         }
+        if (ok) tmem_st_32x32b_x16(p_addr + c * 16, packed);
         l += (l01.x + l01.y) + (l23.x + l23.y);
       }
       };
       if (masked) probabilities(std::true_type{});
       else probabilities(std::false_type{});
       if (ok) {
-        fence_proxy_async_smem();
+        tmem_st_wait();
         tc_fence_before();
         mbar_arrive(p_ready);
       }
     }
     if (ok && nkv > 0) {
-      if (!mbar_wait(o_done, (nkv - 1) & 1, abort_flag, p.st, kTimeoutTmemFull, (2u << 16) | 12)) ok = false;
+      if (!mbar_wait(&o_done[(nkv - 1) & 1], uint32_t((nkv - 1) >> 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (2u << 16) | 12)) ok = false;
     }
     tc_fence_after();
     // the row sum over both halves
