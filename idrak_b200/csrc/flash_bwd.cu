@@ -16,7 +16,10 @@
 // room for two or three stages of every streamed tile at head size 128 too, so loads, products and element-wise steps of
 // neighbouring blocks overlap. With everything staged in shared memory there was one stage of each, and a block's load,
 // scores, element-wise step and accumulation ran one after the other. Measured, 8192 positions, 32 heads on 8, size 128,
-// causal: dQ 1330 -> 747 us, dK / dV 1884 -> 1299 us; 8 x 1024, 12 heads, size 64: 49 -> 47 and 84 -> 77 us.
+// causal: dQ 1330 -> 747 us, dK / dV 1884 -> 1299 us; then with packed fp32 arithmetic 709 and 1263 us, and with one
+// barrier arrival per warp and the scores issued before dP 690 and 1069 us. 8 x 1024, 12 heads, size 64: 49 -> 43 and
+// 84 -> 74 us in all. What bounds them now is the chain of an element-wise step (two warps per scheduler, 64 columns per
+// thread); the tensor pipe is busy 35 to 50 % of the time.
 // A tile in shared memory serves as a K-major operand for one product and as an MN-major operand for the other, so nothing
 // is transposed.
 //
@@ -184,12 +187,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&v_empty[s], 1);
     }
     mbar_init(sdp_full, 1);
-    mbar_init(ds_ready, 256);
+    mbar_init(ds_ready, 8);
     mbar_init(&dq_done[0], 1);
     mbar_init(&dq_done[1], 1);
-    mbar_init(sdp_taken, 256);
+    mbar_init(sdp_taken, 8);
     mbar_init(qdo_free, 1);
-    mbar_init(dq_free, 256);
+    mbar_init(dq_free, 8);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
@@ -338,7 +341,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const int row_lo = bounded ? flash_row_lo(p, t.batch, row, off) : 0;
       for (int j = 0; j < t.nkv && ok; ++j) {
         const int g = g0 + j;
-        if (!mbar_wait(sdp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 10)) { ok = false; break; }
+        if (!warp_wait(sdp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 10)) { ok = false; break; }
         tc_fence_after();
         const int k0 = (t.jlo + j) * 128 + half * 64;          // first key of this thread's 64 columns
         int lim = p.Skv - k0;
@@ -354,7 +357,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_ld_32x32b_x32(tmem_dP + lane_addr + half * 64 + 32, dp[1]);
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(sdp_taken);
+        warp_arrive(sdp_taken);
         uint32_t packed[32];
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
@@ -394,7 +397,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         if (g >= 2) {
           // the dQ product that last read this dS buffer (block g - 2) must be complete
-          if (!mbar_wait(&dq_done[g & 1], uint32_t((g >> 1) - 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 11)) {
+          if (!warp_wait(&dq_done[g & 1], uint32_t((g >> 1) - 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 11)) {
             ok = false;
             break;
           }
@@ -403,11 +406,11 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_st_32x32b_x32(tmem_dS + (g & 1) * 64 + lane_addr + half * 32, packed);
         tmem_st_wait();
         tc_fence_before();
-        mbar_arrive(ds_ready);
+        warp_arrive(ds_ready);
       }
       if (!ok) break;
       const int last = g0 + t.nkv - 1;
-      if (!mbar_wait(&dq_done[last & 1], uint32_t(last >> 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 12)) {
+      if (!warp_wait(&dq_done[last & 1], uint32_t(last >> 1) & 1u, abort_flag, p.st, kTimeoutTmemFull, (3u << 16) | 12)) {
         ok = false;
         break;
       }
@@ -419,7 +422,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_ld_32x32b_x32(tmem_dQ + lane_addr + half * kOC + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[c * 32]));
       tmem_ld_wait();
       tc_fence_before();
-      mbar_arrive(dq_free);
+      warp_arrive(dq_free);
       if (row < p.Sq) {
 #pragma unroll
         for (int gq = 0; gq < kOC / 8; ++gq) {
@@ -545,15 +548,15 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
-    mbar_init(s_taken, 256);
-    mbar_init(dp_taken, 256);
-    mbar_init(p_ready, 256);
-    mbar_init(ds_ready, 256);
+    mbar_init(s_taken, 8);
+    mbar_init(dp_taken, 8);
+    mbar_init(p_ready, 8);
+    mbar_init(ds_ready, 8);
     mbar_init(dv_done, 1);
     mbar_init(&dk_done[0], 1);
     mbar_init(&dk_done[1], 1);
     mbar_init(kv_free, 1);
-    mbar_init(acc_free, 256);
+    mbar_init(acc_free, 8);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
@@ -595,17 +598,20 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tma_load_4d(smem + L::kK + c * 16384, &tmK, kv_full, c * 64, t.k0, t.kv_head, t.batch);
           tma_load_4d(smem + L::kV + c * 16384, &tmV, kv_full, c * 64, t.k0, t.kv_head, t.batch);
         }
+        int head = t.kv_head * group, qi = t.i_min;
         for (int it = 0; it < t.iters; ++it, ++g) {
           const int st = g % NS;
           const uint32_t ph = (g / NS) & 1;
-          const int head = t.kv_head * group + it / t.per_head;
-          const int qi = t.i_min + it % t.per_head;
           if (!mbar_wait(&qdo_empty[st], ph ^ 1, abort_flag, p.st, kTimeoutSmemEmpty, (4u << 16) | st)) { ok = false; break; }
           mbar_expect_tx(&qdo_full[st], 2 * L::kTile);
 #pragma unroll
           for (int c = 0; c < D / 64; ++c) {
             tma_load_4d(smem + L::kQ + st * L::kTile + c * 16384, &tmQ, &qdo_full[st], c * 64, qi * 128, head, t.batch);
             tma_load_4d(smem + L::kDO + st * L::kTile + c * 16384, &tmDO, &qdo_full[st], c * 64, qi * 128, head, t.batch);
+          }
+          if (++qi == t.i_min + t.per_head) {
+            qi = t.i_min;
+            ++head;
           }
         }
         ++n;
@@ -662,8 +668,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int st = g % NS;
           const bool more = it + 1 < t.iters;
           // The next block's scores and dP go out between this block's two accumulations, so the element-wise warps find
-          // them when they are done with this block. Scores with a place of their own go first; scores that share it with
-          // P^T follow dP, whose product covers the wait for dV.
+          // them when they are done with this block: the scores first, which their next step starts from (with a place of
+          // their own even before dV).
           if (more && !kAlias && !issue_s(g + 1)) { ok = false; break; }
           if (!mbar_wait(p_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 9)) { ok = false; break; }
           if (it == 0 && n > 0) {
@@ -677,8 +683,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             tc_mma_f16_ts(tmem_dV, tmem_PT + (kk >> 2) * kPHalf + (kk & 3) * 8, mnmajor_desc(sdo, kk), idesc_acc,
                           (it > 0 || kk > 0) ? 1u : 0u);
           tc_commit(dv_done);
-          if (more && !issue_dp(g + 1)) { ok = false; break; }
           if (more && kAlias && !issue_s(g + 1)) { ok = false; break; }
+          if (more && !issue_dp(g + 1)) { ok = false; break; }
           if (it + 2 == t.iters) tc_commit(kv_free);               // the unit's last score products are on their way
           if (!mbar_wait(ds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 17)) { ok = false; break; }
           tc_fence_after();
@@ -713,40 +719,46 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const KvUnit t = kv_unit<MODES>(p, u, off, nq);
       const int key = t.k0 + r;
       if (t.iters > 0) {
-        auto load_stats = [&](int it, float& l2, float& dl, int& lo) {
-          const int head = t.kv_head * group + it / t.per_head;
-          const int qr = (t.i_min + it % t.per_head) * 128 + r;
-          l2 = -INFINITY;                       // both negated: the addends of the fused multiply-adds below
+        // lse and delta of one row of query block qi, as they are in memory: they are converted only where they are staged
+        auto load_stats = [&](int head, int qi, float& l, float& dl, int& lo) {
+          const int qr = qi * 128 + r;
+          l = -INFINITY;
           dl = 0.f;
           if (qr < p.Sq) {
             const size_t idx = (size_t(t.batch) * p.H + head) * p.Sq + qr;
-            const float l = p.lse[idx];
-            l2 = (l == -INFINITY) ? -INFINITY : -(l * kLog2e);
-            dl = -(p.delta[idx] * p.scale);
+            l = p.lse[idx];
+            dl = p.delta[idx];
           }
           lo = bounded ? flash_row_lo(p, t.batch, qr, off) : 0;
         };
+        // both negated: the addends of the fused multiply-adds below
+        auto staged_lse = [](float l) { return (l == -INFINITY) ? -INFINITY : -(l * kLog2e); };
+        int head = t.kv_head * group, qi = t.i_min;             // of the current block, counted along
         // the previous unit's last block ended with a barrier after its statistics were last read
         if (half == 0) {
-          float l2, dl;
+          float l, dl;
           int lo;
-          load_stats(0, l2, dl, lo);
-          s_lse2[r] = l2;
+          load_stats(head, qi, l, dl, lo);
+          s_lse2[r] = staged_lse(l);
           s_lo[r] = lo;
-          s_delta[r] = dl;
+          s_delta[r] = -(dl * p.scale);
         }
         softmax_bar_sync();
         for (int it = 0; it < t.iters; ++it) {
           const int g = g0 + it;
-          const int qrow0 = (t.i_min + it % t.per_head) * 128;
+          const int qrow0 = qi * 128;
+          if (++qi == t.i_min + t.per_head) {
+            qi = t.i_min;
+            ++head;
+          }
           // The statistics of the next query block are fetched now. Its lse replaces this block's once the probabilities
           // are formed, its delta once dS is: each is written after one of the block's two barriers and read after the
           // other, so neither barrier stands alone in the chain.
-          float n_l2 = -INFINITY, n_dl = 0.f;
+          float n_l = -INFINITY, n_dl = 0.f;
           int n_lo = 0;
           const bool fetch = half == 0 && it + 1 < t.iters;
-          if (fetch) load_stats(it + 1, n_l2, n_dl, n_lo);
-          if (ok && !mbar_wait(s_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 10)) ok = false;
+          if (fetch) load_stats(head, qi, n_l, n_dl, n_lo);
+          if (ok && !warp_wait(s_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 10)) ok = false;
           tc_fence_after();
           // query q (column) sees this key iff key <= q + off  <=>  q >= key - off
           const int first_q = p.causal ? (key - off - qrow0) : 0;    // columns below this are masked
@@ -759,7 +771,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               tmem_ld_32x32b_x32(tmem_ST + lane_addr + half * 64 + 32, s[1]);
               tmem_ld_wait();
               tc_fence_before();
-              if (!kAlias) mbar_arrive(s_taken);
+              if (!kAlias) warp_arrive(s_taken);
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i) s[0][i] = s[1][i] = 0u;
@@ -803,27 +815,27 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
             if (!kAlias && ok && g > 0) {
               // the dV product of the block before has read P^T (over the scores: they came after it)
-              if (!mbar_wait(dv_done, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 18)) ok = false;
+              if (!warp_wait(dv_done, (g - 1) & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 18)) ok = false;
               tc_fence_after();
             }
             if (ok) {
               tmem_st_32x32b_x32(tmem_PT + lane_addr + half * kPHalf, packed);
               tmem_st_wait();
               tc_fence_before();
-              mbar_arrive(p_ready);
+              warp_arrive(p_ready);
             }
           }
           softmax_bar_sync();    // this block's lse is no longer read; its delta is visible
           if (fetch) {
-            s_lse2[r] = n_l2;
+            s_lse2[r] = staged_lse(n_l);
             s_lo[r] = n_lo;
           }
-          if (ok && !mbar_wait(dp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 19)) ok = false;
+          if (ok && !warp_wait(dp_full, g & 1, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 19)) ok = false;
           tc_fence_after();
           uint8_t* sDST = smem + L::kDST + (g % DB) * 32768;
           if (ok && g >= DB) {
             // the dK product that last read this dS^T buffer (block g - DB) must be complete
-            if (!mbar_wait(&dk_done[g % DB], (uint32_t(g / DB) - 1u) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 11)) ok = false;
+            if (!warp_wait(&dk_done[g % DB], (uint32_t(g / DB) - 1u) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 11)) ok = false;
           }
 #pragma unroll
           for (int cc = 0; cc < 2; ++cc) {
@@ -834,7 +846,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               tmem_ld_wait();
               if (cc == 1) {
                 tc_fence_before();
-                mbar_arrive(dp_taken);
+                warp_arrive(dp_taken);
               }
             } else {
 #pragma unroll
@@ -858,14 +870,15 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (ok) {
             fence_proxy_async_smem();
             tc_fence_before();
-            mbar_arrive(ds_ready);
+            __syncwarp();
+            warp_arrive(ds_ready);
           }
           softmax_bar_sync();    // this block's delta is no longer read; the next block's lse is visible
-          if (fetch) s_delta[r] = n_dl;
+          if (fetch) s_delta[r] = -(n_dl * p.scale);
         }
         if (ok) {
           const int last = g0 + t.iters - 1;
-          if (!mbar_wait(&dk_done[last % DB], uint32_t(last / DB) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 12))
+          if (!warp_wait(&dk_done[last % DB], uint32_t(last / DB) & 1u, abort_flag, p.st, kTimeoutTmemFull, (4u << 16) | 12))
             ok = false;
         }
         tc_fence_after();
@@ -879,7 +892,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int c = 0; c < D / 32; ++c) tmem_ld_32x32b_x32(acc + lane_addr + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&o[c * 32]));
         tmem_ld_wait();
         tc_fence_before();
-        mbar_arrive(acc_free);
+        warp_arrive(acc_free);
       } else {
 #pragma unroll
         for (int i = 0; i < D; ++i) o[i] = 0u;

@@ -62,6 +62,20 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 }
 __device__ __forceinline__ float2 as_float2(uint32_t x, uint32_t y) { return make_float2(__uint_as_float(x), __uint_as_float(y)); }
 
+// One arrival per warp: 32 lanes arriving at one barrier are 32 serialised shared-memory atomics, and eight warps did that
+// two to four times in every block. It follows a tcgen05.wait, which ends for all lanes of a warp together; after ordinary
+// stores the warp has to be synchronised first.
+__device__ __forceinline__ void warp_arrive(uint64_t* bar) {
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+
+// A wait of a whole warp: every lane has the same answer, so warp-wide steps after it (tensor-memory loads, votes, one
+// arrival per warp) never meet a diverged warp, also when a wait gives up.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag, Status* st, uint32_t code,
+                                          uint32_t where) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, st, code, where));
+}
+
 // Barrier `id` (1..15) over `threads` threads of the CTA (whole warps).
 __device__ __forceinline__ void flash_bar_sync(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
