@@ -396,6 +396,15 @@ IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn) {
   return min(s, 16);
 }
 
+// Columns of a tile: 256, or 128 where twice as many CTAs still fit the machine at once. A product that small is a chain of
+// set-up, first load and write-out, and the write-out takes as long as a tile is wide. Each element is summed over K in the
+// same order either way. Measured as the training step of a 4-layer model of width 128 on 1024 tokens: 1181 -> 1128 us.
+static int tile_columns(int M, int N, int splits) {
+  if (N <= 128) return 128;
+  const long long units = (long long)((M + kBM - 1) / kBM) * ((N + 255) / 256) * splits;
+  return 2 * units <= sm_count() ? 128 : 256;
+}
+
 // C = epilogue(alpha * op(A) op(B)).
 //   a_mn = 0: A is [M,K] row-major (lda >= K); a_mn = 1: A is stored [K,M] row-major (lda >= M)
 //   b_mn = 0: B is [N,K] row-major (ldb >= K); b_mn = 1: B is stored [K,N] row-major (ldb >= N)
@@ -411,7 +420,6 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -3;
   if (act != kActNone && aux == nullptr) return -4;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-  const int bn = (N <= 128) ? 128 : 256;
   GemmParams p{};
   p.M = M; p.N = N; p.K = K;
   p.C = C; p.ldc = ldc; p.c_fp32 = c_fp32;
@@ -432,6 +440,7 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
     p.splits = (kblocks + per - 1) / per;
   }
   p.workspace = workspace;
+  const int bn = tile_columns(M, N, p.splits);
   p.m_tiles = (M + kBM - 1) / kBM;
   p.n_tiles = (N + bn - 1) / bn;
   p.st = status_device_ptr();

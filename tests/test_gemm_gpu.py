@@ -160,3 +160,23 @@ def test_gemm_large_products(M, N, K, a_mn, b_mn):
     _pair_case(M, N, K, a_mn, b_mn)
     from idrak_b200 import _native
     _native.check_status("large products")
+
+
+@pytest.mark.parametrize("N", [264, 392, 512])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_narrow_tiles_of_a_small_product_give_the_same_bits(N, a_mn, b_mn):
+    """The most row tiles that still get 128 columns per tile, and one more, which gets 256: an element's sum over K has one
+    order, so the rows that both calls share agree to the bit."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows, K = sms // 4 * 128, 136
+    a, b = _rand((rows + 128, K), 1.0, 1), _rand((N, K), 1.0, 2)
+    bias, res = _rand((N,), 1.0, 3), _rand((rows + 128, N), 1.0, 4)
+    def run(m):
+        x = a[:m].t().contiguous() if a_mn else a[:m]
+        w = b.t().contiguous() if b_mn else b
+        return gemm(x, w, a_mn=a_mn, b_mn=b_mn, bias=bias, residual=res[:m], splits=1)
+    narrow = run(rows)
+    assert torch.equal(narrow, run(rows + 128)[:rows])
+    # fp32 accumulation, one rounding to bf16 (half an ulp is 2^-9) and the fp32 reference's own
+    ref = gemm_reference(a[:rows], b, out_dtype=torch.float32) + bias.float() + res[:rows].float()
+    assert ((narrow.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()

@@ -205,3 +205,29 @@ def test_gated_activation_at_the_edges_of_a_block(rows, H):
     ref.backward(do.float())
     _close(o, ref)
     _close(gu.grad, gr.grad)
+
+
+@pytest.mark.parametrize("parts", [1, 24, 25, 32, 33, 57, 128])
+def test_column_sums_over_any_number_of_partials(parts):
+    """One block of rows per partial: fewer than the four a thread keeps in flight, a multiple, and remainders."""
+    x = _rand((64 * parts - 3, 72), 1.0, 7)
+    out = torch.ones(72, device="cuda")
+    ops.colsum(x, out=out, accumulate=True)
+    want = x.double().sum(0) + 1.0
+    # fp32 sums of the rows in a fixed order: at most rows * 2^-24 of the sum of magnitudes
+    assert ((out.double() - want).abs() <= x.shape[0] * 2.0 ** -24 * (x.double().abs().sum(0) + 1.0)).all()
+
+
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_parameter_gradients_from_one_launch(rms):
+    x, dy = _rand((1000, 136), 1.0, 8).requires_grad_(), _rand((1000, 136), 1.0, 9)
+    w, b = _rand((136,), 1.0, 10).requires_grad_(), _rand((136,), 1.0, 11).requires_grad_()
+    (ops.rms_norm(x, w) if rms else ops.layer_norm(x, w, b)).backward(dy)
+    xr = x.detach().double()
+    xh = xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-5) if rms else torch.nn.functional.layer_norm(xr, (136,), eps=1e-5)
+    want = (dy.double() * xh).sum(0)
+    # one rounding to bf16 and fp32 sums of 1000 terms
+    assert ((w.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-2).all()
+    if not rms:
+        want = dy.double().sum(0)
+        assert ((b.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-2).all()
