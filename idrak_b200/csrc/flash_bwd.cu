@@ -472,17 +472,22 @@ struct BwdKVSmem {
 // score products of the next unit. With one launch of 1536 short CTAs the set-up, first-load and write-out latencies
 // (about 12 k cycles per CTA) ran unhidden, a third of the time at 1024 tokens.
 struct KvUnit {
-  int kb, kv_head, batch, k0, i_min, per_head, iters;
+  int kb, kv_head, batch, part, head0, k0, i_min, per_head, iters;
 };
 
 template <bool MODES>
 __device__ __forceinline__ KvUnit kv_unit(const FlashParams& p, int u, int off, int nq) {
   KvUnit t;
-  const int per_kb = p.Hkv * p.B;
+  const int per_kb = p.Hkv * p.B * p.kv_parts;
   t.kb = u / per_kb;                         // ascending key block = most query blocks first under a causal mask
-  const int rem = u - t.kb * per_kb;
+  int rem = u - t.kb * per_kb;
+  t.part = rem % p.kv_parts;
+  rem /= p.kv_parts;
   t.kv_head = rem % p.Hkv;
   t.batch = rem / p.Hkv;
+  const int group = p.H / p.Hkv;
+  const int heads = group / p.kv_parts;      // query heads of this unit
+  t.head0 = t.kv_head * group + t.part * heads;
   t.k0 = t.kb * 128;
   t.i_min = p.causal ? max(0, (t.k0 - off) / 128) : 0;
   // query blocks past the last one that can see these keys are skipped too: a sliding window bounds them directly,
@@ -498,7 +503,7 @@ __device__ __forceinline__ KvUnit kv_unit(const FlashParams& p, int u, int off, 
     i_end = max(i_end, t.i_min);
   }
   t.per_head = max(0, i_end - t.i_min);
-  t.iters = t.per_head * (p.H / p.Hkv);
+  t.iters = t.per_head * heads;
   return t;
 }
 
@@ -534,10 +539,9 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   int* s_lo = reinterpret_cast<int*>(s_delta + 128);      // first key each query of the block may see
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int group = p.H / p.Hkv;
   const int off = p.Skv - p.Sq;
   const int nq = (p.Sq + 127) / 128;
-  const int units = ((p.Skv + 127) / 128) * p.Hkv * p.B;
+  const int units = ((p.Skv + 127) / 128) * p.Hkv * p.B * p.kv_parts;
   const bool bounded = MODES && p.causal && (p.window > 0 || p.row_start != nullptr);
 
   if (threadIdx.x == 0) {
@@ -598,7 +602,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           tma_load_4d(smem + L::kK + c * 16384, &tmK, kv_full, c * 64, t.k0, t.kv_head, t.batch);
           tma_load_4d(smem + L::kV + c * 16384, &tmV, kv_full, c * 64, t.k0, t.kv_head, t.batch);
         }
-        int head = t.kv_head * group, qi = t.i_min;
+        int head = t.head0, qi = t.i_min;
         for (int it = 0; it < t.iters; ++it, ++g) {
           const int st = g % NS;
           const uint32_t ph = (g / NS) & 1;
@@ -733,7 +737,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
         // both negated: the addends of the fused multiply-adds below
         auto staged_lse = [](float l) { return (l == -INFINITY) ? -INFINITY : -(l * kLog2e); };
-        int head = t.kv_head * group, qi = t.i_min;             // of the current block, counted along
+        int head = t.head0, qi = t.i_min;             // of the current block, counted along
         // the previous unit's last block ended with a barrier after its statistics were last read
         if (half == 0) {
           float l, dl;
@@ -897,7 +901,11 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
         for (int i = 0; i < D; ++i) o[i] = 0u;
       }
-      if ((ok || t.iters == 0) && key < p.Skv) {
+      if ((ok || t.iters == 0) && key < p.Skv && p.kv_parts > 1) {
+        float* row = p.kv_partial + ((((size_t(t.part) * 2 + half) * p.B + t.batch) * p.Skv + key) * p.Hkv + t.kv_head) * D;
+#pragma unroll
+        for (int i = 0; i < D / 4; ++i) *reinterpret_cast<uint4*>(row + i * 4) = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      } else if ((ok || t.iters == 0) && key < p.Skv) {
         __nv_bfloat16* drow = (half ? p.dK + (size_t(t.batch) * p.Skv + key) * p.dk_row_stride
                                     : p.dV + (size_t(t.batch) * p.Skv + key) * p.dv_row_stride) + size_t(t.kv_head) * D;
 #pragma unroll
@@ -925,6 +933,53 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
 }
 
+// Sums the parts of dV and dK in part order: one thread per eight columns of a (batch, key, kv head) row.
+__global__ void __launch_bounds__(256) flash_kv_parts_kernel(const FlashParams p, int D) {
+  const int per_row = D / 8;
+  const long long rows = (long long)p.B * p.Skv * p.Hkv, n = rows * per_row;
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (i >= n) return;
+  const bool is_k = blockIdx.y == 1;
+  const size_t plane = size_t(rows) * D;
+  float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int part = 0; part < p.kv_parts; ++part) {
+    const float4* v = reinterpret_cast<const float4*>(p.kv_partial + (size_t(part) * 2 + is_k) * plane + size_t(i) * 8);
+    const float4 x = v[0], y = v[1];
+    a[0] += x.x; a[1] += x.y; a[2] += x.z; a[3] += x.w;
+    a[4] += y.x; a[5] += y.y; a[6] += y.z; a[7] += y.w;
+  }
+  const long long row = i / per_row;
+  const int head = int(row % p.Hkv);
+  const long long pos = row / p.Hkv;          // batch * Skv + key
+  __nv_bfloat16* dst = (is_k ? p.dK + pos * p.dk_row_stride : p.dV + pos * p.dv_row_stride) + size_t(head) * D + (i - row * per_row) * 8;
+  *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
+}
+
+// Into how many units the query heads of a key head are dealt. One unit walks every query head of its key block, so with
+// grouped heads there are few units and the first key block's, which under a causal mask every query block sees, is longer
+// than a CTA's fair share: 3 x 999 tokens with 16 heads on 4 has 96 units of up to 32 blocks for 148 SMs, against 12 blocks
+// a SM if they were even. The smallest divisor of the group that brings the longest unit to a quarter over the fair share
+// is taken; the parts leave as fp32 and are summed in their order. A unit of under four blocks is not worth the extra pass.
+// Measured, causal, size 64: 2 x 2048 tokens, 16 heads on 4: 142 -> 78 + 4 us for the sum; with 8192 tokens the units are
+// even enough and stay whole.
+static int kv_parts_of(int B, int H, int Hkv, int Sq, int Skv, int causal) {
+  const int group = H / Hkv, nq = (Sq + 127) / 128, nkb = (Skv + 127) / 128, off = Skv - Sq;
+  long long blocks = 0;
+  int longest = 0;
+  for (int kb = 0; kb < nkb; ++kb) {
+    const int first = causal ? max(0, (kb * 128 - off) / 128) : 0, seen = max(0, nq - first);
+    blocks += seen;
+    longest = max(longest, seen);
+  }
+  if (longest * group < 4) return 1;
+  const double share = double(blocks) * H * B / sm_count();
+  int parts = 1;
+  while (parts < group && double(longest) * (group / parts) > 1.25 * max(share, 1.0)) {
+    do ++parts; while (group % parts);
+  }
+  return parts;
+}
+
 template <int D, bool MODES>
 static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                       const FlashParams& p, cudaStream_t stream) {
@@ -942,8 +997,13 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
   note_launches(1);
   int rc = int(cudaGetLastError());
   if (rc) return rc;
-  const int kv_units = ((p.Skv + 127) / 128) * p.Hkv * p.B;
+  const int kv_units = ((p.Skv + 127) / 128) * p.Hkv * p.B * p.kv_parts;
   kkv<<<min(kv_units, sm_count()), kBwdThreads, BwdKVSmem<D>::kTotal, stream>>>(tq, tk, tv, tdo, p);
+  note_launches(1);
+  rc = int(cudaGetLastError());
+  if (rc || p.kv_parts == 1) return rc;
+  const long long vecs = (long long)p.B * p.Skv * p.Hkv * (D / 8);
+  flash_kv_parts_kernel<<<dim3(unsigned((vecs + 255) / 256), 2), 256, 0, stream>>>(p, D);
   note_launches(1);
   return int(cudaGetLastError());
 }
@@ -952,18 +1012,26 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 using namespace idrak;
 
+// fp32 elements of workspace a backward call of these sizes needs (0: none).
+IDRAK_API long long idrak_flash_bwd_workspace(int B, int H, int Hkv, int Sq, int Skv, int D, int causal) {
+  if (B <= 0 || Hkv <= 0 || H <= 0 || H % Hkv) return 0;
+  const int parts = kv_parts_of(B, H, Hkv, Sq, Skv, causal);
+  return parts > 1 ? 2LL * parts * B * Skv * Hkv * D : 0;
+}
+
 // out / dout: contiguous [B, Sq, H, D]; lse, delta [B,H,Sq]. dq / dk / dv rows hold heads packed [heads, D] with
 // the given row strides in elements (0 = contiguous), so they may be slices of one fused d(QKV) buffer;
 // their batch stride is rows * row stride.
 // window > 0 and row_start (one int per query row, [B, Sq]) restrict the keys a query sees exactly as in the forward
 // entry point; both need `causal`. `softcap` > 0 differentiates through the tanh cap of the forward.
+// workspace: idrak_flash_bwd_workspace fp32 elements on a 16-byte boundary, or null (the heads of a group then stay together).
 IDRAK_API int idrak_flash_bwd_ex(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                  const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int H, int Hkv,
                                  int Sq, int Skv, int D, long long q_row_stride, long long k_row_stride,
                                  long long v_row_stride, long long q_batch_stride, long long k_batch_stride,
                                  long long v_batch_stride, long long dq_row_stride, long long dk_row_stride,
                                  long long dv_row_stride, float scale, int causal, int window, const int* row_start,
-                                 float softcap, void* stream_) {
+                                 float softcap, float* workspace, void* stream_) {
   if (D != 64 && D != 128) return -2;
   if (H % Hkv) return -3;
   if ((window > 0 || row_start) && !causal) return -4;
@@ -980,6 +1048,8 @@ IDRAK_API int idrak_flash_bwd_ex(const void* q, const void* k, const void* v, co
     if (rc) return rc;
   }
   FlashParams p;
+  p.kv_parts = workspace ? kv_parts_of(B, H, Hkv, Sq, Skv, causal) : 1;
+  p.kv_partial = workspace;
   p.O = nullptr;
   p.o_row_stride = 0;
   p.lse = const_cast<float*>(lse);
@@ -1016,5 +1086,5 @@ IDRAK_API int idrak_flash_bwd(const void* q, const void* k, const void* v, const
                               long long dv_row_stride, float scale, int causal, void* stream_) {
   return idrak_flash_bwd_ex(q, k, v, out, dout, lse, delta, dq, dk, dv, B, H, Hkv, Sq, Skv, D, q_row_stride,
                             k_row_stride, v_row_stride, q_batch_stride, k_batch_stride, v_batch_stride, dq_row_stride,
-                            dk_row_stride, dv_row_stride, scale, causal, 0, nullptr, 0.f, stream_);
+                            dk_row_stride, dv_row_stride, scale, causal, 0, nullptr, 0.f, nullptr, stream_);
 }

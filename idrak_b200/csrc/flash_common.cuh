@@ -26,6 +26,8 @@ struct FlashParams {
   __nv_bfloat16* dK;
   __nv_bfloat16* dV;
   long long dq_row_stride, dk_row_stride, dv_row_stride;
+  int kv_parts;        // into how many units the query heads of a key head are dealt (1: dK and dV are written directly)
+  float* kv_partial;   // [kv_parts][dV, dK][B, Skv, Hkv, D] where kv_parts > 1
 };
 
 // 2^x as one MUFU instruction (flush-to-zero, about 2 ulp): the softmax exponentials are the bulk of the element-wise

@@ -112,12 +112,14 @@ def flash_backward(dout, q, k, v, out, lse, causal=True, scale=None, grads=None,
         for g, rows in ((dq, Sq), (dk, Skv), (dv, Skv)):
             assert g.stride(3) == 1 and g.stride(2) == D and g.stride(0) == rows * g.stride(1)
     rs = _row_start_arg(row_start, B, Sq, q.device)
+    parts = lib.idrak_flash_bwd_workspace(B, H, Hkv, Sq, Skv, D, int(causal))
+    ws = torch.empty(parts, dtype=torch.float32, device=q.device) if parts else None
     rc = lib.idrak_flash_bwd_ex(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),
         delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), B, H, Hkv, Sq, Skv, D,
         q.stride(1), k.stride(1), v.stride(1), q.stride(0), k.stride(0), v.stride(0),
         dq.stride(1), dk.stride(1), dv.stride(1), float(scale), int(causal), int(window or 0), ptr(rs),
-        float(softcap or 0.0), stream_ptr())
+        float(softcap or 0.0), ptr(ws), stream_ptr())
     _native.check(rc, "idrak_flash_bwd_ex")
     return dq, dk, dv
 

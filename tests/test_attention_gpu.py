@@ -83,6 +83,36 @@ def test_flash_backward_walks_many_units(B, Sq, Skv, H, Hkv, D, causal):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("B,Sq,Skv,H,Hkv,D,causal,window,parts", [
+    (3, 515, 515, 16, 4, 64, True, None, 4),       # the last key block three keys tall
+    (3, 515, 515, 16, 4, 128, True, None, 4),
+    (1, 512, 512, 12, 4, 64, True, 100, 3),        # a group of three; key blocks that few query blocks see
+    (2, 256, 700, 8, 4, 64, False, None, 2),
+    (1, 130, 130, 4, 4, 64, True, None, 1),        # no group to deal out
+    (1, 128, 128, 2, 1, 64, True, None, 1),        # too short to be worth it
+    (8, 1024, 1024, 32, 8, 64, True, None, 1),     # units enough
+])
+def test_flash_backward_deals_the_heads_of_a_group(B, Sq, Skv, H, Hkv, D, causal, window, parts):
+    """Key blocks whose query heads go to several units: parts in fp32, summed in their order, written through row strides."""
+    from idrak_b200 import _native
+    need = _native.lib().idrak_flash_bwd_workspace(B, H, Hkv, Sq, Skv, D, int(causal))
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert need == (2 * parts * B * Skv * Hkv * D if parts > 1 else 0)
+    q, k, v = _rand((B, Sq, H, D), 1), _rand((B, Skv, Hkv, D), 2), _rand((B, Skv, Hkv, D), 3)
+    do = _rand((B, Sq, H, D), 4)
+    out, lse = ops.flash_forward(q, k, v, causal, window=window)
+    both = torch.zeros((B, Skv, 2, Hkv, D), dtype=torch.bfloat16, device="cuda")
+    dk, dv = both[:, :, 0], both[:, :, 1]
+    grads = ops.flash_backward(do, q, k, v, out, lse, causal, grads=(torch.empty_like(q), dk, dv), window=window)
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    ops.attention_reference(qr, kr, vr, causal, window=window).backward(do.float())
+    for got, want in zip(grads, (qr.grad, kr.grad, vr.grad)):
+        assert ((got.float() - want).norm() / want.norm()).item() < 2.0 ** -7      # four roundings to bf16, as above
+    again = ops.flash_backward(do, q, k, v, out, lse, causal, window=window)
+    for x, y in zip(grads, again):
+        assert torch.equal(x, y)
+
+
 MODES = [  # B, S, H, Hkv, D, window, spans, softcap
     (2, 512, 4, 4, 64, 128, None, None),
     (1, 640, 4, 2, 128, 200, None, None),
