@@ -91,15 +91,15 @@ def kernel_shapes() -> List[KernelShape]:
     return [
         KernelShape("gemm_kernel<256>", "128 x 256 x 64", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
                     "two accumulators of 256 columns ping-pong between the MMA warp and eight epilogue warps"),
-        KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128"),
+        KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128, and products that fill less than half the machine"),
         KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
                     "cta_group::2: each CTA holds half of the A rows and half of the B columns"),
         KernelShape("skinny_gemm_kernel", "128 features x (16 | 32 | 64) tokens x 64, K over a cluster of up to 8", 4, 320,
                     100352, 64, 2, "partial tiles summed through distributed shared memory"),
-        KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 100 * 1024, 256, 2, ""),
-        KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 197 * 1024, 512, 1, ""),
-        KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 160 * 1024, 320, 1, ""),
-        KernelShape("flash_bwd_kv_kernel<64>", "128 keys x 128 queries per block, persistent", 2, 320, 232192, 384, 1, ""),
+        KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 84 * 1024, 256, 2, "P in tensor memory"),
+        KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 164 * 1024, 512, 1, "P in tensor memory, two buffers"),
+        KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 114 * 1024, 512, 1, "dS in tensor memory, two buffers"),
+        KernelShape("flash_bwd_kv_kernel<64>", "128 keys x 128 queries per block, persistent", 2, 320, 166656, 512, 1, "P in tensor memory, dS in shared memory"),
         KernelShape("qgemm_kernel", "128 x 128 x 64, weights unpacked in shared memory", 4, 448, 4 * 32768 + 2048, 256, 1,
                     "eight unpacking warps"),
         KernelShape("tp_gemm_kernel", "128 x 256 x 64 with peer-memory gather / reduce-scatter", 4, 320,
