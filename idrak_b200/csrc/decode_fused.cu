@@ -120,9 +120,9 @@ __global__ void __launch_bounds__(256) norm_rope_kv_kernel(const NormRopeKvParam
 #pragma unroll
           for (int j = 0; j < PER / 2; ++j) {
             if (j < hj) {
-              // v[j + hj] with hj = 1, 2 or 4: constant indices, so that v stays in registers
+              // v[j + hj], hj any of 1 .. PER / 2 (3 for 192 of 256): constant indices, so that v stays in registers
 #pragma unroll
-              for (int o = 1; o <= PER / 2; o <<= 1) {
+              for (int o = 1; o <= PER / 2; ++o) {
                 if (o == hj && j + o < PER) {
                   const float a = v[j], b = v[j + o];
                   v[j] = a * cs[j] - b * sn[j];

@@ -111,7 +111,8 @@ def test_sampler_ties_do_not_crowd_out_larger_logits():
     assert seen <= allowed and set(big) <= seen, sorted(seen)
 
 
-@pytest.mark.parametrize("H,Hkv,Dh,rot", [(8, 2, 64, 64), (32, 8, 128, 128), (4, 4, 128, 64), (6, 2, 256, 128)])
+@pytest.mark.parametrize("H,Hkv,Dh,rot", [(8, 2, 64, 64), (32, 8, 128, 128), (4, 4, 128, 64), (6, 2, 256, 128), (6, 2, 256, 64),
+                                             (6, 2, 256, 192), (6, 2, 256, 256)])
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_fused_norm_rope_kv_write_matches_the_separate_steps(H, Hkv, Dh, rot, qk_norm):
     """One launch = query / key RMS norm + RoPE (in place on the packed projection) + paged cache write; compared with
