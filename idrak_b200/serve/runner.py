@@ -16,6 +16,7 @@ decode primitives (src/Idrak.Abstraction/Generation/Decoding.cs:243, Tensors/Ten
 from __future__ import annotations
 
 import os
+import weakref
 
 from dataclasses import dataclass
 from typing import List, Optional, Sequence
@@ -89,6 +90,8 @@ class ModelRunner:
         self.max_blocks_per_seq = (s.max_positions + block_size - 1) // block_size
         self._graphs = {}
         self._graph_pool = None
+        self._few_rows_ok = None
+        self._state = self._model_state()
         self.graph_replays = 0
 
     # ------------------------------------------------------------------ sizing
@@ -337,13 +340,36 @@ class ModelRunner:
             x = self._block(blk, x, attend)
         return self._logits(self.model.norm(x))
 
+    # ------------------------------------------------------------------ what the model holds at the moment
+    def _model_state(self) -> list:
+        """What the choice of path and a recorded decode step depend on and a program may change between calls: the blocks'
+        modules, their adapters and packed weights, folded norms. Weak references, equal only while it is the same living
+        object."""
+        ref = weakref.ref
+        state: list = [getattr(self.model, "_norms_folded", False)]
+        for blk in self.model.blocks:
+            for name in ("attn", "mlp"):
+                m = blk._modules[name]
+                state.append(ref(m))
+                adapters = m._modules.get("adapters", m.__dict__.get("adapters"))
+                state.append(adapters if adapters is None else ref(adapters))
+                state += [ref(w) for w in (m.__dict__.get("packed") or {}).values()]
+        return state
+
+    def _follow_model(self) -> None:
+        """Forgets the choice of path and the recorded decode steps when the model no longer holds what they were made for."""
+        state = self._model_state()
+        if state != self._state:
+            self._state, self._few_rows_ok = state, None
+            self._graphs, self._graph_pool = {}, None
+
     # ------------------------------------------------------------------ decode of at most 64 rows: fused projections
     def _few_row_path(self) -> bool:
         """Whether decode steps of up to 64 sequences run on the few-row kernels: one launch per projection with bias,
         residual add, gated activation and (with folded norms) the RMS norm inside it."""
-        cached = getattr(self, "_few_rows_ok", None)
-        if cached is not None:
-            return cached
+        self._follow_model()
+        if self._few_rows_ok is not None:
+            return self._few_rows_ok
         from ..ops import skinny
         from .. import _native
         s = self.spec
@@ -353,7 +379,8 @@ class ModelRunner:
               and s.gated and s.activation in skinny._KINDS and s.dim % 8 == 0 and s.ff_dim % 8 == 0
               and not s.logit_softcap)
         for blk in self.model.blocks:
-            if not ok:
+            if not ok or not isinstance(blk.mlp, FeedForward):
+                ok = False
                 break
             rope = blk.attn.rope
             packed = [w for m in (blk.attn, blk.mlp) for w in (getattr(m, "packed", None) or {}).values()]
@@ -454,6 +481,7 @@ class ModelRunner:
             ctx *= 2
         width = self.max_blocks_per_seq
         key = (bucket, ctx)
+        self._follow_model()
         entry = self._graphs.get(key)
         if entry is None:
             tok = torch.zeros(bucket, dtype=torch.int32, device=self.device)

@@ -150,3 +150,60 @@ def test_prefill_calls_the_same_kernels_as_the_modules(quant, lengths, shared):
     (a, a_all, a_cache), (b, b_all, b_cache) = results
     for x, y in [(a, b), (a_all, b_all)] + list(zip(a_cache, b_cache)):
         assert torch.equal(x, y) and x.isfinite().all()
+
+
+def _small(seed=1):
+    spec = DecoderSpec.llama(layers=2, dim=256, heads=4, kv_heads=2, ff_dim=512, vocab=500, max_positions=256, head_dim=64)
+    return build_decoder(spec, seed=seed).to("cuda", torch.bfloat16)
+
+
+def _step(model_or_runner, graphed=False):
+    """Logits of a prefill of two prompts (every token) and of the decode step after it, on a given or a fresh runner."""
+    runner = model_or_runner if isinstance(model_or_runner, ModelRunner) else ModelRunner(model_or_runner, 8, 16)
+    items = [PrefillItem(list(range(7, 27)), 0, [0, 1]), PrefillItem(list(range(40, 45)), 0, [2])]
+    every = runner.prefill(items, all_logits=True).clone()
+    last = runner.prefill(items).clone()
+    tok, pos = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([3, 4], [20, 5]))
+    table = torch.tensor([[0, 1], [2, 3]], dtype=torch.int32, device="cuda")
+    step = (runner.decode_graphed(tok, pos, table, 21) if graphed else runner.decode(tok, pos, table)).clone()
+    return every, last, step
+
+
+def _same(a, b):
+    return all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("quant", ["", "int8"])
+def test_runner_follows_adapters_that_come_and_go(quant):
+    """Adapters attached after a runner's first calls, taken off for a while, and put back: prefill, decode and recorded
+    decode steps give what a runner made at that moment gives, bit for bit."""
+    from idrak_b200.adapters.lora import add_adapters
+    from idrak_b200.quant import quantize_model
+    from idrak_b200.text.finetuning import adapters_disabled
+    model = _small()
+    if quant:
+        quantize_model(model, quant)
+    plain, graphed = ModelRunner(model, 8, 16), ModelRunner(model, 8, 16)
+    bare, bare_graphed = _step(plain), _step(graphed, True)
+    torch.manual_seed(0)
+    for p in add_adapters(model, rank=4):
+        p.data.normal_(0, 0.05)
+    adapted = _step(model)
+    assert not torch.equal(adapted[0], bare[0]) and not torch.equal(adapted[2], bare[2])
+    assert _same(_step(plain), adapted) and _same(_step(graphed, True), _step(ModelRunner(model, 8, 16), True))
+    with adapters_disabled(model):
+        assert _same(_step(plain), bare) and _same(_step(graphed, True), bare_graphed)
+        inside = ModelRunner(model, 8, 16)                  # its first call finds no adapters
+        assert _same(_step(inside), bare)
+    for r in (plain, inside):
+        assert _same(_step(r), adapted)
+
+
+@pytest.mark.parametrize("kind", ["int8", "int4", "fp8"])
+def test_runner_follows_weights_packed_after_its_first_call(kind):
+    from idrak_b200.quant import quantize_model
+    model = _small()
+    plain, graphed = ModelRunner(model, 8, 16), ModelRunner(model, 8, 16)
+    _step(plain), _step(graphed, True)
+    quantize_model(model, kind)
+    assert _same(_step(plain), _step(model)) and _same(_step(graphed, True), _step(ModelRunner(model, 8, 16), True))
