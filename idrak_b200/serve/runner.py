@@ -23,9 +23,10 @@ from typing import List, Optional, Sequence
 
 import numpy as np
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from .. import ops
-from ..models.decoder import Decoder, FeedForward, apply_rope_table, masked_attention, project
+from ..models.decoder import Decoder, FeedForward, Norm, apply_rope_table, masked_attention, project
 from ..ops import decode as dops
 
 
@@ -63,6 +64,12 @@ def fold_norms_into_projections(model: Decoder) -> bool:
         fold(model.head, model.norm)
     model._norms_folded = True
     return True
+
+
+def _plain(module, cls) -> bool:
+    """Whether calling ``module`` runs ``cls.forward`` and nothing besides (but for hooks on every module there is)."""
+    d = module.__dict__
+    return type(module) is cls and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d)
 
 
 class ModelRunner:
@@ -257,7 +264,7 @@ class ModelRunner:
                     else masked_attention(qi, ki, vi, attn.scale, window, s.attention_softcap))
             return out if out is not None else qkv2.new_empty(qkv2.shape[0], H * D)
 
-        if self.direct_prefill and self._few_row_path():
+        if self._direct_prefill():
             # the kernels of the modules' forwards, in their order, without the modules: a short prompt is bound by the host
             x = self._row_blocks(x.view(ids_t.shape[0], -1), pos_t, slots_t, attention, self._dense)
             return self._logits(self._norm(self.model.norm, x if all_logits else x[last]))
@@ -421,11 +428,24 @@ class ModelRunner:
             y = ops.gemm(x, w, bias=bias, residual=residual)
         return y if gate is None else gated_forward(y, GATE_KINDS[gate])
 
-    direct_prefill = True          # prefill calls the kernels directly (not for a subclass with its own blocks)
+    def _direct_prefill(self) -> bool:
+        """Whether prefill calls the kernels of the modules' forwards itself: the few-row path's models, as long as the modules
+        would run nothing else and the runner's own steps are the library's."""
+        cls = type(self)
+        if not (cls._block is ModelRunner._block and cls._qkv is ModelRunner._qkv and cls._out is ModelRunner._out
+                and self._few_row_path() and _plain(self.model.norm, Norm)) or _has_any_global_hook():
+            return False
+        for blk in self.model.blocks:
+            mods = blk._modules
+            if not (_plain(mods["attn_norm"], Norm) and _plain(mods["mlp_norm"], Norm) and _plain(mods["mlp"], FeedForward)):
+                return False
+        return True
 
     @staticmethod
     def _norm(layer, t):
         """A norm layer's forward without an autograd node."""
+        if not _plain(layer, Norm) or _has_any_global_hook():
+            return layer(t)
         from ..ops.rowops import norm_forward
         return norm_forward(t, layer.effective_weight(), layer.bias, layer.eps, layer.kind != "layer")[0]
 

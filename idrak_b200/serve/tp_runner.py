@@ -36,8 +36,7 @@ class TPModelRunner(ModelRunner):
         self.vocab_offset = lo
         self.vocab_local = max(0, min(hi, self.full_spec.vocabulary) - lo)      # columns of the slice that are real tokens
 
-    few_row_packed = False         # its few-row path below is written over dense slices,
-    direct_prefill = False         # and its prefill sums partial products over ranks
+    few_row_packed = False         # its few-row path below is written over dense slices
 
     def _few_row_path(self) -> bool:
         """Decode steps of up to 64 sequences on the few-row projection kernels, as on one GPU, with the row-parallel

@@ -207,3 +207,36 @@ def test_runner_follows_weights_packed_after_its_first_call(kind):
     _step(plain), _step(graphed, True)
     quantize_model(model, kind)
     assert _same(_step(plain), _step(model)) and _same(_step(graphed, True), _step(ModelRunner(model, 8, 16), True))
+
+
+def test_prefill_runs_hooks_and_replaced_modules():
+    """Hooks on norms and feed-forwards, a feed-forward that is not the library's, a runner with its own block."""
+    model = _small()
+    want, _, _ = _step(model)
+    seen = []
+    blk = model.blocks[1]
+    for m in (blk.attn_norm, blk.mlp_norm, blk.mlp, model.norm):
+        handle = m.register_forward_hook(lambda mod, args, out: seen.append(mod))
+        assert torch.equal(_step(model)[0], want)
+        assert m in seen
+        handle.remove()
+
+    class Doubled(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+        def forward(self, x, residual=None):
+            y = self.inner(x) * 2
+            return y if residual is None else y + residual
+
+    class OwnBlock(ModelRunner):
+        calls = 0
+
+        def _block(self, blk, x, attend):
+            OwnBlock.calls += 1
+            return super()._block(blk, x, attend)
+
+    assert torch.equal(_step(OwnBlock(model, 8, 16))[0], want) and OwnBlock.calls >= 2 * len(model.blocks)
+    blk.mlp = Doubled(blk.mlp)
+    assert not torch.equal(ModelRunner(model, 8, 16).prefill([PrefillItem([5, 6, 7], 0, [0])], all_logits=True), want[:3])
