@@ -186,7 +186,7 @@ def test_runner_follows_adapters_that_come_and_go(quant):
     plain, graphed = ModelRunner(model, 8, 16), ModelRunner(model, 8, 16)
     bare, bare_graphed = _step(plain), _step(graphed, True)
     torch.manual_seed(0)
-    for p in add_adapters(model, rank=4):
+    for p in add_adapters(model, rank=8):
         p.data.normal_(0, 0.05)
     adapted = _step(model)
     assert not torch.equal(adapted[0], bare[0]) and not torch.equal(adapted[2], bare[2])
