@@ -413,6 +413,7 @@ class ModelRunner:
         from ..ops.skinny import packed_linear, skinny_linear
         w, bias = getattr(owner, name + "_weight"), getattr(owner, name + "_bias")
         if w is None:
+            assert norm_eps is None, "no norm inside a product over packed weights"
             return packed_linear(x, owner.packed[name], bias, residual, gate)
         return skinny_linear(x, w, bias, residual, gate, norm_eps)
 
@@ -453,10 +454,10 @@ class ModelRunner:
         """The blocks over rows ``x [n, dim]``: (norm |) qkv | norms of q, k + RoPE + cache write | attention | out + residual
         | (norm |) gate/up, activation | down + residual. ``attention(attn, qkv, layer)`` gives ``[n, H D]`` from the packed
         projection; ``project`` is ``_few`` (at most 64 rows) or ``_dense``. With ``norm_eps`` the norms run inside the
-        projections (folded weights, ``_few`` only)."""
-        fold = {"norm_eps": norm_eps} if norm_eps is not None else {}
+        projections (folded weights, ``_few`` only) of the blocks whose weights are not packed."""
         for li, blk in enumerate(self.model.blocks):
             attn, mlp = blk.attn, blk.mlp
+            fold = {"norm_eps": norm_eps} if norm_eps is not None and attn.qkv_weight is not None else {}
             qkv = project(x if fold else self._norm(blk.attn_norm, x), attn, "qkv", **fold)
             self._rotate_and_cache(attn, qkv, positions, slots, li)
             x = project(attention(attn, qkv, li), attn, "o", residual=x)

@@ -240,3 +240,22 @@ def test_prefill_runs_hooks_and_replaced_modules():
     assert torch.equal(_step(OwnBlock(model, 8, 16))[0], want) and OwnBlock.calls >= 2 * len(model.blocks)
     blk.mlp = Doubled(blk.mlp)
     assert not torch.equal(ModelRunner(model, 8, 16).prefill([PrefillItem([5, 6, 7], 0, [0])], all_logits=True), want[:3])
+
+
+@pytest.mark.parametrize("kind", ["int8", "int4"])
+def test_packed_projections_of_a_model_with_folded_norms(kind):
+    """Norms folded into the projections, the projections packed afterwards: the few-row decode step still normalises."""
+    from idrak_b200.quant import quantize_model
+    from idrak_b200.serve.runner import fold_norms_into_projections
+    model = _small()
+    for blk in model.blocks:
+        blk.attn_norm.weight.data.uniform_(0.5, 2.0)
+    assert fold_norms_into_projections(model)
+    quantize_model(model, kind)
+    runner = ModelRunner(model, 8, 16)
+    fused = _step(runner)[2].float()
+    assert runner._few_row_path()
+    runner._few_rows_ok = False
+    plain = _step(runner)[2].float()
+    # both round activations to bf16 (2^-9) at each of the ten steps of two layers
+    assert (fused - plain).pow(2).mean().sqrt() <= 10 * 2.0 ** -9 * plain.pow(2).mean().sqrt()
