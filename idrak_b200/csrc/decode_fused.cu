@@ -160,15 +160,22 @@ __global__ void __launch_bounds__(256) norm_rope_kv_kernel(const NormRopeKvParam
 }
 
 // Where each sequence's new token goes and how long the sequence is with it: the index arithmetic at the head of a decode
-// step in one launch instead of nine.
-__global__ void decode_slots_kernel(const int* __restrict__ positions, const int* __restrict__ table, int n, int width,
-                                    int block_size, int* __restrict__ slots, int* __restrict__ lens) {
+// step in one launch instead of nine. A position outside its table row is reported in the status word; its token is not
+// cached (slot -1) and the sequence ends with the row.
+__global__ void decode_slots_kernel(const int* __restrict__ positions, const int* __restrict__ table, int n, long long stride,
+                                    int width, int block_size, int* __restrict__ slots, int* __restrict__ lens, Status* st) {
   pdl_launch_dependents();
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int pos = positions[i];
-  slots[i] = table[size_t(i) * width + pos / block_size] * block_size + pos % block_size;
+  const int pos = positions[i], block = pos / block_size;
+  if (pos < 0 || block >= width) {
+    report(st, kBadArgument, (11u << 16) | 1u, uint32_t(i));
+    slots[i] = -1;
+    lens[i] = pos < 0 ? 0 : width * block_size;
+    return;
+  }
+  slots[i] = table[i * stride + block] * block_size + pos % block_size;
   lens[i] = pos + 1;
 }
 
@@ -176,13 +183,14 @@ __global__ void decode_slots_kernel(const int* __restrict__ positions, const int
 
 using namespace idrak;
 
-// slots[i] = table[i, positions[i] / block_size] * block_size + positions[i] % block_size, lens[i] = positions[i] + 1.
-IDRAK_API int idrak_decode_slots(const int* positions, const int* table, int n, int width, int block_size, int* slots,
-                                 int* lens, void* stream_) {
+// slots[i] = table[i, positions[i] / block_size] * block_size + positions[i] % block_size, lens[i] = positions[i] + 1; the
+// table's rows hold `width` blocks and lie `stride` apart.
+IDRAK_API int idrak_decode_slots(const int* positions, const int* table, int n, long long stride, int width, int block_size,
+                                 int* slots, int* lens, void* stream_) {
   if (n <= 0) return 0;
   if (block_size <= 0 || width <= 0) return -2;
   return launch_overlapped(decode_slots_kernel, dim3(unsigned((n + 127) / 128)), 128, 0, static_cast<cudaStream_t>(stream_),
-                           positions, table, n, width, block_size, slots, lens);
+                           positions, table, n, stride, width, block_size, slots, lens, status_device_ptr());
 }
 
 // qkv rows are rotated / normalised in place; keys and values also go to the cache rows named by `slots`.

@@ -28,7 +28,7 @@ def _bind():
     _native.bind("idrak_decode_partial_floats", ll, [i, i, i, i])
     _native.bind("idrak_paged_decode_kv", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, f, i, vp])
     _native.bind("idrak_norm_rope_kv", i, [vp, ll, vp, vp, vp, vp, vp, vp, vp, vp, f, f, f, i, i, i, i, i, i, vp])
-    _native.bind("idrak_decode_slots", i, [vp, vp, i, i, i, vp, vp, vp])
+    _native.bind("idrak_decode_slots", i, [vp, vp, i, ll, i, i, vp, vp, vp])
     _native.bind("idrak_kv_write_paged", i, [vp, vp, ll, vp, vp, vp, i, i, vp])
     _native.bind("idrak_argmax_rows", i, [vp, i, i, i, ll, vp, vp])
     _native.bind("idrak_sample_rows", i, [vp, i, i, i, ll, vp, vp, vp, vp, vp, vp, vp, i, vp, vp, vp, vp, C.c_uint, vp])
@@ -38,14 +38,18 @@ def _bind():
 # --------------------------------------------------------------------------- KV cache
 def decode_slots(positions: torch.Tensor, block_table: torch.Tensor, block_size: int):
     """``(slots, lens)`` int32 of a decode step: the cache slot of every sequence's new token (at ``positions``, looked up in
-    ``block_table [n, width]``) and the sequence's length with it."""
+    ``block_table [n, width]``) and the sequence's length with it. On the GPU a position outside the table's row gives slot
+    -1, which cache writes skip, and a bad argument in the status word."""
+    if positions.is_cuda and block_table.dim() == 2 and block_table.shape[0] < positions.shape[0]:
+        raise IndexError(f"{positions.shape[0]} positions for a block table of {block_table.shape[0]} rows")
     if (positions.is_cuda and positions.dtype == torch.int32 and block_table.dtype == torch.int32
-            and positions.is_contiguous() and block_table.stride(1) == 1):
+            and block_table.device == positions.device and positions.dim() == 1 and block_table.dim() == 2
+            and positions.is_contiguous() and block_table.stride(1) == 1 and block_table.shape[1] > 0):
         _bind()
         out = torch.empty((2, positions.shape[0]), dtype=torch.int32, device=positions.device)
         rc = _native.lib().idrak_decode_slots(positions.data_ptr(), block_table.data_ptr(), positions.shape[0],
-                                              block_table.stride(0), block_size, out[0].data_ptr(), out[1].data_ptr(),
-                                              stream_ptr())
+                                              block_table.stride(0), block_table.shape[1], block_size, out[0].data_ptr(),
+                                              out[1].data_ptr(), stream_ptr())
         _native.check(rc, "idrak_decode_slots")
         return out[0], out[1]
     rows = torch.arange(positions.shape[0], device=positions.device)

@@ -206,3 +206,29 @@ def test_uneven_lengths_share_their_keys_by_the_built_in_rule(int8, Dh, hint, wi
     ref = D.paged_decode_reference(q.float(), kd, vd, table, lens_t, window=window)
     assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * 4
     assert torch.equal(out, D.paged_decode(q, kc, vc, table, lens_t, window=window, max_len_hint=hint, **scales))
+
+
+def test_decode_slots_refuses_what_indexing_refused():
+    """A table on the host or with too few rows raises; a position outside its row of the table - also of a table that is a
+    part of a wider one - gets no slot, shortens the sequence to its row and is reported."""
+    from idrak_b200 import _native
+    wide = torch.arange(100, 140, dtype=torch.int32, device="cuda").view(5, 8)
+    table = wide[:, 2:5]
+    pos = torch.tensor([0, 15, 47, 48, -1], dtype=torch.int32, device="cuda")
+    slots, lens = D.decode_slots(pos[:3], table[:3], 16)
+    want = [102 * 16, 110 * 16 + 15, 120 * 16 + 15]
+    assert slots.tolist() == want and lens.tolist() == [1, 16, 48]
+    _native.check_status("in range")
+    slots, lens = D.decode_slots(pos, table, 16)
+    assert slots.tolist() == want + [-1, -1] and lens.tolist() == [1, 16, 48, 48, 0]
+    with pytest.raises(_native.NativeError, match="bad argument"):
+        _native.check_status("slots")
+    with pytest.raises(RuntimeError):
+        D.decode_slots(pos[:3], table[:3].cpu(), 16)
+    with pytest.raises(IndexError):
+        D.decode_slots(pos, table[:4], 16)
+    for other in (pos[:3].long(), pos[:3].repeat_interleave(2)[::2]):
+        slots, lens = D.decode_slots(other, table, 16)
+        assert slots.tolist() == want and lens.tolist() == [1, 16, 48]
+    empty = D.decode_slots(pos[:0], table, 16)
+    assert empty[0].numel() == 0 and empty[1].numel() == 0
