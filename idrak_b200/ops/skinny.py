@@ -48,14 +48,23 @@ def supported(x: torch.Tensor, w: torch.Tensor, gate: Optional[str] = None) -> b
             and (gate is None or (gate in _KINDS and (w.shape[0] // 2) % 8 == 0)))
 
 
+def _readable(M: int, N: int, outputs: int, bias, residual, out) -> bool:
+    """Whether the few-row kernels read this bias and residual and write this result: bf16, whole, rows of unit stride."""
+    bf16 = torch.bfloat16
+    return ((bias is None or (bias.dtype == bf16 and bias.numel() == outputs))
+            and all(t is None or (t.dtype == bf16 and t.shape == (M, N) and t.stride(1) == 1) for t in (residual, out)))
+
+
 def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                   residual: Optional[torch.Tensor] = None, gate: Optional[str] = None,
                   norm_eps: Optional[float] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x [M <= 64, K]``, ``w [N, K]`` (or ``[2 ff, K]`` with ``gate``) -> ``[M, N]`` (``[M, ff]``)."""
     if not supported(x, w, gate):
-        return skinny_reference(x, w, bias, residual, gate, norm_eps)
+        y = skinny_reference(x, w, bias, residual, gate, norm_eps)
+        return y if out is None else out.copy_(y)
     M, K = x.shape
     N = w.shape[0] // 2 if gate is not None else w.shape[0]
+    assert _readable(M, N, w.shape[0], bias, residual, out), "bias, residual and out are bf16 matrices of the result's shape"
     if out is None:
         out = torch.empty((M, N), dtype=x.dtype, device=x.device)
     rc = _native.lib().idrak_skinny_gemm(
@@ -71,17 +80,31 @@ def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
 # Measured at 32 / 64 activation rows, us, few-row against dense: 28672 x 4096 41 / 45 against 47 / 48, 50304 x 768 21.5 / 25.2
 # against 22.7 / 23.5, 128256 x 4096 165 / 181 against 177 / 179.
 DENSE_FROM_ROWS, DENSE_ABOVE_ROWS = 49152, 32
+# From this many weight rows on, a call that the few-row kernel does not take (more than 64 rows, another gate, an fp32 result)
+# runs on the dense GEMM, and below it as the fp32 statement, whose gated pair is not rounded before the activation.
+WIDE_ROWS = 12288
 
 
 def few_row_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                    residual: Optional[torch.Tensor] = None, gate: Optional[str] = None,
                    norm_eps: Optional[float] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """A decode-sized product on whichever of the two kernels measured faster for the weight's size: the few-row cluster
-    kernel (fused epilogues) or, for a very wide plain product of more rows, the dense GEMM."""
-    if (norm_eps is None and gate is None and w.shape[0] >= DENSE_FROM_ROWS and x.shape[0] > DENSE_ABOVE_ROWS
-            and x.is_cuda):
+    kernel (fused epilogues) or, for a very wide plain product of more rows, the dense GEMM. The dense GEMM (and the activation
+    kernel) also take a wide product that the few-row kernel does not. A folded norm (``norm_eps``) exists only in the few-row
+    kernel."""
+    M, rows = x.shape[0], w.shape[0]
+    N = rows // 2 if gate is not None else rows
+    if (norm_eps is None and rows >= WIDE_ROWS and supported(x[:MAX_ROWS], w) and (gate is None or N % 8 == 0)
+            and (M > (DENSE_ABOVE_ROWS if gate is None and rows >= DENSE_FROM_ROWS else MAX_ROWS)
+                 or not supported(x, w, gate) or not _readable(M, N, rows, bias, residual, out))):
         from .gemm import gemm
-        return gemm(x, w, bias=bias, residual=residual, out=out)
+        if gate is None:
+            return gemm(x, w, bias=bias, residual=residual, out=out)
+        from .rowops import gated_activation
+        y = gated_activation(gemm(x, w, bias=bias), gate)
+        if residual is not None:
+            y = y + residual
+        return y if out is None else out.copy_(y)
     return skinny_linear(x, w, bias, residual, gate, norm_eps, out)
 
 

@@ -1,0 +1,49 @@
+"""``few_row_linear`` and ``skinny_linear`` outside the few-row kernels' own range: which kernel answers, and what is refused."""
+import pytest
+import torch
+
+from idrak_b200.ops import gemm
+from idrak_b200.ops.rowops import gated_activation
+from idrak_b200.ops.skinny import few_row_linear, skinny_linear
+
+pytestmark = pytest.mark.gpu
+
+
+def _rand(*shape, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(*shape, generator=g, device="cuda").to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("M,N", [(65, 12288), (300, 12800), (65, 49152)])
+def test_more_rows_than_the_few_row_kernel_takes_go_to_the_dense_one(M, N):
+    x, w, b, r = _rand(M, 64, seed=1), _rand(N, 64, seed=2), _rand(N, seed=3), _rand(M, N, seed=4)
+    assert torch.equal(few_row_linear(x, w, b, r), gemm(x, w, bias=b, residual=r))
+    assert torch.equal(few_row_linear(x[:9], w, b, gate="tanh"), gated_activation(gemm(x[:9], w, bias=b), "tanh"))
+    gated = gated_activation(gemm(x, w, bias=b), "silu")
+    half = r[:, : N // 2].contiguous()
+    assert torch.equal(few_row_linear(x, w, b, gate="silu"), gated)
+    out = torch.empty_like(half)
+    assert few_row_linear(x, w, b, half, "silu", out=out) is out and torch.equal(out, gated + half)
+
+
+@pytest.mark.parametrize("N", [264, 12288])
+def test_results_go_where_they_were_asked_for(N):
+    """fp32 results of a wide product as the dense kernel gives them, a destination also where the kernel does not take the
+    call, and types that the kernels do not read are refused."""
+    x, w = _rand(5, 64, seed=1), _rand(N, 64, seed=2)
+    want = x.float() @ w.float().t()
+    out = torch.full((5, N), float("nan"), device="cuda")
+    if N >= 12288:
+        few_row_linear(x, w, out=out)
+        assert (out - want).abs().max() <= 1e-4
+    else:
+        with pytest.raises(AssertionError):
+            skinny_linear(x, w, out=out)
+    odd = _rand(5, 67, seed=3)[:, 1:65]                        # rows that start on two-byte boundaries
+    dst = torch.zeros(5, N, dtype=torch.bfloat16, device="cuda")
+    assert skinny_linear(odd, w, out=dst) is dst
+    assert (dst.float() - odd.float() @ w.float().t()).abs().max() <= 2.0 ** -8 * 64
+    for bad in ({"bias": torch.zeros(N, device="cuda")}, {"bias": _rand(N - 1)}, {"residual": torch.zeros(5, N, device="cuda")},
+                {"residual": _rand(4, N)}):
+        with pytest.raises(AssertionError):
+            few_row_linear(x, w, **bad)
