@@ -52,12 +52,13 @@ struct SkinnyOut {
   int ldr;
   int M, N;                      // N = output features (gated: ff)
   int gate_kind;                 // -1: plain; else 0 silu, 1 gelu (tanh), 2 relu
-  int up_offset;                 // gated: first up feature of the weight
+  int up_offset;                 // gated: the weight's first up feature
+  int up_index;                  // gated: its bias and int8 scale
 };
 
 // The end of a few-row product: each of the `csize` CTAs of a cluster holds the partial tile part[token][F] (rows kLd
 // floats apart) of its K range; this CTA finishes the tokens rank, rank + csize, ...: it sums the partials in rank order
-// through distributed shared memory, four features per 16-byte load, multiplies by factor(token, weight row) and runs the
+// through distributed shared memory, four features per 16-byte load, multiplies by factor(token, output) and runs the
 // epilogue. Gated: features [0, F / 2) are gate, [F / 2, F) their up features. t = 0 .. 255. The cluster has met before.
 template <int F, int kLd, class Factor>
 __device__ __forceinline__ void sk_finish(const SkinnyOut& o, const float* part, int csize, int rank, int tile, int t,
@@ -96,8 +97,8 @@ __device__ __forceinline__ void sk_finish(const SkinnyOut& o, const float* part,
       v[e] *= factor(m, n);
       if (o.bias) v[e] += __bfloat162float(o.bias[n]);
       if (gated) {
-        u[e] *= factor(m, o.up_offset + n);
-        if (o.bias) u[e] += __bfloat162float(o.bias[o.up_offset + n]);
+        u[e] *= factor(m, o.up_index + n);
+        if (o.bias) u[e] += __bfloat162float(o.bias[o.up_index + n]);
         v[e] = sk_gate(v[e], o.gate_kind) * u[e];
       }
       if (o.residual) v[e] += __bfloat162float(o.residual[size_t(m) * o.ldr + n]);

@@ -430,7 +430,7 @@ IDRAK_API int idrak_skinny_gemm(const void* X, int ldx, const void* W, int ldw, 
   SkinnyParams p{};
   p.X = static_cast<const __nv_bfloat16*>(X); p.ldx = ldx; p.K = K;
   p.o = {static_cast<__nv_bfloat16*>(C), ldc, static_cast<const __nv_bfloat16*>(bias),
-         static_cast<const __nv_bfloat16*>(residual), ldr, M, N, gated ? gate_kind : -1, gated ? N : 0};
+         static_cast<const __nv_bfloat16*>(residual), ldr, M, N, gated ? gate_kind : -1, gated ? N : 0, gated ? N : 0};
   p.norm_eps = norm_eps;
   p.st = status_device_ptr();
   const int NT = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
@@ -451,13 +451,14 @@ IDRAK_API int idrak_skinny_gemm(const void* X, int ldx, const void* W, int ldw, 
 // them, and C = act(x Wg) * (x Wu)): bits = 8, one code per byte (ld bytes per row) and one fp16 scale per output, or
 // bits = 4, eight codes per 32-bit word (ld bytes per row) and one fp16 scale per 32 inputs and output (scale_ld per group
 // row). M <= 64, K a multiple of 16 (int8) or 32 (int4); rows of X, codes and int4 scales start on 16-byte boundaries, and
-// so does a gated weight's up half (N % 16 == 0, int4: N % 32 == 0). Returns 0, a CUDA error, or a negative argument error.
+// so does a gated weight's up half, which starts at column up_col of the codes: N, or for int8 codes whose halves are padded
+// a multiple of 16 past it (scales and bias are not padded). Returns 0, a CUDA error, or a negative argument error.
 //
 // Up to 16 tokens the register kernel (skinny_packed.cu) is the faster one, above them this file's, whose tensor cores take
 // 64 tokens at the price of 16: 4096 x 28672 int8, us, register / this kernel at 16 tokens 33 / 57, at 64 tokens 97 / 61.
 IDRAK_API int idrak_skinny_packed(const void* X, int ldx, const void* codes, int ld, const void* scales, int scale_ld,
                                   int bits, void* C, int ldc, int M, int N, int K, const void* bias, const void* residual,
-                                  int ldr, int gate_kind, void* stream_) {
+                                  int ldr, int gate_kind, int up_col, void* stream_) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 64) return -2;
   if (bits != 8 && bits != 4) return -7;
@@ -466,12 +467,13 @@ IDRAK_API int idrak_skinny_packed(const void* X, int ldx, const void* codes, int
   if (gate_kind > 2) return -5;
   const bool gated = gate_kind >= 0;
   const int outputs = gated ? 2 * N : N;
-  if (gated && (N % (bits == 8 ? 16 : 32))) return -6;
-  if ((long long)ld * (8 / bits) < outputs || scale_ld < outputs) return -8;
+  if (gated && (up_col % (bits == 8 ? 16 : 32) || up_col < N || (bits == 4 && up_col != N))) return -6;
+  if ((long long)ld * (8 / bits) < (gated ? up_col + N : N) || scale_ld < outputs) return -8;
   if (bits == 4 && ((scale_ld & 7) || (reinterpret_cast<uintptr_t>(scales) & 15))) return -9;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   const SkinnyOut o = {static_cast<__nv_bfloat16*>(C), ldc, static_cast<const __nv_bfloat16*>(bias),
-                       static_cast<const __nv_bfloat16*>(residual), ldr, M, N, gated ? gate_kind : -1, gated ? N : 0};
+                       static_cast<const __nv_bfloat16*>(residual), ldr, M, N, gated ? gate_kind : -1, gated ? up_col : 0,
+                       gated ? N : 0};
   if (M <= kSkinnyRegisterRows)
     return skinny_packed_registers(static_cast<const __nv_bfloat16*>(X), ldx, codes, ld, static_cast<const __half*>(scales),
                                    scale_ld, bits, K, o, stream);

@@ -143,7 +143,9 @@ def packed_linear(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, resid
     they are stored and expand them on the way to the tensor cores."""
     M, K = x.shape
     n_out = w.cols // 2 if gate is not None else w.cols
-    codes = w.tma_codes() if w.bits == 8 else w.codes
+    codes, up_col = w.codes, n_out
+    if w.bits == 8:
+        codes, up_col = w.gate_codes() if gate is not None else (w.tma_codes(), 0)
     if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16:
         x = x.clone(memory_format=torch.contiguous_format)
     if out is None:
@@ -156,15 +158,16 @@ def packed_linear(x: torch.Tensor, w, bias: Optional[torch.Tensor] = None, resid
     rc = _native.lib().idrak_skinny_packed(x.data_ptr(), x.stride(0), codes.data_ptr(), codes.stride(0) * codes.element_size(),
                                            w.scales.data_ptr(), w.scale_ld, w.bits, out.data_ptr(), out.stride(0), M, n_out, K,
                                            ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0,
-                                           _KINDS[gate] if gate is not None else -1, stream_ptr())
+                                           _KINDS[gate] if gate is not None else -1, up_col, stream_ptr())
     _native.check(rc, "idrak_skinny_packed")
     return out
 
 
 def skinny8_linear(x: torch.Tensor, w8, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
                    gate: Optional[str] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``packed_linear`` over an int8 weight, or its fp32 statement where the kernels do not take the call."""
-    if packed_supported(x, w8, gate):
+    """``packed_linear`` over an int8 weight - also a gated one whose up half starts between 16-byte boundaries (a multiple of
+    8 outputs), from a padded copy of the codes - or its fp32 statement where the kernels do not take the call."""
+    if packed_supported(x, w8, gate) or (gate in _KINDS and w8.cols % 16 == 0 and packed_supported(x, w8)):
         return packed_linear(x, w8, bias, residual, gate, out)
     res = skinny8_reference(x, w8, bias, residual, gate)
     if out is not None:

@@ -87,6 +87,20 @@ class Int8Weight:
             self._tma_codes = t
         return t
 
+    def gate_codes(self):
+        """``(codes, first up column)`` of a stacked ``[gate | up]`` weight with both halves on 16-byte boundaries: the codes
+        themselves, or where the half width is not a multiple of 16 a copy with padded halves, made on first use and kept."""
+        half = self.cols // 2
+        if half % 16 == 0:
+            return self.tma_codes(), half
+        pad = (half + 15) // 16 * 16
+        t = getattr(self, "_gate_codes", None)
+        if t is None or t.device != self.codes.device:
+            t = torch.zeros((self.rows, 2 * pad), dtype=torch.int8, device=self.codes.device)
+            t.view(self.rows, 2, pad)[:, :, :half] = self.codes[:, : 2 * half].unflatten(1, (2, half))
+            self._gate_codes = t
+        return t, pad
+
     @property
     def ld(self) -> int:
         return self.codes.stride(0)

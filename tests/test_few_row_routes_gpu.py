@@ -1,10 +1,12 @@
-"""``few_row_linear`` and ``skinny_linear`` outside the few-row kernels' own range: which kernel answers, and what is refused."""
+"""``few_row_linear``, ``skinny_linear`` and ``skinny8_linear`` outside the few-row kernels' own range: which kernel answers, and what is refused."""
 import pytest
 import torch
 
+from idrak_b200 import _native
 from idrak_b200.ops import gemm
 from idrak_b200.ops.rowops import gated_activation
-from idrak_b200.ops.skinny import few_row_linear, skinny_linear
+from idrak_b200.ops.skinny import few_row_linear, skinny8_linear, skinny_linear
+from idrak_b200.quant.weights import Int8Weight
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +49,21 @@ def test_results_go_where_they_were_asked_for(N):
                 {"residual": _rand(4, N)}):
         with pytest.raises(AssertionError):
             few_row_linear(x, w, **bad)
+
+
+@pytest.mark.parametrize("M", [3, 20])
+@pytest.mark.parametrize("ff", [24, 1000])
+def test_int8_gate_whose_halves_start_between_16_byte_boundaries(M, ff):
+    """The up half of the codes starts 8 bytes past a 16-byte boundary: the kernel answers all the same."""
+    x, b, r = _rand(M, 128, seed=1), _rand(2 * ff, seed=2), _rand(M, ff, seed=3)
+    w = Int8Weight.quantize(torch.randn(128, 2 * ff, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda") * 0.05)
+    skinny8_linear(x, w, b, r, "silu")
+    before = _native.lib().idrak_launch_count()
+    got = skinny8_linear(x, w, b, r, "silu")
+    assert _native.lib().idrak_launch_count() == before + 1
+    y = x.double() @ w.dequantize().double() + b.double()
+    a, u = y.chunk(2, -1)
+    want = torch.nn.functional.silu(a) * u + r.double()
+    # one rounding to bf16, fp32 sums of 128 terms and the fp32 activation
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+    _native.check_status("gated int8 product")
