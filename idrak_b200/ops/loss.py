@@ -45,9 +45,11 @@ def softmax_xent_(logits: torch.Tensor, targets: torch.Tensor, vocab: int, grad_
 
 
 def _scaled(x: torch.Tensor, scale: torch.Tensor, dtype: torch.dtype, out: torch.Tensor | None = None) -> torch.Tensor:
-    """``(x * scale).to(dtype)`` with a device scalar, in one pass for bf16 results outside a recorded backward."""
+    """``(x * scale).to(dtype)`` with a device scalar, in one pass for bf16 results outside a recorded backward and outside
+    vmap (several upstream gradients at once are one tensor without an address)."""
     if (dtype == torch.bfloat16 and x.dtype in (torch.float32, torch.bfloat16) and x.is_cuda and x.is_contiguous()
-            and not torch.is_grad_enabled() and x.data_ptr() % 16 == 0
+            and not torch.is_grad_enabled() and torch._C._has_storage(scale)
+            and scale.numel() == 1 and scale.device == x.device and x.data_ptr() % 16 == 0
             and (out is None or (out.is_contiguous() and out.data_ptr() % 16 == 0 and out.dtype == dtype))):
         out = torch.empty_like(x, dtype=dtype) if out is None else out
         scale = scale.float()

@@ -129,3 +129,16 @@ def test_fused_sgd_momentum():
         p.grad, r.grad = g.to(torch.bfloat16), g.to(torch.bfloat16).float()
         opt.step(); ropt.step()
     assert (opt.master[0] - r).abs().max().item() < 1e-5
+
+
+def test_token_cross_entropy_batched_upstream_gradients():
+    """Several upstream gradients at once (``is_grads_batched``): each row is the gradient times its factor."""
+    h, w = _rand((77, 64), 1.0, 1).requires_grad_(), _rand((264, 64), 0.1, 2).requires_grad_()
+    t = torch.randint(0, 264, (77,), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    loss = ops.token_cross_entropy(h, w, t, vocab=264, chunk_rows=None, ignore_index=None)
+    one = torch.autograd.grad(loss, [h, w], retain_graph=True)
+    factors = torch.tensor([1.0, 2.0, -0.5], device="cuda", dtype=loss.dtype)
+    many = torch.autograd.grad(loss, [h, w], grad_outputs=factors, is_grads_batched=True)
+    for g, batch in zip(one, many):
+        for k, f in enumerate((1.0, 2.0, -0.5)):
+            assert torch.equal(batch[k], g * f)               # powers of two: exact
