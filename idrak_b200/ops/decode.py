@@ -162,6 +162,29 @@ def paged_decode_reference(q, k_cache, v_cache, block_table, seq_lens, scale=Non
     return out.to(q.dtype)
 
 
+DECODE_TILE, DECODE_CTAS = 32, 16384
+
+
+def key_shares(seqs: int, kv_heads: int, longest: int, window: int = 0):
+    """``(splits, min_keys)`` of a decode step: by how many CTAs per KV head a sequence's keys are shared at most, and how many
+    keys a share has at least, from a bound on the lengths alone (a power of two above the longest).
+
+    Shares of 128 keys (one tile per warp) to 1024: short ones so that few sequences fill the machine, long ones where there are
+    CTAs enough, since a CTA costs about as much as 200 keys of a busy machine. 1024 CTAs if every sequence had the bound.
+    Measured, us, shares of 128 / 512 / 1024 / unsplit: 1 sequence 9.8 / 11.8 / 11.8 / 11.8, 16 of 128 to 2304 tokens 41 / 28.5 /
+    40 / 51, 64 of those 145 / 91 / 84 / 95.
+
+    At most 64 shares, and 16384 CTAs in all: each has a partial result in HBM and is launched whether its sequence reaches it or
+    not. With less a long sequence's share is longer. 256 sequences of 8 KV heads under a bound of 32768, us, unsplit / 4 / 8 /
+    32 shares: one of 32000 tokens and the others of 300 717 / 294 / 212 / 199, all of 300 94 / 101 / 110 / 161 (136 MB of partial
+    results at 32 query heads of 128, 34 at 8 shares)."""
+    if window > 0:
+        longest = min(longest, window + DECODE_TILE)       # a window may start inside a tile
+    heads = max(seqs * kv_heads, 1)
+    min_keys = max(128, min(1024, (longest * heads // 1024 + 127) // 128 * 128))
+    return max(1, min((longest + min_keys - 1) // min_keys, 64, DECODE_CTAS // heads)), min_keys
+
+
 def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
                  seq_lens: torch.Tensor, scale: Optional[float] = None, window: int = 0,
                  splits: Optional[int] = None, max_len_hint: Optional[int] = None,
@@ -177,13 +200,7 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     lib = _native.lib()
     min_keys = 0
     if splits is None:
-        # Shares of 128 keys (one tile per warp) to 1024: short ones so that few sequences fill the machine, long ones where
-        # there are CTAs enough, since a CTA costs about as much as 200 keys of a busy machine. 1024 CTAs if every sequence
-        # had the bound on the lengths (a power of two above them). Measured, us, shares of 128 / 512 / 1024 / unsplit:
-        # 1 sequence 9.8 / 11.8 / 11.8 / 11.8, 16 of 128 to 2304 tokens 41 / 28.5 / 40 / 51, 64 of those 145 / 91 / 84 / 95
-        longest = max_len_hint if max_len_hint is not None else block_table.shape[1] * bs
-        min_keys = max(128, min(1024, (longest * seqs * Hkv // 1024 + 127) // 128 * 128))
-        splits = max(1, min((longest + min_keys - 1) // min_keys, 64))
+        splits, min_keys = key_shares(seqs, Hkv, max_len_hint if max_len_hint is not None else block_table.shape[1] * bs, window)
     out = torch.empty(seqs, H, D, dtype=q.dtype, device=q.device)
     part = None
     if splits > 1:
