@@ -136,6 +136,7 @@ _SIGNATURES = {
     "idrak_flash_bwd_ex": (c_int, [c_void_p] * 10 + [c_int] * 6 + [c_ll] * 9 + [c_float, c_int, c_int, c_void_p,
                                                                                c_float, c_void_p, c_void_p]),
     "idrak_flash_bwd_workspace": (c_ll, [c_int] * 7),
+    "idrak_flash_bwd_workspace_ex": (c_ll, [c_int] * 9),
 }
 
 

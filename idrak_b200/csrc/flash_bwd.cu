@@ -955,19 +955,27 @@ __global__ void __launch_bounds__(256) flash_kv_parts_kernel(const FlashParams p
   *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]), pack_bf16x2(a[4], a[5]), pack_bf16x2(a[6], a[7]));
 }
 
+// Query blocks that key block kb meets, as kv_unit walks them.
+static int kv_seen(int kb, int nq, int off, int causal, int window) {
+  const int first = causal ? max(0, (kb * 128 - off) / 128) : 0;
+  int last = nq;
+  if (causal && window > 0) last = min(last, (kb * 128 + 127 + window - 1 - off) / 128 + 1);
+  return max(0, last - first);
+}
+
 // Into how many units the query heads of a key head are dealt. One unit walks every query head of its key block, so with
 // grouped heads there are few units and the first key block's, which under a causal mask every query block sees, is longer
 // than a CTA's fair share: 3 x 999 tokens with 16 heads on 4 has 96 units of up to 32 blocks for 148 SMs, against 12 blocks
-// a SM if they were even. The smallest divisor of the group that brings the longest unit to a quarter over the fair share
-// is taken; the parts leave as fp32 and are summed in their order. A unit of under four blocks is not worth the extra pass.
-// Measured, causal, size 64: 2 x 2048 tokens, 16 heads on 4: 142 -> 78 + 4 us for the sum; with 8192 tokens the units are
-// even enough and stay whole.
-static int kv_parts_of(int B, int H, int Hkv, int Sq, int Skv, int causal) {
+// a SM if they were even. Measured, causal, size 64: 2 x 2048 tokens, 16 heads on 4: 142 -> 78 + 4 us for the sum; with 8192
+// tokens the units are even enough and stay whole.
+//
+// The most parts worth a look: the smallest divisor of the group that brings the longest unit to a quarter over the fair share.
+static int kv_parts_bound(int B, int H, int Hkv, int Sq, int Skv, int causal) {
   const int group = H / Hkv, nq = (Sq + 127) / 128, nkb = (Skv + 127) / 128, off = Skv - Sq;
   long long blocks = 0;
   int longest = 0;
   for (int kb = 0; kb < nkb; ++kb) {
-    const int first = causal ? max(0, (kb * 128 - off) / 128) : 0, seen = max(0, nq - first);
+    const int seen = kv_seen(kb, nq, off, causal, 0);
     blocks += seen;
     longest = max(longest, seen);
   }
@@ -978,6 +986,45 @@ static int kv_parts_of(int B, int H, int Hkv, int Sq, int Skv, int causal) {
     do ++parts; while (group % parts);
   }
   return parts;
+}
+// Of the divisors up to that, the one with the least estimated time: 2.1 us for each block of the busiest CTA as the units are
+// handed out and, for more than one part, 0.4 us per MB of fp32 sums written and read again and 4.5 us for the launch that adds
+// them up. Fitted to 140 shapes of 130 to 8192 tokens, head sizes 64 and 128, with and without windows: the choices come within
+// 0.2 % of the best parts on average, and are never more than 4 % slower than whole units (the bound alone: up to 48 %).
+// Measured, us, dealt / whole: 8 x 130 tokens, 32 heads on 8, size 128: 71 / 62, 4 x 256 queries on 700 keys, 8 on 4: 62 / 44, a
+// window of 256 over 2048, 32 on 8: 130 / 110 (whole by the estimate); 2048 tokens, 16 on 4: 114 / 202, with the window 79 / 85.
+// Sequences packed into a row make units shorter by what only the device knows: dealt only where the estimate for one sequence
+// is a third of the whole one, from where on nothing measured slower. Eight sequences in 2048 tokens, 32 on 8, size 128:
+// 108 / 87, in 8192, 8 on 1: 198 / 271.
+static int kv_parts_of(int B, int H, int Hkv, int Sq, int Skv, int D, int causal, int window, bool packed) {
+  const int bound = kv_parts_bound(B, H, Hkv, Sq, Skv, causal);
+  if (bound == 1) return 1;
+  const int group = H / Hkv, nq = (Sq + 127) / 128, nkb = (Skv + 127) / 128, off = Skv - Sq, sms = sm_count();
+  int best = 1;
+  double best_us = 0.0, whole_us = 0.0;
+  for (int parts = 1; parts <= bound; ++parts) {
+    if (group % parts) continue;
+    const int per_kb = Hkv * B * parts;
+    const long long units = (long long)nkb * per_kb;
+    const int ctas = int(units < sms ? units : sms);
+    long long busiest = 0;
+    for (int c = 0; c < ctas; ++c) {                                       // snake_unit
+      long long mine = 0;
+      for (long long round = 0; round * ctas < units; ++round) {
+        const long long u = round * ctas + ((round & 1) ? (ctas - 1 - c) : c);
+        if (u < units) mine += kv_seen(int(u / per_kb), nq, off, causal, window);
+      }
+      busiest = max(busiest, mine);
+    }
+    double us = double(busiest) * (group / parts) * 2.1;
+    if (parts == 1) whole_us = us;
+    else us += 4.5 + 0.4e-6 * 8.0 * parts * B * Skv * Hkv * D;
+    if (parts == 1 || us < best_us) {
+      best = parts;
+      best_us = us;
+    }
+  }
+  return packed && 3.0 * best_us > whole_us ? 1 : best;
 }
 
 template <int D, bool MODES>
@@ -1012,10 +1059,16 @@ static int launch_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
 
 using namespace idrak;
 
-// fp32 elements of workspace a backward call of these sizes needs (0: none).
+// fp32 elements of workspace a backward call of these sizes needs (0: none); packed: with row_start. The form without a window
+// is enough for any.
+IDRAK_API long long idrak_flash_bwd_workspace_ex(int B, int H, int Hkv, int Sq, int Skv, int D, int causal, int window, int packed) {
+  if (B <= 0 || Hkv <= 0 || H <= 0 || H % Hkv) return 0;
+  const int parts = kv_parts_of(B, H, Hkv, Sq, Skv, D, causal, window, packed != 0);
+  return parts > 1 ? 2LL * parts * B * Skv * Hkv * D : 0;
+}
 IDRAK_API long long idrak_flash_bwd_workspace(int B, int H, int Hkv, int Sq, int Skv, int D, int causal) {
   if (B <= 0 || Hkv <= 0 || H <= 0 || H % Hkv) return 0;
-  const int parts = kv_parts_of(B, H, Hkv, Sq, Skv, causal);
+  const int parts = kv_parts_bound(B, H, Hkv, Sq, Skv, causal);
   return parts > 1 ? 2LL * parts * B * Skv * Hkv * D : 0;
 }
 
@@ -1024,7 +1077,7 @@ IDRAK_API long long idrak_flash_bwd_workspace(int B, int H, int Hkv, int Sq, int
 // their batch stride is rows * row stride.
 // window > 0 and row_start (one int per query row, [B, Sq]) restrict the keys a query sees exactly as in the forward
 // entry point; both need `causal`. `softcap` > 0 differentiates through the tanh cap of the forward.
-// workspace: idrak_flash_bwd_workspace fp32 elements on a 16-byte boundary, or null (the heads of a group then stay together).
+// workspace: idrak_flash_bwd_workspace_ex fp32 elements on a 16-byte boundary, or null (the heads of a group then stay together).
 IDRAK_API int idrak_flash_bwd_ex(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                  const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int H, int Hkv,
                                  int Sq, int Skv, int D, long long q_row_stride, long long k_row_stride,
@@ -1048,7 +1101,7 @@ IDRAK_API int idrak_flash_bwd_ex(const void* q, const void* k, const void* v, co
     if (rc) return rc;
   }
   FlashParams p;
-  p.kv_parts = workspace ? kv_parts_of(B, H, Hkv, Sq, Skv, causal) : 1;
+  p.kv_parts = workspace ? kv_parts_of(B, H, Hkv, Sq, Skv, D, causal, window, row_start != nullptr) : 1;
   p.kv_partial = workspace;
   p.O = nullptr;
   p.o_row_stride = 0;

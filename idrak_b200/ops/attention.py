@@ -112,7 +112,7 @@ def flash_backward(dout, q, k, v, out, lse, causal=True, scale=None, grads=None,
         for g, rows in ((dq, Sq), (dk, Skv), (dv, Skv)):
             assert g.stride(3) == 1 and g.stride(2) == D and g.stride(0) == rows * g.stride(1)
     rs = _row_start_arg(row_start, B, Sq, q.device)
-    parts = lib.idrak_flash_bwd_workspace(B, H, Hkv, Sq, Skv, D, int(causal))
+    parts = lib.idrak_flash_bwd_workspace_ex(B, H, Hkv, Sq, Skv, D, int(causal), int(window or 0), int(rs is not None))
     ws = torch.empty(parts, dtype=torch.float32, device=q.device) if parts else None
     rc = lib.idrak_flash_bwd_ex(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), lse.data_ptr(),

@@ -113,6 +113,37 @@ def test_flash_backward_deals_the_heads_of_a_group(B, Sq, Skv, H, Hkv, D, causal
         assert torch.equal(x, y)
 
 
+def _parts(B, Sq, Skv, H, Hkv, D, causal, window, packed):
+    from idrak_b200 import _native
+    need = _native.lib().idrak_flash_bwd_workspace_ex(B, H, Hkv, Sq, Skv, D, int(causal), window or 0, int(packed))
+    assert need <= _native.lib().idrak_flash_bwd_workspace(B, H, Hkv, Sq, Skv, D, int(causal))
+    return need // (2 * B * Skv * Hkv * D) or 1
+
+
+@pytest.mark.parametrize("B,Sq,Skv,H,Hkv,D,causal,window,packed,parts", [
+    (4, 256, 700, 8, 4, 128, False, None, False, 1),     # dealt 62 us, whole 44
+    (8, 130, 130, 32, 8, 128, True, None, False, 1),
+    (1, 2048, 2048, 32, 8, 128, True, 256, False, 1),    # units that a window has evened out
+    (1, 2048, 2048, 16, 4, 128, True, 256, False, 2),
+    (1, 2048, 2048, 16, 4, 128, True, None, False, 4),
+    (1, 2048, 2048, 16, 4, 128, True, None, True, 1),    # lengths that only the device knows
+    (1, 1024, 1024, 8, 1, 64, True, 200, False, 8),
+    (1, 640, 640, 16, 1, 64, True, None, True, 16),
+])
+def test_flash_backward_deals_where_that_is_faster(B, Sq, Skv, H, Hkv, D, causal, window, packed, parts):
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _parts(B, Sq, Skv, H, Hkv, D, causal, window, packed) == parts
+    q, k, v = _rand((B, Sq, H, D), 1), _rand((B, Skv, Hkv, D), 2), _rand((B, Skv, Hkv, D), 3)
+    do = _rand((B, Sq, H, D), 4)
+    rs = ops.row_starts_from_spans([(0, 70), (70, 300), (300, Sq)], B, Sq, "cuda") if packed else None
+    out, lse = ops.flash_forward(q, k, v, causal, window=window, row_start=rs)
+    grads = ops.flash_backward(do, q, k, v, out, lse, causal, window=window, row_start=rs)
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    ops.attention_reference(qr, kr, vr, causal, window=window, row_start=rs).backward(do.float())
+    for got, want in zip(grads, (qr.grad, kr.grad, vr.grad)):
+        assert ((got.float() - want).norm() / want.norm()).item() < 2.0 ** -7      # four roundings to bf16, as above
+
+
 MODES = [  # B, S, H, Hkv, D, window, spans, softcap
     (2, 512, 4, 4, 64, 128, None, None),
     (1, 640, 4, 2, 128, 200, None, None),
