@@ -162,12 +162,12 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* v_full = bars + 7;      // [2]
   uint64_t* v_empty = bars + 9;     // [2]
   uint64_t* sdp_full = bars + 11;
-  uint64_t* ds_ready = bars + 12;
-  uint64_t* dq_done = bars + 13;    // [2]: one per dS buffer
-  uint64_t* sdp_taken = bars + 15;  // the element-wise warps hold S and dP of the block in registers: TMEM may be rewritten
-  uint64_t* qdo_free = bars + 16;   // the unit's last score products have read Q and dO: the next unit's may land
-  uint64_t* dq_free = bars + 17;    // dQ of the unit sits in registers: the next unit may accumulate
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* ds_ready = bars + 12;   // [2]: one per dS buffer, as of P in the forward pass
+  uint64_t* dq_done = bars + 14;    // [2]: one per dS buffer
+  uint64_t* sdp_taken = bars + 16;  // the element-wise warps hold S and dP of the block in registers: TMEM may be rewritten
+  uint64_t* qdo_free = bars + 17;   // the unit's last score products have read Q and dO: the next unit's may land
+  uint64_t* dq_free = bars + 18;    // dQ of the unit sits in registers: the next unit may accumulate
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -187,7 +187,8 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       mbar_init(&v_empty[s], 1);
     }
     mbar_init(sdp_full, 1);
-    mbar_init(ds_ready, 8);
+    mbar_init(&ds_ready[0], 8);
+    mbar_init(&ds_ready[1], 8);
     mbar_init(&dq_done[0], 1);
     mbar_init(&dq_done[1], 1);
     mbar_init(sdp_taken, 8);
@@ -287,7 +288,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             if (!issue_scores(g + 1)) { ok = false; break; }
             if (j + 2 == t.nkv) tc_commit(qdo_free);        // the unit's last score products are on their way
           }
-          if (!mbar_wait(ds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (3u << 16) | 9)) { ok = false; break; }
+          if (!mbar_wait(&ds_ready[g & 1], uint32_t(g >> 1) & 1u, abort_flag, p.st, kTimeoutGeneric, (3u << 16) | 9)) { ok = false; break; }
           if (j == 0 && n > 0) {
             // dQ of the previous unit must have been read out before this unit starts its own sum
             if (!mbar_wait(dq_free, (n - 1) & 1, abort_flag, p.st, kTimeoutTmemEmpty, (3u << 16) | 15)) { ok = false; break; }
@@ -406,7 +407,7 @@ flash_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         tmem_st_32x32b_x32(tmem_dS + (g & 1) * 64 + lane_addr + half * 32, packed);
         tmem_st_wait();
         tc_fence_before();
-        warp_arrive(ds_ready);
+        warp_arrive(&ds_ready[g & 1]);
       }
       if (!ok) break;
       const int last = g0 + t.nkv - 1;
@@ -527,12 +528,12 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* s_taken = bars + 7;     // S^T / dP^T of the block are in registers: TMEM may be rewritten
   uint64_t* dp_taken = bars + 8;
   uint64_t* p_ready = bars + 9;     // P^T is in tensor memory
-  uint64_t* ds_ready = bars + 10;   // dS^T is in shared memory
-  uint64_t* dv_done = bars + 11;    // the dV product has read P^T
-  uint64_t* dk_done = bars + 12;    // [2]: one per dS^T buffer
-  uint64_t* kv_free = bars + 14;    // the unit's last score products have read K and V: the next unit's may land
-  uint64_t* acc_free = bars + 15;   // dV and dK of the unit sit in registers: the next unit may accumulate
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* ds_ready = bars + 10;   // [2]: dS^T is in shared memory, one per buffer
+  uint64_t* dv_done = bars + 12;    // the dV product has read P^T
+  uint64_t* dk_done = bars + 13;    // [2]: one per dS^T buffer
+  uint64_t* kv_free = bars + 15;    // the unit's last score products have read K and V: the next unit's may land
+  uint64_t* acc_free = bars + 16;   // dV and dK of the unit sit in registers: the next unit may accumulate
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* s_lse2 = reinterpret_cast<float*>(smem + L::kStat);
   float* s_delta = s_lse2 + 128;
@@ -555,7 +556,8 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(s_taken, 8);
     mbar_init(dp_taken, 8);
     mbar_init(p_ready, 8);
-    mbar_init(ds_ready, 8);
+    mbar_init(&ds_ready[0], 8);
+    mbar_init(&ds_ready[1], 8);
     mbar_init(dv_done, 1);
     mbar_init(&dk_done[0], 1);
     mbar_init(&dk_done[1], 1);
@@ -690,7 +692,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           if (more && kAlias && !issue_s(g + 1)) { ok = false; break; }
           if (more && !issue_dp(g + 1)) { ok = false; break; }
           if (it + 2 == t.iters) tc_commit(kv_free);               // the unit's last score products are on their way
-          if (!mbar_wait(ds_ready, g & 1, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 17)) { ok = false; break; }
+          if (!mbar_wait(&ds_ready[g % DB], uint32_t(g / DB) & 1u, abort_flag, p.st, kTimeoutGeneric, (4u << 16) | 17)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sdst_b = sdst + (g % DB) * 32768;
 #pragma unroll
@@ -875,7 +877,7 @@ flash_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             fence_proxy_async_smem();
             tc_fence_before();
             __syncwarp();
-            warp_arrive(ds_ready);
+            warp_arrive(&ds_ready[g % DB]);
           }
           softmax_bar_sync();    // this block's delta is no longer read; the next block's lse is visible
           if (fetch) s_delta[r] = -(n_dl * p.scale);

@@ -57,9 +57,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint64_t* v_empty = bars + 7;   // [2]
   uint64_t* s_full = bars + 9;    // [2]
   uint64_t* s_empty = bars + 11;  // [2]
-  uint64_t* p_ready = bars + 13;
-  uint64_t* o_done = bars + 14;   // [2]: the P V products of even and odd blocks
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint64_t* p_ready = bars + 13;  // [2]: one per P buffer
+  uint64_t* o_done = bars + 15;   // [2]: the P V products of even and odd blocks
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -89,7 +89,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       mbar_init(&s_full[b], 1);
       mbar_init(&s_empty[b], 8);       // the softmax warps
     }
-    mbar_init(p_ready, 8);
+    mbar_init(&p_ready[0], 8);
+    mbar_init(&p_ready[1], 8);
     mbar_init(&o_done[0], 1);
     mbar_init(&o_done[1], 1);
     *abort_flag = 0;
@@ -190,14 +191,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const int st = j & 1;
         const uint32_t ph = (j >> 1) & 1;
         if (j + 1 < nkv && !issue_scores(j + 1)) { ok = false; break; }
-        if (!mbar_wait(p_ready, j & 1, abort_flag, p.st, kTimeoutGeneric, (2u << 16) | 9)) { ok = false; break; }
+        // A barrier per P buffer: the softmax warps write a buffer again only after the product that read it, so they are never
+        // two phases ahead of a wait, which could not tell that from none. (With one barrier over two buffers they could be:
+        // nothing but time kept block j + 1's arrivals behind this wait for block j's.)
+        const int pb = j % kPBufs;
+        if (!mbar_wait(&p_ready[pb], uint32_t(j / kPBufs) & 1u, abort_flag, p.st, kTimeoutGeneric, (2u << 16) | 9)) { ok = false; break; }
         if (!mbar_wait(&v_full[st], ph, abort_flag, p.st, kTimeoutSmemFull, (2u << 16) | (2 + st))) { ok = false; break; }
         tc_fence_after();
         const uint32_t sv = smem_u32(smem + L::kV + st * L::kTile);
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint64_t db = make_smem_desc_sw128(sv + kk * 2048, 16384, 1024);
-          tc_mma_f16_ts(tmem_O, tmem_P + ((kPBufs == 2) ? st * 64 : 0) + kk * 8, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+          tc_mma_f16_ts(tmem_O, tmem_P + pb * 64 + kk * 8, db, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
         }
         tc_commit(&v_empty[st]);
         tc_commit(&o_done[st]);
@@ -317,7 +322,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       const float m_sub = (m_used == -INFINITY) ? 0.f : m_used;
       // probabilities -> bf16 A operand of the P V product in tensor memory, two columns of the row per 32-bit column
-      const uint32_t p_addr = tmem_P + ((kPBufs == 2) ? (j & 1) * 64 : 0) + lane_addr + half * 32;
+      const uint32_t p_addr = tmem_P + (j % kPBufs) * 64 + lane_addr + half * 32;
       auto probabilities = [&](auto with_mask) {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
@@ -353,7 +358,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (ok) {
         tmem_st_wait();
         tc_fence_before();
-        warp_arrive(p_ready);
+        warp_arrive(&p_ready[j % kPBufs]);
       }
     }
     if (ok && nkv > 0) {
