@@ -845,7 +845,7 @@ IDRAK_API int idrak_norm_fwd(const void* x, const void* residual, const void* w,
   const int nvec = C / 8;
   // a block per row for few long rows, and for rows of 2048 elements or more however many: a warp per row held them in up to
   // 256 registers a lane (9712 x 4096: 80 us, a block per row 54)
-  if ((rows <= 2 * sm_count() && nvec >= 128) || (nvec >= 256 && nvec <= 1024)) {
+  if ((rows <= 2 * sm_count() && nvec >= 128) || nvec >= 256) {
     return launch_overlapped(norm_fwd_block_kernel, dim3(unsigned(rows)), 256, 0, s, CBF(x), CBF(residual), CBF(w), CBF(b),
                              BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms);
   }
@@ -853,9 +853,7 @@ IDRAK_API int idrak_norm_fwd(const void* x, const void* residual, const void* w,
   if (nvec <= 32 * 1) NF(1);
   else if (nvec <= 32 * 2) NF(2);
   else if (nvec <= 32 * 4) NF(4);
-  else if (nvec <= 32 * 8) NF(8);
-  else if (nvec <= 32 * 16) NF(16);
-  else NF(32);
+  else NF(8);
 #undef NF
   note_launches(1);
   return int(cudaGetLastError());
