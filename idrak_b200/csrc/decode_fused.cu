@@ -3,8 +3,9 @@
 // scale per (token, kv head).
 //
 // The packed projection row of a token is [H query heads | Hkv key heads | Hkv value heads] x D. One warp takes one token and
-// a run of heads, one after another, so that the angles (a power and a range-reduced sincos per pair) are taken once per run:
-// and four heads' loads are in flight at a time (one head per warp: 9712 tokens x 48 heads of 128 128 us, now 63). Lane l holds elements l, l + 32, l + 64, ... of the head, so both members of a rotation pair
+// a run of heads: the angles (a power and a range-reduced sincos per pair) are taken once per run, and the loads of four heads
+// are in flight at a time. 9712 tokens x 48 heads of 128: 128 us with a head per warp, 63 now. Lane l holds elements l, l + 32,
+// l + 64, ... of a head (or neighbouring pairs of them, see the kernel), so both members of a rotation pair
 // (i, i + rot_dim / 2) sit in the same lane.
 //   query head   -> norm, rotate, written back in place (attention reads it from the projection buffer)
 //   key head     -> norm, rotate, written back in place (prefill attention reads it there) and into the cache slot

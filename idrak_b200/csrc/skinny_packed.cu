@@ -6,7 +6,7 @@
 // written back as two bytes of bf16 and read again by the tensor core, and each block would pass a barrier from the
 // converting warps to the MMA and back (57 us for 4096 x 28672 int8 codes at 16 tokens, three times the stream). Here a
 // warp's MMAs take their operands from registers (mma.sync m16n8k16, the weights as the 16-row side; at 8 or 16 tokens the
-// legacy tensor pipe is a third busy): a warp's own ring of TMA boxes brings blocks of 32 inputs x 128 features, its lanes
+// legacy tensor pipe is an eighth to a quarter busy): a warp's own ring of TMA boxes brings blocks of 32 inputs x 128 features, its lanes
 // read the codes, expand them in registers and multiply; no CTA-wide barrier until the sums. The order of the MMA's k
 // index and of its rows is free as long as both operands agree, so a lane takes eight consecutive inputs of 16
 // consecutive features: its part of X is one 16-byte load per token.
@@ -17,7 +17,13 @@
 // A CTA is 8 warps: FW side by side along the features (1; 2 for a gated pair, gate beside up), 8 / FW taking every
 // (8 / FW)-th block of inputs. Their partial tiles are summed in a fixed tree through shared memory, the CTAs of a cluster
 // (which split K further) in rank order through distributed shared memory, and the epilogue (skinny_common.cuh) runs on
-// the sum. Integer instructions bound the kernel (two per pair of codes, half rate), then the stream.
+// the sum.
+//
+// What bounds it (counters, 4096 x 28672): no single unit. The integer pipe, which turns the codes (two instructions per pair,
+// half rate), is the busiest at half of its peak (int8, 16 tokens 50 %, int4, 7 tokens 47 %; tensor pipe 24 and 14 %), DRAM at
+// 37 and 23 %. 224 CTAs share 148 SMs, two on some and one on the others, so 12 of the 16 warps that an SM could hold are
+// there on average, and they wait: for loads of X and scales, for the pipe, for the fixed latency of dependent instructions.
+// At 4096 x 4096 (one CTA per SM) the integer pipe is a quarter busy and the barriers of the sums weigh as much as the loads.
 //
 // Measured, us, 16 tokens int8 / 7 tokens int4 (before: tensor-core tiles expanded by four warps from a K-major copy of the
 // codes / unpacking to bf16 and a dense product): 4096 x 6144 12.0 / 10.6 (15.7 / 35.4), 4096 x 4096 9.0 / 7.9 (12.2 / 28.9),
@@ -80,7 +86,7 @@ __device__ __forceinline__ void sp_prefetch_4d(const CUtensorMap* m, int c0, int
                "r"(c0), "r"(0), "r"(c2)
                : "memory");
 }
-// Codes -> bf16 on as few integer instructions as possible (they run at half rate and bound the kernel): an unsigned
+// Codes -> bf16 on as few integer instructions as possible (they run at half rate, on the busiest pipe): an unsigned
 // integer u < 256 in a 16-bit lane is, read as bf16, the number u * 2^-133 (subnormal, or with the smallest exponent), so
 // one fused multiply-add by a power of two takes it to (u - offset) / 64, exactly; the 64 goes into the scales.
 __device__ __forceinline__ uint32_t sp_fma2(uint32_t a, uint32_t mul, uint32_t add) {
@@ -311,7 +317,7 @@ static int launch_packed(const void* codes, int ld, SkinnyPackedParams& p, cudaS
   auto kern = skinny_packed_kernel<kBits, NT, FW>;
   // One CTA per SM as long as the tiles allow it (enforced by its shared memory: left to itself the device packs the CTAs of
   // a cluster two to an SM), split along K over as many CTAs as keep every cluster resident; with more tiles than SMs two
-  // CTAs per SM and no split. A CTA of eight warps keeps an SM's integer pipes busy by itself. Measured, 16 tokens, int8, us:
+  // CTAs per SM and no split. Measured, 16 tokens, int8, us:
   // 4096 x 4096 (32 tiles) c = 2 / 4 / 8 (two per SM) 11.5 / 9.0 / 10.4; 14336 x 4096 c = 2 / 4 / 8 28.3 / 17.6 / 19.7;
   // 4096 x 28672 (224 tiles) c = 1 / 2 / 4 33 / 38 / 43.
   constexpr int kAlone = S::kTotal > 120 * 1024 ? S::kTotal : 120 * 1024;

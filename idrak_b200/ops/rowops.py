@@ -77,7 +77,8 @@ def norm_forward(x, weight, bias, eps, rms, residual=None):
 
 def norm_backward(dy, x, weight, mean, rstd, rms, has_bias, dres=None, w_param=None, b_param=None,
                   sums_of_dx: bool = False, frozen: bool = False):
-    """Returns (dx, dweight, dbias); with ``frozen`` (weight and bias take no gradient) the latter two may be None. ``x`` is the tensor that was normalised. ``dres`` is added to dx.
+    """Returns (dx, dweight, dbias); with ``frozen`` (weight and bias take no gradient) the latter two may be None. ``x`` is the
+    tensor that was normalised. ``dres`` is added to dx.
     When ``w_param`` (and ``b_param``) take direct gradient writes, dweight / dbias go straight into their
     ``.grad`` and come back as None. With ``sums_of_dx`` the column sums of dx (fp32) are attached to the returned
     dx as ``_idrak_colsum`` where the kernel produces them on the way (rows of up to 1024 elements): dx is the

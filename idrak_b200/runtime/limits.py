@@ -80,7 +80,7 @@ class KernelShape:
     tile: str                 # rows x columns x K per stage (or what the kernel's unit of work is)
     stages: int
     threads: int
-    shared_bytes: int         # dynamic shared memory asked for at launch (the flash and packed kernels: rounded up)
+    shared_bytes: int         # dynamic shared memory asked for at launch (qgemm and tp_gemm: rounded)
     tensor_memory_columns: int
     blocks_per_sm: int
     note: str = ""
@@ -94,12 +94,24 @@ def kernel_shapes() -> List[KernelShape]:
         KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128, and products that fill less than half the machine"),
         KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
                     "cta_group::2: each CTA holds half of the A rows and half of the B columns"),
-        KernelShape("skinny_gemm_kernel", "128 features x (16 | 32 | 64) tokens x 64, K over a cluster of up to 8", 4, 320,
-                    100352, 64, 2, "partial tiles summed through distributed shared memory"),
-        KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 84 * 1024, 256, 2, "P in tensor memory"),
-        KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 164 * 1024, 512, 1, "P in tensor memory, two buffers"),
-        KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 114 * 1024, 512, 1, "dS in tensor memory, two buffers"),
+        KernelShape("skinny_gemm_kernel", "128 features x 64 tokens x 64, K over a cluster of up to 8", 4, 320, 100352, 64, 2,
+                    "partial tiles summed through distributed shared memory"),
+        KernelShape("skinny_gemm_kernel<32>", "the same for up to 32 tokens", 5, 320, 104448, 32, 2),
+        KernelShape("skinny_gemm_kernel<16>", "the same for up to 16 tokens", 6, 320, 112640, 32, 2),
+        KernelShape("skinny_gemm_kernel<64, 8>", "int8 codes, 64 tokens", 3, 320, 100352, 64, 2, "three expanded operand tiles"),
+        KernelShape("skinny_gemm_kernel<32, 8>", "int8 codes, 32 tokens", 5, 320, 112640, 32, 2, "three expanded operand tiles"),
+        KernelShape("skinny_gemm_kernel<64, 4>", "int4 codes, 64 tokens", 5, 320, 112640, 64, 2, "three expanded operand tiles"),
+        KernelShape("skinny_gemm_kernel<32, 4>", "int4 codes, 32 tokens", 7, 320, 108544, 32, 2, "three expanded operand tiles"),
+        KernelShape("skinny_packed_kernel<8>", "128 (gated: 256) features x (8 | 16) tokens x 32 inputs a warp, int8 codes", 3, 256,
+                    122880, 0, 1, "a ring per warp; 99584 bytes and two per SM where there are more tiles than SMs"),
+        KernelShape("skinny_packed_kernel<4>", "the same over int4 codes", 5, 256, 122880, 0, 1,
+                    "83328 bytes and two per SM where there are more tiles than SMs"),
+        KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 85248, 256, 2, "P in tensor memory"),
+        KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 167168, 512, 1, "P in tensor memory, two buffers"),
+        KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 115968, 512, 1, "dS in tensor memory, two buffers"),
+        KernelShape("flash_bwd_q_kernel<128>", "the same, head size 128", 3, 320, 230656, 512, 1, "dS in tensor memory, two buffers"),
         KernelShape("flash_bwd_kv_kernel<64>", "128 keys x 128 queries per block, persistent", 2, 320, 166656, 512, 1, "P in tensor memory, dS in shared memory"),
+        KernelShape("flash_bwd_kv_kernel<128>", "the same, head size 128", 2, 320, 232192, 512, 1, "P over the scores in tensor memory, dS in shared memory"),
         KernelShape("qgemm_kernel", "128 x 128 x 64, weights unpacked in shared memory", 4, 448, 4 * 32768 + 2048, 256, 1,
                     "eight unpacking warps"),
         KernelShape("tp_gemm_kernel", "128 x 256 x 64 with peer-memory gather / reduce-scatter", 4, 320,

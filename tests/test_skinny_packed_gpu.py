@@ -40,7 +40,7 @@ def _check(got, x, w, M, K, bias=None, residual=None, gate=False):
 
 @pytest.mark.parametrize("kind", ["int8", "int4"])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64])
-@pytest.mark.parametrize("N,K", [(136, 64), (1000, 1056), (4096, 512)])
+@pytest.mark.parametrize("N,K", [(136, 64), (1000, 1056), (4096, 512), (160, 64), (1056, 1056)])     # int4 takes the last three
 def test_plain_bias_residual(kind, M, N, K):
     x, w, b, r = _inputs(kind, M, N, K)
     if not packed_supported(x, w):
