@@ -363,29 +363,63 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
   }
 }
 
-// out[seq, head, :] = merge of the partials of a sequence's splits, in split order
-__global__ void decode_merge_kernel(const DecodeParams p) {
+// out[seq, head, :] = merge of the partials of a sequence's splits, in split order. One thread per element of the head (D
+// threads). The shares' weights are taken by a thread each and the loads of eight shares are in flight at a time: one after the
+// other, with the weights taken by every thread, 32 shares of 32 heads of 128 took 12 to 17 us, as long as the attention of 8000 keys.
+constexpr int kMergeShares = 64;
+__global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
   pdl_wait();
-  const int row = blockIdx.x, D = p.D;
+  const int row = blockIdx.x, D = p.D, t = threadIdx.x;
   int first_tile, span;
   key_span(p.seq_lens[row / p.H], p.window, first_tile, span);
   const int per = tiles_per_split(span, p.splits, p.min_tiles);
   if (span <= per) return;                               // written out by its only split
   const int used = (span + per - 1) / per;
-  const float* base = p.partial + size_t(row) * p.splits * (D + 2);
-  float mm = -INFINITY;
-  for (int s = 0; s < used; ++s) mm = fmaxf(mm, base[s * (D + 2) + D]);
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float ll = 0.f, oo = 0.f;
-    for (int s = 0; s < used; ++s) {
-      const float* src = base + s * (D + 2);
-      const float a = (src[D] == -INFINITY) ? 0.f : exp2f(src[D] - mm);
-      ll += src[D + 1] * a;
-      oo += src[d] * a;
+  const float* __restrict__ base = p.partial + size_t(row) * p.splits * (D + 2);
+  __shared__ float weight[kMergeShares], sum[kMergeShares], red[4];
+  float mm = -INFINITY, ll = 0.f, oo = 0.f;
+  if (used <= 8) {                                       // few shares: all of them in flight, no barrier
+    float m[8], l[8], v[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const bool there = s < used;
+      m[s] = there ? base[s * (D + 2) + D] : -INFINITY;
+      l[s] = there ? base[s * (D + 2) + D + 1] : 0.f;
+      v[s] = there ? base[s * (D + 2) + t] : 0.f;
+      mm = fmaxf(mm, m[s]);
     }
-    p.out[size_t(row) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const float a = (m[s] == -INFINITY) ? 0.f : exp2f(m[s] - mm);
+      ll += l[s] * a;
+      oo += v[s] * a;
+    }
+    p.out[size_t(row) * D + t] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
+    return;
   }
+  for (int s = t; s < used; s += blockDim.x) mm = fmaxf(mm, base[s * (D + 2) + D]);
+  mm = warp_max(mm);
+  if ((t & 31) == 0) red[t >> 5] = mm;
+  __syncthreads();
+  for (int w = 0; w < int(blockDim.x >> 5); ++w) mm = fmaxf(mm, red[w]);
+  for (int s0 = 0; s0 < used; s0 += kMergeShares) {
+    const int n = min(kMergeShares, used - s0);
+    if (t < n) {
+      const float m = base[(s0 + t) * (D + 2) + D];
+      weight[t] = (m == -INFINITY) ? 0.f : exp2f(m - mm);
+      sum[t] = base[(s0 + t) * (D + 2) + D + 1];
+    }
+    __syncthreads();
+    const float* src = base + size_t(s0) * (D + 2) + t;
+#pragma unroll 8
+    for (int s = 0; s < n; ++s) {
+      ll += sum[s] * weight[s];
+      oo += src[s * (D + 2)] * weight[s];
+    }
+    __syncthreads();                                     // the next shares' weights take the place of these
+  }
+  p.out[size_t(row) * D + t] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
 }
 
 // k / v rows of new tokens -> their cache slots. src rows hold heads packed [Hkv, D]; slot = block * block_size + offset.

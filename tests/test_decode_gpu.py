@@ -232,3 +232,22 @@ def test_decode_slots_refuses_what_indexing_refused():
         assert slots.tolist() == want and lens.tolist() == [1, 16, 48]
     empty = D.decode_slots(pos[:0], table, 16)
     assert empty[0].numel() == 0 and empty[1].numel() == 0
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("splits", [2, 8, 9, 64, 65, 125])
+def test_any_number_of_shares_merges_in_order(Dh, splits):
+    """Up to eight shares, one round of 64 and more than that, of sequences that fill them, some of them or one."""
+    bs, Hkv, H, lens = 16, 2, 6, [4000, 2500, 33, 0]
+    need = [(n + bs - 1) // bs for n in lens]
+    table, at = torch.zeros(len(lens), max(need), dtype=torch.int32), 0
+    for i, n in enumerate(need):
+        table[i, :n] = torch.arange(at, at + n)
+        at += n
+    kc, vc, q = _rand((at, bs, Hkv, Dh), 1), _rand((at, bs, Hkv, Dh), 2), _rand((len(lens), H, Dh), 3)
+    table, lens_t = table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    out = D.paged_decode(q, kc, vc, table, lens_t, splits=splits)
+    ref = D.paged_decode_reference(q.float(), kc.float(), vc.float(), table, lens_t)
+    # probabilities enter the tensor core as bf16 (2^-9) and the result is rounded to bf16, values up to about 2
+    assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * 2
+    assert torch.equal(out, D.paged_decode(q, kc, vc, table, lens_t, splits=splits))
