@@ -165,24 +165,43 @@ def paged_decode_reference(q, k_cache, v_cache, block_table, seq_lens, scale=Non
 DECODE_TILE, DECODE_CTAS = 32, 16384
 
 
-def key_shares(seqs: int, kv_heads: int, longest: int, window: int = 0):
+def key_shares(seqs: int, kv_heads: int, longest: int, window: int = 0, sms: int = 148):
     """``(splits, min_keys)`` of a decode step: by how many CTAs per KV head a sequence's keys are shared at most, and how many
     keys a share has at least, from a bound on the lengths alone (a power of two above the longest).
 
-    Shares of 128 keys (one tile per warp) to 1024: short ones so that few sequences fill the machine, long ones where there are
-    CTAs enough, since a CTA costs about as much as 200 keys of a busy machine. 1024 CTAs if every sequence had the bound.
-    Measured, us, shares of 128 / 512 / 1024 / unsplit: 1 sequence 9.8 / 11.8 / 11.8 / 11.8, 16 of 128 to 2304 tokens 41 / 28.5 /
-    40 / 51, 64 of those 145 / 91 / 84 / 95.
+    A share costs a CTA's set-up and a partial result to merge, a long one is a long chain. With the machine idle the best share
+    grows like the square root of the length (128 keys below 4096, then 256, 512 from 16384 on), as long as the CTAs are there
+    together, three to an SM: a second round costs as much as the first. With sequences x KV heads from a quarter of the SMs on,
+    each has few shares and unequal lengths weigh more: 1024 CTAs if every sequence had the bound, and 256 keys at least from
+    half of the SMs, 512 from all of them on. From two CTAs per SM on shares only even out a batch: 1024 keys, 2048 from five per
+    SM on. Measured over 476 batches of 50 to 32000 keys, equal, mixed, or one long one among short ones, head sizes 64 and 128:
+    4, 4 and 10 % above the best choice for each on average, where two CTAs per SM and none beyond are 9, 11 and 145 % above it.
+    us, shares of 128 / 256 / 512 / 1024 keys: one sequence of 4000, 8 KV heads 17 / 15 / 18 / 29, of 32000 53 / 52 / 53 / 44;
+    64 of 100 to 4000 192 / 143 / 122 / 115 (unsplit 128), 200 of 300 115 / 97 / 69 unsplit.
 
     At most 64 shares, and 16384 CTAs in all: each has a partial result in HBM and is launched whether its sequence reaches it or
-    not. With less a long sequence's share is longer. 256 sequences of 8 KV heads under a bound of 32768, us, unsplit / 4 / 8 /
-    32 shares: one of 32000 tokens and the others of 300 717 / 294 / 212 / 199, all of 300 94 / 101 / 110 / 161 (136 MB of partial
-    results at 32 query heads of 128, 34 at 8 shares)."""
+    not. 256 sequences of 8 KV heads under a bound of 32768, us, unsplit / 8 / 32 shares: one of 32000 tokens and the others of
+    300 717 / 212 / 199, all of 300 94 / 110 / 161 (136 MB of partial results at 32 query heads of 128, 34 at 8 shares)."""
     if window > 0:
         longest = min(longest, window + DECODE_TILE)       # a window may start inside a tile
+    if longest <= 256:
+        return 1, 128
     heads = max(seqs * kv_heads, 1)
-    min_keys = max(128, min(1024, (longest * heads // 1024 + 127) // 128 * 128))
-    return max(1, min((longest + min_keys - 1) // min_keys, 64, DECODE_CTAS // heads)), min_keys
+    share = 128 << max(0, (longest.bit_length() - 11) // 2)
+    if heads > sms // 4:
+        if heads > 2 * sms:
+            share = max(share, 1024 if heads <= 5 * sms else 2048)
+        elif heads > sms and longest <= 1024:
+            share = max(share, 1024)
+        else:
+            least = 128 if heads <= sms // 2 else 256 if heads <= sms else 512
+            share = max(share, least, min(1024, -(-longest * heads // 1024 // 128) * 128))
+        # to the nearest: a window may leave a share of one tile
+        return max(1, min((longest + share // 2) // share, 64, DECODE_CTAS // heads)), share
+    splits, together = min(-(-longest // share), 64), 3 * sms // heads
+    if splits > together:
+        splits = together if longest <= 8192 or together >= 16 else max(together, min(splits, longest // 1024))
+    return splits, share
 
 
 def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_table: torch.Tensor,
@@ -200,7 +219,8 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     lib = _native.lib()
     min_keys = 0
     if splits is None:
-        splits, min_keys = key_shares(seqs, Hkv, max_len_hint if max_len_hint is not None else block_table.shape[1] * bs, window)
+        longest = max_len_hint if max_len_hint is not None else block_table.shape[1] * bs
+        splits, min_keys = key_shares(seqs, Hkv, longest, window, lib.idrak_sm_count())
     out = torch.empty(seqs, H, D, dtype=q.dtype, device=q.device)
     part = None
     if splits > 1:
