@@ -592,16 +592,19 @@ __global__ void gelu_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
 }
 
 // gate_up: [rows, 2*H] with gate in columns [0,H) and up in [H,2H); out[r, h] = act(gate) * up.
-// One 8-element vector per thread; blockIdx.x = row * chunks + chunk. (A grid-stride loop over eight blocks per SM with a
-// 64-bit division per vector had too few loads in flight: 9712 x 14336 forward 187 us, backward 274; now 165 and 234.)
+// One 8-element vector per thread, counted over the whole matrix; I is 32 bits wide as long as the vectors can be counted in
+// 31 (a 64-bit division costs a vector as much as its memory). A grid-stride loop over eight blocks per SM had too few loads in
+// flight: 9712 x 14336 forward 187 us, backward 274; now 165 and 234. Blocks of a row each, as it was for a while, leave most
+// threads of a narrow row idle: 65536 x 64 forward 70 us, 7 before.
+template <class I>
 __global__ void __launch_bounds__(256) gated_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
-                                                        int H, int kind, int chunks) {
+                                                        I total, int H, int kind) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
   pdl_wait();
-  const int row = blockIdx.x / chunks;
-  const int c = ((blockIdx.x - row * chunks) * 256 + threadIdx.x) * 8;
-  if (c >= H) return;
-  const size_t r = size_t(row);
+  const I i = I(blockIdx.x) * 256 + threadIdx.x, hv = I(H >> 3);
+  if (i >= total) return;
+  const size_t r = size_t(i / hv);
+  const int c = int(i - I(r) * hv) * 8;
   float g[8], u[8];
   load8(gu + r * 2 * H + c, g);
   load8(gu + r * 2 * H + H + c, u);
@@ -609,13 +612,14 @@ __global__ void __launch_bounds__(256) gated_fwd_kernel(const __nv_bfloat16* __r
   for (int j = 0; j < 8; ++j) g[j] = gate_fn(g[j], kind) * u[j];
   store8(out + r * H + c, g);
 }
+template <class I>
 __global__ void __launch_bounds__(256) gated_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                                         const __nv_bfloat16* __restrict__ dout,
-                                                        __nv_bfloat16* __restrict__ dgu, int H, int kind, int chunks) {
-  const int row = blockIdx.x / chunks;
-  const int c = ((blockIdx.x - row * chunks) * 256 + threadIdx.x) * 8;
-  if (c >= H) return;
-  const size_t r = size_t(row);
+                                                        __nv_bfloat16* __restrict__ dgu, I total, int H, int kind) {
+  const I i = I(blockIdx.x) * 256 + threadIdx.x, hv = I(H >> 3);
+  if (i >= total) return;
+  const size_t r = size_t(i / hv);
+  const int c = int(i - I(r) * hv) * 8;
   float g[8], u[8], d[8], dg[8], du[8];
   load8(gu + r * 2 * H + c, g);
   load8(gu + r * 2 * H + H + c, u);
@@ -1001,18 +1005,23 @@ IDRAK_API int idrak_gelu_bwd(const void* x, const void* dy, void* dx, long long 
 IDRAK_API int idrak_gated_fwd(const void* gu, void* out, int rows, int H, int kind, void* stream_) {
   if (H % 8) return -2;
   if (rows <= 0 || H <= 0) return 0;
-  const int chunks = (H / 8 + 255) / 256;
-  if ((long long)rows * chunks > 0x7fffffffll) return -3;
-  return launch_overlapped(gated_fwd_kernel, dim3(unsigned(rows * chunks)), 256, 0, static_cast<cudaStream_t>(stream_),
-                           CBF(gu), BF(out), H, kind, chunks);
+  const long long total = (long long)rows * (H / 8), blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffffll) return -3;
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  if (total <= 0x7fffffffll)
+    return launch_overlapped(gated_fwd_kernel<unsigned>, dim3(unsigned(blocks)), 256, 0, s, CBF(gu), BF(out), unsigned(total), H, kind);
+  return launch_overlapped(gated_fwd_kernel<unsigned long long>, dim3(unsigned(blocks)), 256, 0, s, CBF(gu), BF(out),
+                           (unsigned long long)total, H, kind);
 }
 IDRAK_API int idrak_gated_bwd(const void* gu, const void* dout, void* dgu, int rows, int H, int kind,
                               void* stream_) {
   if (H % 8) return -2;
   if (rows <= 0 || H <= 0) return 0;
-  const int chunks = (H / 8 + 255) / 256;
-  if ((long long)rows * chunks > 0x7fffffffll) return -3;
-  gated_bwd_kernel<<<rows * chunks, 256, 0, static_cast<cudaStream_t>(stream_)>>>(CBF(gu), CBF(dout), BF(dgu), H, kind, chunks);
+  const long long total = (long long)rows * (H / 8), blocks = (total + 255) / 256;
+  if (blocks > 0x7fffffffll) return -3;
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  if (total <= 0x7fffffffll) gated_bwd_kernel<unsigned><<<unsigned(blocks), 256, 0, s>>>(CBF(gu), CBF(dout), BF(dgu), unsigned(total), H, kind);
+  else gated_bwd_kernel<unsigned long long><<<unsigned(blocks), 256, 0, s>>>(CBF(gu), CBF(dout), BF(dgu), (unsigned long long)total, H, kind);
   note_launches(1);
   return int(cudaGetLastError());
 }
