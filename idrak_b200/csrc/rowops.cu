@@ -338,6 +338,65 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_kernel(const __nv_bfloat16* _
   }
 }
 
+// The same for short rows: G lanes hold a row in registers, VPL vectors each, and meet by shuffles. A block per row had blocks
+// of 32 to 128 threads with a barrier each for rows that a warp holds: 327680 x 128 177 us, 65536 x 1024 144 us; the kernel
+// above with the sums of dw that nobody reads 139 and 118 us.
+template <int G, int VPL>
+__global__ void __launch_bounds__(256) norm_bwd_dx_row_kernel(const __nv_bfloat16* __restrict__ dy,
+                                                              const __nv_bfloat16* __restrict__ x,
+                                                              const __nv_bfloat16* __restrict__ w,
+                                                              const float* __restrict__ mean_in,
+                                                              const float* __restrict__ rstd_in,
+                                                              const __nv_bfloat16* __restrict__ dres_in,
+                                                              __nv_bfloat16* __restrict__ dx, int rows, int C, int rms) {
+  const long long row = blockIdx.x * (long long)(256 / G) + threadIdx.x / G;
+  const int nvec = row < rows ? C >> 3 : 0, sub = threadIdx.x % G;       // lanes of a row past the end only meet the others
+  const size_t base = size_t(row) * C;
+  const float mean = rms || nvec == 0 ? 0.f : mean_in[row];
+  const float rstd = nvec == 0 ? 0.f : rstd_in[row];
+  float g[VPL][8], n[VPL][8], s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const int vi = sub + i * G;
+    if (vi < nvec) {
+      float wv[8];
+      load8(dy + base + vi * 8, g[i]);
+      load8(x + base + vi * 8, n[i]);
+      load8(w + vi * 8, wv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        n[i][j] = (n[i][j] - mean) * rstd;
+        g[i][j] *= wv[j];
+        s1 += g[i][j];
+        s2 += g[i][j] * n[i][j];
+      }
+    }
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  }
+  s1 = rms ? 0.f : s1 / float(C);
+  s2 /= float(C);
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    const int vi = sub + i * G;
+    if (vi < nvec) {
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o[j] = (g[i][j] - s1 - n[i][j] * s2) * rstd;
+      if (dres_in) {
+        float r[8];
+        load8(dres_in + base + vi * 8, r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += r[j];
+      }
+      store8(dx + base + vi * 8, o);
+    }
+  }
+}
+
 // out[c] (+)= sum_p part[p, c]. Block = 32 columns x 8 part lanes: lane ty adds parts ty, ty+8, ... in
 // ascending order, then the 8 lane sums are added in lane order, so the result has one fixed order.
 // One launch takes up to three such sums of equal size (blockIdx.y): a normalisation's dw, db and column sums of dx took a
@@ -847,9 +906,10 @@ IDRAK_API int idrak_norm_fwd(const void* x, const void* residual, const void* w,
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const int blocks = (rows + 3) / 4;
   const int nvec = C / 8;
-  // a block per row for few long rows, and for rows of 2048 elements or more however many: a warp per row held them in up to
-  // 256 registers a lane (9712 x 4096: 80 us, a block per row 54)
-  if ((rows <= 2 * sm_count() && nvec >= 128) || nvec >= 256) {
+  // a block per row for few long rows, and for rows of more than 2048 elements however many: a warp per row held them in up to
+  // 256 registers a lane (9712 x 4096: 80 us, a block per row 54; at 2048 elements it is the faster one still, 8192 rows 18 us
+  // against 25)
+  if ((rows <= 2 * sm_count() && nvec >= 128) || nvec > 256) {
     return launch_overlapped(norm_fwd_block_kernel, dim3(unsigned(rows)), 256, 0, s, CBF(x), CBF(residual), CBF(w), CBF(b),
                              BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms);
   }
@@ -883,8 +943,15 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
   if (C % 8 || C > 8192 || rows <= 0) return -2;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   if (!dw && !db && !dx_colsum) {                    // a frozen weight: dx alone
-    const int threads = C / 8 >= 256 ? 256 : (C / 8 + 31) / 32 * 32;
-    norm_bwd_dx_kernel<<<rows, threads, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), C, rms);
+    const int nvec = C / 8;
+#define ND(G, V) norm_bwd_dx_row_kernel<G, V><<<unsigned((rows + 256 / G - 1) / (256 / G)), 256, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), rows, C, rms)
+    if (nvec <= 8) ND(8, 1);
+    else if (nvec <= 16) ND(16, 1);
+    else if (nvec <= 32) ND(32, 1);
+    else if (nvec <= 64) ND(32, 2);
+    else if (nvec <= 128) ND(32, 4);
+    else norm_bwd_dx_kernel<<<rows, nvec >= 256 ? 256 : (nvec + 31) / 32 * 32, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), C, rms);
+#undef ND
     note_launches(1);
     return int(cudaGetLastError());
   }

@@ -231,3 +231,26 @@ def test_norm_parameter_gradients_from_one_launch(rms):
     if not rms:
         want = dy.double().sum(0)
         assert ((b.grad.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-2).all()
+
+
+@pytest.mark.parametrize("C", [8, 64, 72, 128, 136, 256, 264, 512, 520, 1024, 1032, 2048])
+@pytest.mark.parametrize("rows", [1, 7, 300, 1001])
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_backward_with_a_frozen_weight_of_any_width(C, rows, rms):
+    """Rows held by 8, 16 or 32 lanes and by a block, the last block of rows not full, the residual's gradient added."""
+    from idrak_b200.ops.rowops import norm_backward, norm_forward
+    x, w, dy, dres = _rand((rows, C), 1.0, 1), _rand((C,), 1.0, 2), _rand((rows, C), 1.0, 3), _rand((rows, C), 1.0, 4)
+    b = None if rms else _rand((C,), 1.0, 5)
+    _, mean, rstd, _ = norm_forward(x, w, b, 1e-5, rms)
+    xr = x.double().requires_grad_()
+    if rms:
+        yr = xr * torch.rsqrt(xr.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    else:
+        yr = torch.nn.functional.layer_norm(xr, (C,), w.double(), b.double(), 1e-5)
+    yr.backward(dy.double())
+    for extra in (None, dres):
+        dx, dw, db = norm_backward(dy, x, w, mean, rstd, rms, not rms, extra, frozen=True)
+        want = xr.grad if extra is None else xr.grad + extra.double()
+        assert dw is None and db is None
+        # fp32 sums of C terms and one rounding to bf16 (2^-9)
+        assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
