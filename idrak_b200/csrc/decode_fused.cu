@@ -39,14 +39,14 @@ struct NormRopeKvParams {
   int run;                       // heads per warp
 };
 
-// One warp per token and run of heads, four heads in flight at a time; each lane owns PER = D / 32 elements of a head.
+// One warp per token and run of heads, four heads in flight at a time (of 256 elements: one); each lane owns PER = D / 32 elements of a head.
 // kPairs = 0: elements e = lane + 32 j (any rotary width that is a multiple of 64). kPairs = 1 (PER = 4, rotary width = the
 // whole head or none): e = 2 lane, 2 lane + 1 and the same plus D / 2, in four-byte accesses.
 template <int PER, int kPairs>
 __global__ void __launch_bounds__(256) norm_rope_kv_kernel(const NormRopeKvParams p) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int kBatch = 4;
+  constexpr int kBatch = PER == 8 ? 1 : 4;            // heads in flight: more than one of 256 elements only costs registers
   const int heads_total = p.H + 2 * p.Hkv;
   const int runs = (heads_total + p.run - 1) / p.run;
   const long long unit = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -215,8 +215,18 @@ IDRAK_API int idrak_norm_rope_kv(void* qkv, long long row_stride, const int* pos
   p.eps = eps; p.theta = theta; p.freq_scale = freq_scale; p.rot_dim = rot_dim;
   p.T = T; p.H = H; p.Hkv = Hkv; p.D = D; p.kv_int8 = kv_int8;
   const int heads = H + 2 * Hkv;
-  p.run = 1;                     // longer runs as long as there are four warps for every scheduler of the device
-  while (p.run < 16 && (long long)T * ((heads + 2 * p.run - 1) / (2 * p.run)) >= (long long)sm_count() * 16) p.run *= 2;
+  // Heads per warp: the fewest rounds of 32 warps per SM, a round as long as a fixed part (the angles) and its heads. 9000
+  // tokens of 48 heads of 128: 152 us with a head per warp, 58 with 16; 1000 of 36 over an int8 cache 14.3 / 11.5 with four, and
+  // 16.4 with the 16 that merely leave four warps to every scheduler.
+  long long least = 0;
+  for (int run = 1; run <= 16; run *= 2) {
+    const long long warps = (long long)T * ((heads + run - 1) / run), place = 32ll * sm_count();
+    const long long cost = (warps + place - 1) / place * (5 + 2 * run);
+    if (run == 1 || cost < least) {
+      p.run = run;
+      least = cost;
+    }
+  }
   const long long units = (long long)T * ((heads + p.run - 1) / p.run);
   const int blocks = int((units + 7) / 8);
   cudaStream_t s = static_cast<cudaStream_t>(stream_);

@@ -251,3 +251,33 @@ def test_any_number_of_shares_merges_in_order(Dh, splits):
     # probabilities enter the tensor core as bf16 (2^-9) and the result is rounded to bf16, values up to about 2
     assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * 2
     assert torch.equal(out, D.paged_decode(q, kc, vc, table, lens_t, splits=splits))
+
+
+@pytest.mark.parametrize("H,Hkv,Dh,rot", [(12, 12, 256, 128), (12, 12, 128, 128), (12, 12, 128, 64), (9, 3, 64, 64)])
+@pytest.mark.parametrize("T", [700, 3001])
+@pytest.mark.parametrize("int8", [False, True])
+def test_fused_norm_rope_kv_write_in_runs_of_heads(H, Hkv, Dh, rot, T, int8):
+    """Enough tokens that a warp takes runs of heads, the last run of a token shorter: keys rotated once, values as they are."""
+    bs = 16
+    nb = (T + bs - 1) // bs
+    qkv = _rand((T, (H + 2 * Hkv) * Dh), 1)
+    pos = torch.randint(0, 3000, (T,), dtype=torch.int32, device="cuda")
+    slots = torch.randperm(nb * bs)[:T].to(torch.int32).cuda()
+    kc, vc = (torch.zeros((nb, bs, Hkv, Dh), dtype=torch.int8 if int8 else torch.bfloat16, device="cuda") for _ in range(2))
+    ks, vs = (torch.zeros((nb, bs, Hkv), device="cuda") if int8 else None for _ in range(2))
+    got = qkv.clone()
+    D.norm_rope_kv(got, H, Hkv, Dh, pos, slots, kc, vc, ks, vs, None, None, 1e-6, 10000.0, rot)
+    heads = qkv.unflatten(-1, (H + 2 * Hkv, Dh))
+    from idrak_b200.ops.rowops import rope_reference
+    want = rope_reference(heads[:, :H + Hkv].contiguous(), pos, 10000.0, rot).float()
+    mine = got.unflatten(-1, (H + 2 * Hkv, Dh))
+    # both rounded to bf16 (they may fall on neighbours, 2^-7 apart), and fp32 angles of up to 3000 (2^-12 of a pair of up to 8)
+    assert ((mine[:, :H + Hkv].float() - want).abs() <= 2.0 ** -7 * want.abs() + 4e-3).all()
+    assert torch.equal(mine[:, H + Hkv:], heads[:, H + Hkv:])
+    for cache, scale, part in ((kc, ks, mine[:, H:H + Hkv]), (vc, vs, heads[:, H + Hkv:])):
+        held = cache.view(-1, Hkv, Dh)[slots.long()]
+        if int8:
+            codes, sc = D.quantize_kv_reference(part)
+            assert (held.int() - codes.int()).abs().max() <= 1 and torch.allclose(scale.view(-1, Hkv)[slots.long()], sc, rtol=1e-6)
+        else:
+            assert torch.equal(held, part)
