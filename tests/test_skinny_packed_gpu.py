@@ -40,7 +40,7 @@ def _check(got, x, w, M, K, bias=None, residual=None, gate=False):
 
 @pytest.mark.parametrize("kind", ["int8", "int4"])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64])
-@pytest.mark.parametrize("N,K", [(136, 64), (1000, 1056), (4096, 512), (160, 64), (1056, 1056)])     # int4 takes the last three
+@pytest.mark.parametrize("N,K", [(136, 64), (1000, 1056), (4096, 512)])
 def test_plain_bias_residual(kind, M, N, K):
     x, w, b, r = _inputs(kind, M, N, K)
     if not packed_supported(x, w):
@@ -49,6 +49,13 @@ def test_plain_bias_residual(kind, M, N, K):
     _check(a, x, w, M, K)
     assert torch.equal(a, packed_linear(x, w))                    # fixed order of the sums
     _check(packed_linear(x, w, b, r), x, w, M, K, b, r)
+
+
+@pytest.mark.parametrize("kind", ["int8", "int4"])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(160, 64), (1056, 1056)])
+def test_widths_that_end_inside_a_tile(kind, M, N, K):
+    test_plain_bias_residual(kind, M, N, K)       # of the ragged widths above int4 takes none
 
 
 @pytest.mark.parametrize("kind", ["int8", "int4"])
