@@ -75,31 +75,41 @@ class Int8Weight:
     def to(self, device) -> "Int8Weight":
         return Int8Weight(self.codes.to(device), self.scales.to(device), self.rows, self.cols)
 
+    def _kept(self, name: str, make) -> torch.Tensor:
+        """A second layout of the codes, made on first use and kept - but for one made while a CUDA graph is recorded, which holds
+        nothing until a replay and lies in that graph's memory."""
+        t = getattr(self, name, None)
+        if t is None or t.device != self.codes.device:
+            t = make()
+            if not (t.is_cuda and torch.cuda.is_current_stream_capturing()):
+                setattr(self, name, t)
+        return t
+
     def tma_codes(self) -> torch.Tensor:
         """The codes with rows and base on 16-byte boundaries, as the few-row kernels read them: the codes themselves, or
-        for a weight that came with shorter rows (an older file) a padded copy, made on first use and kept."""
+        for a weight that came with shorter rows (an older file) a padded copy."""
         if self.codes.stride(0) % 16 == 0 and self.codes.data_ptr() % 16 == 0:
             return self.codes
-        t = getattr(self, "_tma_codes", None)
-        if t is None or t.device != self.codes.device:
+
+        def make():
             t = torch.zeros((self.rows, (self.cols + 15) // 16 * 16), dtype=torch.int8, device=self.codes.device)
             t[:, : self.cols] = self.codes[:, : self.cols]
-            self._tma_codes = t
-        return t
+            return t
+        return self._kept("_tma_codes", make)
 
     def gate_codes(self):
         """``(codes, first up column)`` of a stacked ``[gate | up]`` weight with both halves on 16-byte boundaries: the codes
-        themselves, or where the half width is not a multiple of 16 a copy with padded halves, made on first use and kept."""
+        themselves, or where the half width is not a multiple of 16 a copy with padded halves."""
         half = self.cols // 2
         if half % 16 == 0:
             return self.tma_codes(), half
         pad = (half + 15) // 16 * 16
-        t = getattr(self, "_gate_codes", None)
-        if t is None or t.device != self.codes.device:
+
+        def make():
             t = torch.zeros((self.rows, 2 * pad), dtype=torch.int8, device=self.codes.device)
             t.view(self.rows, 2, pad)[:, :, :half] = self.codes[:, : 2 * half].unflatten(1, (2, half))
-            self._gate_codes = t
-        return t, pad
+            return t
+        return self._kept("_gate_codes", make), pad
 
     @property
     def ld(self) -> int:

@@ -67,3 +67,22 @@ def test_int8_gate_whose_halves_start_between_16_byte_boundaries(M, ff):
     # one rounding to bf16, fp32 sums of 128 terms and the fp32 activation
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
     _native.check_status("gated int8 product")
+
+
+@pytest.mark.parametrize("gate,cols", [(None, 200), ("silu", 208)])
+def test_codes_padded_while_a_graph_is_recorded_are_not_kept(gate, cols):
+    """The first use of a weight whose codes need another layout may be inside a recording: eager calls before the replay, the
+    replay, and eager calls after the graph is gone all see the codes."""
+    x = _rand(5, 128, seed=1)
+    w = Int8Weight.quantize(torch.randn(128, cols, generator=torch.Generator(device="cuda").manual_seed(4), device="cuda"))
+    want = skinny8_linear(x, Int8Weight(w.codes[:, :cols].clone(), w.scales, 128, cols), gate=gate)
+    fresh = Int8Weight(w.codes[:, :cols].contiguous() if gate is None else w.codes, w.scales, 128, cols)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        recorded = skinny8_linear(x, fresh, gate=gate)
+    assert torch.equal(skinny8_linear(x, fresh, gate=gate), want)
+    graph.replay()
+    assert torch.equal(recorded, want)
+    del graph, recorded
+    torch.cuda.synchronize()
+    assert torch.equal(skinny8_linear(x, fresh, gate=gate), want)
