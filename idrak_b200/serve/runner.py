@@ -68,8 +68,10 @@ def fold_norms_into_projections(model: Decoder) -> bool:
 
 def _plain(module, cls) -> bool:
     """Whether calling ``module`` runs ``cls.forward`` and nothing besides (but for hooks on every module there is)."""
+    if type(module) is not cls:
+        return False
     d = module.__dict__
-    return type(module) is cls and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d)
+    return not (d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d)
 
 
 class ModelRunner:
@@ -356,7 +358,7 @@ class ModelRunner:
         state: list = [getattr(self.model, "_norms_folded", False)]
         for blk in self.model.blocks:
             for name in ("attn", "mlp"):
-                m = blk._modules[name]
+                m = blk._modules.get(name) or getattr(blk, name)      # a block may be wrapped
                 state.append(ref(m))
                 adapters = m._modules.get("adapters", m.__dict__.get("adapters"))
                 state.append(adapters if adapters is None else ref(adapters))
@@ -438,7 +440,8 @@ class ModelRunner:
             return False
         for blk in self.model.blocks:
             mods = blk._modules
-            if not (_plain(mods["attn_norm"], Norm) and _plain(mods["mlp_norm"], Norm) and _plain(mods["mlp"], FeedForward)):
+            if not (_plain(mods.get("attn_norm"), Norm) and _plain(mods.get("mlp_norm"), Norm)
+                    and _plain(mods.get("mlp"), FeedForward)):
                 return False
         return True
 

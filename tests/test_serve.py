@@ -183,3 +183,50 @@ def test_folding_the_norm_weights_into_the_projections_keeps_the_function():
     assert got == want
     tied = build_decoder(DecoderSpec.gpt2(layers=1, dim=32, heads=2, vocab=50, max_positions=16), seed=1)
     assert not fold_norms_into_projections(tied)              # LayerNorm and a tied head: left alone
+
+
+def test_runner_forgets_its_choices_when_the_model_changes():
+    from idrak_b200.adapters.lora import add_adapters
+    from idrak_b200.quant import quantize_model
+    from idrak_b200.serve.runner import ModelRunner
+    from idrak_b200.text.finetuning import adapters_disabled
+    model = build_decoder(DecoderSpec.llama(layers=2, dim=32, heads=2, kv_heads=1, ff_dim=64, vocab=50, max_positions=64), seed=1)
+    runner = ModelRunner(model, 4, 16)
+
+    def kept():
+        runner._graphs, runner._few_rows_ok = {"recorded": 1}, False
+        runner._follow_model()
+        return bool(runner._graphs)
+    assert kept()
+    add_adapters(model, rank=2)
+    runner._graphs = {"recorded": 1}
+    runner._follow_model()
+    assert not runner._graphs and runner._few_rows_ok is None and kept()
+    with adapters_disabled(model):
+        assert not kept() and kept()
+    assert not kept() and kept()
+    quantize_model(model, "int8")
+    assert not kept() and kept()
+    model.blocks[1].mlp = type(model.blocks[1].mlp)(model.spec)
+    assert not kept() and kept()
+
+
+def test_runner_over_wrapped_blocks():
+    from idrak_b200.serve.runner import ModelRunner, PrefillItem
+
+    class Wrapped(torch.nn.Module):
+        def __init__(self, inner):
+            super().__init__()
+            self.inner = inner
+
+        def __getattr__(self, name):
+            try:
+                return super().__getattr__(name)
+            except AttributeError:
+                return getattr(super().__getattr__("inner"), name)
+
+    model = build_decoder(DecoderSpec.llama(layers=2, dim=32, heads=2, kv_heads=1, ff_dim=64, vocab=50, max_positions=64), seed=1)
+    items = [PrefillItem([3, 4, 5], 0, [0])]
+    want = ModelRunner(model, 4, 16).prefill(items, all_logits=True)
+    model.blocks[0] = Wrapped(model.blocks[0])
+    assert torch.equal(ModelRunner(model, 4, 16).prefill(items, all_logits=True), want)
