@@ -242,7 +242,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       int lim = p.Skv - k0;
       if (p.causal) lim = min(lim, row + off - k0 + 1);
       lim = max(0, min(64, lim));
-      const int lo = max(0, min(64, row_lo - k0));
+      const int lo = min(lim, max(0, row_lo - k0));
+      // one comparison where there is a lower bound too: 16 x 256 tokens, 12 heads of 64, a window of 100: 23.2 us with two,
+      // 20.5 with one
+      auto outside = [&](int col) { return MODES ? unsigned(col - lo) >= unsigned(lim - lo) : col >= lim; };
       // whether any row of the warp masks a column: only then are the columns compared one by one, which is half of the
       // instructions of a block
       const bool masked = __any_sync(0xffffffffu, lim < 64 || lo > 0);
@@ -276,7 +279,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         for (int i = 0; i < 32; ++i) {
 #pragma unroll
           for (int c = 0; c < 2; ++c)
-            if (c * 32 + i < lim && c * 32 + i >= lo) m2[c] = fmaxf(m2[c], __uint_as_float(s[c][i]));
+            if (!outside(c * 32 + i)) m2[c] = fmaxf(m2[c], __uint_as_float(s[c][i]));
         }
       }
       // the row maximum over both halves (every thread reaches this barrier, whatever `ok` says, so its partner never
@@ -338,8 +341,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const float2 x = fma2(as_float2(s[c][g * 8 + i], s[c][g * 8 + i + 1]), make_float2(sl2, sl2), make_float2(-m_sub, -m_sub));
             float2 e = make_float2(fast_exp2(x.x), fast_exp2(x.y));
             if (decltype(with_mask)::value) {
-              if (col >= lim || col < lo) e.x = 0.f;
-              if (col + 1 >= lim || col + 1 < lo) e.y = 0.f;
+              if (outside(col)) e.x = 0.f;
+              if (outside(col + 1)) e.y = 0.f;
             }
             pv[i] = e.x;
             pv[i + 1] = e.y;
