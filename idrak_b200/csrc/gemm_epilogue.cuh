@@ -46,6 +46,8 @@ struct GemmParams {
   int group_b_rows;               // per-row-tile mode: rows of one expert in the stacked B array
   const int* group_kb;            // per-expert-K mode: [groups + 1] bounds of each expert's rows in 64-row blocks
   int groups;                     // per-expert-K mode: experts; C is the stacked [groups * M_per, N] array
+  int whole_tiles;                // CTA pairs: tiles taken whole; the others in `parts` parts of `part_blocks` K blocks
+  int parts, part_blocks;
   int extra_kb;                   // second operand pair (low-rank term): its K extent in 64-element blocks, else 0
 };
 
@@ -337,10 +339,10 @@ __device__ __forceinline__ void half_to_smem(uint8_t* buf, int r, int half, cons
   }
 }
 
-__device__ __forceinline__ bool mode_has_side(int mode) {
+__host__ __device__ __forceinline__ bool mode_has_side(int mode) {
   return mode == kEpiBiasRes || mode == kEpiRes || mode == kEpiGeluGrad || mode == kEpiMulAux;
 }
-__device__ __forceinline__ bool mode_side_is_aux(int mode) { return mode == kEpiGeluGrad || mode == kEpiMulAux; }
+__host__ __device__ __forceinline__ bool mode_side_is_aux(int mode) { return mode == kEpiGeluGrad || mode == kEpiMulAux; }
 
 // The side input a thread fetched ahead of the half-slab it will drain next (16 registers carried across halves,
 // slabs and tiles), so the global-memory latency of the residual / saved pre-activation is off the critical path.
@@ -515,8 +517,11 @@ __device__ __forceinline__ void drain_accumulator(const GemmParams& p, const CUt
 // (null unless idrak_gemm_role_timers switched it on).
 int pick_epi_mode(const GemmParams& p);
 unsigned long long* role_timer_buffer();
-// The CTA-pair kernel (gemm2_tcgen05.cu): whether a product should use it, and its launcher.
-bool gemm_pair_wanted(int M, int N, int K, int splits);
+// The CTA-pair kernel (gemm2_tcgen05.cu): whether a product should use it, how many of its 256 x 256 tiles are taken whole and
+// into how many parts along K the others are cut (needs a workspace of gemm_pair_workspace() floats), and its launcher.
+struct PairPlan { bool use; int whole, parts, part_blocks; };
+PairPlan gemm_pair_plan(int M, int N, int K, bool may_cut);
+long long gemm_pair_workspace(const PairPlan& plan, int M, int N);
 int gemm_pair_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const CUtensorMap& tmC,
-                     const CUtensorMap& tmAux, GemmParams p, int fp16, cudaStream_t stream);
+                     const CUtensorMap& tmAux, GemmParams p, int fp16, const PairPlan& plan, cudaStream_t stream);
 }  // namespace idrak

@@ -374,15 +374,20 @@ static int make_operand_map(CUtensorMap* tm, const void* ptr, int mn_extent, int
 
 using namespace idrak;
 
+IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn);
+
 // Switch the role timers on (a device buffer of 8 * SM-count 64-bit words) or off (null).
 IDRAK_API void idrak_gemm_role_timers(void* device_buffer) {
   g_role_timers.store(static_cast<unsigned long long*>(device_buffer), std::memory_order_relaxed);
 }
 
-// Number of fp32 workspace elements a call with these sizes needs (0 when it will not split K).
-IDRAK_API long long idrak_gemm_workspace_elems(int M, int N, int K, int splits) {
-  if (splits <= 1) return 0;
-  return (long long)splits * M * N;
+// fp32 workspace elements that idrak_gemm_bf16 needs when it is left to choose how K is split (splits = 0): 0 where it does
+// not split. Deterministic in (M, N, K, sms).
+IDRAK_API long long idrak_gemm_workspace_elems(int M, int N, int K) {
+  const PairPlan pair = gemm_pair_plan(M, N, K, true);
+  if (pair.use) return gemm_pair_workspace(pair, M, N);
+  const int splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
+  return splits > 1 ? (long long)splits * M * N : 0;
 }
 
 // Pick a split-K factor so a small output still fills the machine. Deterministic in (M, N, K, sms).
@@ -410,6 +415,7 @@ static int tile_columns(int M, int N, int splits) {
 //   b_mn = 0: B is [N,K] row-major (ldb >= K); b_mn = 1: B is stored [K,N] row-major (ldb >= N)
 // Leading dimensions are in elements and must be multiples of 8 for A and B (TMA strides are 16-byte
 // multiples). C, aux and residual may have any leading dimension; unaligned rows take a scalar path.
+// splits: parts that K is cut into; 0 leaves the choice here (workspace: idrak_gemm_workspace_elems floats).
 // Returns 0, a cudaError, or a negative argument error.
 IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, void* C, int ldc,
                               int c_fp32, int M, int N, int K, const void* bias, const void* residual, int ldr,
@@ -431,6 +437,8 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
   p.ld_aux = ld_aux;
   p.beta = beta;
   p.alpha = alpha;
+  const PairPlan pair = splits == 0 || splits == 1 ? gemm_pair_plan(M, N, K, splits == 0 && workspace) : PairPlan{};
+  if (splits == 0 && !pair.use) splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
   p.splits = (splits > 1 && workspace) ? splits : 1;
   {
     // every split must own at least one k-block
@@ -474,9 +482,7 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
   p.epi_mode = pick_epi_mode(p);
   p.prof = role_timer_buffer();
 
-  // large one-pass products go to CTA pairs (256 x 256 tiles, cta_group::2)
-  if (bn == 256 && gemm_pair_wanted(M, N, K, p.splits))
-    return gemm_pair_launch(A, lda, a_mn, B, ldb, b_mn, tmC, tmAux, p, fp16, stream);
+  if (pair.use) return gemm_pair_launch(A, lda, a_mn, B, ldb, b_mn, tmC, tmAux, p, fp16, pair, stream);
 
   const int units = p.m_tiles * p.n_tiles * p.splits;
   const int grid = min(units, sm_count());

@@ -128,14 +128,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     aux_t = aux
     if act_id in _TWO_OUTPUTS and aux_t is None:
         aux_t = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
-    bn = 128 if N <= 128 else 256
     if splits is None:
-        splits = lib.idrak_gemm_pick_splits(M, N, K, bn)
+        splits = 0                          # the library's choice, unless the tuner has measured a better one
         if M <= 256 and not (beta or act_id):
             splits = _tuned_splits(a, b, a_mn, b_mn, M, N, K, splits, out)
-    ws = None
-    if splits > 1:
-        ws = scratch("gemm_splitk", splits * M * N, torch.float32, a.device)
+    ws_elems = lib.idrak_gemm_workspace_elems(M, N, K) if splits == 0 else splits * M * N if splits > 1 else 0
+    ws = scratch("gemm_splitk", ws_elems, torch.float32, a.device) if ws_elems else None
     if bias is not None:
         assert bias.dtype == torch.bfloat16 and bias.numel() == N
     if residual is not None:

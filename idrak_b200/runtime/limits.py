@@ -92,7 +92,7 @@ def kernel_shapes() -> List[KernelShape]:
         KernelShape("gemm_kernel<256>", "128 x 256 x 64", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
                     "two accumulators of 256 columns ping-pong between the MMA warp and eight epilogue warps"),
         KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128, and products that fill less than half the machine"),
-        KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 4, 320, 4 * 49152 + 32768 + 256 + 1024, 512, 1,
+        KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 5, 384, 5 * 32768 + 65536 + 256 + 1024, 512, 1,
                     "cta_group::2: each CTA holds half of the A rows and half of the B columns"),
         KernelShape("skinny_gemm_kernel", "128 features x 64 tokens x 64, K over a cluster of up to 8", 4, 320, 100352, 64, 2,
                     "partial tiles summed through distributed shared memory"),
