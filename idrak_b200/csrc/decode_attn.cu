@@ -5,24 +5,27 @@
 // listed in block_table[seq, :]; token t of a sequence lives in block block_table[seq, t / block_size] at
 // offset t % block_size.
 //
-// paged_decode_kernel: grid (sequences, kv heads, splits). One CTA serves the G = heads / kv_heads query heads
-// that share a KV head over one contiguous share of the sequence's key blocks: each of its 4 warps stages
-// 32-key tiles of K and V in shared memory with asynchronous 16-byte copies and runs Q·K^T and P·V as
-// m16n8k16 tensor-core MMAs with the G query heads as the (padded) 16 rows, keeping an online softmax per row
-// in registers. Splits write (max, sum, partial output) and decode_merge_kernel combines them in split
-// order. The kernel is bound by the bytes of K and V (each is read once); warp-level MMAs are enough to keep up
-// with them - a 16-row tile cannot feed tcgen05's 128-row instruction - while the FMA pipes are not.
+// paged_decode_kernel: grid (sequences, kv heads, splits). One CTA serves the G = heads / kv_heads query heads that share a
+// KV head over one share of the sequence's keys. Its four warps each walk tiles of 16 keys through a ring of their own: the
+// tile's rows arrive by TMA (a box of up to 16 consecutive slots of one cache block, one head), several tiles ahead, and a warp
+// waits for nothing but its next tile. The warp takes both products transposed, so that the keys (S^T = K Q^T) and the head's
+// elements (O^T = V^T P^T) fill the 16 rows of a warp-level m16n8k16 MMA and the query heads its 8 columns; P^T is turned from
+// the layout of a result into that of an operand by four byte-matrix moves. With the query heads as the 16 rows - 4 of them in
+// use where 32 heads share 8 - a tile of 32 keys took 1780 instructions, half of them copies a lane at a time, and the kernel was
+// bound by issuing them; it is about 600 now, and the keys and values on their way bound it. Warp-level MMAs are enough: tcgen05's
+// 128 rows have nothing to fill them.
+//
+// int8 cache: the codes enter the tensor core as exact bf16 numbers (code / 64), converted in registers on their way from
+// shared memory: a lane takes 16 codes of a key at once, and since a sum over d has no order of its own the query operand is laid
+// out to match; values come transposed two codes at a time and their even and odd elements form the two halves of a fragment. A
+// key's scale multiplies its scores and a value's scale its probability in fp32 before the rounding to bf16.
+//
+// Measured, us (32 query heads on 8, head size 128): 64 sequences of 128 to 2304 tokens (386 MB) 92
+// before and 77 now; 150 of 128 to 1024, int8 cache (198 MB) 91 and 54; one of 8000 20.2 and 16.1; 16 of 16 to 60 8.2 and 5.4.
 //
 // The host knows only a bound on the lengths, so a share is at least `min_tiles` tiles and a sequence uses as many of the
-// splits as its own length fills; the other CTAs leave at once, and a sequence with one share is written out directly.
-// Short shares even out a batch whose contexts differ: 64 sequences of 128 to 2304 tokens (8 KV heads, head size 128,
-// 386 MB) took 95 us unsplit - 512 CTAs on 444 places, the longest alone at the end - and 84 us in shares of 1024 keys;
-// 16 of them 51 and 28.5 us in shares of 512.
-//
-// int8 cache: the codes enter the tensor core as exact bf16 numbers (code / 64, one permute and one fused multiply-add per
-// two codes); a key's scale multiplies its column of scores and a value's scale its column of probabilities, so nothing
-// is rounded that a bf16 cache would not round. Converting and scaling every element in fp32 had bound the kernel: 150
-// sequences of 606 tokens on average (192 MB) 152 us, now 88 us.
+// splits as its own length fills; the other CTAs leave at once, and a sequence with one share is written out directly. Splits
+// write (max, sum, partial output) and decode_merge_kernel combines them in split order.
 //
 // Reference counterparts: attention_decode_{f32,int8,bf16} (split over blocks, last block merges;
 // src/Idrak.Gpu/Cuda/PtxKernels.Rows.cs:2047-2060), kv_write_{f32,bf16} (PtxKernels.Decoding.cs:12),
@@ -33,7 +36,7 @@
 namespace idrak {
 
 constexpr int kDecWarps = 4;
-constexpr int kDecTile = 32;       // keys per warp tile
+constexpr int kDecTile = 16;       // keys per warp tile
 constexpr int kDecMaxGroup = 16;   // query heads per KV head
 
 struct DecodeParams {
@@ -51,11 +54,11 @@ struct DecodeParams {
   int min_tiles;                 // tiles per split at least
   float scale_log2;
   int window;                    // 0 = full; else attend to the last `window` positions only
+  int box_log2;                  // slots that one copy brings: the largest power of two up to 16 that divides block_size
+  Status* st;
 };
 
-// ---- warp-level tensor-core pieces (mma.sync m16n8k16, bf16 in, fp32 accumulate). Decode attention is bound by
-// the bytes of K and V; the tensor pipe only has to keep up with them, which these 16-row MMAs do with the G <= 16
-// query heads of a KV head as the rows - the FMA pipes cannot (2 multiply-adds per cache byte).
+// ---- warp-level tensor-core pieces (mma.sync m16n8k16, bf16 in, fp32 accumulate)
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
@@ -63,40 +66,42 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
       : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* smem_row) {
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t smem_row) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem_row)));
+               : "r"(smem_row) : "memory");
 }
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* smem_row) {
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t smem_row) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(smem_u32(smem_row)));
+               : "r"(smem_row) : "memory");
 }
-// 16-byte asynchronous copy global -> shared; `bytes` = 0 writes zeros instead (keys past the sequence's end)
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(bytes)
-               : "memory");
+// an 8 x 8 matrix of 16-bit elements, a row per four lanes, transposed across the warp
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// wait until at most one of this thread's committed groups is still in flight (groups complete in order)
-__device__ __forceinline__ void cp_async_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 
-// 16 int8 codes -> 16 bf16 values code / 64 (two 16-byte words), exactly: an unsigned integer u < 256 in a 16-bit lane is,
-// read as bf16, u * 2^-133, and one fused multiply-add takes it to (u - 128) / 64.
+// 2^x, results below the smallest normal number flushed: the library's routine spends instructions on those.
+__device__ __forceinline__ float dec_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Two int8 codes (biased by 128, in the low bytes of the two halves) -> two bf16 values code / 64, exactly: an unsigned integer
+// u < 256 in a 16-bit lane is, read as bf16, u * 2^-133, and one fused multiply-add takes it to (u - 128) / 64.
 __device__ __forceinline__ uint32_t codes_pair(uint32_t t) {
   const uint32_t mul = 0x7F007F00u, add = 0xC000C000u;      // 2^127, -128 / 64
   const __nv_bfloat162 v = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&t), *reinterpret_cast<const __nv_bfloat162*>(&mul),
                                    *reinterpret_cast<const __nv_bfloat162*>(&add));
   return *reinterpret_cast<const uint32_t*>(&v);
-}
-__device__ __forceinline__ void expand16(const uint4& raw, uint4& lo, uint4& hi) {
-  const uint32_t a = raw.x ^ 0x80808080u, b = raw.y ^ 0x80808080u, c = raw.z ^ 0x80808080u, d = raw.w ^ 0x80808080u;
-  lo = make_uint4(codes_pair(__byte_perm(a, 0, 0x4140)), codes_pair(__byte_perm(a, 0, 0x4342)),
-                  codes_pair(__byte_perm(b, 0, 0x4140)), codes_pair(__byte_perm(b, 0, 0x4342)));
-  hi = make_uint4(codes_pair(__byte_perm(c, 0, 0x4140)), codes_pair(__byte_perm(c, 0, 0x4342)),
-                  codes_pair(__byte_perm(d, 0, 0x4140)), codes_pair(__byte_perm(d, 0, 0x4342)));
 }
 
 // The share of a sequence's tiles that each split takes, and how many splits that leaves with work.
@@ -109,28 +114,60 @@ __device__ __forceinline__ void key_span(int len, int window, int& first_tile, i
   span = (len + kDecTile - 1) / kDecTile - first_tile;
 }
 
-// KV8 = 1: the cache holds int8 codes with one scale per (slot, kv head) (norm_rope_kv's int8 mode). A tile's codes
-// are staged into the upper half of each shared-memory row and expanded to bf16 in place - lane r owns row r and
-// walks it front to back, and the bf16 written for chunk c never reaches the codes of a chunk not yet read - so the
-// tensor-core part below is unchanged and the cache costs half the bytes.
-template <int D, int KV8>
-__global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const DecodeParams p) {
-  pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
-  pdl_wait();
-  constexpr int kRow = D * 2 + 16;                       // padded shared-memory row (bytes): conflict-free ldmatrix
-  constexpr int kChunks = D / 8;                         // 16-byte chunks per key row
-  constexpr int KS = D / 16;                             // k-steps of Q·K^T
-  constexpr int NT = D / 8;                              // n-tiles of P·V
-  extern __shared__ uint8_t dsm[];
+// A tile of keys or values in shared memory: 16 rows, in column blocks of up to 128 bytes as TMA writes them; with SWIZZLE the
+// 16-byte pieces of a row are exchanged by the row's place in the pattern, so that the eight rows of a matrix load touch all banks.
+template <int D, int KV8, bool SWIZZLE>
+struct DecTile {
+  static constexpr int kRowBytes = KV8 ? D : 2 * D;
+  static constexpr int kBlock = kRowBytes < 128 ? kRowBytes : 128;       // bytes of a row in a column block
+  static constexpr int kPitch = SWIZZLE ? kBlock : 128;                  // a copy's place starts at a multiple of 128 bytes
+  static constexpr int kBlocks = kRowBytes / kBlock;
+  static constexpr int kBytes = kDecTile * kPitch * kBlocks;
+  static constexpr int kStage = 2 * kBytes;
+  // Of a warp: three CTAs share an SM over a bf16 cache of head size 128, four otherwise. us, 64 sequences of 128 to 2304 keys /
+  // 64 of 1000 / 16 of 128 to 2304: 16 KB 76.8 / 58.4 / 23.1, 24 KB and two CTAs 79.9 / 55.3 / 27.0; 150 of 128 to 1024, int8: 12 KB
+  // 53.9, 16 KB and three CTAs 59.4, 24 KB 69.6; 32 of 500 to 600, 12 heads of 64: 14.8, 15.1, 19.7.
+  static constexpr int kRing = !KV8 && D == 128 ? 16384 : 12288;
+  static constexpr int kStages = kRing / kStage;
+  static __device__ __forceinline__ uint32_t at(int row, int piece) {
+    constexpr int kPieces = kBlock / 16;
+    const int c = piece % kPieces;
+    const int x = !SWIZZLE ? c : kBlock == 128 ? c ^ (row & 7) : c ^ ((row >> 1) & 3);
+    return uint32_t((piece / kPieces) * kDecTile * kPitch + row * kPitch + x * 16);
+  }
+};
+
+// NH: column tiles of 8 query heads. SWIZZLE: the boxes have 8 rows or more (a smaller block size is taken unswizzled, row groups
+// of fewer rows would not start where the pattern does).
+template <int D, int KV8, int NH, bool SWIZZLE>
+__global__ void __launch_bounds__(kDecWarps * 32)
+paged_decode_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeParams p) {
+  using T = DecTile<D, KV8, SWIZZLE>;
+  constexpr int S = T::kStages;
+  constexpr int KS = D / 16;                             // steps of K Q^T over d, and row tiles of O^T
+  extern __shared__ uint8_t dsm_raw[];
+  uint8_t* dsm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsm_raw) + 1023) & ~uintptr_t(1023));
   const int seq = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
   const int G = p.H / p.Hkv;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* sqb = dsm;                                                          // [16][kRow] queries (bf16), rows >= G zero
-  uint8_t* sk = dsm + 16 * kRow + warp * (2 * kDecTile * kRow);                // this warp's K tile
-  uint8_t* sv = sk + kDecTile * kRow;                                          // and V tile
-  // the warps' partial outputs are merged in the space of the K / V tiles once every warp is done with them: the kernel
-  // then needs 74 KB instead of 107 KB (head size 128) and three CTAs share an SM instead of two
-  float* smerge = reinterpret_cast<float*>(dsm + 16 * kRow);
+  const int g = lane >> 2, t4 = lane & 3;                // row and column pair of this lane in an MMA fragment
+  uint8_t* ring = dsm + warp * T::kRing;                 // [stage][K, V]
+  uint64_t* full = reinterpret_cast<uint64_t*>(dsm + kDecWarps * T::kRing) + warp * S;
+  float* scales = reinterpret_cast<float*>(dsm + kDecWarps * T::kRing + kDecWarps * S * 8) + warp * S * 32;   // int8: [stage][K, V][16]
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(dsm + kDecWarps * T::kRing + kDecWarps * S * (8 + 128));
+  // the warps' partial outputs are merged in the place of the tiles once every warp is done with them
+  float* smerge = reinterpret_cast<float*>(dsm);
+
+  pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
+  if (lane == 0) {
+    for (int i = 0; i < S; ++i) mbar_init(&full[i], KV8 ? 33 : 1);
+    if (warp == 0) *abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+  }
+  __syncthreads();
+  pdl_wait();
 
   const int len = p.seq_lens[seq];
   const int first_pos = (p.window > 0 && len > p.window) ? len - p.window : 0;
@@ -140,219 +177,275 @@ __global__ void __launch_bounds__(kDecWarps * 32) paged_decode_kernel(const Deco
   const bool alone = span <= per;                        // the only split of its sequence with work
   if (split > 0 && split * per >= span) return;
   const int t0 = first_tile + split * per, t1 = min(first_tile + span, t0 + per);
-
-  // queries of the G heads of this KV head -> shared (bf16, rows padded to 16 with zeros)
-  for (int i = threadIdx.x; i < 16 * kChunks; i += blockDim.x) {
-    const int g = i / kChunks, c = i - g * kChunks;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (g < G) v = *reinterpret_cast<const uint4*>(p.q + size_t(seq) * p.q_stride + size_t(kvh * G + g) * D + c * 8);
-    *reinterpret_cast<uint4*>(sqb + g * kRow + c * 16) = v;
-  }
-  __syncthreads();
-  // A fragments of Q for every k-step: ldmatrix.x4 gives (rows 0-7, k 0-7), (rows 8-15, k 0-7), (rows 0-7, k 8-15),
-  // (rows 8-15, k 8-15) = a0..a3
-  uint32_t qa[KS][4];
-#pragma unroll
-  for (int ks = 0; ks < KS; ++ks)
-    ldmatrix_x4(qa[ks], sqb + (lane & 15) * kRow + ks * 32 + (lane >> 4) * 16);
-
-  float o[NT][4];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;      // rows lane / 4 and lane / 4 + 8
-  const size_t tok_stride = size_t(p.Hkv) * D;
   const int* table = p.block_table + size_t(seq) * p.max_blocks;
 
-  // lane r looks up the cache slot of key row r of a tile once (one division and one table read per lane and tile);
-  // the copy loops fetch a row's slot by shuffle, so a 16-byte copy costs a shuffle and a multiply-add, not a
-  // division, a remainder and a table read
-  auto slot_of = [&](int tile) {
-    const int pos = tile * kDecTile + lane;
-    return (tile < t1 && pos < len) ? table[pos / p.block_size] * p.block_size + pos % p.block_size : -1;
+  // The copies of a tile: boxes of `box` slots, each of K and V and each of their column blocks, one to a lane. The slots of the
+  // boxes that the warp comes to next are looked up 32 at a time, a lane each, and the next 32 while these are in use: a lookup
+  // for every tile made the warp wait for it, as long as the tile's arithmetic takes.
+  const int box_log2 = p.box_log2, box_slots = 1 << box_log2, boxes_log2 = 4 - box_log2, boxes = 1 << boxes_log2;
+  const int copies = boxes * 2 * T::kBlocks;
+  const int mine = t1 > t0 + warp ? (t1 - t0 - warp + kDecWarps - 1) / kDecWarps : 0;       // tiles of this warp
+  auto look_up = [&](int chunk) {
+    const int j = chunk * 32 + lane, i = j >> boxes_log2;
+    const int pos = (t0 + warp + i * kDecWarps) * kDecTile + ((j & (boxes - 1)) << box_log2);
+    return i < mine && pos < len ? table[pos / p.block_size] * p.block_size + pos % p.block_size : -1;
   };
-  // one 32-key tile of K or V (bf16 cache) into a warp's buffer, one commit group
-  auto copy_rows = [&](uint8_t* dst, const __nv_bfloat16* cache, int slots) {
-#pragma unroll 4
-    for (int i = lane; i < kDecTile * kChunks; i += 32) {
-      const int r = i / kChunks, c = i - r * kChunks;                // kChunks is a power of two: shifts
-      const int slot = __shfl_sync(0xffffffffu, slots, r);
-      const bool live = slot >= 0;
-      const size_t off = live ? size_t(slot) * tok_stride + size_t(kvh) * D + c * 8 : 0;
-      cp_async16(dst + r * kRow + c * 16, cache + off, live ? 16 : 0);
+  int chunk = 0, slots = look_up(0), next_slots = look_up(1);
+  auto issue = [&](int i, int stage) {
+    const int j = i << boxes_log2;
+    if ((j >> 5) != chunk) {
+      ++chunk;
+      slots = next_slots;
+      next_slots = look_up(chunk + 1);
     }
-    cp_async_commit();
-  };
-  // bf16 cache: the copies run one step ahead of the arithmetic inside the warp's single pair of buffers - the keys of
-  // the next tile are requested as soon as Q K^T of this tile has read its keys (they fly during the softmax and P V),
-  // the values of the next tile once P V has read its values (they fly during the next Q K^T and softmax)
-  // int8 cache: the same, with the codes of a tile staged in the upper half of each row and expanded in place by the
-  // lane that owns the row once they have landed
-  constexpr int kByteChunks = D / 16;                    // 16-byte chunks of int8 codes per key row
-  auto copy_codes = [&](uint8_t* dst, const __nv_bfloat16* cache, int slots) {
-    const int8_t* codes = reinterpret_cast<const int8_t*>(cache);
-#pragma unroll 4
-    for (int i = lane; i < kDecTile * kByteChunks; i += 32) {
-      const int r = i / kByteChunks, c = i - r * kByteChunks;
-      const int slot = __shfl_sync(0xffffffffu, slots, r);
-      const bool live = slot >= 0;
-      const size_t off = live ? size_t(slot) * tok_stride + size_t(kvh) * D + c * 16 : 0;
-      cp_async16(dst + r * kRow + D + c * 16, codes + off, live ? 16 : 0);
+    const int pos0 = (t0 + warp + i * kDecWarps) * kDecTile;
+    if (lane == 0) {
+      const int used = (min(len - pos0, kDecTile) + box_slots - 1) >> box_log2;       // boxes with a key in them
+      mbar_expect_tx(&full[stage], uint32_t((used << box_log2) * (T::kRowBytes * 2)));
     }
-    cp_async_commit();
-  };
-  auto expand_row = [&](uint8_t* row) {                  // this lane's row: codes -> bf16, front to back
-#pragma unroll
-    for (int c = 0; c < kByteChunks; ++c) {
-      const uint4 codes = *reinterpret_cast<const uint4*>(row + D + c * 16);
-      uint4 lo, hi;
-      expand16(codes, lo, hi);
-      *reinterpret_cast<uint4*>(row + c * 32) = lo;
-      *reinterpret_cast<uint4*>(row + c * 32 + 16) = hi;
-    }
-  };
-  int next_slots = -1;
-  if (t0 + warp < t1) {
-    next_slots = slot_of(t0 + warp);
-    if (!KV8) {
-      copy_rows(sk, p.k_cache, next_slots);
-      copy_rows(sv, p.v_cache, next_slots);
+    __syncwarp();
+    uint8_t* to = ring + stage * T::kStage;
+    if (box_log2 == 4) {                                 // a box a tile: one lane a column block of K or V
+      const int slot = __shfl_sync(0xffffffffu, slots, j & 31);
+      if (lane < 2 * T::kBlocks)
+        tma_load_3d(to + (lane & 1) * T::kBytes + (lane >> 1) * kDecTile * T::kPitch, (lane & 1) ? &tmV : &tmK, &full[stage],
+                    (lane >> 1) * (KV8 ? T::kBlock : T::kBlock / 2), kvh, slot);
     } else {
-      copy_codes(sk, p.k_cache, next_slots);
-      copy_codes(sv, p.v_cache, next_slots);
+      for (int c0 = 0; c0 < copies; c0 += 32) {
+        const int c = c0 + lane, box = min(c / (2 * T::kBlocks), boxes - 1), which = c & 1, column = (c % (2 * T::kBlocks)) >> 1;
+        const int slot = __shfl_sync(0xffffffffu, slots, (j + box) & 31);
+        if (c < copies && slot != -1)
+          tma_load_3d(to + which * T::kBytes + column * kDecTile * T::kPitch + (box << box_log2) * T::kPitch, which ? &tmV : &tmK,
+                      &full[stage], column * (KV8 ? T::kBlock : T::kBlock / 2), kvh, slot);
+      }
+    }
+    if (KV8) {
+      // the scales of the tile's 16 keys and 16 values, a lane each, 0 outside the sequence
+      const int row = lane & 15;
+      const int slot = __shfl_sync(0xffffffffu, slots, (j + (row >> box_log2)) & 31);
+      const bool live = slot != -1 && pos0 + row < len;
+      const float* src = (lane < 16 ? p.k_scale : p.v_scale) + (live ? (size_t(slot) + (row & (box_slots - 1))) * p.Hkv + kvh : 0);
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(scales + stage * 32 + lane)), "l"(src), "r"(live ? 4 : 0)
+                   : "memory");
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(&full[stage])) : "memory");
+    }
+  };
+  for (int i = 0; i < S && i < mine; ++i) issue(i, i);
+
+  // the queries of the heads of this KV head as B operand: column = head, and the elements of d that step ks has for this lane
+  uint32_t qb[NH][KS][2];
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+    const int head = h * 8 + g;
+    const __nv_bfloat16* src = p.q + size_t(seq) * p.q_stride + size_t(kvh * G + head) * D;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      // bf16 keys: elements 2t, 2t + 1 and 2t + 8, 2t + 9 of the step's 16; codes: a lane holds 16 codes in a row of its key's 64,
+      // four of them in each of the four steps
+      const int d = KV8 ? (ks >> 2) * 64 + t4 * 16 + (ks & 3) * 4 : ks * 16 + t4 * 2;
+      qb[h][ks][0] = head < G ? *reinterpret_cast<const uint32_t*>(src + d) : 0u;
+      qb[h][ks][1] = head < G ? *reinterpret_cast<const uint32_t*>(src + d + (KV8 ? 2 : 8)) : 0u;
     }
   }
 
-  for (int t = t0 + warp; t < t1; t += kDecWarps) {
-    const int key0 = t * kDecTile;
-    // int8 cache: this lane's row scales (0 for a key past the end: the codes are zeros there anyway)
-    float ks = 0.f, vs = 0.f;
-    if (KV8 && next_slots >= 0) {
-      ks = p.k_scale[size_t(next_slots) * p.Hkv + kvh] * (64.f * p.scale_log2);
-      vs = p.v_scale[size_t(next_slots) * p.Hkv + kvh] * 64.f;
-    }
-    cp_async_wait_but_one();                             // this tile's keys have landed; its values may still fly
-    __syncwarp();
+  float o[NH][KS][4];
+  float m[NH][2], l[NH][2];                              // of heads 8 h + 2 t4 and the next; sums of this lane's keys only
+#pragma unroll
+  for (int h = 0; h < NH; ++h) {
+#pragma unroll
+    for (int n = 0; n < KS; ++n) { o[h][n][0] = o[h][n][1] = o[h][n][2] = o[h][n][3] = 0.f; }
+    m[h][0] = m[h][1] = -INFINITY;
+    l[h][0] = l[h][1] = 0.f;
+  }
+  // Where this lane's pieces of a tile stand. The swizzle exchanges pieces within 128 bytes by an exclusive or, so the pieces of
+  // the other steps are one exclusive or away: 32 bytes a step of two pieces.
+  const uint32_t k_at = KV8 ? T::at(g, t4) : T::at(lane & 15, lane >> 4);
+  const uint32_t v_at = KV8 ? T::at((lane & 7) + (((lane >> 3) & 1) << 3), lane >> 4) : T::at((lane & 7) + ((lane >> 4) << 3), (lane >> 3) & 1);
+  auto step_at = [](uint32_t at, int step) {              // the piece 2 * step further on
+    constexpr int kSteps = T::kBlock / 32;
+    return (at ^ uint32_t((step % kSteps) * 32)) + uint32_t((step / kSteps) * kDecTile * T::kPitch);
+  };
+
+  bool ok = true;
+  int stage = 0;
+  uint32_t phase = 0;
+  for (int i = 0; i < mine; ++i) {
+    ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, p.st, kTimeoutSmemFull, (9u << 16) | stage));
+    if (!ok) break;
+    // factors of this lane's two keys, rows g and g + 8
+    float ks[2] = {p.scale_log2, p.scale_log2}, vs[2] = {1.f, 1.f};
     if (KV8) {
-      expand_row(sk + lane * kRow);
-      __syncwarp();
-    }
-    // ---- S[16 x 32] = Q · K^T: 4 n-tiles of 8 keys
-    float s[4][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-#pragma unroll
-      for (int ks = 0; ks < KS; ks += 2) {
-        // matrices: (keys n*8.., d ks*16 + 0..7), (.., +8..15), (.., (ks+1)*16 + 0..7), (.., +8..15)
-        uint32_t kb[4];
-        ldmatrix_x4(kb, sk + (n * 8 + (lane & 7)) * kRow + ks * 32 + (lane >> 3) * 16);
-        mma_bf16_16816(s[n], qa[ks], kb[0], kb[1]);
-        mma_bf16_16816(s[n], qa[ks + 1], kb[2], kb[3]);
+      for (int e = 0; e < 2; ++e) {
+        ks[e] = scales[stage * 32 + g + e * 8] * (64.f * p.scale_log2);
+        vs[e] = scales[stage * 32 + 16 + g + e * 8] * 64.f;
       }
     }
-    __syncwarp();                                        // every lane has read this tile's keys
-    next_slots = slot_of(t + kDecWarps);
-    if (!KV8) copy_rows(sk, p.k_cache, next_slots);      // (an empty group when there is no next tile)
-    else copy_codes(sk, p.k_cache, next_slots);
-    // ---- mask, online softmax (log2 domain) for rows r0 = lane / 4 and r0 + 8
-    float mx0 = -INFINITY, mx1 = -INFINITY;
+    uint8_t* tile_k = ring + stage * T::kStage;
+    const uint32_t sk = smem_u32(tile_k), sv = sk + T::kBytes;
+    const int key0 = (t0 + warp + i * kDecWarps) * kDecTile;
+    const bool whole = key0 + kDecTile <= len && key0 >= first_pos;        // every key of the tile is seen
+    if (!KV8 && key0 + kDecTile > len) {
+      // values past the end get probability 0, but may be anything
+      for (int c = lane; c < kDecTile * T::kRowBytes / 16; c += 32) {
+        const int row = c / (T::kRowBytes / 16), piece = c % (T::kRowBytes / 16);
+        if (key0 + row >= len)
+          *reinterpret_cast<uint4*>(tile_k + T::kBytes + T::at(row, piece)) = make_uint4(0, 0, 0, 0);
+      }
+      __syncwarp();
+    }
+    // ---- S^T [16 keys x heads] = K Q^T, two sums over alternate steps
+    float s[NH][2][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
+    for (int h = 0; h < NH; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) { s[h][e][0] = s[h][e][1] = s[h][e][2] = s[h][e][3] = 0.f; }
+    if (!KV8) {
+#pragma unroll
+      for (int k = 0; k < KS; ++k) {
+        uint32_t a[4];
+        ldmatrix_x4(a, sk + step_at(k_at, k));
+#pragma unroll
+        for (int h = 0; h < NH; ++h) mma_bf16_16816(s[h][k & 1], a, qb[h][k][0], qb[h][k][1]);
+      }
+    } else {
+#pragma unroll
+      for (int kk = 0; kk < D / 64; ++kk) {
+        const uint4 lo = lds128(sk + step_at(k_at, kk * 2)), hi = lds128(sk + step_at(k_at, kk * 2) + 8 * T::kPitch);
+        const uint32_t w0[4] = {lo.x, lo.y, lo.z, lo.w}, w1[4] = {hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint32_t x0 = w0[w] ^ 0x80808080u, x1 = w1[w] ^ 0x80808080u;
+          const uint32_t a[4] = {codes_pair(__byte_perm(x0, 0, 0x4140)), codes_pair(__byte_perm(x1, 0, 0x4140)),
+                                 codes_pair(__byte_perm(x0, 0, 0x4342)), codes_pair(__byte_perm(x1, 0, 0x4342))};
+#pragma unroll
+          for (int h = 0; h < NH; ++h) mma_bf16_16816(s[h][w & 1], a, qb[h][kk * 4 + w][0], qb[h][kk * 4 + w][1]);
+        }
+      }
+    }
+    // ---- online softmax (log2 domain) over the keys, per head
+    uint32_t pb[NH][2];                                  // P^T as B operand
+    bool moved = false;
+    float mn[NH][2];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int pos = key0 + n * 8 + 2 * (lane & 3) + j;
-        const bool valid = pos < len && pos >= first_pos;
-        const float f = KV8 ? __shfl_sync(0xffffffffu, ks, n * 8 + 2 * (lane & 3) + j) : p.scale_log2;
-        s[n][j] = valid ? s[n][j] * f : -INFINITY;
-        s[n][2 + j] = valid ? s[n][2 + j] * f : -INFINITY;
-        mx0 = fmaxf(mx0, s[n][j]);
-        mx1 = fmaxf(mx1, s[n][2 + j]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          s[h][0][e * 2 + j] = (s[h][0][e * 2 + j] + s[h][1][e * 2 + j]) * ks[e];
+          if (!whole) {
+            const int pos = key0 + g + e * 8;
+            if (pos >= len || pos < first_pos) s[h][0][e * 2 + j] = -INFINITY;
+          }
+        }
+        float mx = fmaxf(s[h][0][j], s[h][0][2 + j]);
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+        mn[h][j] = fmaxf(m[h][j], mx);
+        moved = moved || mn[h][j] > m[h][j];
       }
     }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-    const float a0 = (m0 == -INFINITY) ? 0.f : exp2f(m0 - mn0);
-    const float a1 = (m1 == -INFINITY) ? 0.f : exp2f(m1 - mn1);
-    float sum0 = 0.f, sum1 = 0.f;
-    uint32_t pa[2][4];                                   // P as A fragments of the two 16-key k-steps
+    if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const float p00 = (mn0 == -INFINITY) ? 0.f : exp2f(s[n][0] - mn0);
-      const float p01 = (mn0 == -INFINITY) ? 0.f : exp2f(s[n][1] - mn0);
-      const float p10 = (mn1 == -INFINITY) ? 0.f : exp2f(s[n][2] - mn1);
-      const float p11 = (mn1 == -INFINITY) ? 0.f : exp2f(s[n][3] - mn1);
-      sum0 += p00 + p01;
-      sum1 += p10 + p11;
-      const float v0 = KV8 ? __shfl_sync(0xffffffffu, vs, n * 8 + 2 * (lane & 3)) : 1.f;
-      const float v1 = KV8 ? __shfl_sync(0xffffffffu, vs, n * 8 + 2 * (lane & 3) + 1) : 1.f;
-      pa[n >> 1][(n & 1) * 2 + 0] = KV8 ? pack_bf16x2(p00 * v0, p01 * v1) : pack_bf16x2(p00, p01);
-      pa[n >> 1][(n & 1) * 2 + 1] = KV8 ? pack_bf16x2(p10 * v0, p11 * v1) : pack_bf16x2(p10, p11);
-    }
-    sum0 += __shfl_xor_sync(0xffffffffu, sum0, 1);
-    sum0 += __shfl_xor_sync(0xffffffffu, sum0, 2);
-    sum1 += __shfl_xor_sync(0xffffffffu, sum1, 1);
-    sum1 += __shfl_xor_sync(0xffffffffu, sum1, 2);
-    l0 = l0 * a0 + sum0;
-    l1 = l1 * a1 + sum1;
-    m0 = mn0;
-    m1 = mn1;
+      for (int h = 0; h < NH; ++h) {
+        float a[2];
 #pragma unroll
-    for (int n = 0; n < NT; ++n) { o[n][0] *= a0; o[n][1] *= a0; o[n][2] *= a1; o[n][3] *= a1; }
-    cp_async_wait_but_one();                             // this tile's values have landed; the next keys may still fly
-    __syncwarp();
-    if (KV8) {
-      expand_row(sv + lane * kRow);
-      __syncwarp();
-    }
-    // ---- O[16 x D] += P[16 x 32] · V[32 x D]: V is [key][d], so its B fragments come through transposing loads
+        for (int j = 0; j < 2; ++j) {
+          a[j] = (m[h][j] == -INFINITY) ? 0.f : dec_exp2(m[h][j] - mn[h][j]);
+          m[h][j] = mn[h][j];
+          l[h][j] *= a[j];
+        }
 #pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
-#pragma unroll
-      for (int n = 0; n < NT; n += 2) {
-        // matrices: (keys kk*16 + 0..7, d n*8..), (keys +8..15, d n*8..), (keys 0..7, d (n+1)*8..), (keys 8..15, ..)
-        uint32_t vb[4];
-        ldmatrix_x4_trans(vb, sv + (kk * 16 + (lane & 15)) * kRow + (n + (lane >> 4)) * 16);
-        mma_bf16_16816(o[n], pa[kk], vb[0], vb[1]);
-        mma_bf16_16816(o[n + 1], pa[kk], vb[2], vb[3]);
+        for (int n = 0; n < KS; ++n) { o[h][n][0] *= a[0]; o[h][n][1] *= a[1]; o[h][n][2] *= a[0]; o[h][n][3] *= a[1]; }
       }
     }
-    __syncwarp();
-    if (!KV8) copy_rows(sv, p.v_cache, next_slots);      // every lane has read this tile's values
-    else copy_codes(sv, p.v_cache, next_slots);
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      float e[4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float base = m[h][j] == -INFINITY ? 0.f : m[h][j];
+        e[j] = dec_exp2(s[h][0][j] - base);
+        e[2 + j] = dec_exp2(s[h][0][2 + j] - base);
+        l[h][j] += e[j] + e[2 + j];
+      }
+      pb[h][0] = transpose_8x8(pack_bf16x2(e[0] * vs[0], e[1] * vs[0]));
+      pb[h][1] = transpose_8x8(pack_bf16x2(e[2] * vs[1], e[3] * vs[1]));
+    }
+    // ---- O^T [d x heads] += V^T P^T
+    if (!KV8) {
+#pragma unroll
+      for (int n = 0; n < KS; ++n) {
+        uint32_t a[4];
+        ldmatrix_x4_trans(a, sv + step_at(v_at, n));
+#pragma unroll
+        for (int h = 0; h < NH; ++h) mma_bf16_16816(o[h][n], a, pb[h][0], pb[h][1]);
+      }
+    } else {
+#pragma unroll
+      for (int n = 0; n < KS; n += 2) {
+        uint32_t r[4];
+        ldmatrix_x4_trans(r, sv + step_at(v_at, n / 2));
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          // two keys' codes of elements 2u and 2u + 1: the even elements are rows 0..7 of the fragment, the odd ones rows 8..15
+          const uint32_t x0 = r[e * 2] ^ 0x80808080u, x1 = r[e * 2 + 1] ^ 0x80808080u;
+          const uint32_t a[4] = {codes_pair(__byte_perm(x0, 0, 0x4240)), codes_pair(__byte_perm(x0, 0, 0x4341)),
+                                 codes_pair(__byte_perm(x1, 0, 0x4240)), codes_pair(__byte_perm(x1, 0, 0x4341))};
+#pragma unroll
+          for (int h = 0; h < NH; ++h) mma_bf16_16816(o[h][n + e], a, pb[h][0], pb[h][1]);
+        }
+      }
+    }
+    __syncwarp();                                        // every lane has read the tile
+    if (i + S < mine) issue(i + S, stage);
+    if (++stage == S) { stage = 0; phase ^= 1; }
   }
-  cp_async_wait_all();
+  if (!ok) {                                             // let the copies on their way land before the CTA leaves
+    const uint64_t from = global_timer_ns();
+    while (global_timer_ns() - from < 200000ull) { }
+  }
 
   // ---- combine the 4 warps of the CTA (in warp order), then write the split's partial or the final output
-  // smerge layout: [warp][16][D + 2], over the tiles: nobody may still be reading a tile
-  __syncthreads();
-  {
-    const int r0 = lane >> 2, c0 = 2 * (lane & 3);
-    float* d0 = smerge + (size_t(warp) * 16 + r0) * (D + 2);
-    float* d1 = smerge + (size_t(warp) * 16 + r0 + 8) * (D + 2);
+  // smerge layout: [warp][head][D + 2], over the tiles: nobody may still be reading a tile
 #pragma unroll
-    for (int n = 0; n < NT; ++n) {
-      d0[n * 8 + c0] = o[n][0]; d0[n * 8 + c0 + 1] = o[n][1];
-      d1[n * 8 + c0] = o[n][2]; d1[n * 8 + c0 + 1] = o[n][3];
+  for (int h = 0; h < NH; ++h)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      l[h][j] += __shfl_xor_sync(0xffffffffu, l[h][j], 4);
+      l[h][j] += __shfl_xor_sync(0xffffffffu, l[h][j], 8);
+      l[h][j] += __shfl_xor_sync(0xffffffffu, l[h][j], 16);
     }
-    if ((lane & 3) == 0) { d0[D] = m0; d0[D + 1] = l0; d1[D] = m1; d1[D + 1] = l1; }
-  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < NH; ++h)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int head = h * 8 + t4 * 2 + j;
+      if (head >= G) continue;
+      float* dst = smerge + (size_t(warp) * G + head) * (D + 2);
+#pragma unroll
+      for (int n = 0; n < KS; ++n) {
+        dst[n * 16 + (KV8 ? 2 * g : g)] = o[h][n][j];
+        dst[n * 16 + (KV8 ? 2 * g + 1 : g + 8)] = o[h][n][2 + j];
+      }
+      if (g == 0) { dst[D] = m[h][j]; dst[D + 1] = l[h][j]; }
+    }
   __syncthreads();
   for (int i = threadIdx.x; i < G * D; i += blockDim.x) {
-    const int g = i / D, d = i - g * D;
+    const int hd = i / D, d = i - hd * D;
     float mm = -INFINITY;
-    for (int w = 0; w < kDecWarps; ++w) mm = fmaxf(mm, smerge[(size_t(w) * 16 + g) * (D + 2) + D]);
+    for (int w = 0; w < kDecWarps; ++w) mm = fmaxf(mm, smerge[(size_t(w) * G + hd) * (D + 2) + D]);
     float ll = 0.f, oo = 0.f;
     for (int w = 0; w < kDecWarps; ++w) {
-      const float* src = smerge + (size_t(w) * 16 + g) * (D + 2);
+      const float* src = smerge + (size_t(w) * G + hd) * (D + 2);
       const float a = (src[D] == -INFINITY) ? 0.f : exp2f(src[D] - mm);
       ll += src[D + 1] * a;
       oo += src[d] * a;
     }
-    const int head = kvh * G + g;
+    const int head = kvh * G + hd;
     if (alone) {
       p.out[(size_t(seq) * p.H + head) * D + d] = __float2bfloat16(ll > 0.f ? oo / ll : 0.f);
     } else {
@@ -441,11 +534,27 @@ __global__ void kv_write_paged_kernel(const __nv_bfloat16* __restrict__ k_src, c
   }
 }
 
-template <int D>
-static size_t decode_smem() {
-  const size_t tiles = size_t(kDecWarps) * 2 * kDecTile * (D * 2 + 16);
-  const size_t merge = size_t(kDecWarps) * 16 * (D + 2) * 4;
-  return size_t(16) * (D * 2 + 16) + (tiles > merge ? tiles : merge);
+template <int D, int KV8, int NH, bool SWIZZLE>
+static int launch_decode(DecodeParams p, int seqs, long long slots, cudaStream_t stream) {
+  using T = DecTile<D, KV8, SWIZZLE>;
+  constexpr size_t kSmem = size_t(kDecWarps) * T::kRing + kDecWarps * T::kStages * (8 + 128) + 16 + 1024;
+  static_assert(size_t(kDecWarps) * kDecMaxGroup * (D + 2) * 4 <= size_t(kDecWarps) * T::kRing, "the merge fits in the rings");
+  auto kern = paged_decode_kernel<D, KV8, NH, SWIZZLE>;
+  static DeviceOnce configured;
+  if (int e = configured.run([&] { return int(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem))); }))
+    return e;
+  if (T::kPitch != T::kBlock) p.box_log2 = 0;
+  // (elements of a head, head, slot)
+  constexpr int kElem = KV8 ? 1 : 2;
+  uint64_t dims[3] = {uint64_t(D), uint64_t(p.Hkv), uint64_t(slots)};
+  uint64_t strides[2] = {uint64_t(D) * kElem, uint64_t(p.Hkv) * D * kElem};
+  uint32_t box[3] = {uint32_t(T::kBlock / kElem), 1, 1u << p.box_log2};
+  const CUtensorMapDataType type = KV8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const CUtensorMapSwizzle swizzle = !SWIZZLE ? CU_TENSOR_MAP_SWIZZLE_NONE : T::kBlock == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  CUtensorMap tk, tv;
+  if (encode_tensor_map(&tk, type, 3, const_cast<__nv_bfloat16*>(p.k_cache), dims, strides, box, swizzle)) return -10;
+  if (encode_tensor_map(&tv, type, 3, const_cast<__nv_bfloat16*>(p.v_cache), dims, strides, box, swizzle)) return -11;
+  return launch_overlapped(kern, dim3(seqs, p.Hkv, p.splits), kDecWarps * 32, kSmem, stream, tk, tv, p);
 }
 
 }  // namespace idrak
@@ -457,13 +566,14 @@ IDRAK_API long long idrak_decode_partial_floats(int seqs, int H, int D, int spli
 }
 
 // Over an int8 cache when k_scale / v_scale are given (one fp32 scale per (slot, kv head)). A sequence's keys are shared by
-// at most `splits` CTAs per KV head, at least `min_keys` keys each (rounded up to tiles).
+// at most `splits` CTAs per KV head, at least `min_keys` keys each (rounded up to tiles). cache_slots: blocks x block_size.
 IDRAK_API int idrak_paged_decode_kv(const void* q, long long q_stride, const void* k_cache, const void* v_cache,
                                     const float* k_scale, const float* v_scale, const int* block_table,
                                     const int* seq_lens, void* out, float* partial, int seqs, int H, int Hkv, int D,
-                                    int block_size, int max_blocks, int splits, int min_keys, float scale, int window,
+                                    int block_size, int max_blocks, long long cache_slots, int splits, int min_keys, float scale, int window,
                                     void* stream_) {
   if (D != 64 && D != 128) return -2;
+  if (block_size < 1) return -7;
   const bool kv8 = k_scale != nullptr;
   if (kv8 && !v_scale) return -6;
   if (H % Hkv || H / Hkv > kDecMaxGroup) return -3;
@@ -486,27 +596,24 @@ IDRAK_API int idrak_paged_decode_kv(const void* q, long long q_stride, const voi
   p.min_tiles = min_keys <= kDecTile ? 1 : (min_keys + kDecTile - 1) / kDecTile;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.window = window;
-  dim3 grid(seqs, Hkv, p.splits);
-  static DeviceOnce configured;
-  if (int e = configured.run([&] {
-        cudaError_t e1 = cudaFuncSetAttribute(paged_decode_kernel<64, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              int(decode_smem<64>()));
-        if (e1 == cudaSuccess)
-          e1 = cudaFuncSetAttribute(paged_decode_kernel<64, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(decode_smem<64>()));
-        if (e1 == cudaSuccess)
-          e1 = cudaFuncSetAttribute(paged_decode_kernel<128, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(decode_smem<128>()));
-        if (e1 == cudaSuccess)
-          e1 = cudaFuncSetAttribute(paged_decode_kernel<128, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(decode_smem<128>()));
-        return int(e1);
-      }))
-    return e;
-  const int threads = kDecWarps * 32;
+  p.box_log2 = 0;
+  while (p.box_log2 < 4 && block_size % (2 << p.box_log2) == 0) ++p.box_log2;
+  p.st = status_device_ptr();
+  if (seqs <= 0) return 0;
+  const bool swizzle = p.box_log2 >= 3;
   int rc;
-  if (D == 64) rc = launch_overlapped(kv8 ? paged_decode_kernel<64, 1> : paged_decode_kernel<64, 0>, grid, threads, decode_smem<64>(), s, p);
-  else rc = launch_overlapped(kv8 ? paged_decode_kernel<128, 1> : paged_decode_kernel<128, 0>, grid, threads, decode_smem<128>(), s, p);
+#define IDRAK_DECODE(D_, Q_, N_) \
+  rc = swizzle ? launch_decode<D_, Q_, N_, true>(p, seqs, cache_slots, s) : launch_decode<D_, Q_, N_, false>(p, seqs, cache_slots, s)
+#define IDRAK_DECODE_HEADS(D_, Q_) \
+  if (H / Hkv <= 8) IDRAK_DECODE(D_, Q_, 1); \
+  else IDRAK_DECODE(D_, Q_, 2)
+  if (D == 64) {
+    if (kv8) { IDRAK_DECODE_HEADS(64, 1); } else { IDRAK_DECODE_HEADS(64, 0); }
+  } else {
+    if (kv8) { IDRAK_DECODE_HEADS(128, 1); } else { IDRAK_DECODE_HEADS(128, 0); }
+  }
+#undef IDRAK_DECODE_HEADS
+#undef IDRAK_DECODE
   if (rc == 0 && p.splits > 1)
     rc = launch_overlapped(decode_merge_kernel, dim3(unsigned(seqs * H)), D < 128 ? 64 : 128, 0, s, p);
   return rc;

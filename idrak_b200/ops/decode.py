@@ -26,7 +26,7 @@ def _bind():
         return
     vp, i, f, ll = C.c_void_p, C.c_int, C.c_float, C.c_longlong
     _native.bind("idrak_decode_partial_floats", ll, [i, i, i, i])
-    _native.bind("idrak_paged_decode_kv", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, i, i, f, i, vp])
+    _native.bind("idrak_paged_decode_kv", i, [vp, C.c_longlong, vp, vp, vp, vp, vp, vp, vp, vp, i, i, i, i, i, i, ll, i, i, f, i, vp])
     _native.bind("idrak_norm_rope_kv", i, [vp, ll, vp, vp, vp, vp, vp, vp, vp, vp, f, f, f, i, i, i, i, i, i, vp])
     _native.bind("idrak_decode_slots", i, [vp, vp, i, ll, i, i, vp, vp, vp])
     _native.bind("idrak_kv_write_paged", i, [vp, vp, ll, vp, vp, vp, i, i, vp])
@@ -162,7 +162,7 @@ def paged_decode_reference(q, k_cache, v_cache, block_table, seq_lens, scale=Non
     return out.to(q.dtype)
 
 
-DECODE_TILE, DECODE_CTAS = 32, 16384
+DECODE_TILE, DECODE_CTAS = 16, 16384
 
 
 def key_shares(seqs: int, kv_heads: int, longest: int, window: int = 0, sms: int = 148):
@@ -230,7 +230,7 @@ def paged_decode(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, 
     assert block_table.dtype == torch.int32 and seq_lens.dtype == torch.int32
     rc = lib.idrak_paged_decode_kv(q.data_ptr(), q.stride(0), k_cache.data_ptr(), v_cache.data_ptr(), ptr(k_scale),
                                    ptr(v_scale), block_table.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), ptr(part),
-                                   seqs, H, Hkv, D, bs, block_table.shape[1], splits, min_keys, float(scale), int(window),
+                                   seqs, H, Hkv, D, bs, block_table.shape[1], k_cache.shape[0] * bs, splits, min_keys, float(scale), int(window),
                                    stream_ptr())
     _native.check(rc, "idrak_paged_decode_kv")
     return out

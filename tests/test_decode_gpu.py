@@ -187,7 +187,7 @@ def test_int8_kv_cache_write_and_decode(H, Hkv, Dh, splits):
 @pytest.mark.parametrize("Dh", [64, 128])
 @pytest.mark.parametrize("hint,window", [(None, 0), (4096, 0), (4096, 300)])
 def test_uneven_lengths_share_their_keys_by_the_built_in_rule(int8, Dh, hint, window):
-    """Lengths at the edges of tiles (32) and shares (128 to 512), empty and long ones in one batch, with the split that the
+    """Lengths at the edges of tiles (16) and shares (128 to 512), empty and long ones in one batch, with the split that the
     length bound gives. Probabilities enter the tensor core as bf16 (relative 2^-9) and the result is rounded to bf16:
     2^-8 of the largest value, which is at most about 4 here."""
     bs, Hkv, H = 16, 2, 8
@@ -286,3 +286,39 @@ def test_fused_norm_rope_kv_write_in_runs_of_heads(H, Hkv, Dh, rot, T, int8):
             assert (held.int() - codes.int()).abs().max() <= 1 and torch.allclose(scale.view(-1, Hkv)[slots.long()], sc, rtol=1e-6)
         else:
             assert torch.equal(held, part)
+
+
+@pytest.mark.parametrize("int8", [False, True])
+@pytest.mark.parametrize("bs,H,Hkv,Dh", [(1, 4, 2, 64), (3, 8, 2, 128), (8, 9, 1, 128), (8, 8, 1, 64), (12, 16, 1, 64), (16, 2, 2, 128),
+                                         (24, 16, 1, 128), (32, 10, 5, 64), (48, 8, 1, 128), (64, 6, 2, 128)])
+@pytest.mark.parametrize("window", [0, 37])
+def test_block_sizes_and_groups(int8, bs, H, Hkv, Dh, window):
+    """Blocks that divide a tile of 16 keys, are divided by it, or neither; groups of 1 to 16 query heads, on either side of a column
+    tile of 8; lengths at the edges of tiles and blocks. Slots past a sequence's end hold NaN (bf16) or scales of NaN (int8), which
+    nothing may read into a result. The bound is that of the test of uneven lengths."""
+    lens = [1, 7, 8, 15, 16, 17, 33, 64, 100, 257]
+    need = [(n + bs - 1) // bs for n in lens]
+    order = torch.randperm(sum(need), generator=torch.Generator().manual_seed(2)).tolist()
+    table, at = torch.full((len(lens), max(need) + 1), -7, dtype=torch.int32), 0
+    live = torch.zeros(sum(need), bs, dtype=torch.bool)
+    for i, n in enumerate(need):
+        blocks = order[at:at + n]
+        table[i, :n] = torch.tensor(blocks, dtype=torch.int32)
+        for j, b in enumerate(blocks):
+            live[b, : min(bs, lens[i] - j * bs)] = True
+        at += n
+    table, lens_t, live = table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda"), live.cuda()
+    kc, vc, q = _rand((sum(need), bs, Hkv, Dh), 1), _rand((sum(need), bs, Hkv, Dh), 2), _rand((len(lens), H, Dh), 3)
+    scales = {}
+    if int8:
+        codes = [D.quantize_kv_reference(t.view(-1, Hkv, Dh)) for t in (kc, vc)]
+        (kc, ks), (vc, vs) = ((c.view(-1, bs, Hkv, Dh), s.view(-1, bs, Hkv).contiguous()) for c, s in codes)
+        kd, vd = kc.float() * ks[..., None], vc.float() * vs[..., None]
+        ks[~live], vs[~live] = float("nan"), float("nan")
+        scales = {"k_scale": ks, "v_scale": vs}
+    else:
+        kd, vd = kc.float(), vc.float()
+        kc[~live], vc[~live] = float("nan"), float("nan")
+    out = D.paged_decode(q, kc, vc, table, lens_t, window=window, **scales)
+    ref = D.paged_decode_reference(q.float(), kd, vd, table, lens_t, window=window)
+    assert (out.float() - ref).abs().max().item() <= 2.0 ** -8 * 4
