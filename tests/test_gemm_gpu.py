@@ -180,3 +180,26 @@ def test_narrow_tiles_of_a_small_product_give_the_same_bits(N, a_mn, b_mn):
     # fp32 accumulation, one rounding to bf16 (half an ulp is 2^-9) and the fp32 reference's own
     ref = gemm_reference(a[:rows], b, out_dtype=torch.float32) + bias.float() + res[:rows].float()
     assert ((narrow.float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 63, 64, 65])
+@pytest.mark.parametrize("N,K", [(8, 1024), (136, 72), (768, 768), (4096, 1032), (9216, 1024), (9728, 1024), (100, 2048), (128, 8)])
+def test_products_of_few_rows_keep_the_contract(M, N, K):
+    """Calls on either side of the rule that sends them to the few-row kernel: rows and widths at its edges, rows that it cannot read
+    (strides between 16 bytes), an output, bias and residual given. One fp32 sum over K and one rounding to bf16 either way: half an
+    ulp (2^-9 relative) each for kernel and reference, and sums of K products of magnitude about 1 in another order."""
+    a, b = _rand((M, K), 1.0, 41), _rand((N, K), 0.2, 42)
+    bias, res, out = _rand((N,), 1.0, 43), _rand((M, N), 1.0, 44), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    ref = gemm_reference(a, b, out_dtype=torch.float32)
+    full = ref + bias.float() + res.float()
+    for got, want in ((gemm(a, b), ref), (gemm(a, b, bias=bias, residual=res, out=out), full), (gemm(a, b, splits=1), ref)):
+        assert ((got.float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    assert gemm(a, b, bias=bias, residual=res, out=out) is out
+    wide = torch.zeros(M, K + 3, dtype=torch.bfloat16, device="cuda")
+    if M > 1:
+        wide[:, :K] = a
+        with pytest.raises(Exception):
+            gemm(wide[:, :K], b)
+    assert gemm(a, b, out_dtype=torch.float32).dtype == torch.float32
+    from idrak_b200 import _native
+    _native.check_status("few rows")
