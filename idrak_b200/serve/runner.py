@@ -268,7 +268,9 @@ class ModelRunner:
 
         if self._direct_prefill():
             # the kernels of the modules' forwards, in their order, without the modules: a short prompt is bound by the host
-            x = self._row_blocks(x.view(ids_t.shape[0], -1), pos_t, slots_t, attention, self._dense)
+            x = x.view(ids_t.shape[0], -1)
+            done = self._native_blocks(x, pos_t, slots_t, bounds, runs) if all(it.start == 0 for it in items) else None
+            x = done if done is not None else self._row_blocks(x, pos_t, slots_t, attention, self._dense)
             return self._logits(self._norm(self.model.norm, x if all_logits else x[last]))
 
         layer_index = {id(blk.attn): i for i, blk in enumerate(self.model.blocks)}
@@ -444,6 +446,15 @@ class ModelRunner:
                     and _plain(mods.get("mlp"), FeedForward)):
                 return False
         return True
+
+    def _native_blocks(self, x, positions, slots, bounds, runs):
+        """The blocks over fresh prompts as one native call, or ``None`` where the runner's own steps are a subclass's, or the call
+        is not covered."""
+        cls = type(self)
+        if any(n in self.__dict__ or getattr(cls, n) is not getattr(ModelRunner, n) for n in ("_row_blocks", "_rotate_and_cache", "_dense", "_flash", "_norm")):
+            return None
+        from . import native_prefill
+        return native_prefill.run(self, x, positions, slots, bounds, runs)
 
     @staticmethod
     def _norm(layer, t):

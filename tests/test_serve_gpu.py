@@ -259,3 +259,50 @@ def test_packed_projections_of_a_model_with_folded_norms(kind):
     plain = _step(runner)[2].float()
     # both round activations to bf16 (2^-9) at each of the ten steps of two layers
     assert (fused - plain).pow(2).mean().sqrt() <= 10 * 2.0 ** -9 * plain.pow(2).mean().sqrt()
+
+
+@pytest.mark.parametrize("dim,heads,kv_heads,head_dim", [(256, 4, 2, 64), (512, 4, 1, 128)])
+@pytest.mark.parametrize("extra", [{}, {"qk_norm": True}, {"qkv_bias": True}, {"norm_offset": 1.0, "activation": "gelu"}, {"int8": True}])
+def test_native_prefill_launches_what_the_runner_would(dim, heads, kv_heads, head_dim, extra, monkeypatch):
+    """The blocks as one native call against the runner's own launches: the same kernels on the same operands, so logits and caches
+    agree bit for bit - one token, prompts of one length side by side, odd lengths, on both sides of 64 rows."""
+    import dataclasses
+    from idrak_b200.models import DecoderSpec, build_decoder
+    from idrak_b200.serve import ModelRunner, PrefillItem, native_prefill
+    extra = dict(extra)
+    int8 = extra.pop("int8", False)
+    spec = dataclasses.replace(DecoderSpec.llama(layers=2, dim=dim, heads=heads, kv_heads=kv_heads, ff_dim=1152, vocab=300, max_positions=512,
+                                                 head_dim=head_dim), **extra)
+    model = build_decoder(spec, seed=2).to("cuda", torch.bfloat16)
+    ran = []
+    inner = native_prefill.run
+    monkeypatch.setattr(native_prefill, "run", lambda *a: ran.append(inner(*a)) or ran[-1])
+    g = torch.Generator().manual_seed(1)
+    for lengths in ((1,), (45,), (16, 16, 7), (8, 8), (300, 33)):
+        out = []
+        for native in (True, False):
+            runner = ModelRunner(model, 80, 16, cache_dtype=torch.int8 if int8 else None)
+            if not native:
+                runner._native_blocks = lambda *a: None
+            items, block = [], 0
+            g.manual_seed(sum(lengths))
+            for n in lengths:
+                items.append(PrefillItem(torch.randint(0, 300, (n,), generator=g).tolist(), 0, list(range(block, block + (n + 15) // 16))))
+                block += (n + 15) // 16
+            caches = runner.k_cache + runner.v_cache + (runner.k_scale + runner.v_scale if int8 else [])
+            out.append([runner.prefill(items).clone(), runner.prefill(items, all_logits=True).clone()] + [c[:-1].clone() for c in caches])
+        assert all(torch.equal(x, y) and x.float().isfinite().all() for x, y in zip(*out))
+    assert len(ran) == 10 and all(r is not None for r in ran)
+
+
+def test_native_prefill_refuses_what_it_does_not_cover():
+    from idrak_b200.models import DecoderSpec, build_decoder
+    from idrak_b200.serve import ModelRunner, PrefillItem
+    model = _small()
+    runner = ModelRunner(model, 20, 16)
+    items = [PrefillItem([1, 2, 3], 0, [0]), PrefillItem([4] * 20, 0, [1, 2])]
+    want = runner.prefill(items).clone()
+    w = model.blocks[0].attn.o_weight
+    model.blocks[0].attn.o_weight = torch.nn.Parameter(torch.cat([w.data, w.data], 1)[:, : w.shape[1]])      # rows not side by side
+    assert torch.equal(runner.prefill(items), want)
+    assert torch.equal(runner.prefill([PrefillItem([4] * 4, 16, [1, 2])])[0], want[1])                       # behind a cached prefix
