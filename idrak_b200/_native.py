@@ -41,6 +41,7 @@ _SIGNATURES = {
     "idrak_device_limits": (c_int, [C.POINTER(c_ll), c_int]),
     "idrak_gemm_workspace_elems": (c_ll, [c_int, c_int, c_int]),
     "idrak_gemm_pick_splits": (c_int, [c_int, c_int, c_int, c_int]),
+    "idrak_gemm_few_rows": (c_int, [c_int, c_int, c_int]),
     "idrak_gemm_bf16": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                 c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int,
                                 c_int, c_float, c_int, c_void_p, c_int, c_void_p]),
@@ -87,7 +88,7 @@ _SIGNATURES = {
     "idrak_gemm_grouped_k": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                                      c_int, c_void_p, c_void_p]),
     "idrak_skinny_gemm": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_void_p,
-                                  c_void_p, c_int, c_int, c_float, c_void_p]),
+                                  c_void_p, c_int, c_int, c_float, c_int, c_void_p]),
     "idrak_skinny_packed": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,
                                     c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "idrak_flash_fwd_ex": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_ll] * 7 + [c_float, c_int, c_int, c_void_p, c_float,

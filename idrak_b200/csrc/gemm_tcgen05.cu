@@ -401,6 +401,20 @@ IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn) {
   return min(s, 16);
 }
 
+// Whether x W^T of this size goes to the few-row kernel (skinny_gemm.cu): 0 no, 1 yes, 2 yes with K in one pass. That kernel has
+// the weights on the 128-row side of its tiles, sums the parts of K inside a cluster and is set up while the kernel before it runs.
+// Where K is not cut here it is not cut there either, and the bits are the same: a row then has the same bits whatever the number
+// of rows, which a prompt that finds its first blocks in the cache relies on to be continued as before. In one pass a short K is
+// no longer the faster one there from 33 rows on, and neither are weights so wide that the tiles here fill the machine many times.
+// us, here / there, at 1, 32, 64 rows: 1024 x 1024 10.2, 10.7, 11.3 / 4.6, 5.4, 6.0; 4096 x 4096 17.7, 18.7, 20.0 / 10.5, 11.8, 13.8;
+// 4096 x 14336 34.8, 36.8, 38.9 / 27.6, 28.7, 31.4; in one pass: 768 x 768 10.1, 10.4, 10.6 / 7.2, 9.2, 11.5; 28672 x 4096 63.5, 57.3,
+// 57.3 / 50.2, 53.2, 57.3; 128256 x 4096 206, 189, 193 / 166, 183, 207.
+IDRAK_API int idrak_gemm_few_rows(int M, int N, int K) {
+  if (M > 64) return 0;
+  if (idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1) return 1;
+  return M <= 32 || (K >= 1024 && N < 49152) ? 2 : 0;
+}
+
 // Columns of a tile: 256, or 128 where twice as many CTAs still fit the machine at once. A product that small is a chain of
 // set-up, first load and write-out, and the write-out takes as long as a tile is wide. Each element is summed over K in the
 // same order either way. Measured as the training step of a 4-layer model of width 128 on 1024 tokens: 1181 -> 1128 us.

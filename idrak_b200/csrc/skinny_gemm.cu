@@ -383,7 +383,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 // (32 tiles) c = 2 / 4 / 8 14.8 / 10.7 / 11.0; 4096 x 14336 c = 4 / 7 / 8 27.2 / 24.3 / 24.4; 28672 x 4096 (224 tiles)
 // c = 1 / 2 / 4 45.2 / 46.5 / 54.6; int8 codes 6144 x 4096 c = 2 / 4 / 5 / 8 21.8 / 16.3 / 14.7 / 20.4.
 template <int NT, int kBits>
-static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyParams& p, cudaStream_t stream) {
+static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyParams& p, cudaStream_t stream, bool one_pass = false) {
   using L = SkinnySmem<NT, kBits>;
   auto kern = skinny_gemm_kernel<NT, kBits>;
   static DeviceOnce configured;
@@ -393,7 +393,7 @@ static int launch_skinny(const CUtensorMap& tmW, const CUtensorMap& tmX, SkinnyP
     return e;
   const int half = kSkFeat / 2, kblocks = (p.K + kSkBK - 1) / kSkBK;
   const int tiles = p.o.gate_kind >= 0 ? (p.o.N + half - 1) / half : (p.o.N + kSkFeat - 1) / kSkFeat;
-  int c = skinny_forced_splits();
+  int c = one_pass ? 1 : skinny_forced_splits();
   if (!c)
     for (c = 8; c > 1 && tiles * c > sm_count() * 2 * 6 / 7;) --c;
   p.csize = c < kblocks ? c : kblocks;
@@ -414,11 +414,11 @@ using namespace idrak;
 
 // C[M, N] = epilogue(X[M, K] W^T), M <= 64. W is [N, K] (ldw elements per row), or with gate_kind >= 0 the stacked
 // [gate; up] matrix of 2 * N rows and C = act(x Wg^T) * (x Wu^T). norm_eps >= 0 folds an RMS norm over K in (the norm
-// weight must already be multiplied into W's columns). K % 8 == 0, rows 16-byte aligned. Returns 0, a CUDA error, or
-// a negative argument error.
+// weight must already be multiplied into W's columns). one_pass: K is not cut, an element has the bits of the dense kernel's
+// uncut sum. K % 8 == 0, rows 16-byte aligned. Returns 0, a CUDA error, or a negative argument error.
 IDRAK_API int idrak_skinny_gemm(const void* X, int ldx, const void* W, int ldw, void* C, int ldc, int M, int N, int K,
                                 const void* bias, const void* residual, int ldr, int gate_kind, float norm_eps,
-                                void* stream_) {
+                                int one_pass, void* stream_) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 64) return -2;
   if ((K & 7) || (ldx & 7) || (ldw & 7)) return -3;
@@ -442,9 +442,9 @@ IDRAK_API int idrak_skinny_gemm(const void* X, int ldx, const void* W, int ldw, 
                         CU_TENSOR_MAP_SWIZZLE_128B))
     return -10;
   if (encode_tokens(&tmX, X, ldx, M, K, NT)) return -11;
-  if (NT == 16) return launch_skinny<16, 16>(tmW, tmX, p, stream);
-  if (NT == 32) return launch_skinny<32, 16>(tmW, tmX, p, stream);
-  return launch_skinny<64, 16>(tmW, tmX, p, stream);
+  if (NT == 16) return launch_skinny<16, 16>(tmW, tmX, p, stream, one_pass);
+  if (NT == 32) return launch_skinny<32, 16>(tmW, tmX, p, stream, one_pass);
+  return launch_skinny<64, 16>(tmW, tmX, p, stream, one_pass);
 }
 
 // C[M, N] = epilogue(X[M, K] W) over a packed weight stored [K inputs, outputs] (gated: outputs = [gate | up], 2 * N of

@@ -85,19 +85,6 @@ def _tuned_splits(a, b, a_mn, b_mn, M, N, K, default, out) -> int:
     return int(t.choose("gemm.splits", shape, cands, default=str(default), cold_l2=True))
 
 
-def _few_rows(a, b, M, N, K, bias, residual, out) -> bool:
-    """Whether ``a @ b.T`` (+ bias) (+ residual) goes to the few-row kernel: up to 64 rows of a product whose K the dense kernel would
-    cut. The few-row kernel has the weights on the 128-row side of its tiles, sums the parts of K inside a cluster and is set up
-    while the kernel before it runs. us, dense and few-row, at 1 / 32 / 64 rows: 1024 x 1024 10.5, 4.6 / 10.5, 5.4 / 11.3, 6.0;
-    4096 x 4096 18.2, 10.2 / 18.9, 11.8 / 20.2, 13.8; 4096 x 14336 35.5, 27.6 / 36.9, 29.0 / 38.2, 31.1; 6144 x 4096 20.5, 14.0 / 22.9,
-    15.4 / 24.9, 16.7. Where the dense kernel does not cut K a row has the same bits whatever the number of rows, which a prompt that
-    finds its first blocks in the cache relies on to be continued as before: those products stay there (768 x 768 10.1, 4.4 /
-    10.1, 5.1 / 10.6, 5.9; 28672 x 4096 60.4, 50.2 / 57.3, 52.8 / 57.9, 58.4)."""
-    from . import skinny
-    return (_native.lib().idrak_gemm_pick_splits(M, N, K, 128 if N <= 128 else 256) > 1 and skinny.supported(a, b)
-            and skinny._readable(M, N, N, bias, residual, out))
-
-
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          bias: torch.Tensor | None = None, residual: torch.Tensor | None = None, act: str | None = None,
          aux: torch.Tensor | None = None, out: torch.Tensor | None = None, beta: bool = False,
@@ -145,10 +132,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         splits = 0                          # the library's choice, unless the tuner has measured a better one
         if M <= 256 and not (beta or act_id):
             splits = _tuned_splits(a, b, a_mn, b_mn, M, N, K, splits, out)
-    if (M <= 64 and splits == 0 and not (a_mn or b_mn or act_id or beta) and alpha == 1.0 and M * N > 0
-            and _few_rows(a, b, M, N, K, bias, residual, out)):
-        from .skinny import skinny_linear
-        return skinny_linear(a, b, bias, residual, out=out)
+    if M <= 64 and splits == 0 and not (a_mn or b_mn or act_id or beta) and alpha == 1.0 and M * N > 0:
+        from . import skinny
+        few = lib.idrak_gemm_few_rows(M, N, K)
+        if few and skinny.supported(a, b) and skinny._readable(M, N, N, bias, residual, out):
+            return skinny.skinny_linear(a, b, bias, residual, out=out, one_pass=few == 2)
     ws_elems = lib.idrak_gemm_workspace_elems(M, N, K) if splits == 0 else splits * M * N if splits > 1 else 0
     ws = scratch("gemm_splitk", ws_elems, torch.float32, a.device) if ws_elems else None
     if bias is not None:

@@ -57,8 +57,9 @@ def _readable(M: int, N: int, outputs: int, bias, residual, out) -> bool:
 
 def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None,
                   residual: Optional[torch.Tensor] = None, gate: Optional[str] = None,
-                  norm_eps: Optional[float] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``x [M <= 64, K]``, ``w [N, K]`` (or ``[2 ff, K]`` with ``gate``) -> ``[M, N]`` (``[M, ff]``)."""
+                  norm_eps: Optional[float] = None, out: Optional[torch.Tensor] = None, one_pass: bool = False) -> torch.Tensor:
+    """``x [M <= 64, K]``, ``w [N, K]`` (or ``[2 ff, K]`` with ``gate``) -> ``[M, N]`` (``[M, ff]``). With ``one_pass`` K is not cut:
+    the bits of the dense kernel's uncut sum."""
     if not supported(x, w, gate):
         y = skinny_reference(x, w, bias, residual, gate, norm_eps)
         return y if out is None else out.copy_(y)
@@ -70,7 +71,7 @@ def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     rc = _native.lib().idrak_skinny_gemm(
         x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K, ptr(bias),
         ptr(residual), residual.stride(0) if residual is not None else 0, _KINDS[gate] if gate is not None else -1,
-        float(norm_eps) if norm_eps is not None else -1.0, stream_ptr())
+        float(norm_eps) if norm_eps is not None else -1.0, int(one_pass), stream_ptr())
     _native.check(rc, "idrak_skinny_gemm")
     return out
 

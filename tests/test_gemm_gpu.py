@@ -183,7 +183,7 @@ def test_narrow_tiles_of_a_small_product_give_the_same_bits(N, a_mn, b_mn):
 
 
 @pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 63, 64, 65])
-@pytest.mark.parametrize("N,K", [(8, 1024), (136, 72), (768, 768), (4096, 1032), (9216, 1024), (9728, 1024), (100, 2048), (128, 8)])
+@pytest.mark.parametrize("N,K", [(8, 1024), (136, 72), (768, 768), (4096, 1032), (18944, 1024), (19200, 1024), (100, 2048), (128, 8)])
 def test_products_of_few_rows_keep_the_contract(M, N, K):
     """Calls on either side of the rule that sends them to the few-row kernel: rows and widths at its edges, rows that it cannot read
     (strides between 16 bytes), an output, bias and residual given. One fp32 sum over K and one rounding to bf16 either way: half an
@@ -195,6 +195,9 @@ def test_products_of_few_rows_keep_the_contract(M, N, K):
     for got, want in ((gemm(a, b), ref), (gemm(a, b, bias=bias, residual=res, out=out), full), (gemm(a, b, splits=1), ref)):
         assert ((got.float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
     assert gemm(a, b, bias=bias, residual=res, out=out) is out
+    if K < 1024 or N > 18944:                                     # the dense kernel does not cut K: the same bits for any number of rows
+        assert torch.equal(gemm(a, b), gemm(a, b, splits=1))
+        assert torch.equal(gemm(a, b), gemm(torch.cat([a, a[:1].expand(200, K)]), b, splits=1)[:M])
     wide = torch.zeros(M, K + 3, dtype=torch.bfloat16, device="cuda")
     if M > 1:
         wide[:, :K] = a
