@@ -93,6 +93,7 @@ _SIGNATURES = {
                                     c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "idrak_flash_fwd_ex": (c_int, [c_void_p] * 5 + [c_int] * 6 + [c_ll] * 7 + [c_float, c_int, c_int, c_void_p, c_float,
                                                                               c_void_p]),
+    "idrak_small_attention": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_float, c_void_p]),
     "idrak_gemm_lowrank": (c_int, [c_void_p, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                    c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p]),
     "idrak_pw_unary": (c_int, [c_int, c_int, c_void_p, c_void_p, c_ll, c_float, c_float, c_void_p]),

@@ -17,7 +17,9 @@ import math
 
 import torch
 
+from .. import _native
 from . import rowops
+from ._util import stream_ptr
 from .attention import attention_reference, flash_backward, flash_forward
 from .gemm import bias_grad, gemm, weight_grad
 from .rowops import GATE_KINDS, _gate_ref, colsum, rope_, rope_reference
@@ -68,6 +70,70 @@ class _QkvAttention(torch.autograd.Function):
         return (dqkv,) + (None,) * 12
 
 
+def _small_attention_grad(qkv, dout, H, Hkv, D, causal, scale):
+    """d(qkv) of ``attention_reference`` over a packed projection in plain operations (fp32): differentiable once more, and over
+    several upstream gradients at once."""
+    B, S, _ = qkv.shape
+    q, k, v = (t.float().transpose(1, 2) for t in _split_qkv(qkv, H, Hkv, D))
+    G = H // Hkv
+    k, v = k.repeat_interleave(G, dim=1), v.repeat_interleave(G, dim=1)
+    do = dout.reshape(B, S, H, D).float().transpose(1, 2)
+    s = torch.matmul(q, k.transpose(-1, -2)) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=qkv.device).triu(1), float("-inf"))
+    p = torch.softmax(s, dim=-1)
+    dp = torch.matmul(do, v.transpose(-1, -2))
+    ds = p * (dp - (p * dp).sum(-1, keepdim=True)) * scale
+    dq, dk, dv = torch.matmul(ds, k), torch.matmul(ds.transpose(-1, -2), q), torch.matmul(p.transpose(-1, -2), do)
+    dk, dv = (t.reshape(B, Hkv, G, S, D).sum(2) for t in (dk, dv))
+    return torch.cat([t.transpose(1, 2).reshape(B, S, -1) for t in (dq, dk, dv)], -1).to(qkv.dtype)
+
+
+class _SmallQkvAttention(torch.autograd.Function):
+    """Attention over a packed projection with heads below 64 on the fp32 kernels (``csrc/small_attn.cu``)."""
+
+    @staticmethod
+    def forward(ctx, qkv, H, Hkv, D, causal, scale):
+        B, S, _ = qkv.shape
+        out = torch.empty(B, S, H * D, dtype=qkv.dtype, device=qkv.device)
+        o32 = torch.empty(B, S, H * D, dtype=torch.float32, device=qkv.device)
+        lse = torch.empty(B, H, S, dtype=torch.float32, device=qkv.device)
+        rc = _native.lib().idrak_small_attention(qkv.data_ptr(), None, out.data_ptr(), None, o32.data_ptr(), lse.data_ptr(), B, S,
+                                                 H, Hkv, D, int(causal), float(scale), stream_ptr())
+        _native.check(rc, "idrak_small_attention")
+        ctx.save_for_backward(qkv, o32, lse)
+        ctx.cfg = (H, Hkv, D, causal, scale)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        qkv, o32, lse = ctx.saved_tensors
+        H, Hkv, D, causal, scale = ctx.cfg
+        if torch.is_grad_enabled() or not torch._C._has_storage(dout) or dout.dtype != torch.bfloat16:
+            return (_small_attention_grad(qkv, dout, H, Hkv, D, causal, scale),) + (None,) * 5
+        B, S, _ = qkv.shape
+        qkv, dout = _whole(qkv), _whole(dout)               # a hook may hand the saved tensor back in another place
+        dqkv = torch.empty_like(qkv)
+        rc = _native.lib().idrak_small_attention(qkv.data_ptr(), dout.data_ptr(), None, dqkv.data_ptr(), o32.contiguous().data_ptr(),
+                                                 lse.contiguous().data_ptr(), B, S, H, Hkv, D, int(causal),
+                                                 float(scale), stream_ptr())
+        _native.check(rc, "idrak_small_attention")
+        return (dqkv,) + (None,) * 5
+
+
+def _whole(t):
+    return t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
+def _plain_call(t: torch.Tensor) -> bool:
+    """Whether an operation on this tensor just runs: no transform, trace, forward-mode derivative or dispatch mode around it and
+    an ordinary tensor. Everything else goes through torch's own operations, which take part in all of those."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t)
+            and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
+            and not torch.compiler.is_compiling() and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0)
+
+
 def qkv_attention(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, causal: bool = True,
                   scale: float | None = None, rope_theta: float | None = None, rope_dim: int | None = None,
                   rope_scale: float = 1.0, positions: torch.Tensor | None = None, window: int | None = None,
@@ -88,6 +154,12 @@ def qkv_attention(qkv: torch.Tensor, heads: int, kv_heads: int, head_dim: int, c
         pos = positions if positions is not None else torch.arange(S, device=qkv.device).repeat(B)
         q = rope_reference(q.reshape(B * S, heads, head_dim), pos, rope_theta, rope_dim, rope_scale).reshape(q.shape)
         k = rope_reference(k.reshape(B * S, kv_heads, head_dim), pos, rope_theta, rope_dim, rope_scale).reshape(k.shape)
+    if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and head_dim < 64 and head_dim % 8 == 0 and qkv.numel() > 0
+            and not (window or row_start is not None or softcap) and heads % kv_heads == 0 and max(heads, B) <= 65535
+            and _plain_call(qkv)):
+        packed = qkv if rope_theta is None else torch.cat([t.flatten(2) for t in (q, k, v)], -1)
+        return _SmallQkvAttention.apply(_whole(packed), heads, kv_heads, head_dim, causal,
+                                        scale if scale is not None else 1.0 / math.sqrt(head_dim))
     return attention_reference(q, k, v, causal, scale, window, row_start, softcap).reshape(B, S, heads * head_dim)
 
 
