@@ -83,6 +83,15 @@ __device__ __forceinline__ void flash_bar_sync(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The query rows of forward CTA blockIdx.x, blocks of `rows`: row block by row block over all heads and batches, causal ones from
+// the last, which sees the most keys.
+struct FwdUnit { int qb, head, batch; };
+__device__ __forceinline__ FwdUnit fwd_unit(const FlashParams& p, int rows) {
+  const unsigned heads = unsigned(p.H) * unsigned(p.B), slot = blockIdx.x / heads, rem = blockIdx.x - slot * heads;
+  const int blocks = (p.Sq + rows - 1) / rows;
+  return FwdUnit{p.causal ? blocks - 1 - int(slot) : int(slot), int(rem % unsigned(p.H)), int(rem / unsigned(p.H))};
+}
+
 // First key index query `row` (position in its batch entry) may see; off = Skv - Sq.
 __device__ __forceinline__ int flash_row_lo(const FlashParams& p, int batch, int row, int off) {
   int lo = 0;

@@ -108,6 +108,7 @@ def kernel_shapes() -> List[KernelShape]:
                     "83328 bytes and two per SM where there are more tiles than SMs"),
         KernelShape("flash_fwd_kernel<64>", "128 queries x 128 keys, head size 64", 2, 320, 85248, 256, 2, "P in tensor memory"),
         KernelShape("flash_fwd_kernel<128>", "128 queries x 128 keys, head size 128", 2, 320, 167168, 512, 1, "P in tensor memory, two buffers"),
+        KernelShape("flash_fwd_pair_kernel<128>", "2 x 128 queries x 128 keys, head size 128", 4, 640, 201984, 512, 1, "P over the scores in tensor memory"),
         KernelShape("flash_bwd_q_kernel<64>", "128 queries x 128 keys per block, persistent", 3, 320, 115968, 512, 1, "dS in tensor memory, two buffers"),
         KernelShape("flash_bwd_q_kernel<128>", "the same, head size 128", 3, 320, 230656, 512, 1, "dS in tensor memory, two buffers"),
         KernelShape("flash_bwd_kv_kernel<64>", "128 keys x 128 queries per block, persistent", 2, 320, 166656, 512, 1, "P in tensor memory, dS in shared memory"),

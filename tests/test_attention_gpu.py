@@ -183,3 +183,24 @@ def test_packed_row_equals_the_sequences_run_one_by_one():
     for lo, hi in spans:
         alone, _ = ops.flash_forward(q[:, lo:hi].contiguous(), k[:, lo:hi].contiguous(), v[:, lo:hi].contiguous(), True)
         _close(packed[:, lo:hi], alone, 1e-2)
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Skv,causal", [(5, 32, 8, 200, 200, True), (40, 4, 1, 257, 257, True), (5, 32, 8, 129, 500, True),
+                                                   (1, 32, 4, 1281, 1281, True), (3, 64, 8, 128, 128, True), (3, 32, 8, 300, 300, False),
+                                                   (3, 50, 10, 256, 640, False), (10, 16, 16, 385, 400, True)])
+def test_two_query_tiles_have_the_bits_of_one(B, H, Hkv, Sq, Skv, causal):
+    """Calls with a CTA of two query tiles for every SM against calls that one tile per CTA takes: the same arithmetic in the same
+    order, at sizes where the second tile is empty, short or sees more keys. Rows of a warp move their maxima together on both."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q, k, v = (torch.randn(B, s, h, 128, generator=g, device="cuda").to(torch.bfloat16) for s, h in ((Sq, H), (Skv, Hkv), (Skv, Hkv)))
+    o, lse = ops.flash_forward(q, k, v, causal)
+    for b in range(B):                                                       # one sequence and few heads at a time: one tile per CTA
+        for h in range(0, H, H // Hkv):
+            part = slice(h, h + H // Hkv)
+            ob, lb = ops.flash_forward(q[b:b + 1, :, part].contiguous(), k[b:b + 1, :, h * Hkv // H][:, :, None].contiguous(),
+                                       v[b:b + 1, :, h * Hkv // H][:, :, None].contiguous(), causal)
+            assert torch.equal(ob[0], o[b, :, part]) and torch.equal(lb[0], lse[b, part])
+    if Sq <= Skv:
+        ref = ops.attention_reference(q.float(), k.float(), v.float(), causal)
+        # probabilities enter the product as bf16 (2^-9) and the result is rounded to bf16, values up to about 5
+        assert (o.float() - ref).abs().max().item() <= 2.0 ** -8 * 5
