@@ -19,6 +19,8 @@ int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, int ldb, in
                     int splits, float* workspace, int fp16, void* stream_);
 int idrak_skinny_gemm(const void* X, int ldx, const void* W, int ldw, void* C, int ldc, int M, int N, int K, const void* bias,
                       const void* residual, int ldr, int gate_kind, float norm_eps, int one_pass, void* stream_);
+int idrak_skinny_wide(const void* X, int ldx, const void* W, int ldw, void* C, int ldc, int M, int N, int K, const void* bias,
+                      const void* residual, int ldr, int one_pass, void* stream_);
 int idrak_norm_rope_kv(void* qkv, long long row_stride, const int* positions, const int* slots, void* k_cache, void* v_cache,
                        float* k_scale, float* v_scale, const void* q_norm, const void* k_norm, float eps, float theta,
                        float freq_scale, int rot_dim, int T, int H, int Hkv, int D, int kv_int8, void* stream_);
@@ -57,7 +59,9 @@ struct PrefillArgs {
 // x W^T (+ bias) (+ residual) on the kernel that ops.gemm takes for a product of this size.
 static int product(const void* x, const void* w, void* out, int M, int N, int K, const void* bias, const void* residual, float* workspace,
                    void* stream) {
-  if (const int few = idrak_gemm_few_rows(M, N, K))
+  const int few = idrak_gemm_few_rows(M, N, K);
+  if (few == 3) return idrak_skinny_wide(x, K, w, K, out, N, M, N, K, bias, residual, residual ? N : 0, 0, stream);
+  if (few)
     return idrak_skinny_gemm(x, K, w, K, out, N, M, N, K, bias, residual, residual ? N : 0, -1, -1.f, few == 2, stream);
   return idrak_gemm_bf16(x, K, 0, w, K, 0, out, N, 0, M, N, K, bias, residual, residual ? N : 0, 0, nullptr, 0, 0, 1.f, 0, workspace, 0,
                          stream);

@@ -132,10 +132,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         splits = 0                          # the library's choice, unless the tuner has measured a better one
         if M <= 256 and not (beta or act_id):
             splits = _tuned_splits(a, b, a_mn, b_mn, M, N, K, splits, out)
-    if M <= 64 and splits == 0 and not (a_mn or b_mn or act_id or beta) and alpha == 1.0 and M * N > 0:
+    if M <= 256 and splits == 0 and not (a_mn or b_mn or act_id or beta) and alpha == 1.0 and M * N > 0:
         from . import skinny
         few = lib.idrak_gemm_few_rows(M, N, K)
-        if few and skinny.supported(a, b) and skinny._readable(M, N, N, bias, residual, out):
+        if few and skinny.supported(a[: skinny.MAX_ROWS], b) and skinny._readable(M, N, N, bias, residual, out):
+            if few == 3:
+                return skinny.wide_linear(a, b, bias, residual, out)
             return skinny.skinny_linear(a, b, bias, residual, out=out, one_pass=few == 2)
     ws_elems = lib.idrak_gemm_workspace_elems(M, N, K) if splits == 0 else splits * M * N if splits > 1 else 0
     ws = scratch("gemm_splitk", ws_elems, torch.float32, a.device) if ws_elems else None

@@ -76,6 +76,21 @@ def skinny_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]
     return out
 
 
+def wide_linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, residual: Optional[torch.Tensor] = None,
+                out: Optional[torch.Tensor] = None, one_pass: bool = False) -> torch.Tensor:
+    """``x [M <= 256, K]`` times ``w [N, K]`` on the kernel for some more rows (``csrc/skinny_wide.cu``); operands as ``supported``
+    asks of the few-row kernel's."""
+    M, K = x.shape
+    N = w.shape[0]
+    if out is None:
+        out = torch.empty((M, N), dtype=x.dtype, device=x.device)
+    rc = _native.lib().idrak_skinny_wide(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(), out.stride(0), M, N, K,
+                                         ptr(bias), ptr(residual), residual.stride(0) if residual is not None else 0, int(one_pass),
+                                         stream_ptr())
+    _native.check(rc, "idrak_skinny_wide")
+    return out
+
+
 # From this many weight rows on, and with more than 32 activation rows, the dense GEMM is level with the few-row kernel or
 # ahead of it: many waves of tiles hide its split-K, and the few-row kernel reads the activations once per 128 weight rows.
 # Measured at 32 / 64 activation rows, us, few-row against dense: 28672 x 4096 41 / 45 against 47 / 48, 50304 x 768 21.5 / 25.2

@@ -498,7 +498,7 @@ class ModelRunner:
         return logits.reshape(-1, logits.shape[-1])
 
     # ------------------------------------------------------------------ decode as a replayed CUDA graph
-    BATCH_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
+    BATCH_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 96, 128, 160, 192, 224, 256)     # above 64 a row that is padded costs as any other
 
     @torch.no_grad()
     def decode_graphed(self, tokens: torch.Tensor, positions: torch.Tensor, block_table: torch.Tensor,

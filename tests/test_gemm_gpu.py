@@ -206,3 +206,22 @@ def test_products_of_few_rows_keep_the_contract(M, N, K):
     assert gemm(a, b, out_dtype=torch.float32).dtype == torch.float32
     from idrak_b200 import _native
     _native.check_status("few rows")
+
+
+@pytest.mark.parametrize("M", [65, 80, 127, 128, 129, 160, 192, 193, 255, 256])
+@pytest.mark.parametrize("N,K", [(8, 1024), (264, 1032), (768, 3072), (4096, 1024), (300, 136)])
+def test_products_of_some_more_rows(M, N, K):
+    """The kernel for 65 to 256 rows on either side of the rule that sends products to it, and called by itself at sizes that the rule
+    does not give it: one pass of 128 rows, two, a ragged last tile of features, an uncut K with the dense kernel's bits."""
+    from idrak_b200.ops.skinny import wide_linear
+    a, b = _rand((M, K), 1.0, 51), _rand((N, K), 0.2, 52)
+    bias, res, out = _rand((N,), 1.0, 53), _rand((M, N), 1.0, 54), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    ref = gemm_reference(a, b, out_dtype=torch.float32)
+    full = ref + bias.float() + res.float()
+    for got, want in ((gemm(a, b), ref), (gemm(a, b, bias=bias, residual=res, out=out), full), (wide_linear(a, b), ref),
+                      (wide_linear(a, b, bias, res, torch.empty_like(out)), full)):
+        # fp32 sums in another order and one rounding to bf16, as in the test of few rows
+        assert ((got.float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5).all()
+    assert torch.equal(wide_linear(a, b, one_pass=True), gemm(a, b, splits=1)) and torch.equal(wide_linear(a, b), wide_linear(a, b))
+    from idrak_b200 import _native
+    _native.check_status("wide")
