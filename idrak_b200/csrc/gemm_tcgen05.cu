@@ -459,7 +459,12 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
   p.beta = beta;
   p.alpha = alpha;
   const PairPlan pair = splits == 0 || splits == 1 ? gemm_pair_plan(M, N, K, splits == 0 && workspace) : PairPlan{};
-  if (splits == 0 && !pair.use) splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
+  if (splits == 0) {
+    if (!pair.use) splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
+    const bool cut = workspace && (pair.use ? pair.parts > 1 : splits > 1);
+    const int parts = fp16 ? 0 : gemm_small_cuts(M, N, K, !a_mn && !b_mn && !cut, cut);
+    if (parts) return gemm_small_launch(A, lda, a_mn, B, ldb, b_mn, p, parts, stream);
+  }
   p.splits = (splits > 1 && workspace) ? splits : 1;
   {
     // every split must own at least one k-block

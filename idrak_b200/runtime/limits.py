@@ -94,6 +94,8 @@ def kernel_shapes() -> List[KernelShape]:
         KernelShape("gemm_kernel<128>", "128 x 128 x 64", 6, 320, 6 * 32768 + 32768 + 256 + 1024, 256, 1, "N <= 128, and products that fill less than half the machine"),
         KernelShape("gemm_pair_kernel", "256 x 256 x 64 over two SMs", 5, 384, 5 * 32768 + 65536 + 256 + 1024, 512, 1,
                     "cta_group::2: each CTA holds half of the A rows and half of the B columns"),
+        KernelShape("small_gemm_kernel", "64 x 64 x 64, K over a cluster of up to 8", 4, 256, 4 * 16384, 0, 3,
+                    "warp-level MMAs: nothing to set up, for products of a few tiles"),
         KernelShape("skinny_gemm_kernel", "128 features x 64 tokens x 64, K over a cluster of up to 8", 4, 320, 100352, 64, 2,
                     "partial tiles summed through distributed shared memory"),
         KernelShape("skinny_gemm_kernel<32>", "the same for up to 32 tokens", 5, 320, 104448, 32, 2),
@@ -102,6 +104,8 @@ def kernel_shapes() -> List[KernelShape]:
         KernelShape("skinny_gemm_kernel<32, 8>", "int8 codes, 32 tokens", 5, 320, 112640, 32, 2, "three expanded operand tiles"),
         KernelShape("skinny_gemm_kernel<64, 4>", "int4 codes, 64 tokens", 5, 320, 112640, 64, 2, "three expanded operand tiles"),
         KernelShape("skinny_gemm_kernel<32, 4>", "int4 codes, 32 tokens", 7, 320, 108544, 32, 2, "three expanded operand tiles"),
+        KernelShape("skinny_wide_kernel", "256 features x 128 tokens x 64, K over a cluster of up to 8", 4, 320, 232448, 512, 1,
+                    "65 to 256 tokens"),
         KernelShape("skinny_packed_kernel<8>", "128 (gated: 256) features x (8 | 16) tokens x 32 inputs a warp, int8 codes", 3, 256,
                     122880, 0, 1, "a ring per warp; 99584 bytes and two per SM where there are more tiles than SMs"),
         KernelShape("skinny_packed_kernel<4>", "the same over int4 codes", 5, 256, 122880, 0, 1,

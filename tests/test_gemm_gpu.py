@@ -225,3 +225,34 @@ def test_products_of_some_more_rows(M, N, K):
     assert torch.equal(wide_linear(a, b, one_pass=True), gemm(a, b, splits=1)) and torch.equal(wide_linear(a, b), wide_linear(a, b))
     from idrak_b200 import _native
     _native.check_status("wide")
+
+
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (72, 64, 64), (264, 128, 512), (64, 192, 1032), (520, 392, 200), (296, 72, 1000), (64, 64, 8192),
+                                   (1024, 520, 128), (3072, 576, 64), (1024, 64, 1024), (1032, 256, 1024)])
+def test_small_products(M, N, K, a_mn, b_mn):
+    """The kernel of products of a few tiles on either side of the rules that send them to it, ragged in each direction, in each
+    operand order, over views whose rows lie further apart than they are long; every form of the epilogue."""
+    def operand(rows, cols, sd, seed):
+        return _rand((rows, cols + 24), sd, seed)[:, 8 : 8 + cols]
+    a = operand(K, M, 1.0, 61) if a_mn else operand(M, K, 1.0, 61)
+    b = operand(K, N, 0.2, 62) if b_mn else operand(N, K, 0.2, 62)
+    bias, res, aux = _rand((N,), 1.0, 63), operand(M, N, 1.0, 64), _rand((M, N), 1.0, 65)
+    order = dict(a_mn=a_mn, b_mn=b_mn)
+    # sums of K products of standard deviation 0.2 in fp32 in another order, and one rounding to bf16 (half an ulp: 2^-8)
+    tol = lambda want: 2.0 ** -8 * want.abs() + 1e-5 * K ** 0.5
+    for kw in (dict(), dict(bias=bias, residual=res, alpha=0.5), dict(act="mul_aux", aux=aux), dict(act="gelu_d", bias=bias)):
+        got, want = gemm(a, b, **order, **kw), gemm_reference(a, b, **order, **kw, out_dtype=torch.float32)
+        pairs = zip(got, want) if isinstance(got, tuple) else ((got, want),)
+        for g, w in pairs:                  # the derivative that the oracle returns is itself rounded: one ulp
+            assert ((g.float() - w.float()).abs() <= tol(w.float()) * (2 if isinstance(got, tuple) else 1)).all()
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.ones(M, N + 3, device="cuda", dtype=dtype)[:, 1 : N + 1]          # rows that start anywhere
+        want = gemm_reference(a, b, **order, out_dtype=torch.float32) + 1
+        got = gemm(a, b, **order, out=out, beta=True)
+        assert ((got.float() - want).abs() <= tol(want)).all()
+    assert torch.equal(gemm(a, b, **order, splits=0), gemm(a, b, **order, splits=0))
+    if not (a_mn or b_mn) and K <= 960:      # up to 15 blocks K is not cut: in one pass, with the bits of the kernel for larger products
+        assert torch.equal(gemm(a, b, bias=bias, residual=res, splits=0), gemm(a, b, bias=bias, residual=res, splits=1))
+    from idrak_b200 import _native
+    _native.check_status("small")
