@@ -47,6 +47,8 @@ __device__ __forceinline__ float load_grad(const OptTensor& t, long long i) {
 __global__ void __launch_bounds__(kOptThreads) multi_sumsq_kernel(const OptTensor* __restrict__ tensors,
                                                                   const OptChunk* __restrict__ chunks,
                                                                   float* __restrict__ partial) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[kOptThreads / 32];
   const OptChunk c = chunks[blockIdx.x];
   const OptTensor t = tensors[c.tensor];
@@ -72,6 +74,8 @@ __global__ void __launch_bounds__(kOptThreads) multi_sumsq_kernel(const OptTenso
 __global__ void __launch_bounds__(1024) clip_factor_kernel(const float* __restrict__ partial, int n,
                                                            const float* __restrict__ extra_sumsq,
                                                            float* __restrict__ hyper) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += partial[i];
@@ -96,6 +100,8 @@ __global__ void __launch_bounds__(1024) clip_factor_kernel(const float* __restri
 __global__ void __launch_bounds__(kOptThreads) multi_adamw_kernel(const OptTensor* __restrict__ tensors,
                                                                   const OptChunk* __restrict__ chunks,
                                                                   const float* __restrict__ hyper, int zero_grad) {
+  pdl_launch_dependents();
+  pdl_wait();
   const OptChunk c = chunks[blockIdx.x];
   const OptTensor t = tensors[c.tensor];
   const long long end = min(t.n, c.first + kOptChunk);
@@ -163,22 +169,19 @@ IDRAK_API int idrak_opt_hyper_floats() { return kHCount; }
 IDRAK_API int idrak_opt_grad_norm(const void* tensors, const void* chunks, int n_chunks, float* partial,
                                   const float* extra_sumsq, float* hyper, void* stream_) {
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  if (n_chunks > 0)
-    multi_sumsq_kernel<<<n_chunks, kOptThreads, 0, s>>>(static_cast<const OptTensor*>(tensors),
-                                                        static_cast<const OptChunk*>(chunks), partial);
-    note_launches(1);
-  clip_factor_kernel<<<1, 1024, 0, s>>>(partial, n_chunks, extra_sumsq, hyper);
-  note_launches(1);
-  return int(cudaGetLastError());
+  if (n_chunks > 0) {
+    const int rc = launch_overlapped(multi_sumsq_kernel, dim3(unsigned(n_chunks)), kOptThreads, 0, s,
+                                     static_cast<const OptTensor*>(tensors), static_cast<const OptChunk*>(chunks), partial);
+    if (rc) return rc;
+  }
+  return launch_overlapped(clip_factor_kernel, dim3(1), 1024, 0, s, partial, n_chunks, extra_sumsq, hyper);
 }
 
 IDRAK_API int idrak_opt_adamw(const void* tensors, const void* chunks, int n_chunks, const float* hyper,
                               int zero_grad, void* stream_) {
   if (n_chunks <= 0) return 0;
-  multi_adamw_kernel<<<n_chunks, kOptThreads, 0, static_cast<cudaStream_t>(stream_)>>>(
-      static_cast<const OptTensor*>(tensors), static_cast<const OptChunk*>(chunks), hyper, zero_grad);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(multi_adamw_kernel, dim3(unsigned(n_chunks)), kOptThreads, 0, static_cast<cudaStream_t>(stream_),
+                           static_cast<const OptTensor*>(tensors), static_cast<const OptChunk*>(chunks), hyper, zero_grad);
 }
 
 IDRAK_API int idrak_opt_sgd(const void* tensors, const void* chunks, int n_chunks, const float* hyper,

@@ -352,7 +352,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const int pair = blockIdx.x >> 1;
   const int pairs = gridDim.x >> 1;
 
-  pdl_launch_dependents();                           // the kernel that adds the parts may take an SM as soon as it is free
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
@@ -380,6 +379,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_wait();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                           // what follows may take an SM as soon as it is free
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (one per CTA)
@@ -689,9 +690,7 @@ static int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
         return int(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kTotal));
       }))
     return e;
-  kern<<<grid, kPairThreads, PairSmem::kTotal, stream>>>(tmA, tmB, tmC, tmAux, tmSide, tmPart, p);
-  note_launches(1);
-  int rc = int(cudaGetLastError());
+  int rc = launch_overlapped(kern, dim3(unsigned(grid)), kPairThreads, PairSmem::kTotal, stream, tmA, tmB, tmC, tmAux, tmSide, tmPart, p);
   const int cut = p.m_tiles * p.n_tiles - p.whole_tiles;
   if (rc == 0 && cut) rc = launch_overlapped(pair_reduce_kernel, dim3(unsigned(cut * 32)), 256, 0, stream, p);
   return rc;

@@ -10,7 +10,9 @@
 // and MMAs, and the second warp of a scheduler fills them (K = 512: 7.2 -> 6.1 us). us, back to back, before and now:
 //   1024 x 384 x 128          6.3, 4.1     its input gradient (K 384)    7.3, 5.1     its weight gradient (K 1024)   11.7, 6.0
 //   200 x 1024 x 256          7.0, 4.6                       (K 1024)  11.9, 6.3                      (K 200)      6.8, 4.6
-// The training step of a 4-layer model of width 128 on 1024 tokens: 837, 644.
+// The training step of a 4-layer model of width 128 on 1024 tokens: 837, 612. Launched the ordinary way: with programmatic
+// serialization a chain of these back to back is faster, but in that step, among other kernels of 2 to 8 us, each took 1 us longer
+// to start (612 -> 644, 714 where the others are launched so as well).
 //
 // Reference counterparts: gemm_tc_{nn,nt,tn,tt}_f32 (src/Idrak.Gpu/Cuda/PtxKernels.TensorCore.cs:24-29) at small sizes.
 #include "gemm_epilogue.cuh"
@@ -63,8 +65,7 @@ small_gemm_kernel(const SmallOperand a, const SmallOperand b, const GemmParams p
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;       // this warp's 32 x 16 of the tile
   const int csize = int(gridDim.x), rank = int(blockIdx.x);    // the cluster: the parts of K of one tile
   const int all = (p.K + kSmK - 1) / kSmK, first = all * rank / csize, blocks = all * (rank + 1) / csize;
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_launch_dependents();                                     // what follows may be set up meanwhile
   auto issue = [&](int kb) {
     if (kb < blocks) {
       const uint32_t at = base + (kb % kSmStages) * 2 * kSmTile;
@@ -153,16 +154,17 @@ static int launch_small(const SmallOperand& a, const SmallOperand& b, const Gemm
   cfg.blockDim = dim3(kSmThreads);
   cfg.dynamicSmemBytes = kSmBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = unsigned(cuts);
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(cuts);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = cuts > 1 ? 2 : 1;
-  return int(cudaLaunchKernelEx(&cfg, kern, a, b, p));
+  cfg.numAttrs = cuts > 1 ? 1 : 0;
+  const int rc = int(cudaLaunchKernelEx(&cfg, kern, a, b, p));
+  if (rc) cudaGetLastError();
+  note_launches(1);
+  return rc;
 }
 
 // How many CTAs share K of a tile here, or 0: the tcgen05 kernels. Measured over widths of 128 to 768 and 64 to 3072 rows, in us

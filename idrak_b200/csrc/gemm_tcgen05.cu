@@ -68,6 +68,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   constexpr int kKB = F8 ? 2 * kBK : kBK;          // elements of K per shared-memory stage
+  if (GROUPED == 1 || GROUPED == 2) pdl_wait();    // the tiles to work on come from memory
   const int k_blocks_total = (p.K + kKB - 1) / kKB;
   const int kb_per_split = (k_blocks_total + p.splits - 1) / p.splits;
   const int m_tiles = (GROUPED == 1) ? min(p.m_tiles, *p.tiles_in_use) : p.m_tiles;
@@ -109,6 +110,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();                         // after the allocation: a dependent's could take the columns first and wait for this kernel
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -282,6 +285,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
 // Sum split-K partials in split order and run the fused epilogue. One thread per 8 columns.
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const GemmParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int groups_per_row = (p.N + 7) / 8;
   const long long total = (long long)p.M * groups_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -322,9 +327,8 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUt
         return int(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
       }))
     return e;
-  kern<<<grid, kDenseThreads, L::kTotal, stream>>>(tmA, tmB, tmC, tmAux, tmA2 ? *tmA2 : tmA, tmB2 ? *tmB2 : tmB, p);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(kern, dim3(unsigned(grid)), kDenseThreads, L::kTotal, stream, tmA, tmB, tmC, tmAux, tmA2 ? *tmA2 : tmA,
+                           tmB2 ? *tmB2 : tmB, p);
 }
 
 int pick_epi_mode(const GemmParams& p) {
@@ -531,9 +535,7 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
     const long long groups = (long long)M * ((N + 7) / 8);
     long long want = (groups + 255) / 256, cap = (long long)sm_count() * 8;
     int blocks = int(want < cap ? want : cap);
-    splitk_reduce_kernel<<<blocks, 256, 0, stream>>>(p);
-    note_launches(1);
-    rc = int(cudaGetLastError());
+    rc = launch_overlapped(splitk_reduce_kernel, dim3(unsigned(blocks)), 256, 0, stream, p);
   }
   return rc;
 }

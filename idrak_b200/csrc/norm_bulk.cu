@@ -92,6 +92,8 @@ __global__ void __launch_bounds__(kNbThreads, 1) norm_bwd_bulk_kernel(const Norm
     fence_barrier_init();
   }
   __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (wid == kNbWarps) {
     // ------------------------------------------------------------------ producer
@@ -292,9 +294,7 @@ int norm_bwd_bulk_launch(const NormBulkParams& base, int blocks, cudaStream_t st
         return int(cudaFuncSetAttribute(norm_bwd_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
       }))
     return e;
-  norm_bwd_bulk_kernel<<<blocks, kNbThreads, smem, stream>>>(p);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(norm_bwd_bulk_kernel, dim3(unsigned(blocks)), kNbThreads, smem, stream, p);
 }
 
 }  // namespace idrak

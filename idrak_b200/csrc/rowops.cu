@@ -44,6 +44,7 @@ __global__ void __launch_bounds__(128) norm_fwd_kernel(const __nv_bfloat16* __re
                                                        float* __restrict__ mean_out, float* __restrict__ rstd_out,
                                                        int rows, int C, float eps, int rms) {
   pdl_launch_dependents();     // a dependent launched programmatically may set itself up while this kernel runs
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= rows) return;
@@ -204,6 +205,8 @@ __global__ void __launch_bounds__(128) norm_bwd_kernel(const __nv_bfloat16* __re
                                                        __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part,
                                                        float* __restrict__ db_part, int rows, int C, int rms,
                                                        int rows_per_block) {
+  pdl_launch_dependents();
+  pdl_wait();
   // A block walks its rows one after another; each thread owns fixed columns (vectors tid + i*128), so
   // the dw / db partial sums stay in registers and are added in row order.
   __shared__ float red[2][4];
@@ -289,6 +292,8 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_kernel(const __nv_bfloat16* _
                                                           const float* __restrict__ rstd_in,
                                                           const __nv_bfloat16* __restrict__ dres_in,
                                                           __nv_bfloat16* __restrict__ dx, int C, int rms) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[2][8];
   const int row = blockIdx.x, nvec = C >> 3, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const size_t base = size_t(row) * C;
@@ -349,6 +354,8 @@ __global__ void __launch_bounds__(256) norm_bwd_dx_row_kernel(const __nv_bfloat1
                                                               const float* __restrict__ rstd_in,
                                                               const __nv_bfloat16* __restrict__ dres_in,
                                                               __nv_bfloat16* __restrict__ dx, int rows, int C, int rms) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long row = blockIdx.x * (long long)(256 / G) + threadIdx.x / G;
   const int nvec = row < rows ? C >> 3 : 0, sub = threadIdx.x % G;       // lanes of a row past the end only meet the others
   const size_t base = size_t(row) * C;
@@ -407,6 +414,8 @@ struct ColsumJobs {
   int out_fp32[3], accumulate[3];
 };
 __global__ void __launch_bounds__(256) colsum_final_kernel(const ColsumJobs jobs, int parts, int C) {
+  pdl_launch_dependents();
+  pdl_wait();
   const float* __restrict__ part = jobs.part[blockIdx.y];
   void* __restrict__ out = jobs.out[blockIdx.y];
   const int out_fp32 = jobs.out_fp32[blockIdx.y], accumulate = jobs.accumulate[blockIdx.y];
@@ -446,6 +455,8 @@ __global__ void __launch_bounds__(256) colsum_final_kernel(const ColsumJobs jobs
 // the rows of the block's chunk. Needs ld % 8 == 0 and a 16-byte aligned base; C may be ragged.
 __global__ void __launch_bounds__(256) colsum_part_kernel(const __nv_bfloat16* __restrict__ x, int rows, int C,
                                                           int ld, int rows_per_block, float* __restrict__ part) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[8][256];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 256 + tx * 8;
@@ -481,6 +492,8 @@ __global__ void __launch_bounds__(256) colsum_part_kernel(const __nv_bfloat16* _
 __global__ void __launch_bounds__(256) colsum_part_scalar_kernel(const __nv_bfloat16* __restrict__ x, int rows,
                                                                  int C, int ld, int rows_per_block,
                                                                  float* __restrict__ part) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[8][64];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int col = blockIdx.x * 64 + tx * 2;
@@ -519,6 +532,8 @@ __global__ void __launch_bounds__(256, 2) norm_bwd_warp_kernel(const __nv_bfloat
                                                             __nv_bfloat16* __restrict__ dx,
                                                             float* __restrict__ dw_part, float* __restrict__ db_part,
                                                             int rows, int C, int rms, int rows_per_block) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float sm_acc[];   // [2][C]
   float* sdw = sm_acc;
   float* sdb = sm_acc + C;
@@ -675,6 +690,8 @@ template <class I>
 __global__ void __launch_bounds__(256) gated_bwd_kernel(const __nv_bfloat16* __restrict__ gu,
                                                         const __nv_bfloat16* __restrict__ dout,
                                                         __nv_bfloat16* __restrict__ dgu, I total, int H, int kind) {
+  pdl_launch_dependents();
+  pdl_wait();
   const I i = I(blockIdx.x) * 256 + threadIdx.x, hv = I(H >> 3);
   if (i >= total) return;
   const size_t r = size_t(i / hv);
@@ -744,6 +761,8 @@ template <int kLanes>
 __global__ void __launch_bounds__(256) rope_token_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ positions,
                                                          int tokens, int heads, int D, int row_stride, float theta,
                                                          float freq_scale, int inverse, int heads_per_warp) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int kHalf = 2 * kLanes, kGroup = 32 / kLanes;
   const int runs = (heads + heads_per_warp - 1) / heads_per_warp;
   const long long unit = blockIdx.x * 8ll + (threadIdx.x >> 5);
@@ -798,6 +817,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
 __global__ void embedding_fwd_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ wte,
                                      const __nv_bfloat16* __restrict__ wpe, __nv_bfloat16* __restrict__ out,
                                      int tokens, int seq, int C) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int cv = C >> 3;
   const size_t total = size_t(tokens) * cv;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -818,6 +839,8 @@ __global__ void embedding_fwd_kernel(const int* __restrict__ ids, const __nv_bfl
 // Position-table gradient: dwpe[s, :] (+)= sum_b dout[b*seq + s, :], b ascending.
 __global__ void wpe_bwd_kernel(const __nv_bfloat16* __restrict__ dout, void* __restrict__ dwpe, int batch, int seq,
                                int C, int out_fp32, int accumulate) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int cv = C >> 3;
   const size_t total = size_t(seq) * cv;
   for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -855,6 +878,8 @@ __global__ void wpe_bwd_kernel(const __nv_bfloat16* __restrict__ dout, void* __r
 __global__ void wte_bwd_kernel(const int* __restrict__ sorted_ids, const int* __restrict__ order,
                                const __nv_bfloat16* __restrict__ dout, void* __restrict__ dwte, int tokens, int C,
                                int out_fp32) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int i0 = blockIdx.x;
   if (i0 >= tokens) return;
   const int id = sorted_ids[i0];
@@ -913,14 +938,12 @@ IDRAK_API int idrak_norm_fwd(const void* x, const void* residual, const void* w,
     return launch_overlapped(norm_fwd_block_kernel, dim3(unsigned(rows)), 256, 0, s, CBF(x), CBF(residual), CBF(w), CBF(b),
                              BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms);
   }
-#define NF(V) norm_fwd_kernel<V><<<blocks, 128, 0, s>>>(CBF(x), CBF(residual), CBF(w), CBF(b), BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms)
+#define NF(V) return launch_overlapped(norm_fwd_kernel<V>, dim3(unsigned(blocks)), 128, 0, s, CBF(x), CBF(residual), CBF(w), CBF(b), BF(out), BF(sum_out), mean, rstd, rows, C, eps, rms)
   if (nvec <= 32 * 1) NF(1);
   else if (nvec <= 32 * 2) NF(2);
   else if (nvec <= 32 * 4) NF(4);
   else NF(8);
 #undef NF
-  note_launches(1);
-  return int(cudaGetLastError());
 }
 
 IDRAK_API int idrak_colsum(const void* x, int rows, int C, int ld, float* part, void* out, int out_fp32,
@@ -944,16 +967,14 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   if (!dw && !db && !dx_colsum) {                    // a frozen weight: dx alone
     const int nvec = C / 8;
-#define ND(G, V) norm_bwd_dx_row_kernel<G, V><<<unsigned((rows + 256 / G - 1) / (256 / G)), 256, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), rows, C, rms)
+#define ND(G, V) return launch_overlapped(norm_bwd_dx_row_kernel<G, V>, dim3(unsigned((rows + 256 / G - 1) / (256 / G))), 256, 0, s, CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), rows, C, rms)
     if (nvec <= 8) ND(8, 1);
     else if (nvec <= 16) ND(16, 1);
     else if (nvec <= 32) ND(32, 1);
     else if (nvec <= 64) ND(32, 2);
     else if (nvec <= 128) ND(32, 4);
-    else norm_bwd_dx_kernel<<<rows, nvec >= 256 ? 256 : (nvec + 31) / 32 * 32, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), C, rms);
+    else return launch_overlapped(norm_bwd_dx_kernel, dim3(unsigned(rows)), nvec >= 256 ? 256 : (nvec + 31) / 32 * 32, 0, s, CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), C, rms);
 #undef ND
-    note_launches(1);
-    return int(cudaGetLastError());
   }
   int blocks = norm_bwd_bulk_blocks(rows, C);
   static int use_bulk = -1;
@@ -989,8 +1010,8 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
     db_part = part + size_t(blocks) * C;
     const int rpb = (rows + blocks - 1) / blocks;
     const int nvec = C / 8;
-#define NW(V) norm_bwd_warp_kernel<V><<<blocks, 256, size_t(2) * C * sizeof(float), s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), dw_part, rms ? nullptr : db_part, rows, C, rms, rpb)
-#define NB(V) norm_bwd_kernel<V><<<blocks, 128, 0, s>>>(CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), dw_part, rms ? nullptr : db_part, rows, C, rms, rpb)
+#define NW(V) rc = launch_overlapped(norm_bwd_warp_kernel<V>, dim3(unsigned(blocks)), 256, size_t(2) * C * sizeof(float), s, CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), dw_part, rms ? nullptr : db_part, rows, C, rms, rpb)
+#define NB(V) rc = launch_overlapped(norm_bwd_kernel<V>, dim3(unsigned(blocks)), 128, 0, s, CBF(dy), CBF(x), CBF(w), mean, rstd, CBF(dres_in), BF(dx), dw_part, rms ? nullptr : db_part, rows, C, rms, rpb)
     if (nvec <= 32 * 1) NW(1);
     else if (nvec <= 32 * 2) NW(2);
     else if (nvec <= 32 * 3) NW(3);
@@ -1000,8 +1021,6 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
     else NB(8);
 #undef NW
 #undef NB
-    note_launches(1);
-    rc = int(cudaGetLastError());
     if (rc) return rc;
     if (dx_colsum) {
       rc = idrak_colsum(dx, rows, C, C, part + size_t(2) * blocks * C, dx_colsum, 1, 0, stream_);
@@ -1010,9 +1029,7 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
   }
   add_job(dw_part, dw, grads_fp32, accumulate);
   if (!rms && db) add_job(db_part, db, grads_fp32, accumulate);
-  colsum_final_kernel<<<dim3(unsigned((C + 31) / 32), unsigned(n_jobs)), 256, 0, s>>>(jobs, blocks, C);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(colsum_final_kernel, dim3(unsigned((C + 31) / 32), unsigned(n_jobs)), 256, 0, s, jobs, blocks, C);
 }
 
 // Whether a call of these sizes gets the column sums of dx without a pass of their own (1) or not (0).
@@ -1038,22 +1055,21 @@ IDRAK_API int idrak_colsum(const void* x, int rows, int C, int ld, float* part, 
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   const int yb = idrak_colsum_blocks(rows);
   const int rpb = (rows + yb - 1) / yb;
+  int rc;
   if ((ld % 8) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     dim3 grid((C + 255) / 256, yb);
-    colsum_part_kernel<<<grid, 256, 0, s>>>(CBF(x), rows, C, ld, rpb, part);
+    rc = launch_overlapped(colsum_part_kernel, grid, 256, 0, s, CBF(x), rows, C, ld, rpb, part);
   } else {
     dim3 grid((C + 63) / 64, yb);
-    colsum_part_scalar_kernel<<<grid, 256, 0, s>>>(CBF(x), rows, C, ld, rpb, part);
+    rc = launch_overlapped(colsum_part_scalar_kernel, grid, 256, 0, s, CBF(x), rows, C, ld, rpb, part);
   }
-  note_launches(1);
+  if (rc) return rc;
   ColsumJobs jobs{};
   jobs.part[0] = part;
   jobs.out[0] = out;
   jobs.out_fp32[0] = out_fp32;
   jobs.accumulate[0] = accumulate;
-  colsum_final_kernel<<<(C + 31) / 32, 256, 0, s>>>(jobs, yb, C);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(colsum_final_kernel, dim3(unsigned((C + 31) / 32)), 256, 0, s, jobs, yb, C);
 }
 
 IDRAK_API int idrak_gelu_fwd(const void* x, void* y, long long n, void* stream_) {
@@ -1087,10 +1103,10 @@ IDRAK_API int idrak_gated_bwd(const void* gu, const void* dout, void* dgu, int r
   const long long total = (long long)rows * (H / 8), blocks = (total + 255) / 256;
   if (blocks > 0x7fffffffll) return -3;
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
-  if (total <= 0x7fffffffll) gated_bwd_kernel<unsigned><<<unsigned(blocks), 256, 0, s>>>(CBF(gu), CBF(dout), BF(dgu), unsigned(total), H, kind);
-  else gated_bwd_kernel<unsigned long long><<<unsigned(blocks), 256, 0, s>>>(CBF(gu), CBF(dout), BF(dgu), (unsigned long long)total, H, kind);
-  note_launches(1);
-  return int(cudaGetLastError());
+  if (total <= 0x7fffffffll)
+    return launch_overlapped(gated_bwd_kernel<unsigned>, dim3(unsigned(blocks)), 256, 0, s, CBF(gu), CBF(dout), BF(dgu), unsigned(total), H, kind);
+  return launch_overlapped(gated_bwd_kernel<unsigned long long>, dim3(unsigned(blocks)), 256, 0, s, CBF(gu), CBF(dout), BF(dgu),
+                           (unsigned long long)total, H, kind);
 }
 IDRAK_API int idrak_add(const void* a, const void* b, void* y, long long n, void* stream_) {
   if (n % 8) return -2;
@@ -1121,10 +1137,8 @@ IDRAK_API int idrak_rope(void* x, const int* positions, int tokens, int heads, i
     const long long units = (long long)tokens * ((heads + run - 1) / run);
     const int blocks = int((units + 7) / 8);
     cudaStream_t s = static_cast<cudaStream_t>(stream_);
-    if (rot_dim == 128) rope_token_kernel<32><<<blocks, 256, 0, s>>>(BF(x), positions, tokens, heads, D, row_stride, theta, freq_scale, inverse, run);
-    else rope_token_kernel<16><<<blocks, 256, 0, s>>>(BF(x), positions, tokens, heads, D, row_stride, theta, freq_scale, inverse, run);
-    note_launches(1);
-    return int(cudaGetLastError());
+    return launch_overlapped(rot_dim == 128 ? rope_token_kernel<32> : rope_token_kernel<16>, dim3(unsigned(blocks)), 256, 0, s, BF(x),
+                             positions, tokens, heads, D, row_stride, theta, freq_scale, inverse, run);
   }
   rope_kernel<<<grid_for(size_t(tokens) * heads * (rot_dim / 2), 256), 256, 0,
                 static_cast<cudaStream_t>(stream_)>>>(BF(x), positions, tokens, heads, D, row_stride, rot_dim, theta,
@@ -1135,25 +1149,19 @@ IDRAK_API int idrak_rope(void* x, const int* positions, int tokens, int heads, i
 IDRAK_API int idrak_embedding_fwd(const int* ids, const void* wte, const void* wpe, void* out, int tokens, int seq,
                                   int C, void* stream_) {
   if (C % 8) return -2;
-  embedding_fwd_kernel<<<grid_for(size_t(tokens) * (C / 8), 256), 256, 0, static_cast<cudaStream_t>(stream_)>>>(
-      ids, CBF(wte), CBF(wpe), BF(out), tokens, seq, C);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(embedding_fwd_kernel, dim3(unsigned(grid_for(size_t(tokens) * (C / 8), 256))), 256, 0,
+                           static_cast<cudaStream_t>(stream_), ids, CBF(wte), CBF(wpe), BF(out), tokens, seq, C);
 }
 IDRAK_API int idrak_wpe_bwd(const void* dout, void* dwpe, int batch, int seq, int C, int out_fp32, int accumulate,
                             void* stream_) {
   if (C % 8) return -2;
-  wpe_bwd_kernel<<<grid_for(size_t(seq) * (C / 8), 128), 128, 0, static_cast<cudaStream_t>(stream_)>>>(
-      CBF(dout), dwpe, batch, seq, C, out_fp32, accumulate);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(wpe_bwd_kernel, dim3(unsigned(grid_for(size_t(seq) * (C / 8), 128))), 128, 0,
+                           static_cast<cudaStream_t>(stream_), CBF(dout), dwpe, batch, seq, C, out_fp32, accumulate);
 }
 IDRAK_API int idrak_wte_bwd(const int* sorted_ids, const int* order, const void* dout, void* dwte, int tokens, int C,
                             int out_fp32, void* stream_) {
   if (C % 8) return -2;
   int threads = C / 8 < 128 ? ((C / 8 + 31) / 32) * 32 : 128;
-  wte_bwd_kernel<<<tokens, threads, 0, static_cast<cudaStream_t>(stream_)>>>(sorted_ids, order, CBF(dout), dwte,
-                                                                            tokens, C, out_fp32);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(wte_bwd_kernel, dim3(unsigned(tokens)), threads, 0, static_cast<cudaStream_t>(stream_), sorted_ids, order,
+                           CBF(dout), dwte, tokens, C, out_fp32);
 }

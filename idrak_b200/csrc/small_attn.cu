@@ -111,6 +111,8 @@ __device__ __forceinline__ void sa_put(float* w, int lane, const float (&v)[R]) 
 // R: rows of a warp, 4 R a block
 template <int DP, int R>
 __global__ void __launch_bounds__(kSaThreads) small_attn_fwd_kernel(const SmallAttnParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int kPitch = DP + 4, kE = (DP + 31) / 32, kRows = 4 * R;
   __shared__ __align__(16) float sq[kRows * kPitch], sk[kSaCols * kPitch], sv[kSaCols * kPitch];
   __shared__ __align__(16) float sp[kSaThreads / 32][kSaCols * R];
@@ -186,6 +188,8 @@ __global__ void __launch_bounds__(kSaThreads) small_attn_fwd_kernel(const SmallA
 // group. Both find delta for themselves, so that they are one launch.
 template <int DP, int R>
 __global__ void __launch_bounds__(kSaThreads) small_attn_bwd_kernel(const SmallAttnParams p, int tiles) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int kPitch = DP + 4, kE = (DP + 31) / 32, kRows = 4 * R;
   extern __shared__ __align__(16) float sa_smem[];
   float *ra = sa_smem, *rb = ra + kRows * kPitch, *ca = rb + kRows * kPitch, *cb = ca + kSaCols * kPitch, *sw = cb + kSaCols * kPitch;
@@ -338,19 +342,14 @@ __global__ void __launch_bounds__(kSaThreads) small_attn_bwd_kernel(const SmallA
 template <int DP, int R>
 static int launch_small(const SmallAttnParams& p, bool backward, cudaStream_t stream) {
   const int tiles = (p.S + 4 * R - 1) / (4 * R);
-  note_launches(1);
-  if (!backward) {
-    small_attn_fwd_kernel<DP, R><<<dim3(tiles, p.H, p.B), kSaThreads, 0, stream>>>(p);
-    return int(cudaGetLastError());
-  }
+  if (!backward) return launch_overlapped(small_attn_fwd_kernel<DP, R>, dim3(tiles, p.H, p.B), kSaThreads, 0, stream, p);
   constexpr size_t kSmem = (2 * 4 * R + 2 * kSaCols) * (DP + 4) * 4 + kSaThreads / 32 * 2 * kSaCols * R * 4;
   static DeviceOnce configured;
   if (int e = configured.run([&] {
         return int(cudaFuncSetAttribute(small_attn_bwd_kernel<DP, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmem)));
       }))
     return e;
-  small_attn_bwd_kernel<DP, R><<<dim3(2 * tiles, p.H, p.B), kSaThreads, kSmem, stream>>>(p, tiles);
-  return int(cudaGetLastError());
+  return launch_overlapped(small_attn_bwd_kernel<DP, R>, dim3(2 * tiles, p.H, p.B), kSaThreads, kSmem, stream, p, tiles);
 }
 
 // Four rows a warp while blocks of 16 rows are few to an SM: the chain of a step is half as long; eight share the broadcasts of a

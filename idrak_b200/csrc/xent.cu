@@ -176,6 +176,8 @@ __global__ void __launch_bounds__(kXentThreads) xent_stream_kernel(__nv_bfloat16
 // out[0] = sum(losses) * scale, summed in index order by one block (deterministic).
 __global__ void __launch_bounds__(1024) sum_rows_kernel(const float* __restrict__ v, int n, float scale,
                                                         float* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sm[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
@@ -188,6 +190,8 @@ __global__ void __launch_bounds__(1024) sum_rows_kernel(const float* __restrict_
 template <class T>
 __global__ void __launch_bounds__(256) scale_cast_kernel(const T* __restrict__ x, const float* __restrict__ scale,
                                                          __nv_bfloat16* __restrict__ out, long long n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const float s = *scale;
   const long long n8 = n >> 3, step = (long long)gridDim.x * blockDim.x;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8; i += step) {
@@ -256,9 +260,7 @@ IDRAK_API int idrak_softmax_xent(void* logits, const int* targets, float* losses
 }
 
 IDRAK_API int idrak_sum_rows(const float* v, int n, float scale, float* out, void* stream_) {
-  sum_rows_kernel<<<1, 1024, 0, static_cast<cudaStream_t>(stream_)>>>(v, n, scale, out);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(sum_rows_kernel, dim3(1), 1024, 0, static_cast<cudaStream_t>(stream_), v, n, scale, out);
 }
 
 // out[n] (bf16) = x[n] (fp32 or bf16) * scale[0]; x and out start on 16-byte boundaries.
@@ -269,8 +271,6 @@ IDRAK_API int idrak_scale_cast(const void* x, int x_fp32, const float* scale, vo
   const int blocks = int(want < 1 ? 1 : (want < cap ? want : cap));
   cudaStream_t s = static_cast<cudaStream_t>(stream_);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
-  if (x_fp32) scale_cast_kernel<float><<<blocks, 256, 0, s>>>(static_cast<const float*>(x), scale, o, n);
-  else scale_cast_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), scale, o, n);
-  note_launches(1);
-  return int(cudaGetLastError());
+  if (x_fp32) return launch_overlapped(scale_cast_kernel<float>, dim3(unsigned(blocks)), 256, 0, s, static_cast<const float*>(x), scale, o, n);
+  return launch_overlapped(scale_cast_kernel<__nv_bfloat16>, dim3(unsigned(blocks)), 256, 0, s, static_cast<const __nv_bfloat16*>(x), scale, o, n);
 }

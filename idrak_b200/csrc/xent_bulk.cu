@@ -83,6 +83,8 @@ __global__ void __launch_bounds__(kXbThreads, 1) xent_bulk_kernel(const XentBulk
     fence_barrier_init();
   }
   __syncthreads();
+  pdl_launch_dependents();
+  pdl_wait();
 
   if (threadIdx.x >= kXbConsumers) {
     // ------------------------------------------------------------------ producer (one thread): loads and stores
@@ -249,9 +251,7 @@ int xent_bulk_launch(void* logits, const int* targets, float* losses, float* lse
   p.ignore_index = ignore_index; p.write_grad = write_grad;
   p.st = status_device_ptr();
   const int grid = rows < sm_count() ? rows : sm_count();
-  xent_bulk_kernel<<<grid, kXbThreads, smem, stream>>>(p);
-  note_launches(1);
-  return int(cudaGetLastError());
+  return launch_overlapped(xent_bulk_kernel, dim3(unsigned(grid)), kXbThreads, smem, stream, p);
 }
 
 }  // namespace idrak
