@@ -45,6 +45,9 @@ _SIGNATURES = {
     "idrak_gemm_bf16": (c_int, [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                                 c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int,
                                 c_int, c_float, c_int, c_void_p, c_int, c_void_p]),
+    "idrak_weight_bias_grad_fits": (c_int, [c_int, c_int, c_int]),
+    "idrak_weight_bias_grad": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                       c_int, c_int, c_int, c_void_p]),
     "idrak_norm_fwd": (c_int, [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_void_p]),
     "idrak_norm_bwd_blocks": (c_int, [c_int]),
     "idrak_norm_bwd": (c_int, [c_void_p] * 11 + [c_int, c_int, c_int, c_int, c_int, c_void_p]),

@@ -519,6 +519,7 @@ int pick_epi_mode(const GemmParams& p);
 unsigned long long* role_timer_buffer();
 // The kernel for small products (gemm_small.cu): in how many parts it would take K (0: not at all), and its launcher.
 int gemm_small_cuts(int M, int N, int K, bool ordered, bool cut_there);
+bool gemm_cuts_k(int M, int N, int K);      // whether the tcgen05 kernels, left the choice, cut K of this product
 int gemm_small_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, GemmParams p, int cuts, cudaStream_t stream);
 // The CTA-pair kernel (gemm2_tcgen05.cu): whether a product should use it, how many of its 256 x 256 tiles are taken whole and
 // into how many parts along K the others are cut (needs a workspace of gemm_pair_workspace() floats), and its launcher.

@@ -405,6 +405,11 @@ IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn) {
   return min(s, 16);
 }
 
+bool idrak::gemm_cuts_k(int M, int N, int K) {
+  const PairPlan pair = gemm_pair_plan(M, N, K, true);
+  return pair.use ? pair.parts > 1 : idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1;
+}
+
 // Whether x W^T of this size goes to a few-row kernel: 0 no, 1 yes, 2 yes with K in one pass (both skinny_gemm.cu, up to 64 rows), 3 yes
 // (skinny_wide.cu, up to 192 rows). More than 64 rows of a product whose K is cut here: up to 128 whatever its size, and up to 192 of
 // a weight of at most 8 M elements - of larger ones the pairs' tiles take as long (figures in skinny_wide.cu; 2048 x 2048 at 192 rows
@@ -417,11 +422,7 @@ IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn) {
 // 4096 x 14336 34.8, 36.8, 38.9 / 27.6, 28.7, 31.4; in one pass: 768 x 768 10.1, 10.4, 10.6 / 7.2, 9.2, 11.5; 28672 x 4096 63.5, 57.3,
 // 57.3 / 50.2, 53.2, 57.3; 128256 x 4096 206, 189, 193 / 166, 183, 207.
 IDRAK_API int idrak_gemm_few_rows(int M, int N, int K) {
-  if (M > 64) {
-    const PairPlan pair = gemm_pair_plan(M, N, K, true);
-    const bool cut = pair.use ? pair.parts > 1 : idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1;
-    return cut && (M <= 128 || (M <= 192 && (long long)N * K <= (8ll << 20))) ? 3 : 0;
-  }
+  if (M > 64) return gemm_cuts_k(M, N, K) && (M <= 128 || (M <= 192 && (long long)N * K <= (8ll << 20))) ? 3 : 0;
   if (idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1) return 1;
   return M <= 32 || (K >= 1024 && N < 49152) ? 2 : 0;
 }

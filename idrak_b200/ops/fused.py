@@ -21,7 +21,7 @@ from .. import _native
 from . import rowops
 from ._util import stream_ptr
 from .attention import attention_reference, flash_backward, flash_forward
-from .gemm import bias_grad, gemm, weight_grad
+from .gemm import gemm, weight_bias_grad, weight_grad
 from .rowops import GATE_KINDS, _gate_ref, colsum, rope_, rope_reference
 
 
@@ -184,11 +184,9 @@ class _MlpGelu(torch.autograd.Function):
         if dy2.stride(1) != 1 or dy2.stride(0) != dy2.shape[1]:
             dy2 = dy2.contiguous()
         p_w1, p_b1, p_w2, p_b2 = ctx.params
-        dw2 = weight_grad(dy2, h, p_w2)
-        db2 = bias_grad(dy2, p_b2, dy) if has_b2 else None
+        dw2, db2 = weight_bias_grad(dy2, h, p_w2, p_b2, dy) if has_b2 else (weight_grad(dy2, h, p_w2), None)
         dpre = gemm(dy2, w2, b_mn=True, act="mul_aux", aux=dact)
-        dw1 = weight_grad(dpre, x2, p_w1)
-        db1 = bias_grad(dpre, p_b1) if has_b1 else None
+        dw1, db1 = weight_bias_grad(dpre, x2, p_w1, p_b1) if has_b1 else (weight_grad(dpre, x2, p_w1), None)
         dx = gemm(dpre, w1, b_mn=True).reshape(*dy.shape[:-1], w1.shape[1])
         return dx, dw1, db1, dw2, db2, (dy if has_res else None)
 
@@ -231,15 +229,13 @@ class _MlpGated(torch.autograd.Function):
         if dy2.stride(1) != 1 or dy2.stride(0) != dy2.shape[1]:
             dy2 = dy2.contiguous()
         p_wgu, p_bgu, p_w2, p_b2 = ctx.params
-        dw2 = weight_grad(dy2, act, p_w2)
-        db2 = bias_grad(dy2, p_b2, dy) if has_b2 else None
+        dw2, db2 = weight_bias_grad(dy2, act, p_w2, p_b2, dy) if has_b2 else (weight_grad(dy2, act, p_w2), None)
         dact = gemm(dy2, w2, b_mn=True)
         dgu = torch.empty_like(gu)
         Hd = gu.shape[1] // 2
         _native.check(_native.lib().idrak_gated_bwd(gu.data_ptr(), dact.data_ptr(), dgu.data_ptr(), gu.shape[0], Hd,
                                                     kind, stream_ptr()), "gated_bwd")
-        dwgu = weight_grad(dgu, x2, p_wgu)
-        dbgu = bias_grad(dgu, p_bgu) if has_bgu else None
+        dwgu, dbgu = weight_bias_grad(dgu, x2, p_wgu, p_bgu) if has_bgu else (weight_grad(dgu, x2, p_wgu), None)
         dx = gemm(dgu, wgu, b_mn=True).reshape(*dy.shape[:-1], wgu.shape[1])
         return dx, dwgu, dbgu, dw2, db2, (dy if has_res else None), None
 

@@ -173,10 +173,7 @@ def bias_grad(dy2: torch.Tensor, param: torch.Tensor | None, dy: torch.Tensor | 
     it left its column sums on it (``_idrak_colsum``, see ``rowops.norm_backward``) no pass over dy is made."""
     from . import _grad
     from .rowops import colsum
-    ready = None
-    tagged = getattr(dy, "_idrak_colsum", None) if dy is not None else None
-    if tagged is not None and tagged[1] == dy._version and tagged[0].numel() == dy2.shape[1]:
-        ready = tagged[0]
+    ready = _tagged_colsum(dy2, dy)
     tgt = _grad.target(param)
     if tgt is None:
         return colsum(dy2) if ready is None else ready.to(dy2.dtype)
@@ -189,6 +186,36 @@ def bias_grad(dy2: torch.Tensor, param: torch.Tensor | None, dy: torch.Tensor | 
         g.copy_(ready)
     _grad.written(param)
     return None
+
+
+def _tagged_colsum(dy2, dy):
+    tagged = getattr(dy, "_idrak_colsum", None) if dy is not None else None
+    return tagged[0] if tagged is not None and tagged[1] == dy._version and tagged[0].numel() == dy2.shape[1] else None
+
+
+def weight_bias_grad(dy2: torch.Tensor, x2: torch.Tensor, w_param, b_param, dy: torch.Tensor | None = None):
+    """``(weight_grad(dy2, x2, w_param), bias_grad(dy2, b_param, dy))``, in one launch where the weight gradient is small and nobody has
+    summed the columns of dy yet."""
+    lib = _native.lib() if dy2.is_cuda else None
+    K, M = dy2.shape
+    N = x2.shape[1]
+    if (lib is None or dy2.dtype != torch.bfloat16 or x2.dtype != torch.bfloat16 or dy2.stride(1) != 1 or x2.stride(1) != 1
+            or _tagged_colsum(dy2, dy) is not None or not lib.idrak_weight_bias_grad_fits(K, M, N)
+            or (M <= 256 and _tuned_splits(dy2, x2, True, True, M, N, K, 0, x2.new_empty((M, N))))):
+        return weight_grad(dy2, x2, w_param), bias_grad(dy2, b_param, dy)
+    from . import _grad
+    targets = [_grad.target(p) for p in (w_param, b_param)]
+    (dw, w_acc), (db, b_acc) = [t if t is not None else (dy2.new_empty(s), False) for t, s in zip(targets, ((M, N), (M,)))]
+    assert dw.stride(1) == 1 and dw.shape == (M, N) and db.is_contiguous() and db.numel() == M
+    assert {dw.dtype, db.dtype} <= {torch.float32, torch.bfloat16}, (dw.dtype, db.dtype)
+    rc = lib.idrak_weight_bias_grad(dy2.data_ptr(), dy2.stride(0), x2.data_ptr(), x2.stride(0), dw.data_ptr(), dw.stride(0),
+                                    int(dw.dtype == torch.float32), int(w_acc), db.data_ptr(), int(db.dtype == torch.float32), int(b_acc),
+                                    K, M, N, stream_ptr())
+    _native.check(rc, "idrak_weight_bias_grad")
+    for t, p in zip(targets, (w_param, b_param)):
+        if t is not None:
+            _grad.written(p)
+    return tuple(None if t is not None else g for t, g in zip(targets, (dw, db)))
 
 
 class _Linear(torch.autograd.Function):
@@ -218,9 +245,11 @@ class _Linear(torch.autograd.Function):
         dx = dw = db = dres = None
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, weight, b_mn=True).reshape(*dy.shape[:-1], weight.shape[1])
-        if ctx.needs_input_grad[1]:
+        if ctx.needs_input_grad[1] and ctx.has_bias and ctx.needs_input_grad[2]:
+            dw, db = weight_bias_grad(dy2, x2, w_param, b_param, dy)
+        elif ctx.needs_input_grad[1]:
             dw = weight_grad(dy2, x2, w_param)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
+        elif ctx.has_bias and ctx.needs_input_grad[2]:
             db = bias_grad(dy2, b_param, dy)
         if ctx.has_res and ctx.needs_input_grad[3]:
             dres = dy
@@ -305,9 +334,11 @@ class _LowRankLinear(torch.autograd.Function):
         dt = gemm(dy2, B, b_mn=True)                                          # [M, R]
         if ctx.needs_input_grad[0]:
             dx = gemm_lowrank(dy2, weight, dt, A, b_mn=True).reshape(*dy.shape[:-1], weight.shape[1])
-        if ctx.needs_input_grad[1]:
+        if ctx.needs_input_grad[1] and ctx.has_bias and ctx.needs_input_grad[2]:
+            dw, db = weight_bias_grad(dy2, x2, w_param, b_param, dy)
+        elif ctx.needs_input_grad[1]:
             dw = weight_grad(dy2, x2, w_param)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
+        elif ctx.has_bias and ctx.needs_input_grad[2]:
             db = bias_grad(dy2, b_param, dy)
         if ctx.has_res and ctx.needs_input_grad[3]:
             dres = dy

@@ -1,4 +1,6 @@
 """tcgen05 GEMM against a plain PyTorch fp32 statement of the same contract."""
+import math
+
 import pytest
 import torch
 
@@ -256,3 +258,37 @@ def test_small_products(M, N, K, a_mn, b_mn):
         assert torch.equal(gemm(a, b, bias=bias, residual=res, splits=0), gemm(a, b, bias=bias, residual=res, splits=1))
     from idrak_b200 import _native
     _native.check_status("small")
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("tokens,M,N", [(8, 8, 8), (65, 72, 136), (1000, 384, 128), (1024, 512, 128), (1500, 200, 64), (8192, 64, 64), (4096, 2304, 768)])
+def test_weight_and_bias_gradient(tokens, M, N, accumulate, dtype):
+    """One launch for both where the weight gradient is small (all sizes but the last): the weight gradient has the bits it has alone, and
+    the column sums are as close to the 64-bit ones as a tree of fp32 sums has to be."""
+    from idrak_b200.ops import _grad
+    from idrak_b200.ops.gemm import bias_grad, weight_bias_grad, weight_grad
+    dy, x = _rand((tokens, M + 8), 1.0, 71)[:, :M], _rand((tokens, N), 1.0, 72)
+    times, grads = 2 if accumulate else 1, []
+    for fused in (True, False):
+        w, b = (torch.nn.Parameter(torch.zeros(s, device="cuda", dtype=dtype)) for s in ((M, N), (M,)))
+        w.grad, b.grad = torch.ones_like(w), torch.ones_like(b)
+        _grad.enable((w, b))
+        for _ in range(times):
+            if fused:
+                assert weight_bias_grad(dy, x, w, b, dy) == (None, None)
+            else:
+                weight_grad(dy, x, w), bias_grad(dy, b, dy)
+        grads.append((w.grad, b.grad))
+        _grad.next_step()
+    assert torch.equal(grads[0][0], grads[1][0])
+    want = dy.double().sum(0)
+    # every fp32 addition is off by 2^-24 of its partial sum, and a value passes fewer than log2(tokens) + 16 of them; a bf16 store by 2^-8
+    bound = dy.double().abs().sum(0) * 2.0 ** -24 * (math.log2(tokens) + 16) * times
+    if dtype == torch.bfloat16:
+        bound = bound + want.abs() * 2.0 ** -8 * (3 if accumulate else 1)      # the first store of 1 x, the second of 2 x
+    assert ((grads[0][1].double() - times * want).abs() <= bound).all()
+    new = weight_bias_grad(dy, x, None, None)
+    assert torch.equal(new[0], gemm(dy, x, a_mn=True, b_mn=True)) and new[1].dtype == torch.bfloat16
+    from idrak_b200 import _native
+    _native.check_status("weight and bias gradient")
