@@ -1007,6 +1007,7 @@ IDRAK_API int idrak_norm_bwd_fused(const void* dy, const void* x, const void* w,
     if (dx_colsum) add_job(dxs_part, dx_colsum, 1, 0);
   } else {
     blocks = idrak_norm_bwd_blocks(rows);
+    if (C <= 1024) blocks = min(blocks, (rows + 7) / 8);       // a row for every warp: half as many parts to add for 1024 rows
     db_part = part + size_t(blocks) * C;
     const int rpb = (rows + blocks - 1) / blocks;
     const int nvec = C / 8;
