@@ -41,6 +41,8 @@
 #include <cstdlib>
 #include <cstring>
 
+IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn);
+
 namespace idrak {
 
 constexpr int kPairBN = 256;        // columns of the pair's tile; each CTA stages half of the B rows
@@ -720,20 +722,37 @@ static int pair_env() {
   return enabled;
 }
 
-// Whether a product of this size goes to CTA pairs, and how its tiles are cut (`may_cut`: parts may be used).
+// Where a product of this size goes, and how its K is cut (`may_cut`: parts may be used). Costs are in K blocks of a wave (0.4 us);
+// the figures are us, back to back, single CTAs / pairs:
+//  - Of as many waves (128 x 256 on each SM, 256 x 256 on each two) pairs are 8 % faster, operands come from L2 once for 256 rows:
+//    3000 x 28672 x 4096 527 / 491; a wave alone is a tie (2997 x 1024 x 1024 12.8 / 13.8, with a residual 15.4 / 14.6; the training step
+//    that it is from takes 3303 with the one and 3264 with the other). But an odd number of 128 rows costs pairs a tile more, and where
+//    that is a wave more single CTAs win: 300 x 28672 x 4096 88 / 104, 520 rows 118 / 131, 1030 rows 198 / 209, 1030 x 4096 x 4096 31 / 45,
+//    x 14336 97 / 111; not 2100 x 28672 x 4096, 13 waves and 14, 383 / 368.
+//  - The last tiles in parts along K, where they leave pairs idle: kCutCost for the second kernel and the fp32 parts through L2, of
+//    which kPartsPerBlock take as long as a block. Whole and cut: 1500 x 4096 x 4096 54.0, 47.4, x 14336 163, 133; weight gradients over
+//    16384 rows of 768 x 768 90, 29, of 3072 x 768 98, 64; not cut is 1030 x 6144 x 4096 (two rounds of parts, 55).
+//  - Where all tiles are cut, single CTAs may have fewer to cut: 300 x 4096 x 4096 23.0 / 25.8, x 14336 50 / 56; 512 rows 27.1 / 26.5.
 PairPlan gemm_pair_plan(int M, int N, int K, bool may_cut) {
-  PairPlan plan{false, 0, 1, 0};
+  const int sms = sm_count(), pairs = sms / 2, kb = (K + kBK - 1) / kBK;
+  PairPlan plan{false, 0, 1, 0, may_cut ? idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) : 1};
   const int enabled = pair_env();
   if (!enabled || M <= 128 || N < 256 || K < 128) return plan;
   const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
-  const int pairs = sm_count() / 2, kb = (K + kBK - 1) / kBK;
   if (tiles > (1 << 24)) return plan;
+  const long long units = (long long)((M + 127) / 128) * ((N + 255) / 256), waves = (tiles + pairs - 1) / pairs;
   plan.whole = int(tiles);
   plan.part_blocks = kb;
   plan.use = enabled == 2 || 2 * tiles >= pairs;
+  const long long single_waves = (units + sms - 1) / sms;
+  if (enabled == 1 && plan.use && single_waves < waves && single_waves * 1.085f * kb < waves * kb + 5.f) {
+    plan.use = false;
+    plan.splits = 1;
+    return plan;
+  }
   const int full = int(tiles / pairs) * pairs, cut = int(tiles) - full;
   if (!may_cut || cut == 0) return plan;
-  // in K blocks of a pair: the last tiles whole, or in parts taken in `rounds` rounds
+  // the last tiles whole, or in parts taken in `rounds` rounds
   int best = kb;
   for (int rounds = 1; rounds <= 4; ++rounds) {
     int parts = rounds * pairs / cut;
@@ -748,6 +767,11 @@ PairPlan gemm_pair_plan(int M, int N, int K, bool may_cut) {
       plan.parts = parts;
       plan.part_blocks = blocks;
     }
+  }
+  const int s = plan.splits;
+  if (enabled == 1 && plan.parts > 1 && full == 0 && s > 1 && 1.085f * ((kb + s - 1) / s) + 12.f + float(units * s / 2 / kPartsPerBlock) < best) {
+    plan.use = false;
+    plan.parts = 1;
   }
   return plan;
 }

@@ -523,7 +523,9 @@ bool gemm_cuts_k(int M, int N, int K);      // whether the tcgen05 kernels, left
 int gemm_small_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, GemmParams p, int cuts, cudaStream_t stream);
 // The CTA-pair kernel (gemm2_tcgen05.cu): whether a product should use it, how many of its 256 x 256 tiles are taken whole and
 // into how many parts along K the others are cut (needs a workspace of gemm_pair_workspace() floats), and its launcher.
-struct PairPlan { bool use; int whole, parts, part_blocks; };
+// `use`: on pairs, `whole` tiles taken whole and the others in `parts` parts of `part_blocks` K blocks; else on single CTAs with K in
+// `splits` parts.
+struct PairPlan { bool use; int whole, parts, part_blocks, splits; };
 PairPlan gemm_pair_plan(int M, int N, int K, bool may_cut);
 long long gemm_pair_workspace(const PairPlan& plan, int M, int N);
 int gemm_pair_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const CUtensorMap& tmC,

@@ -388,10 +388,8 @@ IDRAK_API void idrak_gemm_role_timers(void* device_buffer) {
 // fp32 workspace elements that idrak_gemm_bf16 needs when it is left to choose how K is split (splits = 0): 0 where it does
 // not split. Deterministic in (M, N, K, sms).
 IDRAK_API long long idrak_gemm_workspace_elems(int M, int N, int K) {
-  const PairPlan pair = gemm_pair_plan(M, N, K, true);
-  if (pair.use) return gemm_pair_workspace(pair, M, N);
-  const int splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
-  return splits > 1 ? (long long)splits * M * N : 0;
+  const PairPlan plan = gemm_pair_plan(M, N, K, true);
+  return plan.use ? gemm_pair_workspace(plan, M, N) : plan.splits > 1 ? (long long)plan.splits * M * N : 0;
 }
 
 // Pick a split-K factor so a small output still fills the machine. Deterministic in (M, N, K, sms).
@@ -406,8 +404,8 @@ IDRAK_API int idrak_gemm_pick_splits(int M, int N, int K, int bn) {
 }
 
 bool idrak::gemm_cuts_k(int M, int N, int K) {
-  const PairPlan pair = gemm_pair_plan(M, N, K, true);
-  return pair.use ? pair.parts > 1 : idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1;
+  const PairPlan plan = gemm_pair_plan(M, N, K, true);
+  return plan.use ? plan.parts > 1 : plan.splits > 1;
 }
 
 // Whether x W^T of this size goes to a few-row kernel: 0 no, 1 yes, 2 yes with K in one pass (both skinny_gemm.cu, up to 64 rows), 3 yes
@@ -422,8 +420,9 @@ bool idrak::gemm_cuts_k(int M, int N, int K) {
 // 4096 x 14336 34.8, 36.8, 38.9 / 27.6, 28.7, 31.4; in one pass: 768 x 768 10.1, 10.4, 10.6 / 7.2, 9.2, 11.5; 28672 x 4096 63.5, 57.3,
 // 57.3 / 50.2, 53.2, 57.3; 128256 x 4096 206, 189, 193 / 166, 183, 207.
 IDRAK_API int idrak_gemm_few_rows(int M, int N, int K) {
-  if (M > 64) return gemm_cuts_k(M, N, K) && (M <= 128 || (M <= 192 && (long long)N * K <= (8ll << 20))) ? 3 : 0;
-  if (idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1) return 1;
+  const bool cut = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256) > 1;
+  if (M > 64) return cut && (M <= 128 || (M <= 192 && (long long)N * K <= (8ll << 20))) ? 3 : 0;
+  if (cut) return 1;
   return M <= 32 || (K >= 1024 && N < 49152) ? 2 : 0;
 }
 
@@ -465,7 +464,7 @@ IDRAK_API int idrak_gemm_bf16(const void* A, int lda, int a_mn, const void* B, i
   p.alpha = alpha;
   const PairPlan pair = splits == 0 || splits == 1 ? gemm_pair_plan(M, N, K, splits == 0 && workspace) : PairPlan{};
   if (splits == 0) {
-    if (!pair.use) splits = idrak_gemm_pick_splits(M, N, K, N <= 128 ? 128 : 256);
+    if (!pair.use) splits = pair.splits;
     const bool cut = workspace && (pair.use ? pair.parts > 1 : splits > 1);
     const int parts = fp16 ? 0 : gemm_small_cuts(M, N, K, !a_mn && !b_mn && !cut, cut);
     if (parts) return gemm_small_launch(A, lda, a_mn, B, ldb, b_mn, p, parts, stream);

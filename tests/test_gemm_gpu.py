@@ -292,3 +292,15 @@ def test_weight_and_bias_gradient(tokens, M, N, accumulate, dtype):
     assert torch.equal(new[0], gemm(dy, x, a_mn=True, b_mn=True)) and new[1].dtype == torch.bfloat16
     from idrak_b200 import _native
     _native.check_status("weight and bias gradient")
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 4096, 4096), (384, 4096, 1032), (300, 28672, 256), (1030, 4096, 200), (520, 28672, 192), (2100, 28672, 128)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_products_of_an_odd_number_of_row_tiles(M, N, K, b_mn):
+    """Sizes on either side of the rule that keeps a product on single CTAs: a tile fewer than pairs, a wave fewer, all tiles cut."""
+    a, b, res = _rand((M, K), 1.0, 81), _rand((K, N) if b_mn else (N, K), 0.2, 82), _rand((M, N), 1.0, 83)
+    ref = gemm_reference(a, b, b_mn=b_mn, residual=res, out_dtype=torch.float32)
+    # fp32 sums in another order and one rounding to bf16, as in the test of few rows
+    assert ((gemm(a, b, b_mn=b_mn, residual=res).float() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-5 * K ** 0.5).all()
+    from idrak_b200 import _native
+    _native.check_status("row tiles")
